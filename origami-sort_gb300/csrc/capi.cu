@@ -75,7 +75,32 @@ void prof_end(int slot, cudaStream_t st) {
 std::atomic<uint32_t> g_wait_limit{BULK_SPIN_LIMIT};
 uint32_t wait_limit() { return g_wait_limit.load(std::memory_order_relaxed); }
 
+// Whether the radix passes sort n items in chunks of sort_n under this shape
+// code: the size class asks for them, the geometry fits, and the runs that are
+// to be sorted are long enough. A radix sort costs the same for any chunk
+// size, a merge sort one level less for every halving: 2^28 uint32 keys in
+// chunks of 2^18 / 2^19 / 2^20 / 2^21 keys take 3.66 / 4.03 / 4.40 / 4.77 ms
+// by merge passes, 3.99 by radix passes.
+bool radix_takes(int kind, uint64_t n, uint64_t sort_n, int code) {
+    if (!(code & SHAPE_RADIX)) return false;
+    const bool chunks = chunk_limit(n, sort_n) < n;
+    switch (kind) {
+        case ORIGAMI_U32: return radix_fits_u32(n, sort_n) && (!chunks || sort_n >= (1u << 19));
+        case ORIGAMI_U64:
+        case ORIGAMI_I64: return radix_fits_u64(n, sort_n) && (!chunks || sort_n >= (1u << 20));
+        default: return radix_fits_kv(n, sort_n) && (!chunks || sort_n >= (1u << 19));
+    }
+}
+
 uint64_t scratch_bytes(int kind, uint64_t n, uint64_t sort_n, int fan) {
+    if (radix_takes(kind, n, sort_n, fan)) {
+        switch (kind) {
+            case ORIGAMI_U32: return radix_scratch_bytes_u32(n, sort_n);
+            case ORIGAMI_U64:
+            case ORIGAMI_I64: return radix_scratch_bytes_u64(n, sort_n);
+            default: return radix_scratch_bytes_kv(n, sort_n);
+        }
+    }
     switch (kind) {
         case ORIGAMI_U32: return scratch_bytes_u32(n, sort_n, fan);
         case ORIGAMI_U64:
@@ -258,8 +283,9 @@ int size_class(uint64_t n) {
 
 void tune_init();
 
-// Pass shape code for a sort of n items: min_k = 0 takes the table's choice,
-// min_k <= 2 binary passes with the table's tile shape, larger min_k k-way.
+// Pass shape code for a sort of n items: min_k = 0 takes the table's choice
+// (radix passes included), min_k <= 2 binary passes with the table's tile shape,
+// larger min_k k-way.
 int shape_for(int kind, uint64_t n, unsigned min_k) {
     std::call_once(g_tune_once, tune_init);
     const int code = g_tune[kind][size_class(n)].load(std::memory_order_relaxed);
@@ -282,6 +308,14 @@ int seg_shape_for(int kind, uint64_t n, uint64_t nseg) {
 cudaError_t run_typed(int kind, void* d, void* tmp, uint64_t n, uint64_t sort_n, void* want,
                       int fan, void* scratch, cudaStream_t st) {
     const uint64_t m = key_mask(kind);
+    if (radix_takes(kind, n, sort_n, fan)) {
+        switch (kind) {
+            case ORIGAMI_U32: return radix_sort_u32(d, tmp, n, sort_n, m, want, scratch, st);
+            case ORIGAMI_U64:
+            case ORIGAMI_I64: return radix_sort_u64(d, tmp, n, sort_n, m, want, scratch, st);
+            default: return radix_sort_kv(d, tmp, n, sort_n, m, want, scratch, st);
+        }
+    }
     switch (kind) {
         case ORIGAMI_U32: return sort_u32(d, tmp, n, sort_n, m, want, fan, scratch, st, nullptr);
         case ORIGAMI_U64:
@@ -341,9 +375,15 @@ int sort_device_impl(int kind, void* d, void* tmp, uint64_t n, uint64_t sort_n, 
     }
     void* scratch = nullptr;
     if (!tmp) CK(cudaMallocAsync(&scratch, n * item_bytes(kind), st), "scratch allocation");
-    const int fan = shape_for(kind, n, min_k);
+    int fan = shape_for(kind, n, min_k);
     void* work = nullptr;
     cudaError_t e = cudaMallocAsync(&work, scratch_bytes(kind, n, sort_n, fan), st);
+    if (e == cudaErrorMemoryAllocation && radix_takes(kind, n, sort_n, fan)) {
+        // the merge passes need less scratch
+        cudaGetLastError();
+        fan &= ~SHAPE_RADIX;
+        e = cudaMallocAsync(&work, scratch_bytes(kind, n, sort_n, fan), st);
+    }
     if (e != cudaSuccess) {
         if (scratch) cudaFreeAsync(scratch, st);
         return cuda_fail(e, "splitter allocation");
@@ -566,7 +606,7 @@ uint64_t a256(uint64_t b) { return (b + 255) & ~255ull; }
 HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_k) {
     HostPipePlan p;
     const uint64_t limit = (sort_n == 0 || sort_n >= n) ? n : sort_n;
-    p.fan = shape_for(kind, n, min_k);
+    p.fan = shape_for(kind, n, min_k) & ~SHAPE_RADIX;
     p.chunk_n = 1ull << 22;
     // at most 16 chunks, so that one k-way pass of fan-in 16 merges them, and
     // more than 8 where the chunks are larger than the smallest size. The
@@ -745,9 +785,13 @@ int sort_host_direct(int kind, void* host_in, void* host_out, const void* vin, v
     return rc;
 }
 
+int tune_builtin(int kind, int cls);
+void tune_store(int kind, int cls, int code);
+
 // Tuning file: one entry per line. "kind class fan variant": the plain sort's
-// pass shape for a size class; "seg kind class shape": the segmented sort's
-// merge shape for a class of mean segment length. Other lines are skipped.
+// merge shape for a size class; "radix kind class on": whether the class sorts
+// by radix passes, after its shape line; "seg kind class shape": the segmented
+// sort's merge shape for a class of mean segment length. Other lines are skipped.
 int tune_load_file(const char* path) {
     FILE* f = std::fopen(path, "r");
     if (!f) return fail(ORIGAMI_ERR_INVALID, "cannot open tuning file %s", path);
@@ -760,11 +804,18 @@ int tune_load_file(const char* path) {
             ++loaded;
             continue;
         }
+        if (std::sscanf(line, "radix %d %d %d", &kind, &cls, &var) == 3) {
+            if (kind < 0 || kind > 4 || cls < 0 || cls >= TUNE_CLASSES || (var != 0 && var != 1)) continue;
+            const int c = g_tune[kind][cls].load(std::memory_order_relaxed);
+            g_tune[kind][cls].store(var ? c | SHAPE_RADIX : c & ~SHAPE_RADIX, std::memory_order_relaxed);
+            ++loaded;
+            continue;
+        }
         if (std::sscanf(line, "%d %d %d %d", &kind, &cls, &fan, &var) != 4) continue;
         if (kind < 0 || kind > 4 || cls < 0 || cls >= TUNE_CLASSES) continue;
         if (fan != 2 && fan != 4 && fan != 8 && fan != 16) continue;
         if (var < 0 || var > 3 || (fan != 2 && var != 0)) continue;
-        g_tune[kind][cls].store(shape_code(fan, var), std::memory_order_relaxed);
+        tune_store(kind, cls, shape_code(fan, var));
         ++loaded;
     }
     std::fclose(f);
@@ -781,6 +832,13 @@ int tune_load_file(const char* path) {
 struct TuneDefault {
     int kind, cls, fan, variant;
 };
+// First size class that sorts by radix passes. Below it the launches decide,
+// and a merge sort of a few levels has fewer: 131,072 uint32 keys take 43 us by
+// radix passes and 55 by the better merge shape, 65,536 keys 42 and 47, 32,768
+// keys are two merge levels (38); 131,072 uint64 keys 74 and 71, 262,144 keys 78
+// and 85; 131,072 pairs 74 and 83, 91,750 pairs
+// 83 by merges.
+constexpr int RADIX_FROM_U32 = 16, RADIX_FROM_U64 = 18, RADIX_FROM_KV = 17;
 constexpr TuneDefault kTuneDefaults[] = {
     {ORIGAMI_U32, 18, 16, 0},  {ORIGAMI_U32, 19, 2, 3},   {ORIGAMI_U32, 20, 2, 3},   {ORIGAMI_U32, 21, 16, 0},
     {ORIGAMI_U32, 22, 2, 3},   {ORIGAMI_U32, 23, 2, 2},   {ORIGAMI_U32, 25, 16, 0},  {ORIGAMI_U64, 17, 16, 0},
@@ -790,14 +848,27 @@ constexpr TuneDefault kTuneDefaults[] = {
     {ORIGAMI_KV64, 25, 2, 1},  {ORIGAMI_KV64, 26, 2, 1},   {ORIGAMI_KV64, 27, 2, 1},   {ORIGAMI_KV64, 28, 2, 1},
 };
 
+// Built-in choice of a size class: the merge shape above, and radix passes from
+// the class on where they were faster (RADIX_FROM below).
+int tune_builtin(int kind, int cls) {
+    const int k = kind == ORIGAMI_I64 ? ORIGAMI_U64 : (kind == ORIGAMI_KVU64 ? ORIGAMI_KV64 : kind);
+    int code = shape_code(2, 0);
+    for (const TuneDefault& t : kTuneDefaults)
+        if (t.kind == k && t.cls == cls) code = shape_code(t.fan, t.variant);
+    const int from = k == ORIGAMI_U32 ? RADIX_FROM_U32 : (k == ORIGAMI_U64 ? RADIX_FROM_U64 : RADIX_FROM_KV);
+    return cls >= from ? code | SHAPE_RADIX : code;
+}
+
+// Sets a class to a merge shape. The class's own built-in shape restores its
+// built-in choice (radix passes included); any other shape selects merge passes.
+void tune_store(int kind, int cls, int code) {
+    const int b = tune_builtin(kind, cls);
+    g_tune[kind][cls].store(code == (b & ~SHAPE_RADIX) ? b : code, std::memory_order_relaxed);
+}
+
 void tune_init() {
-    for (auto& row : g_tune)
-        for (auto& c : row) c.store(shape_code(2, 0), std::memory_order_relaxed);
-    for (const TuneDefault& t : kTuneDefaults) {
-        g_tune[t.kind][t.cls].store(shape_code(t.fan, t.variant), std::memory_order_relaxed);
-        const int twin = t.kind == ORIGAMI_U64 ? ORIGAMI_I64 : (t.kind == ORIGAMI_KV64 ? ORIGAMI_KVU64 : -1);
-        if (twin >= 0) g_tune[twin][t.cls].store(shape_code(t.fan, t.variant), std::memory_order_relaxed);
-    }
+    for (int k = 0; k < 5; ++k)
+        for (int c = 0; c < TUNE_CLASSES; ++c) g_tune[k][c].store(tune_builtin(k, c), std::memory_order_relaxed);
     for (auto& row : g_seg_tune)
         for (auto& c : row) c.store(0, std::memory_order_relaxed);
     if (const char* path = std::getenv("ORIGAMI_TUNING")) tune_load_file(path);
@@ -1151,7 +1222,7 @@ int origami_tuning_set(int kind, uint64_t n, int fan, int variant) {
     if (variant < 0 || variant > 3 || (fan != 2 && variant != 0))
         return fail(ORIGAMI_ERR_INVALID, "variant must be 0 to 3 (1 to 3 only with fan 2)");
     std::call_once(g_tune_once, tune_init);
-    g_tune[kind][size_class(n)].store(shape_code(fan, variant), std::memory_order_relaxed);
+    tune_store(kind, size_class(n), shape_code(fan, variant));
     return ORIGAMI_OK;
 }
 
@@ -1162,8 +1233,12 @@ int origami_tuning_save(const char* path) {
     if (!f) return fail(ORIGAMI_ERR_INVALID, "cannot write tuning file %s", path);
     for (int k = 0; k < 5; ++k)
         for (int c = 0; c < TUNE_CLASSES; ++c) {
-            const int code = g_tune[k][c].load(std::memory_order_relaxed);
-            if (code != shape_code(2, 0)) std::fprintf(f, "%d %d %d %d\n", k, c, shape_fan(code), shape_variant(code));
+            const int code = g_tune[k][c].load(std::memory_order_relaxed), shape = code & ~SHAPE_RADIX;
+            if (shape != shape_code(2, 0)) std::fprintf(f, "%d %d %d %d\n", k, c, shape_fan(code), shape_variant(code));
+            // the radix choice, where loading the shape alone would give another
+            const int b = tune_builtin(k, c);
+            if (code != (shape == (b & ~SHAPE_RADIX) ? b : shape))
+                std::fprintf(f, "radix %d %d %d\n", k, c, (code & SHAPE_RADIX) ? 1 : 0);
         }
     for (int k = 0; k < 5; ++k)
         for (int c = 0; c < TUNE_CLASSES; ++c) {
@@ -1198,7 +1273,8 @@ int origami_autotune(int kind, uint64_t n, char* report, uint64_t cap) {
     if (e == cudaSuccess) e = cudaMallocAsync(&t, bytes, st);
     const int codes[] = {shape_code(2, 0), shape_code(2, 1), shape_code(2, 2), shape_code(2, 3),
                          shape_code(4, 0), shape_code(8, 0), shape_code(16, 0)};
-    uint64_t wbytes = 0;
+    const int radix = shape_code(2, 0) | SHAPE_RADIX;
+    uint64_t wbytes = scratch_bytes(kind, n, 0, radix);
     for (int c : codes) wbytes = std::max<uint64_t>(wbytes, scratch_bytes(kind, n, 0, c));
     if (e == cudaSuccess) e = cudaMallocAsync(&work, wbytes, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1209,9 +1285,7 @@ int origami_autotune(int kind, uint64_t n, char* report, uint64_t cap) {
     std::string rep;
     int best = codes[0];
     float best_ms = 1e30f;
-    for (int c : codes) {
-        if (e != cudaSuccess) break;
-        if (shape_fan(c) > 2 && (n + k1_tile_of(kind) - 1) / k1_tile_of(kind) <= 2) continue;  // one level
+    auto timed = [&](int c) {
         float ms_best = 1e30f;
         for (int it = 0; it < 4 && e == cudaSuccess; ++it) {
             e = cudaMemcpyAsync(d, p, bytes, cudaMemcpyDeviceToDevice, st);
@@ -1222,13 +1296,25 @@ int origami_autotune(int kind, uint64_t n, char* report, uint64_t cap) {
             float ms = 0;
             if (e == cudaSuccess && it > 0 && cudaEventElapsedTime(&ms, a, b) == cudaSuccess) ms_best = std::min(ms_best, ms);
         }
-        char line[128];
+        return ms_best;
+    };
+    char line[128];
+    for (int c : codes) {
+        if (e != cudaSuccess) break;
+        if (shape_fan(c) > 2 && (n + k1_tile_of(kind) - 1) / k1_tile_of(kind) <= 2) continue;  // one level
+        const float ms_best = timed(c);
         std::snprintf(line, sizeof line, "fan=%d variant=%d ms=%.4f\n", shape_fan(c), shape_variant(c), ms_best);
         rep += line;
         if (ms_best < best_ms) {
             best_ms = ms_best;
             best = c;
         }
+    }
+    if (e == cudaSuccess && radix_takes(kind, n, 0, radix)) {
+        const float ms = timed(radix);
+        std::snprintf(line, sizeof line, "radix ms=%.4f\n", ms);
+        rep += line;
+        if (ms < best_ms) best |= SHAPE_RADIX;
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
@@ -1240,9 +1326,8 @@ int origami_autotune(int kind, uint64_t n, char* report, uint64_t cap) {
     if (e != cudaSuccess) return cuda_fail(e, "autotune");
     if (es != cudaSuccess) return cuda_fail(es, "autotune");
     g_tune[kind][size_class(n)].store(best, std::memory_order_relaxed);
-    char line[128];
-    std::snprintf(line, sizeof line, "chosen fan=%d variant=%d size_class=%d\n", shape_fan(best), shape_variant(best),
-                  size_class(n));
+    std::snprintf(line, sizeof line, "chosen %sfan=%d variant=%d size_class=%d\n", (best & SHAPE_RADIX) ? "radix " : "",
+                  shape_fan(best), shape_variant(best), size_class(n));
     rep += line;
     if (report && cap) {
         std::strncpy(report, rep.c_str(), cap - 1);

@@ -29,6 +29,18 @@ ORIGAMI_DECLARE_SORT(u64)
 ORIGAMI_DECLARE_SORT(kv)
 #undef ORIGAMI_DECLARE_SORT
 
+// Radix passes (radix.cuh): whether they take a sort of n items in chunks of
+// sort_n, the scratch they need (error word in its last 256 bytes) and the sort.
+#define ORIGAMI_DECLARE_RADIX(name)                                                                        \
+    bool radix_fits_##name(uint64_t n, uint64_t sort_n);                                                   \
+    uint64_t radix_scratch_bytes_##name(uint64_t n, uint64_t sort_n);                                      \
+    cudaError_t radix_sort_##name(void* d, void* tmp, uint64_t n, uint64_t sort_n, uint64_t key_mask, void* want, \
+                                  void* scratch, cudaStream_t st);
+ORIGAMI_DECLARE_RADIX(u32)
+ORIGAMI_DECLARE_RADIX(u64)
+ORIGAMI_DECLARE_RADIX(kv)
+#undef ORIGAMI_DECLARE_RADIX
+
 // Batched segmented sort (segmented.cuh): levels to plan for, scratch bytes,
 // the launch sequence, and where the error word sits inside the scratch.
 #define ORIGAMI_DECLARE_SEG(name)                                                                 \

@@ -187,8 +187,11 @@ static_assert(Config<uint32_t>::P2_TILE >= Config<uint32_t>::P_TILE && Config<ui
 // A pass shape code: merge fan-in in the low byte (2 = binary passes, 4/8/16 =
 // k-way), the binary-pass merge shape above it (0 = P_*, 1 = P2_*, 2 = P_* one
 // tile per CTA). Chosen per kind and size by the tuning table (capi.cu).
+// SHAPE_RADIX on top: the size class sorts by radix passes (radix.cuh) where
+// they take the call, and by the merge shape elsewhere.
+constexpr int SHAPE_RADIX = 1 << 16;
 inline int shape_fan(int code) { return code & 0xFF; }
-inline int shape_variant(int code) { return code >> 8; }
+inline int shape_variant(int code) { return (code >> 8) & 0xFF; }
 inline int shape_code(int fan, int variant) { return fan | (variant << 8); }
 
 // Number of binary merge passes after K1 for runs to reach `limit` items.

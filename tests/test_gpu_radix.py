@@ -1,0 +1,147 @@
+"""Radix passes (the default of device sorts from some size on): tile edges,
+ragged ends, digits with one, two and sixteen values, both result buffers,
+chunks, and their bounded waits. Integer work: the tolerance is zero."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle as orc
+import origami_gpu as og
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    import __graft_entry__ as g
+    g.build()
+    assert torch.cuda.is_available()
+
+
+def keys(dist, n, seed):
+    rng = np.random.default_rng(seed)
+    k = rng.integers(0, 2**64, n, dtype=np.uint64)
+    if dist == "equal":
+        k[:] = k[0]
+    elif dist == "two":  # every digit has two values
+        k = np.where(k & np.uint64(1), np.uint64(0), ~np.uint64(0))
+    elif dist == "sixteen":
+        k = (k & np.uint64(15)) * np.uint64(0x9E3779B97F4A7C15)
+    elif dist == "small":  # constant high digits
+        k &= np.uint64(0xFFFFF)
+    elif dist == "one_high":  # all but one key share the high digits
+        k &= np.uint64(0xFFFF)
+        k[n // 2] = ~np.uint64(0)
+    elif dist == "sorted":
+        k.sort()
+    return k
+
+
+def items(kind, dist, n, seed):
+    k = keys(dist, n, seed)
+    a = orc.empty(kind, n)
+    if kind == og.U32:
+        a[:] = (k >> np.uint64(32) if dist in ("uniform", "sorted") else k).astype(np.uint32)
+    elif a.dtype.names:
+        a["key"] = k.view(a.dtype["key"])
+        a["value"] = np.arange(n)
+    else:
+        a[:] = k.view(a.dtype)
+    return a
+
+
+def expected(a, sort_n=0):
+    out = a.copy()
+    for i in range(0, len(a), sort_n or len(a)):
+        c = a[i:i + (sort_n or len(a))]
+        out[i:i + len(c)] = c[np.argsort(orc.keys_of(c), kind="stable")]
+    return out
+
+
+def device_sort(a, kind, **kw):
+    d = torch.from_numpy(a.view(np.uint8).copy()).cuda()
+    t = torch.empty_like(d)
+    r = og.sort(d, t, kind=kind, **kw)
+    torch.cuda.synchronize()
+    assert r.data_ptr() == (t if kw.get("result_in_tmp") else d).data_ptr()
+    return r.cpu().numpy().view(a.dtype)
+
+
+@pytest.mark.parametrize("in_tmp", [False, True])
+@pytest.mark.parametrize("dist", ["uniform", "equal", "two", "sixteen", "small", "one_high", "sorted"])
+@pytest.mark.parametrize("kind", [og.U32, og.U64, og.I64, og.KV64, og.KVU64])
+@pytest.mark.parametrize("n", [1 << 17, 135_167, 1_310_721])
+def test_radix_matches_stable_sort(kind, dist, n, in_tmp):
+    a = items(kind, dist, n, seed=n + kind)
+    assert np.array_equal(device_sort(a, kind, result_in_tmp=in_tmp), expected(a))
+
+
+@pytest.mark.parametrize("kind", [og.U32, og.I64, og.KV64])
+@pytest.mark.parametrize("sort_n", [1 << 19, 1 << 20])
+def test_radix_chunks(kind, sort_n):
+    n = (1 << 21) + 4099  # the last chunk is short
+    a = items(kind, "uniform", n, seed=3)
+    a[sort_n:2 * sort_n] = items(kind, "small", sort_n, seed=4)  # one chunk with constant digits
+    assert np.array_equal(device_sort(a, kind, sort_n=sort_n), expected(a, sort_n))
+
+
+def test_radix_long_segment():
+    # 2^30 items and more: the counts of one segment need the wide words
+    n = (1 << 30) + 5
+    g = torch.Generator(device="cuda").manual_seed(9)
+    src = torch.randint(-(2**31), 2**31, (n,), dtype=torch.int32, device="cuda", generator=g)
+    want = int(src.sum(dtype=torch.int64))
+    t = torch.empty_like(src)
+    out = og.sort(src, t, kind="u32")
+    del t
+    assert int(out.sum(dtype=torch.int64)) == want
+    for i in range(0, n, 1 << 28):
+        x = out[i:i + (1 << 28) + 1] ^ torch.tensor(-(2**31), dtype=torch.int32, device="cuda")
+        assert bool((x[1:] >= x[:-1]).all())
+
+
+@pytest.mark.parametrize("kind", [og.U32, og.KV64])
+def test_radix_reports_expired_wait_then_recovers(kind):
+    n = 1 << 20
+    a = items(kind, "uniform", n, seed=5)
+    d = torch.from_numpy(a.view(np.uint8).copy()).cuda()
+    t = torch.empty_like(d)
+    res = ctypes.c_void_p()
+    default = og.wait_limit()
+    og.set_wait_limit(0)
+    try:
+        rc = og.lib().origami_sort_device(kind, d.data_ptr(), t.data_ptr(), n, 0, 0, og.FLAG_SYNC,
+                                          ctypes.byref(res), None)
+        assert rc == og.ERR_TIMEOUT
+    finally:
+        og.set_wait_limit(default)
+    assert np.array_equal(device_sort(a, kind), expected(a))
+
+
+def test_tuning_selects_radix_or_merges(tmp_path):
+    # another shape selects merge passes, the built-in one restores the built-in
+    # choice; both travel through a tuning file
+    n = 1 << 20
+    a = items(og.U32, "uniform", n, seed=6)
+    prev = og.tuning_get(og.U32, n)
+
+    def launched():
+        og.profile_enable(True)
+        assert np.array_equal(device_sort(a, og.U32), expected(a))
+        names = set(og.profile_report())
+        og.profile_enable(False)
+        return any(k.startswith("radix") for k in names)
+
+    try:
+        assert launched()
+        og.tuning_set(og.U32, n, 2, 1)
+        assert not launched()
+        og.tuning_save(tmp_path / "t")
+        og.tuning_set(og.U32, n, *prev)
+        assert launched()
+        og.tuning_load(tmp_path / "t")
+        assert not launched()
+    finally:
+        og.tuning_set(og.U32, n, *prev)
