@@ -1,0 +1,799 @@
+// Bucket sort: the default path (min_k = 0) of device sorts whose keys spread
+// evenly enough. Radix passes from the lowest digit up (radix.cuh) need one pass
+// per digit of the key; from the top down the array is cut into buckets that
+// fit shared memory after log2(n / bucket) bits, 16 for 2^28 keys, and one more
+// pass sorts every bucket whole. So a sort is two partition passes and a bucket
+// pass (one partition pass up to 256 buckets) whatever the width of the key.
+//
+//   bk_sample_kernel  samples the keys of a segment, chooses the range that is
+//                     cut into 2^(b1+b2) equal slices, and sees whether a slice
+//                     is far too full
+//   bk_hist_kernel    counts a level's slices, one read
+//   bk_scan_kernel    slice starts; bucket sizes against what the last kernel
+//                     can take; the next level's tiles
+//   bk_pass_kernel    one partition level for keys, one read and one write
+//   radix_pass_kernel the same for pairs, whose order has to be kept
+//   bk_sort_kernel    one bucket per CTA, sorted in shared memory
+//
+// Measured (one GB300): 2^28 uint32 keys 3.79 ms by radix passes, 2.84 by buckets
+// (counting 2 x 0.20, partition 2 x 0.60, buckets 1.2); 2^27 uint64 keys 5.17 and
+// 2.21 (2 x 0.20, 2 x 0.47, 0.82); 2^27 pairs 8.47 and 4.27 (2 x 0.35, 2 x 1.08,
+// 1.38). A plain copy takes 0.32, 0.32 and 0.64 ms.
+//
+// A slice is a monotone function of the key (keys outside the sampled range
+// fall into the end slices), so any data is sorted correctly as long as every
+// bucket fits. Where one does not (heavy duplicates, clustered keys), *route is
+// set on the device, the remaining kernels return at once, and the radix passes
+// that follow in the stream sort the array instead.
+//
+// Equal keys of keys-only items are identical, so their order does not matter:
+// bk_pass_kernel takes places with shared-memory atomics, one CTA per tile in
+// any order, and claims each slice's output range with one global atomic. No
+// kernel here waits for another CTA. The kernels start early (programmatic
+// dependent launch), some while the buffers they will read are still being
+// written, so no pointer here is __restrict__ (no loads through the read-only
+// path) and everything shared is read after grid_dep_wait().
+#pragma once
+#include <cstdint>
+
+#include "bulk.cuh"
+#include "common.cuh"
+#include "radix.cuh"
+
+namespace origami {
+
+// *route: 0 buckets; 1 radix passes from the input buffer; 2 radix passes from
+// the other buffer (the first partition pass has moved the items there).
+enum BucketRoute : int { ROUTE_BUCKETS = 0, ROUTE_RADIX = 1, ROUTE_RADIX_MOVED = 2 };
+
+template <class T>
+struct BucketCfg;
+template <>
+struct BucketCfg<uint32_t> {
+    static constexpr int NT = 256, IPT = 32, MINB = 3;        // partition tile: 8192 keys
+    static constexpr int S_NT = 256, S_IPT = 24, S_MINB = 4;  // bucket: up to 6144 keys
+    static constexpr int BINS = 4096;                         // bins of the bucket sort
+    static constexpr int LOG_TARGET = 12;                     // mean bucket of 2048 to 4096 keys
+};
+template <>
+struct BucketCfg<uint64_t> {
+    static constexpr int NT = 256, IPT = 16, MINB = 3;
+    static constexpr int S_NT = 256, S_IPT = 16, S_MINB = 4;
+    static constexpr int BINS = 2048;
+    static constexpr int LOG_TARGET = 11;
+};
+template <>
+struct BucketCfg<KV64> {
+    static constexpr int NT = 256, IPT = 16, MINB = 2;  // (radix_pass_kernel's tile)
+    static constexpr int S_NT = 512, S_IPT = 8, S_MINB = 2;
+    static constexpr int BINS = 2048;
+    static constexpr int LOG_TARGET = 11;
+};
+template <class T>
+struct BucketShape {
+    using C = BucketCfg<T>;
+    static constexpr bool STABLE = Traits<T>::kStable;
+    static constexpr int TILE = C::NT * C::IPT;
+    static constexpr size_t PASS_SMEM = (size_t)TILE * sizeof(T);
+    static constexpr int CAP = C::S_NT * C::S_IPT;  // largest bucket
+    static constexpr int CROWDED = 32;              // largest bin that neighbours settle
+    static constexpr int SIDE = STABLE ? 0 : CROWDED;  // guard keys on either side of the bucket
+    static constexpr size_t KEYS_BYTES = (size_t)(CAP + 2 * SIDE) * sizeof(T);
+    // bins and original places (pairs), or the byte passes' words
+    static constexpr size_t BIN_BYTES = (size_t)C::BINS * 4 + (STABLE ? (size_t)CAP * 2 : 0);
+    static constexpr size_t BYTE_BYTES = (size_t)(C::S_NT / 16) * RADIX_BINS * 4;
+    static constexpr size_t SORT_SMEM = KEYS_BYTES + (BIN_BYTES > BYTE_BYTES ? BIN_BYTES : BYTE_BYTES);
+    static_assert(TILE == RadixShape<T>::TILE || !STABLE, "pairs partition by radix_pass_kernel");
+};
+constexpr int BK_SAMPLES = 8192;     // keys sampled per segment
+constexpr int BK_MAX_BITS = 16;      // slices of both levels
+
+// How a segment's keys map to slices: x = the key's distance from lo, scaled so
+// that hi's fills 32 bits; slice = x * mul >> 32. mul is a multiple of 2^b2, so
+// the first level's digit is x * (mul >> b2) >> 32.
+template <class K>
+struct SliceMap {
+    K lo, hi;
+    uint32_t mul;
+    int c;
+    __device__ __forceinline__ uint32_t scaled(K k) const {
+        k = k < lo ? lo : (k > hi ? hi : k);
+        k -= lo;
+        if constexpr (sizeof(K) == 8)
+            return (uint32_t)((k << c) >> 32);
+        else
+            return k << c;
+    }
+    // 2^(b1 + b2) slices of [lo, hi]
+    __device__ __forceinline__ void set(K lo_, K hi_, int b1, int b2) {
+        lo = lo_;
+        hi = hi_;
+        const K r = hi - lo;
+        uint32_t x;
+        if constexpr (sizeof(K) == 8) {
+            c = r ? __clzll((long long)r) : 0;
+            x = (uint32_t)((r << c) >> 32);
+        } else {
+            c = r ? __clz((int)r) : 0;
+            x = r << c;
+        }
+        // x >= 2^31 (r == 0: one slice)
+        mul = r ? (uint32_t)(((1ull << 32) << b1) / ((uint64_t)x + 1)) << b2 : 0u;
+    }
+};
+
+// Items to the keys' unsigned order (32-bit keys are unsigned already).
+template <class T>
+__device__ __forceinline__ T bk_flip(const T& v, uint64_t xmask) {
+    if constexpr (sizeof(typename Traits<T>::Key) == 4)
+        return v;
+    else
+        return Traits<T>::flip(v, xmask);
+}
+
+// Digit of a partition level: the first level's is the slice without its low b2
+// bits, the second's is those bits.
+template <class T>
+struct SliceDigit {
+    SliceMap<typename Traits<T>::Key> map;  // mul as the level wants it (level())
+    uint64_t xmask;
+    uint32_t mask;
+    __device__ __forceinline__ void level(const SliceMap<typename Traits<T>::Key>& m, int shift) {
+        map = m;
+        map.mul >>= shift;
+    }
+    __device__ __forceinline__ unsigned operator()(const T& v) const {
+        return __umulhi(map.scaled(Traits<T>::key(bk_flip(v, xmask))), map.mul) & mask;
+    }
+};
+// The same for radix_pass_kernel, with the slice starts of the scan.
+template <class T>
+struct SliceDigitStable : SliceDigit<T> {
+    static constexpr bool kHeavy = false;  // the sample sends crowded slices to the radix passes
+    const SliceMap<typename Traits<T>::Key>* maps;
+    uint32_t map_shift;
+    const uint32_t* start;
+    int shift, bits;
+    __device__ __forceinline__ void enter(uint32_t seg) { this->level(maps[seg >> map_shift], shift); }
+    __device__ __forceinline__ uint32_t count(uint32_t seg, int bin) const {
+        if (bin >= (1 << bits)) return 0;
+        const uint32_t* s = start + ((size_t)seg << bits) + bin;
+        return s[1] - s[0];
+    }
+    __device__ __forceinline__ uint32_t first(uint32_t seg, uint64_t sbase, uint32_t*) const {
+        const int bin = threadIdx.x;
+        return bin < (1 << bits) ? start[((size_t)seg << bits) + bin] - (uint32_t)sbase : 0u;
+    }
+};
+
+// One tile of the second level (written by bk_scan_kernel).
+struct __align__(16) BkTile {
+    uint64_t base, sbase;           // first item; the first-level bucket's first item
+    uint32_t slen, seg, ti, cnt;    // the bucket's length and number; tile inside it; items
+};
+
+// Where a level's tiles are: level 1 cuts segments of equal length, level 2 the
+// tiles listed by the scan.
+struct BkListed {
+    using Tile = RadixUniform::Tile;
+    const BkTile* rec;
+    const uint32_t* count;
+    __device__ __forceinline__ uint32_t total(uint32_t) const { return *count; }
+    template <int TILE>
+    __device__ __forceinline__ Tile tile(uint32_t t) const {
+        const BkTile r = rec[t];
+        Tile q;
+        q.base = r.base;
+        q.sbase = r.sbase;
+        q.slen = r.slen;
+        q.seg = r.seg;
+        q.ti = r.ti;
+        q.cnt = (int)r.cnt;
+        return q;
+    }
+};
+
+// ---------------------------------------------------------------- sample ---
+// One CTA per segment of len items (the last may be shorter). The range is the
+// samples', widened by 1/512 at each end: of n evenly spread keys about n/8192
+// lie outside the samples at either end.
+template <class T>
+__global__ void __launch_bounds__(1024) bk_sample_kernel(const T* in, uint64_t n, uint64_t len, uint64_t xmask, int b1,
+                                                         int b2, uint64_t cap, SliceMap<typename Traits<T>::Key>* maps,
+                                                         int* route) {
+    using K = typename Traits<T>::Key;
+    constexpr int PER = BK_SAMPLES / 1024;
+    extern __shared__ __align__(16) uint32_t half[];  // 2^(b1+b2) 16-bit counters
+    __shared__ K smin[32], smax[32];
+    __shared__ SliceMap<K> map;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, bits = b1 + b2;
+    const uint64_t base = (uint64_t)blockIdx.x * len;
+    const uint64_t m = n - base < len ? n - base : len;
+    K v[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        // evenly spaced, each moved inside its stretch by a hash
+        const uint32_t j = (uint32_t)(i * 1024 + tid);
+        const uint64_t a = (m * j) / BK_SAMPLES;
+        const uint32_t gap = (uint32_t)((m * (j + 1)) / BK_SAMPLES - a);
+        const uint64_t p = a + __umulhi(j * 2654435761u, gap);
+        v[i] = Traits<T>::key(bk_flip(in[base + (p < m ? p : m - 1)], xmask));
+    }
+    for (int i = tid; i < (1 << bits) / 2 + 1; i += 1024) half[i] = 0;
+    K lo = v[0], hi = v[0];
+#pragma unroll
+    for (int i = 1; i < PER; ++i) {
+        lo = v[i] < lo ? v[i] : lo;
+        hi = v[i] > hi ? v[i] : hi;
+    }
+    auto reduce = [&] {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            const K a = __shfl_xor_sync(0xFFFFFFFFu, lo, o), b = __shfl_xor_sync(0xFFFFFFFFu, hi, o);
+            lo = a < lo ? a : lo;
+            hi = b > hi ? b : hi;
+        }
+    };
+    reduce();
+    if (lane == 0) {
+        smin[warp] = lo;
+        smax[warp] = hi;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        lo = smin[lane];
+        hi = smax[lane];
+        reduce();
+        if (lane == 0) {
+            const K add = (K)((hi - lo) / 512 + 1), top = (K)~(K)0;
+            lo = lo > add ? (K)(lo - add) : (K)0;
+            hi = top - hi > add ? (K)(hi + add) : top;
+            map.set(lo, hi, b1, b2);
+            maps[blockIdx.x] = map;
+        }
+    }
+    __syncthreads();
+    bool full = false;
+    const SliceMap<K> mp = map;
+    // far too full: at least 16 samples, and twice the largest bucket by estimate
+    const uint32_t most = max(15u, (uint32_t)min((unsigned long long)(2 * cap * BK_SAMPLES / m), 60000ull));
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const uint32_t s = __umulhi(mp.scaled(v[i]), mp.mul);
+        const uint32_t h = (atomicAdd(&half[s >> 1], (s & 1) ? 0x10000u : 1u) >> ((s & 1) * 16) & 0xFFFFu) + 1;
+        full |= h > most;
+    }
+    if (__syncthreads_or(full) && tid == 0) *route = ROUTE_RADIX;
+}
+
+// ------------------------------------------------------------------ hist ---
+// Counts of a level's slices: hist[seg << log2(mask+1) | digit]. The lanes of a
+// warp spread over COPIES copies of the counters.
+template <class T, class G>
+__global__ void __launch_bounds__(512) bk_hist_kernel(const T* in, G geo, uint32_t tiles,
+                                                      const SliceMap<typename Traits<T>::Key>* maps,
+                                                      uint32_t map_shift, uint64_t xmask, int shift, int bits,
+                                                      uint32_t* hist, const int* route) {
+    using Sh = BucketShape<T>;
+    constexpr int COPIES = 16, TILE = Sh::TILE, V = Vec<T>::N, STEPS = TILE / V / 512;
+    static_assert(STEPS * V * 512 == TILE, "whole vector steps");
+    __shared__ uint32_t cnt[RADIX_BINS * COPIES];
+    const int tid = threadIdx.x, col = tid & (COPIES - 1), nb = 1 << bits;
+    grid_dep_launch();
+    grid_dep_wait();
+    if (route_load(route) != ROUTE_BUCKETS) return;
+    const uint32_t total = geo.total(tiles);
+    const uint32_t t0 = (uint32_t)((uint64_t)total * blockIdx.x / gridDim.x);
+    const uint32_t t1 = (uint32_t)((uint64_t)total * (blockIdx.x + 1) / gridDim.x);
+    if (t0 >= t1) return;
+    for (int i = tid; i < nb * COPIES; i += 512) cnt[i] = 0;
+    __syncthreads();
+    auto flush = [&](uint32_t seg) {
+        __syncthreads();
+        for (int i = tid; i < nb; i += 512) {
+            uint32_t s = 0;
+#pragma unroll
+            for (int c = 0; c < COPIES; ++c) {
+                s += cnt[i * COPIES + c];
+                cnt[i * COPIES + c] = 0;
+            }
+            if (s) atomicAdd(hist + ((size_t)seg << bits) + i, s);
+        }
+        __syncthreads();
+    };
+    uint32_t seg = 0xFFFFFFFFu;
+    SliceDigit<T> dig;
+    dig.xmask = xmask;
+    dig.mask = (uint32_t)nb - 1;
+    for (uint32_t t = t0; t < t1; ++t) {
+        const auto q = geo.template tile<TILE>(t);
+        if (q.seg != seg) {
+            if (seg != 0xFFFFFFFFu) flush(seg);
+            seg = q.seg;
+            dig.level(maps[seg >> map_shift], shift);
+        }
+        const T* p = in + q.base;
+        // (second-level buckets start anywhere: items, not vectors)
+        if (((uintptr_t)p & 15) == 0 && q.cnt == TILE) {
+            uint4 x[STEPS];
+#pragma unroll
+            for (int j = 0; j < STEPS; ++j) x[j] = reinterpret_cast<const uint4*>(p)[j * 512 + tid];
+#pragma unroll
+            for (int j = 0; j < STEPS; ++j) {
+                const T* e = reinterpret_cast<const T*>(&x[j]);
+#pragma unroll
+                for (int k = 0; k < V; ++k) atomicAdd(&cnt[dig(e[k]) * COPIES + col], 1u);
+            }
+        } else {
+#pragma unroll 8
+            for (int i = tid; i < q.cnt; i += 512) atomicAdd(&cnt[dig(p[i]) * COPIES + col], 1u);
+        }
+    }
+    if (seg != 0xFFFFFFFFu) flush(seg);
+}
+
+// ------------------------------------------------------------------ scan ---
+// One CTA per segment of the level (256 threads, one slice each): slice starts
+// into start[] and cursor[], and either the next level's tiles (tiles2 given)
+// or the check that every bucket fits.
+template <class T>
+__global__ void __launch_bounds__(RADIX_BINS)
+    bk_scan_kernel(const uint32_t* hist, int bits, const uint32_t* seg_start, uint64_t len,
+                   uint32_t* start, uint32_t* cursor, uint64_t n, uint32_t last_seg,
+                   BkTile* tiles2, uint32_t* count2, int* route, int full_route) {
+    constexpr uint32_t TILE = BucketShape<T>::TILE;
+    __shared__ uint32_t ws[RADIX_BINS / 32], ws2[RADIX_BINS / 32], at2;
+    const int tid = threadIdx.x, nb = 1 << bits;
+    const uint32_t seg = blockIdx.x;
+    grid_dep_launch();
+    grid_dep_wait();
+    if (route_load(route) != ROUTE_BUCKETS) return;
+    const size_t at = ((size_t)seg << bits) + tid;
+    const uint32_t h = tid < nb ? hist[at] : 0;
+    const uint32_t base = seg_start ? seg_start[seg] : (uint32_t)(seg * len);
+    const uint32_t s = base + radix_bin_scan<uint32_t>(h, ws);
+    if (tid < nb) {
+        start[at] = s;
+        if (cursor) cursor[at] = s;
+        if (seg == last_seg && tid == nb - 1) start[at + 1] = (uint32_t)n;
+    }
+    if (tiles2) {
+        // the segment's tiles stand together in the list, bucket by bucket
+        const uint32_t nt = (h + TILE - 1) / TILE;
+        uint32_t t0 = radix_bin_scan<uint32_t>(nt, ws2);
+        if (tid == RADIX_BINS - 1) at2 = atomicAdd(count2, t0 + nt);
+        __syncthreads();
+        t0 += at2;
+        for (uint32_t i = 0; i < nt; ++i) {
+            BkTile r;
+            r.sbase = s;
+            r.base = (uint64_t)s + (uint64_t)i * TILE;
+            r.slen = h;
+            r.seg = (seg << bits) + (uint32_t)tid;
+            r.ti = i;
+            r.cnt = h - i * TILE < TILE ? h - i * TILE : TILE;
+            tiles2[t0 + i] = r;
+        }
+    } else if (h > (uint32_t)BucketShape<T>::CAP) {
+        *route = full_route;
+    }
+}
+
+// ------------------------------------------------------------------ pass ---
+// One partition level of keys-only items: count the tile's digits, claim each
+// digit's output range, place the items in digit order in shared memory, write
+// them out run by run. Per 32 keys the shared-memory pipe takes three random
+// accesses of 3.5 bank conflicts (count, place, store). Atomics of lanes with
+// one digit would be serialised (31 cycles), so in a tile whose neighbours
+// share digits (sorted or nearly sorted input: a warp's first step is uniform)
+// one lane counts and places for all where a step is uniform.
+template <class T, class G>
+__global__ void __launch_bounds__(BucketCfg<T>::NT, BucketCfg<T>::MINB)
+    bk_pass_kernel(const T* src, T* dst, G geo, uint32_t tiles, const SliceMap<typename Traits<T>::Key>* maps,
+                   uint32_t map_shift, uint64_t xmask, int shift, int bits, uint32_t* cursor, uint32_t n,
+                   const int* route) {
+    using Sh = BucketShape<T>;
+    constexpr int NT = Sh::C::NT, IPT = Sh::C::IPT, TILE = Sh::TILE;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* skeys = reinterpret_cast<T*>(smem_raw);
+    __shared__ uint32_t tab[RADIX_BINS], goff[RADIX_BINS], ws[RADIX_BINS / 32];
+    static_assert(NT == RADIX_BINS && IPT % 4 == 0, "one thread per slice; four digits to a register");
+    const int tid = threadIdx.x, lane = tid & 31, nb = 1 << bits;
+    tab[tid] = 0;
+    grid_dep_launch();
+    grid_dep_wait();
+    if (route_load(route) != ROUTE_BUCKETS) return;
+    const uint32_t t = blockIdx.x;
+    if (t >= geo.total(tiles)) return;
+    const auto q = geo.template tile<TILE>(t);
+    SliceDigit<T> dig;
+    dig.level(maps[q.seg >> map_shift], shift);
+    dig.xmask = xmask;
+    dig.mask = (uint32_t)nb - 1;
+    T v[IPT];
+    uint32_t dp[IPT / 4];  // the items' digits
+    const bool whole = q.cnt == TILE;
+    const T* p = src + q.base + tid;
+    if (whole) {
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) v[i] = p[i * NT];
+    } else {
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) v[i] = src[q.base + min(i * NT + tid, q.cnt - 1)];
+    }
+#pragma unroll
+    for (int i = 0; i < IPT; i += 4)
+        dp[i / 4] = dig(v[i]) | dig(v[i + 1]) << 8 | dig(v[i + 2]) << 16 | dig(v[i + 3]) << 24;
+    auto digit = [&](int i) -> uint32_t { return __byte_perm(dp[i / 4], 0, 0x4440 | (i & 3)); };
+    const bool plain = whole && !__all_sync(0xFFFFFFFFu, digit(0) == __shfl_sync(0xFFFFFFFFu, digit(0), 0));
+    const int mine = q.cnt - tid;
+    __syncthreads();
+    if (plain) {
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) atomicAdd(&tab[digit(i)], 1u);
+    } else {
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            const uint32_t d = digit(i), d0 = __shfl_sync(0xFFFFFFFFu, d, 0);
+            const bool in = i * NT < mine;
+            if (__all_sync(0xFFFFFFFFu, in && d == d0)) {
+                if (lane == 0) atomicAdd(&tab[d], 32u);
+            } else if (in) {
+                atomicAdd(&tab[d], 1u);
+            }
+        }
+    }
+    __syncthreads();
+    const uint32_t c = tab[tid];
+    uint32_t g = 0;
+    if (c) g = atomicAdd(cursor + ((size_t)q.seg << bits) + tid, c);
+    const uint32_t start = radix_bin_scan<uint32_t>(c, ws);
+    tab[tid] = start;
+    __syncthreads();
+    if (plain) {
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) skeys[atomicAdd(&tab[digit(i)], 1u)] = v[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            const uint32_t d = digit(i), d0 = __shfl_sync(0xFFFFFFFFu, d, 0);
+            const bool in = i * NT < mine;
+            uint32_t r = 0;
+            if (__all_sync(0xFFFFFFFFu, in && d == d0)) {
+                if (lane == 0) r = atomicAdd(&tab[d], 32u);
+                r = __shfl_sync(0xFFFFFFFFu, r, 0) + lane;
+            } else if (in) {
+                r = atomicAdd(&tab[d], 1u);
+            }
+            if (in) skeys[r] = v[i];
+        }
+    }
+    goff[tid] = g - start;
+    __syncthreads();
+    // (o < n always holds while the input does not change under the sort)
+    if (whole) {
+#pragma unroll 8
+        for (int i = 0; i < IPT; ++i) {
+            const T x = skeys[i * NT + tid];
+            const uint32_t o = goff[dig(x)] + (uint32_t)(i * NT + tid);
+            if (o < n) dst[o] = x;
+        }
+    } else {
+        for (int j = tid; j < q.cnt; j += NT) {
+            const T x = skeys[j];
+            const uint32_t o = goff[dig(x)] + (uint32_t)j;
+            if (o < n) dst[o] = x;
+        }
+    }
+}
+
+// ------------------------------------------------------------ bucket sort ---
+// Sorts one bucket per CTA in shared memory: the keys' range in the bucket is
+// cut into BINS bins of equal width, about as many as there are items, and the
+// items are placed bin by bin. A place then differs from the item's rank by the
+// items of its own bin that stand on the wrong side of it, and bins are ordered,
+// so an item is compared with its W neighbours on either side, W + 1 the largest
+// bin of the bucket: conflict-free loads, no bin bounds, one trip count for the
+// CTA. (Pairs compare original positions on equal keys and so are stable.)
+// Crowded bins (a few distinct keys, or clustered ones): where every crowded bin
+// holds one key only, keys are in order as placed; any other such bucket is
+// sorted by stable byte passes over the keys' distance from the smallest, in
+// shared memory.
+template <class T>
+__device__ __forceinline__ bool bk_before(const T& a, int ia, const T& b, int ib) {
+    return less(a, b) || (!less(b, a) && ia < ib);
+}
+
+// Byte passes over the bucket in sk[0, cnt), as radix_pass_kernel ranks: every
+// 16 lanes own a stretch of items and 256 words of `table`.
+template <class T, int NT, int IPT>
+__device__ __forceinline__ void bk_byte_passes(T* sk, uint32_t* table, uint32_t* ws, int cnt,
+                                               typename Traits<T>::Key klo, int bytes) {
+    constexpr int NG = NT / 16;
+    const int tid = threadIdx.x, hl = tid & 15, grp = tid >> 4;
+    const unsigned one = 1u << hl, lt = one - 1u;
+    uint32_t* gt = table + grp * RADIX_BINS;
+    const int i0 = grp * (16 * IPT) + hl;
+    T w[IPT];
+#pragma unroll 1
+    for (int b = 0; b < bytes; ++b) {
+#pragma unroll
+        for (int i = 0; i < IPT; ++i)
+            if (i0 + i * 16 < cnt) w[i] = sk[i0 + i * 16];
+        uint4* z = reinterpret_cast<uint4*>(gt);
+#pragma unroll
+        for (int i = 0; i < RADIX_BINS / 64; ++i) z[i * 16 + hl] = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+        auto digit = [&](int i) -> unsigned { return (unsigned)((Traits<T>::key(w[i]) - klo) >> (8 * b)) & 255u; };
+#pragma unroll
+        for (int i = 0; i < IPT; ++i)
+            if (i0 + i * 16 < cnt) atomicAdd(&gt[digit(i)], 1u << 16);
+        __syncthreads();
+        uint32_t total = 0;
+        if (tid < RADIX_BINS)
+            for (int g = 0; g < NG; ++g) total += table[g * RADIX_BINS + tid] >> 16;
+        uint32_t run = radix_bin_scan<uint32_t>(total, ws);
+        if (tid < RADIX_BINS)
+            for (int g = 0; g < NG; ++g) {
+                const uint32_t c = table[g * RADIX_BINS + tid] >> 16;
+                table[g * RADIX_BINS + tid] = run << 16;
+                run += c;
+            }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            const bool in = i0 + i * 16 < cnt;
+            const unsigned d = in ? digit(i) : 0;
+            if (in) atomicOr(&gt[d], one);
+            __syncwarp();
+            const uint32_t x = gt[d], m = x & 0xFFFFu;
+            const uint32_t r = (x >> 16) + __popc(m & lt);
+            __syncwarp();
+            if (in && (m >> hl) == 1u) gt[d] = (r + 1) << 16;
+            __syncwarp();
+            if (in) sk[r] = w[i];
+        }
+        __syncthreads();
+    }
+}
+
+template <class T>
+__global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
+    bk_sort_kernel(const T* src, T* dst, const uint32_t* start, uint64_t xmask, uint32_t n, const int* route) {
+    using Sh = BucketShape<T>;
+    using K = typename Traits<T>::Key;
+    constexpr int NT = Sh::C::S_NT, IPT = Sh::C::S_IPT, CAP = Sh::CAP, BINS = Sh::C::BINS;
+    constexpr int BPT = BINS / NT;     // bins per thread of the scan
+    constexpr uint32_t CROWDED = Sh::CROWDED;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* sk = reinterpret_cast<T*>(smem_raw) + Sh::SIDE;
+    uint32_t* tab = reinterpret_cast<uint32_t*>(smem_raw + Sh::KEYS_BYTES);
+    uint16_t* si = reinterpret_cast<uint16_t*>(tab + BINS);  // pairs: original places
+    __shared__ uint32_t ws[NT / 32];
+    __shared__ uint32_t rlo[2], rhi[2], widest;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < 2) {
+        rlo[tid] = 0xFFFFFFFFu;
+        rhi[tid] = 0;
+        widest = 1;
+    }
+#pragma unroll
+    for (int i = 0; i < BPT; ++i) tab[i * NT + tid] = 0;
+    grid_dep_launch();
+    grid_dep_wait();
+    if (route_load(route) != ROUTE_BUCKETS) return;
+    const uint32_t b0 = start[blockIdx.x], b1 = start[blockIdx.x + 1];
+    if (b1 <= b0 || b1 > n || b1 - b0 > (uint32_t)CAP) return;
+    const int cnt = (int)(b1 - b0);
+    const int mine = cnt - tid;  // this thread's item i exists when i * NT < mine
+    T v[IPT];
+    const T* p = src + b0 + tid;
+    // the range of the bucket's keys; 64-bit keys by their upper halves first
+    auto hi32 = [](K k) -> uint32_t {
+        if constexpr (sizeof(K) == 8) return (uint32_t)(k >> 32);
+        return (uint32_t)k;
+    };
+#pragma unroll
+    for (int i = 0; i < IPT; ++i)
+        if (i * NT < mine) v[i] = bk_flip(p[i * NT], xmask);
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
+#pragma unroll
+    for (int i = 0; i < IPT; ++i)
+        if (i * NT < mine) {
+            const uint32_t x = hi32(Traits<T>::key(v[i]));
+            lo = min(lo, x);
+            hi = max(hi, x);
+        }
+    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+    __syncthreads();
+    if (lane == 0) {
+        atomicMin(&rlo[0], lo);
+        atomicMax(&rhi[0], hi);
+    }
+    __syncthreads();
+    K klo, kr;
+    lo = rlo[0];
+    hi = rhi[0];
+    if constexpr (sizeof(K) == 8) {
+        if (lo == hi) {
+            uint32_t a = 0xFFFFFFFFu, b = 0;
+#pragma unroll
+            for (int i = 0; i < IPT; ++i)
+                if (i * NT < mine) {
+                    const uint32_t x = (uint32_t)Traits<T>::key(v[i]);
+                    a = min(a, x);
+                    b = max(b, x);
+                }
+            a = __reduce_min_sync(0xFFFFFFFFu, a);
+            b = __reduce_max_sync(0xFFFFFFFFu, b);
+            if (lane == 0) {
+                atomicMin(&rlo[1], a);
+                atomicMax(&rhi[1], b);
+            }
+            __syncthreads();
+            klo = ((K)lo << 32) | rlo[1];
+            kr = (K)(rhi[1] - rlo[1]);
+        } else {
+            klo = (K)lo << 32;
+            kr = ((K)(hi - lo) << 32) | 0xFFFFFFFFu;
+        }
+    } else {
+        klo = lo;
+        kr = hi - lo;
+    }
+    T* out = dst + b0;
+    if (kr == 0) {  // one key: the bucket is sorted
+#pragma unroll
+        for (int i = 0; i < IPT; ++i)
+            if (i * NT < mine) out[i * NT + tid] = bk_flip(v[i], xmask);
+        return;
+    }
+    int c;
+    uint32_t xr;
+    if constexpr (sizeof(K) == 8) {
+        c = __clzll((long long)kr);
+        xr = (uint32_t)((kr << c) >> 32);
+    } else {
+        c = __clz((int)kr);
+        xr = kr << c;
+    }
+    // bins of equal width; rounded down, and never past the last bin (xr >= 2^31)
+    const uint32_t mul = (uint32_t)(((float)BINS * 4294967296.0f) / ((float)xr + 512.0f)) - 1u;
+    auto bin = [&](K k) -> uint32_t {
+        k -= klo;
+        if constexpr (sizeof(K) == 8)
+            return __umulhi((uint32_t)((k << c) >> 32), mul);
+        else
+            return __umulhi(k << c, mul);
+    };
+    uint32_t bp[(IPT + 1) / 2];  // the items' bins
+#pragma unroll
+    for (int i = 0; i < IPT; ++i)
+        if (i * NT < mine) {
+            const uint32_t b = bin(Traits<T>::key(v[i]));
+            bp[i / 2] = (i & 1) ? __byte_perm(bp[i / 2], b, 0x5410) : b;
+            atomicAdd(&tab[b], 1u);
+        }
+    __syncthreads();
+    bool crowded = false;
+    {
+        uint32_t h[BPT], sum = 0, wide = 0;
+        if constexpr (BPT % 4 == 0) {
+#pragma unroll
+            for (int i = 0; i < BPT; i += 4) {
+                const uint4 x = reinterpret_cast<const uint4*>(tab)[(tid * BPT + i) / 4];
+                h[i] = x.x;
+                h[i + 1] = x.y;
+                h[i + 2] = x.z;
+                h[i + 3] = x.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < BPT; ++i) h[i] = tab[tid * BPT + i];
+        }
+#pragma unroll
+        for (int i = 0; i < BPT; ++i) {
+            const uint32_t x = h[i];
+            crowded |= x > CROWDED;
+            wide = max(wide, x > CROWDED ? 0u : x);
+            h[i] = sum;
+            sum += x;
+        }
+        wide = __reduce_max_sync(0xFFFFFFFFu, wide);
+        if (lane == 0) atomicMax(&widest, wide);
+        uint32_t inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        if (lane == 31) ws[warp] = inc;
+        crowded = __syncthreads_or(crowded);
+        uint32_t first = inc - sum;
+#pragma unroll
+        for (int w = 0; w < NT / 32; ++w)
+            if (w < warp) first += ws[w];
+        if constexpr (BPT % 4 == 0) {
+#pragma unroll
+            for (int i = 0; i < BPT; i += 4)
+                reinterpret_cast<uint4*>(tab)[(tid * BPT + i) / 4] =
+                    make_uint4(first + h[i], first + h[i + 1], first + h[i + 2], first + h[i + 3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < BPT; ++i) tab[tid * BPT + i] = first + h[i];
+        }
+    }
+    __syncthreads();
+    const bool by_bytes = Sh::STABLE && crowded;
+    if (!by_bytes) {
+#pragma unroll
+        for (int i = 0; i < IPT; ++i)
+            if (i * NT < mine) {
+                const uint32_t r = atomicAdd(&tab[__byte_perm(bp[i / 2], 0, (i & 1) ? 0x4432 : 0x4410)], 1u);
+                sk[r] = v[i];
+                if constexpr (Sh::STABLE) si[r] = (uint16_t)(i * NT + tid);
+            }
+        if constexpr (!Sh::STABLE) {
+            if (tid < Sh::SIDE) {
+                sk[-1 - tid] = 0;
+                sk[cnt + tid] = Traits<T>::max_item();
+            }
+        }
+        __syncthreads();
+    }
+    if (crowded) {
+        // keys only: does every crowded bin hold one key?
+        bool mixed = Sh::STABLE;
+        if constexpr (!Sh::STABLE) {
+            for (int j = tid; j < cnt; j += NT) {
+                const uint32_t b = bin(Traits<T>::key(sk[j]));
+                const uint32_t e = tab[b], s = b ? tab[b - 1] : 0;
+                mixed |= e - s > CROWDED && sk[j] != sk[s];
+            }
+        }
+        if (__syncthreads_or(mixed)) {
+#pragma unroll
+            for (int i = 0; i < IPT; ++i)
+                if (i * NT < mine) sk[i * NT + tid] = v[i];
+            __syncthreads();
+            int bytes;
+            if constexpr (sizeof(K) == 8)
+                bytes = (71 - __clzll((long long)kr)) / 8;
+            else
+                bytes = (39 - __clz((int)kr)) / 8;
+            bk_byte_passes<T, NT, IPT>(sk, tab, ws, cnt, klo, bytes);
+            for (int i = tid; i < cnt; i += NT) out[i] = bk_flip(sk[i], xmask);
+            return;
+        }
+    }
+    if constexpr (Sh::STABLE) {
+        // a bin's word is its end now, and so the start of the next
+        for (int j = tid; j < cnt; j += NT) {
+            const T x = sk[j];
+            const uint32_t b = bin(Traits<T>::key(x));
+            const int e = (int)tab[b], s = b ? (int)tab[b - 1] : 0;
+            int r = s;
+            if (e - s > 1) {
+                const int ix = (int)si[j];
+                for (int i = s; i < e; ++i) r += bk_before(sk[i], (int)si[i], x, ix) ? 1 : 0;
+            }
+            out[r] = bk_flip(x, xmask);
+        }
+    } else {
+        const int w = (int)widest;
+#pragma unroll 2
+        for (int j = tid; j < cnt; j += NT) {
+            const T x = sk[j];
+            int r = j;
+#pragma unroll 2
+            for (int k = 1; k < w; ++k) {
+                r += sk[j + k] < x ? 1 : 0;
+                r -= sk[j - k] > x ? 1 : 0;
+            }
+            out[r] = bk_flip(x, xmask);
+        }
+    }
+}
+
+}  // namespace origami

@@ -75,20 +75,22 @@ void prof_end(int slot, cudaStream_t st) {
 std::atomic<uint32_t> g_wait_limit{BULK_SPIN_LIMIT};
 uint32_t wait_limit() { return g_wait_limit.load(std::memory_order_relaxed); }
 
-// Whether the radix passes sort n items in chunks of sort_n under this shape
-// code: the size class asks for them, the geometry fits, and the runs that are
-// to be sorted are long enough. A radix sort costs the same for any chunk
-// size, a merge sort one level less for every halving: 2^28 uint32 keys in
-// chunks of 2^18 / 2^19 / 2^20 / 2^21 keys take 3.66 / 4.03 / 4.40 / 4.77 ms
-// by merge passes, 3.99 by radix passes.
+// Smallest chunk that sorts by the radix path: 2^28 uint32 keys in chunks of
+// 2^16 / 2^18 / 2^20 / 2^21 keys take 2.15 / 2.07 / 2.01 / 2.77 ms by buckets, 2.92 /
+// 3.66 / 4.41 / 4.78 by merge passes; shorter chunks have too few buckets.
+constexpr uint64_t RADIX_CHUNK = 1 << 16;
+// Whether the radix path (bucket sort, radix passes behind it) sorts n items in
+// chunks of sort_n under this shape code: the size class asks for it, the
+// geometry fits, and the chunks are long enough. Its cost hardly depends on the
+// chunk size, a merge sort's is one level less for every halving.
 bool radix_takes(int kind, uint64_t n, uint64_t sort_n, int code) {
     if (!(code & SHAPE_RADIX)) return false;
-    const bool chunks = chunk_limit(n, sort_n) < n;
+    if (chunk_limit(n, sort_n) < n && sort_n < RADIX_CHUNK) return false;
     switch (kind) {
-        case ORIGAMI_U32: return radix_fits_u32(n, sort_n) && (!chunks || sort_n >= (1u << 19));
+        case ORIGAMI_U32: return radix_fits_u32(n, sort_n);
         case ORIGAMI_U64:
-        case ORIGAMI_I64: return radix_fits_u64(n, sort_n) && (!chunks || sort_n >= (1u << 20));
-        default: return radix_fits_kv(n, sort_n) && (!chunks || sort_n >= (1u << 19));
+        case ORIGAMI_I64: return radix_fits_u64(n, sort_n);
+        default: return radix_fits_kv(n, sort_n);
     }
 }
 

@@ -1,5 +1,6 @@
-// Radix passes: the sort's default path (min_k = 0) for arrays and chunks of
-// more than a few tiles.
+// Radix passes: what device sorts with min_k = 0 use where the bucket sort
+// (buckets.cuh) does not take the call or gives up; its partition of pairs is
+// the pass kernel here.
 //
 // A merge level moves every item once through HBM and doubles the runs; a
 // radix pass moves every item once and settles eight bits of the key, whatever
@@ -61,7 +62,7 @@ struct RadixCfg<uint32_t> {
 };
 template <>
 struct RadixCfg<uint64_t> {
-    static constexpr int NT = 256, IPT = 20, MINB = 3;  // 5120 keys, 40 KiB
+    static constexpr int NT = 256, IPT = 16, MINB = 3;  // 4096 keys, 32 KiB
     static constexpr int HIST_COPIES = 8;
 };
 template <>
@@ -129,6 +130,13 @@ __device__ __forceinline__ uint64_t look_load(const uint64_t* p) {
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
+// The route word of a bucket sort (buckets.cuh): from L2, because kernels that
+// overlap (programmatic dependent launch) read it while one of them may set it.
+__device__ __forceinline__ int route_load(const int* p) {
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void look_store(uint32_t* p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
 }
@@ -146,6 +154,7 @@ struct RadixUniform {
         uint32_t seg, ti;            // segment; the tile's number inside it
         int cnt;                     // items in the tile
     };
+    __device__ __forceinline__ uint32_t total(uint32_t tiles) const { return tiles; }
     template <int TILE>
     __device__ __forceinline__ Tile tile(uint32_t t) const {
         Tile r;
@@ -164,16 +173,22 @@ struct RadixUniform {
 // warp's lanes spread over HIST_COPIES copies of the counters, so that lanes
 // with equal digits mostly meet different banks. A CTA takes a contiguous range
 // of tiles and flushes its counters when the segment changes. Also clears the
-// first pass's look-back words and, with COPY, copies the input (when the
-// result has to land in the other buffer: the number of passes is even).
-template <class T, class S, class G, bool COPY>
-__global__ void __launch_bounds__(512) radix_hist_kernel(const T* __restrict__ in, T* __restrict__ copy, G geo,
-                                                         uint32_t tiles, uint64_t xmask, S* __restrict__ hist,
-                                                         S* __restrict__ look0) {
+// first pass's look-back words, and copies the input to `want` where it is not
+// there yet (the passes are an even number and end where they start).
+// route (optional): the radix passes stand behind a bucket sort (buckets.cuh);
+// 0: it has done the work, return; 2: the items are in `moved` instead of `in`.
+template <class T, class S, class G>
+__global__ void __launch_bounds__(512) radix_hist_kernel(const T* in0, const T* moved, T* want, G geo, uint32_t tiles,
+                                                         uint64_t xmask, S* hist, S* look0, const int* route) {
     using Sh = RadixShape<T>;
     constexpr int D = Sh::DIGITS, C = Sh::C::HIST_COPIES, TILE = Sh::TILE;
     extern __shared__ __align__(16) uint32_t cnt_sm[];
     const int tid = threadIdx.x, col = tid & (C - 1);
+    grid_dep_wait();
+    const int r = route ? route_load(route) : 1;
+    if (r == 0) return;
+    const T* in = r == 2 ? moved : in0;
+    const bool copy = in != want;
     const uint32_t t0 = (uint32_t)((uint64_t)tiles * blockIdx.x / gridDim.x);
     const uint32_t t1 = (uint32_t)((uint64_t)tiles * (blockIdx.x + 1) / gridDim.x);
     for (int i = tid; i < D * RADIX_BINS * C; i += 512) cnt_sm[i] = 0;
@@ -217,7 +232,7 @@ __global__ void __launch_bounds__(512) radix_hist_kernel(const T* __restrict__ i
             for (int j = 0; j < TILE / V / 512; ++j) {
                 const int i = j * 512 + tid;
                 const uint4 x = reinterpret_cast<const uint4*>(p)[i];
-                if constexpr (COPY) reinterpret_cast<uint4*>(copy + q.base)[i] = x;
+                if (copy) reinterpret_cast<uint4*>(want + q.base)[i] = x;
                 const T* e = reinterpret_cast<const T*>(&x);
 #pragma unroll
                 for (int k = 0; k < V; ++k) count(e[k]);
@@ -225,14 +240,14 @@ __global__ void __launch_bounds__(512) radix_hist_kernel(const T* __restrict__ i
         } else {
             for (int i = tid; i < nvec; i += 512) {
                 const uint4 x = reinterpret_cast<const uint4*>(p)[i];
-                if constexpr (COPY) reinterpret_cast<uint4*>(copy + q.base)[i] = x;
+                if (copy) reinterpret_cast<uint4*>(want + q.base)[i] = x;
                 const T* e = reinterpret_cast<const T*>(&x);
 #pragma unroll
                 for (int k = 0; k < V; ++k) count(e[k]);
             }
             for (int i = nvec * V + tid; i < q.cnt; i += 512) {
                 const T x = p[i];
-                if constexpr (COPY) copy[q.base + i] = x;
+                if (copy) want[q.base + i] = x;
                 count(x);
             }
         }
@@ -261,13 +276,39 @@ __device__ __forceinline__ S radix_bin_scan(S v, S* ws) {
     return base + inc - v;
 }
 
-// One pass: src -> dst by digit `byte`. look: this pass's words, 256 per tile,
-// zero at launch; look_next (optional): the next pass's, cleared here.
-template <class T, class S, class G>
+// The digit of a radix pass: byte `byte` of the key. Also what a pass asks about
+// its segments: the count of a bin, and where the bin starts in the segment.
+template <class T, class S>
+struct ByteDigit {
+    static constexpr bool kHeavy = true;  // any share of the items may have one digit
+    const S* hist;
+    uint64_t xmask;
+    int byte;
+    unsigned dx;
+    ByteDigit(const S* h, uint64_t x, int b) : hist(h), xmask(x), byte(b), dx((unsigned)(x >> (8 * b)) & 255u) {}
+    __device__ __forceinline__ unsigned operator()(const T& v) const {
+        return radix_digit(Traits<T>::key(v), byte, dx);
+    }
+    __device__ __forceinline__ void enter(uint32_t) {}  // a tile of this segment follows
+    __device__ __forceinline__ S count(uint32_t seg, int bin) const {
+        return hist[((size_t)seg * RadixShape<T>::DIGITS + byte) * RADIX_BINS + bin];
+    }
+    // every thread of the CTA calls it (a barrier inside)
+    __device__ __forceinline__ S first(uint32_t seg, uint64_t, S* ws) const {
+        const int bin = threadIdx.x;
+        return radix_bin_scan<S>(bin < RADIX_BINS ? count(seg, bin) : (S)0, ws);
+    }
+};
+
+// One pass: src -> dst by one digit. look: this pass's words, 256 per tile, zero
+// at launch; look_next (optional): the next pass's, cleared here. route
+// (optional): run only where it holds `run` (radix passes behind a bucket sort
+// run unless it is 0, the stable partition of a bucket sort while it is 0).
+template <class T, class S, class G, class D>
 __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
-    radix_pass_kernel(const T* __restrict__ src, T* __restrict__ dst, G geo, uint32_t tiles, int byte, uint64_t xmask,
-                      const S* __restrict__ hist, S* look, S* __restrict__ look_next, unsigned* __restrict__ claim,
-                      int* err, uint32_t spin) {
+    radix_pass_kernel(const T* __restrict__ src, T* __restrict__ dst, G geo, uint32_t tiles, D digit, S* look,
+                      S* __restrict__ look_next, unsigned* __restrict__ claim, int* err, uint32_t spin,
+                      const int* route, bool buckets) {
     using Sh = RadixShape<T>;
     using W = LookWord<S>;
     constexpr int NT = Sh::NT, IPT = Sh::IPT, NG = Sh::NG, TILE = Sh::TILE;
@@ -279,20 +320,21 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
     __shared__ S ws2[RADIX_BINS / 32];
     __shared__ uint32_t next_tile;
     const int tid = threadIdx.x, hl = tid & 15, grp = tid >> 4;
-    const unsigned dx = (unsigned)(xmask >> (8 * byte)) & 255u;
     uint32_t* gt = table + grp * RADIX_BINS;
     const unsigned one = 1u << hl, lt = one - 1u;
 
     grid_dep_wait();
+    if (route && (route_load(route) == 0) != buckets) return;
+    tiles = geo.total(tiles);
     if (tid == 0) next_tile = atomicAdd(claim, 1u);
     if (__syncthreads_or(tid == 0 && err_wait_set(err))) return;
     uint32_t t = next_tile, seg = 0xFFFFFFFFu;
     bool heavy = false;
     for (; t < tiles; t = next_tile) {
         const typename G::Tile q = geo.template tile<TILE>(t);
-        if (q.seg != seg) {
-            seg = q.seg;
-            const S h = tid < RADIX_BINS ? hist[((size_t)seg * Sh::DIGITS + byte) * RADIX_BINS + tid] : (S)0;
+        if (q.seg != seg) digit.enter(q.seg);
+        if (D::kHeavy && q.seg != seg) {
+            const S h = tid < RADIX_BINS ? digit.count(q.seg, tid) : (S)0;
             heavy = __syncthreads_or(h > (S)(q.slen / 24));
             if (heavy && __syncthreads_or(h == (S)q.slen)) {
                 // one digit only: the segment keeps its order. (A tile of it
@@ -301,11 +343,11 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
                 if (look_next)
                     for (int i = tid; i < RADIX_BINS; i += NT) look_next[(size_t)t * RADIX_BINS + i] = 0;
                 if (tid == 0) next_tile = atomicAdd(claim, 1u);
-                seg = 0xFFFFFFFFu;
                 __syncthreads();
                 continue;
             }
         }
+        seg = q.seg;
         T v[IPT];
         const int i0 = grp * (16 * IPT) + hl;
         const int mine = q.cnt - i0;  // item i of this thread exists when i * 16 < mine
@@ -315,13 +357,8 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
 #pragma unroll
                 for (int i = 0; i < IPT; ++i) v[i] = p[i0 + i * 16];
             } else {
-                // the tail is filled with the item that sorts last; only the
-                // ranking by ballots places it, behind every real item
 #pragma unroll
                 for (int i = 0; i < IPT; ++i) v[i] = p[min(i0 + i * 16, q.cnt - 1)];
-#pragma unroll
-                for (int i = 0; i < IPT; ++i)
-                    if (i0 + i * 16 >= q.cnt) v[i] = Traits<T>::flip(Traits<T>::max_item(), xmask);
             }
         }
         {
@@ -330,17 +367,22 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
             for (int i = 0; i < RADIX_BINS / 64; ++i) z[i * 16 + hl] = make_uint4(0, 0, 0, 0);
         }
         __syncwarp();
+        // lanes of the group whose item of step i exists
+        auto present = [&](int i) -> unsigned {
+            const int k = min(max(mine + hl - i * 16, 0), 16);
+            return 0xFFFFu >> (16 - k);
+        };
         // count the group's digits (upper half of its words)
-        if (!heavy) {
+        if (!D::kHeavy || !heavy) {
 #pragma unroll
             for (int i = 0; i < IPT; ++i)
-                if (i * 16 < mine) atomicAdd(&gt[radix_digit(Traits<T>::key(v[i]), byte, dx)], 1u << 16);
+                if (i * 16 < mine) atomicAdd(&gt[digit(v[i])], 1u << 16);
         } else {
 #pragma unroll
             for (int i = 0; i < IPT; ++i) {
-                const unsigned d = radix_digit(Traits<T>::key(v[i]), byte, dx);
-                const unsigned m = (radix_match(d) >> (tid & 16)) & 0xFFFFu;
-                if (!(m & lt)) atomicAdd(&gt[d], (unsigned)__popc(m) << 16);
+                const unsigned d = digit(v[i]);
+                const unsigned m = (radix_match(d) >> (tid & 16)) & present(i);
+                if ((m & one) && !(m & lt)) atomicAdd(&gt[d], (unsigned)__popc(m) << 16);
             }
         }
         __syncthreads();
@@ -365,10 +407,10 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
         }
         __syncthreads();
         // rank and order the tile by digit in shared memory
-        if (!heavy) {
+        if (!D::kHeavy || !heavy) {
 #pragma unroll
             for (int i = 0; i < IPT; ++i) {
-                const unsigned d = radix_digit(Traits<T>::key(v[i]), byte, dx);
+                const unsigned d = digit(v[i]);
                 if (i * 16 < mine) atomicOr(&gt[d], one);
                 __syncwarp();
                 const uint32_t w = gt[d], m = w & 0xFFFFu;
@@ -381,22 +423,20 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
         } else {
 #pragma unroll
             for (int i = 0; i < IPT; ++i) {
-                const unsigned d = radix_digit(Traits<T>::key(v[i]), byte, dx);
-                const unsigned m = (radix_match(d) >> (tid & 16)) & 0xFFFFu;
+                const unsigned d = digit(v[i]);
+                const unsigned m = (radix_match(d) >> (tid & 16)) & present(i);
                 const uint32_t r = (gt[d] >> 16) + __popc(m & lt);
                 __syncwarp();
                 if ((m >> hl) == 1u) gt[d] = (r + 1) << 16;
                 __syncwarp();
-                skeys[r] = v[i];
+                if (m & one) skeys[r] = v[i];
             }
         }
         // where this tile's items of bin `tid` go inside the segment
         S excl = 0;
         bool ok = true;
         if (q.ti == 0) {
-            S h = 0;
-            if (tid < RADIX_BINS) h = hist[((size_t)q.seg * Sh::DIGITS + byte) * RADIX_BINS + tid];
-            excl = radix_bin_scan<S>(h, ws2);
+            excl = digit.first(q.seg, q.sbase, ws2);
         } else if (tid < RADIX_BINS) {
             constexpr int LB = 4;
             const S* p = my - RADIX_BINS;
@@ -450,7 +490,7 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
         for (int i = 0; i < IPT; ++i) {
             const int p = i * NT + tid;
             const T x = skeys[p];
-            const S o = goff[radix_digit(Traits<T>::key(x), byte, dx)] + (S)p;
+            const S o = goff[digit(x)] + (S)p;
             // (o < slen always holds while the input does not change under the sort)
             if (p < q.cnt && o < (S)q.slen) out[o] = x;
         }

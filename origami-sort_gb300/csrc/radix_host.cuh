@@ -1,8 +1,10 @@
-// Host launcher of the radix passes (radix.cuh).
+// Host launchers of the radix passes (radix.cuh) and the bucket sort
+// (buckets.cuh).
 #pragma once
 #include <algorithm>
 #include <string>
 
+#include "buckets.cuh"
 #include "pipeline.cuh"
 #include "profiler.h"
 #include "radix.cuh"
@@ -32,19 +34,54 @@ struct RadixPlan {
     }
 };
 
-// Device scratch of one radix sort (each part 256-byte aligned):
-//   look 0/1   look-back words of the even / odd passes, 256 per tile
-//   hist       digit counts, [segment][digit][256]
-//   tail       256 bytes: the error word, the passes' tile counters (+64)
-// hist and tail start at zero (one memset).
+// Bucket sort of a full sort or of chunks: bits per level, 0 when it does not
+// take the call (buckets would be larger than half of what fits, or the items
+// too few for 16 buckets).
+template <class T>
+struct BucketPlan {
+    using Sh = BucketShape<T>;
+    int b1 = 0, b2 = 0;
+    uint64_t tiles = 0, tiles2 = 0, nbuckets = 0;
+    BucketPlan(const RadixPlan<T>& p) {
+        if (p.n >= (1ull << 31)) return;
+        int bits = 0;
+        while ((p.len >> bits) > (1ull << Sh::C::LOG_TARGET)) ++bits;
+        if (bits < 4 || bits > BK_MAX_BITS) return;
+        if (p.nseg > 1 && (p.len % Sh::TILE != 0 || p.nseg > (1u << 20))) return;
+        // two levels of about equal width: few slices would serialise the atomics
+        b1 = bits > 8 ? (bits + 1) / 2 : bits;
+        b2 = bits - b1;
+        tiles = (p.n + Sh::TILE - 1) / Sh::TILE;
+        tiles2 = b2 ? tiles + (p.nseg << b1) : 0;
+        nbuckets = p.nseg << bits;
+    }
+    bool on() const { return b1 > 0; }
+};
+
+// Device scratch of one sort (each part 256-byte aligned):
+//   look 1/0   look-back words of the odd / even passes, 256 per tile
+//   bucket sort: slice starts and cursors of both levels, slice maps, tiles of
+//   the second level and their count
+//   hist 1/2   counts of the bucket sort's levels
+//   hist       digit counts of the radix passes, [segment][digit][256]
+//   tail       256 bytes: the error word, the passes' tile counters (+64), the
+//              bucket sort's route (+128)
+// From `zero` on everything starts at 0 (one memset).
 template <class T>
 struct RadixScratch {
+    using K = typename Traits<T>::Key;
     uint64_t bytes = 0, zero_bytes = 0;
+    char* zero = nullptr;
     void* look[2] = {nullptr, nullptr};
+    uint32_t *start1 = nullptr, *start2 = nullptr, *cursor1 = nullptr, *cursor2 = nullptr, *count2 = nullptr;
+    SliceMap<K>* maps = nullptr;
+    BkTile* tiles2 = nullptr;
+    uint32_t *hist1 = nullptr, *hist2 = nullptr;
     void* hist = nullptr;
-    int* err = nullptr;
+    int *err = nullptr, *route = nullptr;
     unsigned* claim = nullptr;
-    RadixScratch(void* base, const RadixPlan<T>& p) {
+    RadixScratch(void* base, const RadixPlan<T>& p, const BucketPlan<T>& bk) {
+        constexpr bool ST = BucketShape<T>::STABLE;
         const uint64_t w = p.wide ? 8 : 4;
         char* b = static_cast<char*>(base);
         uint64_t o = 0;
@@ -53,85 +90,201 @@ struct RadixScratch {
             o += (sz + 255) & ~255ull;
             return r;
         };
-        for (void*& l : look) l = take(p.tiles * RADIX_BINS * w);
-        zero_bytes = o;
+        auto words = [&](uint64_t k) { return reinterpret_cast<uint32_t*>(take(k * 4)); };
+        if (bk.on()) {
+            start1 = words((p.nseg << bk.b1) + 1);
+            if (!ST) cursor1 = words(p.nseg << bk.b1);
+            maps = reinterpret_cast<SliceMap<K>*>(take(p.nseg * sizeof(SliceMap<K>)));
+            if (bk.b2) {
+                start2 = words(bk.nbuckets + 1);
+                if (!ST) cursor2 = words(bk.nbuckets);
+                tiles2 = reinterpret_cast<BkTile*>(take(bk.tiles2 * sizeof(BkTile)));
+            }
+        }
+        // the second level's words: the first pass clears those of its own tiles
+        look[1] = take(std::max(p.tiles, ST ? bk.tiles2 : 0) * RADIX_BINS * w);
+        uint64_t z = o;
+        if (ST && bk.b2) z -= (bk.tiles2 - bk.tiles) * RADIX_BINS * w;
+        look[0] = take(p.tiles * RADIX_BINS * w);
+        if (!(ST && bk.on())) z = o;  // (cleared by radix_hist_kernel)
+        if (bk.on()) {
+            hist1 = words(p.nseg << bk.b1);
+            if (bk.b2) hist2 = words(bk.nbuckets);
+        }
         hist = take(p.nseg * RadixShape<T>::DIGITS * RADIX_BINS * w);
         err = reinterpret_cast<int*>(take(256));
-        claim = b ? reinterpret_cast<unsigned*>(reinterpret_cast<char*>(err) + 64) : nullptr;
-        zero_bytes = o - zero_bytes;
+        if (b) {
+            claim = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(err) + 64);
+            route = reinterpret_cast<int*>(reinterpret_cast<char*>(err) + 128);
+            count2 = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(err) + 132);
+            zero = b + z;
+        }
+        zero_bytes = o - z;
         bytes = o;
     }
 };
 
 template <class T>
 uint64_t radix_scratch_bytes(uint64_t n, uint64_t sort_n) {
-    return RadixScratch<T>(nullptr, RadixPlan<T>(n, sort_n)).bytes;
+    const RadixPlan<T> p(n, sort_n);
+    return RadixScratch<T>(nullptr, p, BucketPlan<T>(p)).bytes;
 }
 
+inline uint32_t resident_ctas(const void* kernel, int nt, size_t smem) {
+    int dev = 0, sms = 0, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, nt, smem);
+    return (uint32_t)(sms * (per > 0 ? per : 1));
+}
+
+// The radix passes: d -> want (d or tmp). With `route` they stand behind a
+// bucket sort and run only where it gave up.
 template <class T, class S>
-cudaError_t radix_launch(T* d, T* other, bool copy, const RadixPlan<T>& p, uint64_t xmask, const RadixScratch<T>& sc,
-                         cudaStream_t st) {
+void radix_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, uint64_t xmask, const RadixScratch<T>& sc,
+                  const int* route, cudaStream_t st) {
     using Sh = RadixShape<T>;
     using G = RadixUniform;
-    struct Grids {
-        uint32_t hist, pass;
-    };
-    static const Grids g = [] {  // kernel attributes and grids, once per process
-        int dev = 0, sms = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(radix_pass_kernel<T, S, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM);
-        cudaFuncSetAttribute(radix_hist_kernel<T, S, G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)Sh::HIST_SMEM);
-        cudaFuncSetAttribute(radix_hist_kernel<T, S, G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)Sh::HIST_SMEM);
-        Grids r;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, radix_hist_kernel<T, S, G, false>, 512, Sh::HIST_SMEM);
-        r.hist = (uint32_t)(sms * (per > 0 ? per : 1));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, radix_pass_kernel<T, S, G>, Sh::NT, Sh::SMEM);
-        r.pass = (uint32_t)(sms * (per > 0 ? per : 1));
-        return r;
-    }();
+    using D = ByteDigit<T, S>;
+    // kernel attributes and grids, once per process
+    static const uint32_t g_hist = resident_ctas((const void*)radix_hist_kernel<T, S, G>, 512, Sh::HIST_SMEM);
+    static const uint32_t g_pass = resident_ctas((const void*)radix_pass_kernel<T, S, G, D>, Sh::NT, Sh::SMEM);
     static const std::string n_hist = std::string("radix_hist<") + TypeName<T>::v + ">";
     static const std::string n_pass = std::string("radix_pass<") + TypeName<T>::v + ">";
     const uint32_t tiles = (uint32_t)p.tiles;
     const G geo{p.n, p.len, p.shift};
     S* hist = static_cast<S*>(sc.hist);
-    cudaMemsetAsync(hist, 0, sc.zero_bytes, st);
     launch(n_hist.c_str(), st, [&] {
-        const uint32_t gh = std::min(tiles, g.hist);
-        S* l0 = static_cast<S*>(sc.look[0]);
-        if (copy)
-            radix_hist_kernel<T, S, G, true><<<gh, 512, Sh::HIST_SMEM, st>>>(d, other, geo, tiles, xmask, hist, l0);
-        else
-            radix_hist_kernel<T, S, G, false><<<gh, 512, Sh::HIST_SMEM, st>>>(d, nullptr, geo, tiles, xmask, hist, l0);
+        launch_dependent(radix_hist_kernel<T, S, G>, dim3(std::min(tiles, g_hist)), dim3(512), Sh::HIST_SMEM, st,
+                         (const T*)d, (const T*)tmp, want, geo, tiles, xmask, hist, static_cast<S*>(sc.look[0]), route);
     });
-    T* src = copy ? other : d;
-    T* dst = copy ? d : other;
+    T* src = want;
+    T* dst = want == d ? tmp : d;
     static_assert(Sh::DIGITS % 2 == 0, "the passes end in the buffer they start from");
     for (int b = 0; b < Sh::DIGITS; ++b) {
         launch(n_pass.c_str(), st, [&] {
-            launch_dependent(radix_pass_kernel<T, S, G>, dim3(std::min(tiles, g.pass)), dim3(Sh::NT), Sh::SMEM, st,
-                             (const T*)src, dst, geo, tiles, b, xmask, (const S*)hist, static_cast<S*>(sc.look[b & 1]),
+            launch_dependent(radix_pass_kernel<T, S, G, D>, dim3(std::min(tiles, g_pass)), dim3(Sh::NT), Sh::SMEM, st,
+                             (const T*)src, dst, geo, tiles, D(hist, xmask, b), static_cast<S*>(sc.look[b & 1]),
                              b + 1 < Sh::DIGITS ? static_cast<S*>(sc.look[(b + 1) & 1]) : (S*)nullptr, sc.claim + b,
-                             sc.err, wait_limit());
+                             sc.err, wait_limit(), route, false);
         });
         std::swap(src, dst);
     }
-    return cudaGetLastError();
 }
 
-// Sorts d[0..n) in chunks of sort_n (0 = one full sort) into `want` (d or tmp).
-// The passes are an even number, so they end in the buffer they start from:
-// with want == tmp the counting kernel copies the input there as it reads it.
-// `scratch` holds radix_scratch_bytes<T>(n, sort_n) bytes.
+// The bucket sort: d -> want (d or tmp), *route set where it gives up.
+template <class T>
+void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPlan<T>& bk, uint64_t xmask,
+                   const RadixScratch<T>& sc, cudaStream_t st) {
+    using Sh = BucketShape<T>;
+    using RSh = RadixShape<T>;
+    using K = typename Traits<T>::Key;
+    using G1 = RadixUniform;
+    using G2 = BkListed;
+    using D = SliceDigitStable<T>;
+    constexpr bool ST = Sh::STABLE;
+    constexpr size_t SAMPLE_SMEM = ((1u << BK_MAX_BITS) / 2 + 1) * 4;
+    static const uint32_t g_hist = resident_ctas((const void*)bk_hist_kernel<T, G1>, 512, 0);
+    static const uint32_t g_part = [] {
+        cudaFuncSetAttribute(bk_sample_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SAMPLE_SMEM);
+        cudaFuncSetAttribute(bk_sort_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SORT_SMEM);
+        if constexpr (ST) {
+            resident_ctas((const void*)radix_pass_kernel<T, uint32_t, G2, D>, RSh::NT, RSh::SMEM);
+            return resident_ctas((const void*)radix_pass_kernel<T, uint32_t, G1, D>, RSh::NT, RSh::SMEM);
+        } else {
+            cudaFuncSetAttribute(bk_pass_kernel<T, G1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::PASS_SMEM);
+            cudaFuncSetAttribute(bk_pass_kernel<T, G2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::PASS_SMEM);
+            return 0u;
+        }
+    }();
+    static const std::string n_sample = std::string("bucket_sample<") + TypeName<T>::v + ">";
+    static const std::string n_hist = std::string("bucket_hist<") + TypeName<T>::v + ">";
+    static const std::string n_scan = std::string("bucket_scan<") + TypeName<T>::v + ">";
+    static const std::string n_pass = std::string("bucket_pass<") + TypeName<T>::v + ">";
+    static const std::string n_sort = std::string("bucket_sort<") + TypeName<T>::v + ">";
+    const int bits = bk.b1 + bk.b2;
+    const uint32_t nseg = (uint32_t)p.nseg, tiles = (uint32_t)bk.tiles, n32 = (uint32_t)p.n;
+    // (the partition tile may differ from the radix passes')
+    uint32_t shift = 31;
+    if (nseg > 1)
+        for (shift = 0; ((uint64_t)Sh::TILE << shift) < p.len;) ++shift;
+    const G1 geo{p.n, p.len, shift};
+    launch(n_sample.c_str(), st, [&] {
+        bk_sample_kernel<T><<<nseg, 1024, ((1u << bits) / 2 + 1) * 4, st>>>(d, p.n, p.len, xmask, bk.b1, bk.b2,
+                                                                            (uint64_t)Sh::CAP, sc.maps, sc.route);
+    });
+    auto level = [&](auto geo_l, const T* src, T* dst, uint32_t tiles_l, int shift_l, int bits_l, uint32_t map_shift,
+                     uint32_t segs, const uint32_t* seg_start, uint32_t* hist, uint32_t* start, uint32_t* cursor,
+                     bool last, int full_route, void* look, void* look_next, unsigned* claim) {
+        using G = decltype(geo_l);
+        launch(n_hist.c_str(), st, [&] {
+            launch_dependent(bk_hist_kernel<T, G>, dim3(std::min(tiles_l, g_hist)), dim3(512), 0, st, src, geo_l, tiles_l,
+                             (const SliceMap<K>*)sc.maps, map_shift, xmask, shift_l, bits_l, hist,
+                             (const int*)sc.route);
+        });
+        launch(n_scan.c_str(), st, [&] {
+            launch_dependent(bk_scan_kernel<T>, dim3(segs), dim3(RADIX_BINS), 0, st, (const uint32_t*)hist, bits_l,
+                             seg_start, p.len, start, cursor, p.n, segs - 1, last ? (BkTile*)nullptr : sc.tiles2,
+                             sc.count2, sc.route, full_route);
+        });
+        launch(n_pass.c_str(), st, [&] {
+            if constexpr (ST) {
+                D dig;
+                dig.xmask = xmask;
+                dig.shift = shift_l;
+                dig.mask = (1u << bits_l) - 1;
+                dig.maps = sc.maps;
+                dig.map_shift = map_shift;
+                dig.start = start;
+                dig.bits = bits_l;
+                launch_dependent(radix_pass_kernel<T, uint32_t, G, D>, dim3(std::min(tiles_l, g_part)), dim3(RSh::NT),
+                                 RSh::SMEM, st, src, dst, geo_l, tiles_l, dig, static_cast<uint32_t*>(look),
+                                 static_cast<uint32_t*>(look_next), claim, sc.err, wait_limit(), (const int*)sc.route,
+                                 true);
+            } else {
+                launch_dependent(bk_pass_kernel<T, G>, dim3(tiles_l), dim3(Sh::C::NT), Sh::PASS_SMEM, st, src, dst, geo_l,
+                                 tiles_l, (const SliceMap<K>*)sc.maps, map_shift, xmask, shift_l, bits_l, cursor, n32,
+                                 (const int*)sc.route);
+            }
+        });
+    };
+    const T* cur = tmp;
+    level(geo, d, tmp, tiles, bk.b2, bk.b1, 0u, nseg, (const uint32_t*)nullptr, sc.hist1, sc.start1, sc.cursor1, !bk.b2,
+          (int)ROUTE_RADIX, sc.look[0], bk.b2 ? sc.look[1] : nullptr, sc.claim + 8);
+    if (bk.b2) {
+        level(G2{sc.tiles2, sc.count2}, tmp, d, (uint32_t)bk.tiles2, 0, bk.b2, (uint32_t)bk.b1, nseg << bk.b1,
+              (const uint32_t*)sc.start1, sc.hist2, sc.start2, sc.cursor2, true, (int)ROUTE_RADIX_MOVED, sc.look[1],
+              (void*)nullptr, sc.claim + 9);
+        cur = d;
+    }
+    launch(n_sort.c_str(), st, [&] {
+        launch_dependent(bk_sort_kernel<T>, dim3((unsigned)bk.nbuckets), dim3(Sh::C::S_NT), Sh::SORT_SMEM, st, cur, want,
+                         (const uint32_t*)(bk.b2 ? sc.start2 : sc.start1), xmask, n32, (const int*)sc.route);
+    });
+}
+
+// Sorts d[0..n) in chunks of sort_n (0 = one full sort) into `want` (d or tmp):
+// by buckets where the geometry allows it, with the radix passes behind them
+// for what does not spread; else by radix passes. `scratch` holds
+// radix_scratch_bytes<T>(n, sort_n) bytes.
 template <class T>
 cudaError_t radix_sort(T* d, T* tmp, uint64_t n, uint64_t sort_n, uint64_t key_mask, T* want, void* scratch,
                        cudaStream_t st) {
     const RadixPlan<T> p(n, sort_n);
-    const RadixScratch<T> sc(scratch, p);
-    if (p.wide) return radix_launch<T, uint64_t>(d, tmp, want == tmp, p, key_mask, sc, st);
-    return radix_launch<T, uint32_t>(d, tmp, want == tmp, p, key_mask, sc, st);
+    const BucketPlan<T> bk(p);
+    const RadixScratch<T> sc(scratch, p, bk);
+    cudaMemsetAsync(sc.zero, 0, sc.zero_bytes, st);
+    const int* route = nullptr;
+    if (bk.on()) {
+        bucket_launch<T>(d, tmp, want, p, bk, key_mask, sc, st);
+        route = sc.route;
+    }
+    if (p.wide)
+        radix_launch<T, uint64_t>(d, tmp, want, p, key_mask, sc, route, st);
+    else
+        radix_launch<T, uint32_t>(d, tmp, want, p, key_mask, sc, route, st);
+    return cudaGetLastError();
 }
 
 }  // namespace origami

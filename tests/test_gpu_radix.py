@@ -1,6 +1,8 @@
-"""Radix passes (the default of device sorts from some size on): tile edges,
-ragged ends, digits with one, two and sixteen values, both result buffers,
-chunks, and their bounded waits. Integer work: the tolerance is zero."""
+"""Bucket sort and the radix passes behind it (the default of device sorts from
+some size on): tile edges, ragged ends, one and two partition levels, digits
+with one, two and sixteen values, clustered, duplicated and outlying keys, both
+result buffers, chunks, and the bounded waits. Integer work: the tolerance is
+zero."""
 import ctypes
 
 import numpy as np
@@ -36,6 +38,17 @@ def keys(dist, n, seed):
         k[n // 2] = ~np.uint64(0)
     elif dist == "sorted":
         k.sort()
+    elif dist == "normal":  # slices of very different sizes
+        k = (np.clip(rng.normal(0.5, 0.1, n), 0, 1) * (2.0**64 - 4096)).astype(np.uint64)
+    elif dist == "repeated":  # every key some 200 times
+        d = rng.integers(0, 2**64, max(1, n // 200), dtype=np.uint64)
+        k = d[rng.integers(0, len(d), n)]
+    elif dist == "clusters":  # 100 neighbouring keys around each of many centres
+        d = rng.integers(0, 2**64, max(1, n // 1000), dtype=np.uint64) & ~np.uint64(0x7F00000000)
+        k = d[rng.integers(0, len(d), n)] + (rng.integers(0, 100, n).astype(np.uint64) << np.uint64(32))
+    elif dist == "outliers":  # a narrow range and a few keys far outside it
+        k = (k >> np.uint64(22)) + (np.uint64(5) << np.uint64(60))
+        k[:: max(1, n // 5)] = rng.integers(0, 2**64, len(k[:: max(1, n // 5)]), dtype=np.uint64)
     return k
 
 
@@ -43,7 +56,7 @@ def items(kind, dist, n, seed):
     k = keys(dist, n, seed)
     a = orc.empty(kind, n)
     if kind == og.U32:
-        a[:] = (k >> np.uint64(32) if dist in ("uniform", "sorted") else k).astype(np.uint32)
+        a[:] = (k if dist in ("equal", "two", "sixteen", "small", "one_high") else k >> np.uint64(32)).astype(np.uint32)
     elif a.dtype.names:
         a["key"] = k.view(a.dtype["key"])
         a["value"] = np.arange(n)
@@ -78,6 +91,16 @@ def test_radix_matches_stable_sort(kind, dist, n, in_tmp):
     assert np.array_equal(device_sort(a, kind, result_in_tmp=in_tmp), expected(a))
 
 
+# the largest one-level sort and the smallest two-level one of each kind are
+# 2^20 / 2^20 + 1 items (u32) and 2^19 / 2^19 + 1 (64-bit keys)
+@pytest.mark.parametrize("dist", ["uniform", "normal", "repeated", "clusters", "outliers"])
+@pytest.mark.parametrize("kind", [og.U32, og.U64, og.I64, og.KV64, og.KVU64])
+@pytest.mark.parametrize("n", [1 << 19, (1 << 19) + 1, 1 << 20, (1 << 20) + 1, (1 << 22) + 8191])
+def test_buckets_match_stable_sort(kind, dist, n):
+    a = items(kind, dist, n, seed=n + kind)
+    assert np.array_equal(device_sort(a, kind, result_in_tmp=bool(n & 1)), expected(a))
+
+
 @pytest.mark.parametrize("kind", [og.U32, og.I64, og.KV64])
 @pytest.mark.parametrize("sort_n", [1 << 19, 1 << 20])
 def test_radix_chunks(kind, sort_n):
@@ -105,7 +128,7 @@ def test_radix_long_segment():
 @pytest.mark.parametrize("kind", [og.U32, og.KV64])
 def test_radix_reports_expired_wait_then_recovers(kind):
     n = 1 << 20
-    a = items(kind, "uniform", n, seed=5)
+    a = items(kind, "sixteen", n, seed=5)  # (buckets of keys wait for nothing)
     d = torch.from_numpy(a.view(np.uint8).copy()).cuda()
     t = torch.empty_like(d)
     res = ctypes.c_void_p()
