@@ -136,8 +136,10 @@ int origami_merge_series_device(int kind, void* src, void* dst, uint64_t n, uint
  * is sorted independently and in place (the result is in d; tmp is scratch of
  * n items). All segments go through the same short launch sequence, planned
  * on the device (no host synchronisation, so it can be captured in a CUDA
- * graph): one tile-sort launch for every segment's tiles (a short segment is
- * one tile, sorted in registers and shared memory), then for each merge level
+ * graph): by default the segments longer than a bucket that shared memory holds
+ * are cut into slices, level by level, and one launch sorts all buckets, short
+ * segments among them; where the tuning table (below) says so, or the scratch
+ * for that cannot be had, one tile-sort launch and then for each merge level
  * a partition and a persistent merge launch over the segments still merging.
  * Key-value segments are sorted stably.
  *   _device: d, tmp, offsets are device memory, d and tmp 16-byte aligned,
@@ -356,7 +358,8 @@ int origami_generate_device(int kind, void* d, uint64_t n, int dist, uint64_t se
  *                      "kind class fan variant"
  *                      lines, radix choices that differ from the built-in ones
  *                      as "radix kind class on" lines, and the segmented
- *                      table's (below) as "seg kind class shape" lines. The file named by
+ *                      table's (below) as "seg kind class shape" and
+ *                      "segbuckets kind class on" lines. The file named by
  *                      ORIGAMI_TUNING, if set, is loaded at first use.
  */
 int origami_autotune(int kind, uint64_t n, char* report, uint64_t cap);
@@ -367,17 +370,19 @@ int origami_tuning_load(const char* path);
 
 /*
  * Segmented-sort tuning (no counterpart in the reference; its analogue is the
- * compile-time config.h tables and the bench_sort_phases sweeps). The level
- * merges of a batched segmented sort use one of two merge shapes: 0 (the
- * default) is the binary pass's first tile shape, 1 its second (twice the tile,
- * more threads). The table is keyed by item kind and the size class
- * floor(log2(n / nseg)) of the mean segment length; every segmented launch
- * (origami_sort_segmented*, origami_seg_plan_create, the serving loop's
- * batches) takes its shape from it.
- *   origami_autotune_segmented  times both shapes on the caller's own device
- *                      segments (d is left holding its input), stores the
- *                      faster; `report` (may be NULL) gets "shape= ms=" lines.
- *   get / set          read or write one entry (shape 0 or 1).
+ * compile-time config.h tables and the bench_sort_phases sweeps). The table is
+ * keyed by item kind and the size class floor(log2(n / nseg)) of the mean
+ * segment length; every segmented launch (origami_sort_segmented*,
+ * origami_seg_plan_create, the serving loop's batches) takes its choice from it:
+ * buckets (the built-in choice) or merges, and the shape of the level merges: 0
+ * is the binary pass's first tile shape, 1 its second (twice the tile, more
+ * threads).
+ *   origami_autotune_segmented  times both merge shapes and the buckets on the
+ *                      caller's own device segments (d is left holding its
+ *                      input), stores the fastest; `report` (may be NULL) gets
+ *                      "shape= ms=" lines and a "buckets ms=" line.
+ *   get / set          read or write one entry's merge shape (0 or 1). Setting 0
+ *                      restores the built-in choice; 1 selects merges.
  */
 int origami_autotune_segmented(int kind, void* d, void* tmp, const uint64_t* offsets, uint64_t nseg, uint64_t n,
                                char* report, uint64_t cap);

@@ -24,6 +24,7 @@ namespace origami {
 
 constexpr uint32_t BULK_SPIN_LIMIT = 1u << 20;
 constexpr int ERR_WAIT_EXPIRED = 1;
+constexpr int ERR_BAD_OFFSETS = 2;
 constexpr int ERR_WAIT_UNDRAINED = 3;
 constexpr int ERR_BAD_RUNS = 5;
 

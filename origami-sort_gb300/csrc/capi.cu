@@ -296,8 +296,11 @@ int shape_for(int kind, uint64_t n, unsigned min_k) {
     return shape_code(fan_of(min_k), 0);
 }
 
-// Segmented sorts: the level merges' merge shape (0 / 1, SegMergeCfg) per
-// kind and size class of the mean segment length. Default 0.
+// Segmented sorts, per kind and size class of the mean segment length: buckets
+// (SEG_BUCKETS, the built-in choice), and the level merges' merge shape (0 / 1,
+// SegMergeCfg) where merges run.
+constexpr int SEG_BUCKETS = 1 << 8;
+inline int seg_builtin(int shape) { return shape == 0 ? SEG_BUCKETS : shape; }
 std::atomic<int> g_seg_tune[5][TUNE_CLASSES];
 
 int seg_class(uint64_t n, uint64_t nseg) { return size_class(nseg ? n / nseg : n); }
@@ -793,7 +796,8 @@ void tune_store(int kind, int cls, int code);
 // Tuning file: one entry per line. "kind class fan variant": the plain sort's
 // merge shape for a size class; "radix kind class on": whether the class sorts
 // by radix passes, after its shape line; "seg kind class shape": the segmented
-// sort's merge shape for a class of mean segment length. Other lines are skipped.
+// sort's merge shape for a class of mean segment length; "segbuckets kind class
+// on": whether it sorts by buckets, after its shape line. Other lines are skipped.
 int tune_load_file(const char* path) {
     FILE* f = std::fopen(path, "r");
     if (!f) return fail(ORIGAMI_ERR_INVALID, "cannot open tuning file %s", path);
@@ -802,7 +806,14 @@ int tune_load_file(const char* path) {
     while (std::fgets(line, sizeof line, f)) {
         if (std::sscanf(line, "seg %d %d %d", &kind, &cls, &var) == 3) {
             if (kind < 0 || kind > 4 || cls < 0 || cls >= TUNE_CLASSES || (var != 0 && var != 1)) continue;
-            g_seg_tune[kind][cls].store(var, std::memory_order_relaxed);
+            g_seg_tune[kind][cls].store(seg_builtin(var), std::memory_order_relaxed);
+            ++loaded;
+            continue;
+        }
+        if (std::sscanf(line, "segbuckets %d %d %d", &kind, &cls, &var) == 3) {
+            if (kind < 0 || kind > 4 || cls < 0 || cls >= TUNE_CLASSES || (var != 0 && var != 1)) continue;
+            const int c = g_seg_tune[kind][cls].load(std::memory_order_relaxed);
+            g_seg_tune[kind][cls].store(var ? c | SEG_BUCKETS : c & ~SEG_BUCKETS, std::memory_order_relaxed);
             ++loaded;
             continue;
         }
@@ -872,7 +883,7 @@ void tune_init() {
     for (int k = 0; k < 5; ++k)
         for (int c = 0; c < TUNE_CLASSES; ++c) g_tune[k][c].store(tune_builtin(k, c), std::memory_order_relaxed);
     for (auto& row : g_seg_tune)
-        for (auto& c : row) c.store(0, std::memory_order_relaxed);
+        for (auto& c : row) c.store(seg_builtin(0), std::memory_order_relaxed);
     if (const char* path = std::getenv("ORIGAMI_TUNING")) tune_load_file(path);
 }
 
@@ -950,9 +961,32 @@ int noalloc_check(int kind, const void* d, const void* tmp, uint64_t n, uint64_t
 int api_fail(int code, const char* msg) { return fail(code, "%s", msg); }
 int arena_init() { return ensure_device(); }
 
-SegPlan seg_plan(int kind, uint64_t n, uint64_t nseg) {
+// The bucket sort's plan, where it takes the sort.
+static bool seg_bucket_plan(int kind, uint64_t n, uint64_t nseg, SegPlan& p) {
+    switch (kind) {
+        case ORIGAMI_U32:
+            p.buckets = segbucket_fits_u32(n, nseg);
+            if (p.buckets) p.scratch_bytes = segbucket_scratch_bytes_u32(n, nseg);
+            break;
+        case ORIGAMI_U64:
+        case ORIGAMI_I64:
+            p.buckets = segbucket_fits_u64(n, nseg);
+            if (p.buckets) p.scratch_bytes = segbucket_scratch_bytes_u64(n, nseg);
+            break;
+        default:
+            p.buckets = segbucket_fits_kv(n, nseg);
+            if (p.buckets) p.scratch_bytes = segbucket_scratch_bytes_kv(n, nseg);
+            break;
+    }
+    p.err_offset = p.scratch_bytes - 256;
+    return p.buckets;
+}
+
+SegPlan seg_plan(int kind, uint64_t n, uint64_t nseg, bool merges) {
     SegPlan p{};
-    p.shape = seg_shape_for(kind, n, nseg);
+    const int code = seg_shape_for(kind, n, nseg);
+    p.shape = code & 0xFF;
+    if (!merges && (code & SEG_BUCKETS) && seg_bucket_plan(kind, n, nseg, p)) return p;
     switch (kind) {
         case ORIGAMI_U32:
             p.maxl = seg_levels_u32(n);
@@ -976,16 +1010,33 @@ SegPlan seg_plan(int kind, uint64_t n, uint64_t nseg) {
 
 void seg_prepare(int kind) {
     switch (kind) {
-        case ORIGAMI_U32: seg_prepare_u32(); break;
+        case ORIGAMI_U32:
+            seg_prepare_u32();
+            segbucket_prepare_u32();
+            break;
         case ORIGAMI_U64:
-        case ORIGAMI_I64: seg_prepare_u64(); break;
-        default: seg_prepare_kv(); break;
+        case ORIGAMI_I64:
+            seg_prepare_u64();
+            segbucket_prepare_u64();
+            break;
+        default:
+            seg_prepare_kv();
+            segbucket_prepare_kv();
+            break;
     }
 }
 
 cudaError_t seg_launch(int kind, void* d, void* tmp, const uint64_t* off, uint64_t nseg, uint64_t n,
                        void* scratch, const SegPlan& p, cudaStream_t st) {
     const uint64_t m = key_mask(kind);
+    if (p.buckets) {
+        switch (kind) {
+            case ORIGAMI_U32: return segbucket_sort_u32(d, tmp, off, nseg, n, m, scratch, st);
+            case ORIGAMI_U64:
+            case ORIGAMI_I64: return segbucket_sort_u64(d, tmp, off, nseg, n, m, scratch, st);
+            default: return segbucket_sort_kv(d, tmp, off, nseg, n, m, scratch, st);
+        }
+    }
     switch (kind) {
         case ORIGAMI_U32: return seg_sort_u32(d, tmp, off, nseg, n, m, scratch, p.maxl, p.shape, st);
         case ORIGAMI_U64:
@@ -1071,10 +1122,17 @@ int origami_sort_segmented_device(int kind, void* d, void* tmp, const uint64_t* 
     int rc = ensure_device();
     if (rc != ORIGAMI_OK) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    const SegPlan plan = seg_plan(kind, n, nseg);
+    SegPlan plan = seg_plan(kind, n, nseg);
     void* scratch = nullptr;
-    CK(cudaMallocAsync(&scratch, plan.scratch_bytes, st), "segmented scratch");
-    cudaError_t e = seg_launch(kind, d, tmp, offsets, nseg, n, scratch, plan, st);
+    cudaError_t e = cudaMallocAsync(&scratch, plan.scratch_bytes, st);
+    if (e == cudaErrorMemoryAllocation && plan.buckets) {
+        // the merges need less scratch
+        cudaGetLastError();
+        plan = seg_plan(kind, n, nseg, true);
+        e = cudaMallocAsync(&scratch, plan.scratch_bytes, st);
+    }
+    CK(e, "segmented scratch");
+    e = seg_launch(kind, d, tmp, offsets, nseg, n, scratch, plan, st);
     int herr = 0;
     if (e == cudaSuccess && (flags & ORIGAMI_FLAG_SYNC)) {
         e = cudaMemcpyAsync(&herr, static_cast<char*>(scratch) + plan.err_offset, sizeof(int),
@@ -1244,8 +1302,9 @@ int origami_tuning_save(const char* path) {
         }
     for (int k = 0; k < 5; ++k)
         for (int c = 0; c < TUNE_CLASSES; ++c) {
-            const int shape = g_seg_tune[k][c].load(std::memory_order_relaxed);
+            const int code = g_seg_tune[k][c].load(std::memory_order_relaxed), shape = code & 0xFF;
             if (shape != 0) std::fprintf(f, "seg %d %d %d\n", k, c, shape);
+            if (code != seg_builtin(shape)) std::fprintf(f, "segbuckets %d %d %d\n", k, c, code & SEG_BUCKETS ? 1 : 0);
         }
     std::fclose(f);
     return ORIGAMI_OK;
@@ -1343,7 +1402,7 @@ int origami_autotune(int kind, uint64_t n, char* report, uint64_t cap) {
 int origami_seg_tuning_get(int kind, uint64_t n, uint64_t nseg, int* shape) {
     if (!valid_kind(kind)) return fail(ORIGAMI_ERR_DTYPE, "unknown item kind %d", kind);
     if (!shape) return fail(ORIGAMI_ERR_INVALID, "shape is NULL");
-    *shape = seg_shape_for(kind, n, nseg);
+    *shape = seg_shape_for(kind, n, nseg) & 0xFF;
     return ORIGAMI_OK;
 }
 
@@ -1351,7 +1410,7 @@ int origami_seg_tuning_set(int kind, uint64_t n, uint64_t nseg, int shape) {
     if (!valid_kind(kind)) return fail(ORIGAMI_ERR_DTYPE, "unknown item kind %d", kind);
     if (shape != 0 && shape != 1) return fail(ORIGAMI_ERR_INVALID, "shape must be 0 or 1");
     std::call_once(g_tune_once, tune_init);
-    g_seg_tune[kind][seg_class(n, nseg)].store(shape, std::memory_order_relaxed);
+    g_seg_tune[kind][seg_class(n, nseg)].store(seg_builtin(shape), std::memory_order_relaxed);
     return ORIGAMI_OK;
 }
 
@@ -1370,10 +1429,11 @@ int origami_autotune_segmented(int kind, void* d, void* tmp, const uint64_t* off
     std::call_once(g_tune_once, tune_init);
     const uint64_t bytes = n * item_bytes(kind);
     cudaStream_t st = worker_stream();
-    SegPlan plan = seg_plan(kind, n, nseg);
+    SegPlan plan = seg_plan(kind, n, nseg, true), bplan{};
+    seg_bucket_plan(kind, n, nseg, bplan);
     void *keep = nullptr, *scratch = nullptr;
     CK(cudaMallocAsync(&keep, bytes, st), "autotune buffers");
-    cudaError_t e = cudaMallocAsync(&scratch, plan.scratch_bytes, st);
+    cudaError_t e = cudaMallocAsync(&scratch, std::max(plan.scratch_bytes, bplan.scratch_bytes), st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(keep, d, bytes, cudaMemcpyDeviceToDevice, st);
     cudaEvent_t a = nullptr, b = nullptr;
     cudaEventCreate(&a);
@@ -1381,26 +1441,37 @@ int origami_autotune_segmented(int kind, void* d, void* tmp, const uint64_t* off
     std::string rep;
     int best = 0;
     float best_ms = 1e30f;
-    for (int shape = 0; shape < 2 && e == cudaSuccess; ++shape) {
-        plan.shape = shape;
+    char line[128];
+    auto timed = [&](const SegPlan& pl) {
         float ms_best = 1e30f;
         for (int it = 0; it < 4 && e == cudaSuccess; ++it) {
             e = cudaMemcpyAsync(d, keep, bytes, cudaMemcpyDeviceToDevice, st);
             if (e == cudaSuccess) e = cudaEventRecord(a, st);
-            if (e == cudaSuccess) e = seg_launch(kind, d, tmp, offsets, nseg, n, scratch, plan, st);
+            if (e == cudaSuccess) e = seg_launch(kind, d, tmp, offsets, nseg, n, scratch, pl, st);
             if (e == cudaSuccess) e = cudaEventRecord(b, st);
             if (e == cudaSuccess) e = cudaEventSynchronize(b);
             float ms = 0;
             if (e == cudaSuccess && it > 0 && cudaEventElapsedTime(&ms, a, b) == cudaSuccess)
                 ms_best = std::min(ms_best, ms);
         }
-        char line[128];
+        return ms_best;
+    };
+    for (int shape = 0; shape < 2 && e == cudaSuccess; ++shape) {
+        plan.shape = shape;
+        const float ms_best = timed(plan);
         std::snprintf(line, sizeof line, "shape=%d ms=%.4f\n", shape, ms_best);
         rep += line;
         if (ms_best < best_ms) {
             best_ms = ms_best;
             best = shape;
         }
+    }
+    bool buckets = false;
+    if (e == cudaSuccess && bplan.buckets) {
+        const float ms = timed(bplan);
+        std::snprintf(line, sizeof line, "buckets ms=%.4f\n", ms);
+        rep += line;
+        buckets = ms < best_ms;
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(d, keep, bytes, cudaMemcpyDeviceToDevice, st);
     cudaEventDestroy(a);
@@ -1410,9 +1481,9 @@ int origami_autotune_segmented(int kind, void* d, void* tmp, const uint64_t* off
     const cudaError_t es = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "segmented autotune");
     if (es != cudaSuccess) return cuda_fail(es, "segmented autotune");
-    g_seg_tune[kind][seg_class(n, nseg)].store(best, std::memory_order_relaxed);
-    char line[128];
-    std::snprintf(line, sizeof line, "chosen shape=%d mean_len_class=%d\n", best, seg_class(n, nseg));
+    g_seg_tune[kind][seg_class(n, nseg)].store(buckets ? best | SEG_BUCKETS : best, std::memory_order_relaxed);
+    std::snprintf(line, sizeof line, "chosen %sshape=%d mean_len_class=%d\n", buckets ? "buckets " : "", best,
+                  seg_class(n, nseg));
     rep += line;
     if (report && cap) {
         std::strncpy(report, rep.c_str(), cap - 1);

@@ -41,6 +41,20 @@ ORIGAMI_DECLARE_RADIX(u64)
 ORIGAMI_DECLARE_RADIX(kv)
 #undef ORIGAMI_DECLARE_RADIX
 
+// Segmented sort by buckets (seg_buckets.cuh): whether it takes nseg segments of n
+// items in all, the scratch it needs (error word in its last 256 bytes), the sort
+// (result in d), and one-time kernel attributes (call outside stream capture).
+#define ORIGAMI_DECLARE_SEGBUCKET(name)                                                                      \
+    bool segbucket_fits_##name(uint64_t n, uint64_t nseg);                                                   \
+    uint64_t segbucket_scratch_bytes_##name(uint64_t n, uint64_t nseg);                                      \
+    cudaError_t segbucket_sort_##name(void* d, void* tmp, const uint64_t* off, uint64_t nseg, uint64_t n,    \
+                                      uint64_t key_mask, void* scratch, cudaStream_t st);                    \
+    void segbucket_prepare_##name();
+ORIGAMI_DECLARE_SEGBUCKET(u32)
+ORIGAMI_DECLARE_SEGBUCKET(u64)
+ORIGAMI_DECLARE_SEGBUCKET(kv)
+#undef ORIGAMI_DECLARE_SEGBUCKET
+
 // Batched segmented sort (segmented.cuh): levels to plan for, scratch bytes,
 // the launch sequence, and where the error word sits inside the scratch.
 #define ORIGAMI_DECLARE_SEG(name)                                                                 \
@@ -63,10 +77,12 @@ ORIGAMI_DECLARE_SEG(kv)
 struct SegPlan {
     int maxl;
     uint64_t scratch_bytes;
-    int err_offset;
-    int shape;  // merge shape of the level merges (0 or 1), from the segmented tuning table
+    uint64_t err_offset;
+    int shape;     // merge shape of the level merges (0 or 1), from the segmented tuning table
+    bool buckets;  // sorted by buckets instead
 };
-SegPlan seg_plan(int kind, uint64_t n, uint64_t nseg);
+// merges: leave the bucket sort out (its scratch could not be had).
+SegPlan seg_plan(int kind, uint64_t n, uint64_t nseg, bool merges = false);
 void seg_prepare(int kind);
 cudaError_t seg_launch(int kind, void* d, void* tmp, const uint64_t* off, uint64_t nseg, uint64_t n,
                        void* scratch, const SegPlan& p, cudaStream_t st);

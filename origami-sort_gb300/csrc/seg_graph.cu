@@ -61,8 +61,16 @@ int origami_seg_plan_create(int kind, void* d, void* tmp, const uint64_t* offset
     p->n = n;
     p->nseg = nseg;
     p->plan = origami::seg_plan(kind, n, nseg);
-    if (cudaMalloc(&p->scratch, p->plan.scratch_bytes) != cudaSuccess) {
+    cudaError_t em = cudaMalloc(&p->scratch, p->plan.scratch_bytes);
+    if (em == cudaErrorMemoryAllocation && p->plan.buckets) {
+        // the merges need less scratch
         cudaGetLastError();
+        p->plan = origami::seg_plan(kind, n, nseg, true);
+        em = cudaMalloc(&p->scratch, p->plan.scratch_bytes);
+    }
+    if (em != cudaSuccess) {
+        cudaGetLastError();
+        p->scratch = nullptr;
         destroy(p);
         return api_fail(ORIGAMI_ERR_OOM, "plan scratch allocation failed");
     }

@@ -175,7 +175,8 @@ struct Layout {
     uint64_t tmp, off, scratch, total;
     SegPlan plan;
 };
-Layout layout(int kind, uint64_t items, uint64_t nseg) {
+// Where the bucket sort's scratch would take it past `limit`, the merges sort it.
+Layout layout(int kind, uint64_t items, uint64_t nseg, uint64_t limit) {
     Layout l;
     l.plan = origami::seg_plan(kind, items, nseg);
     const uint64_t data = r256(items * item_bytes(kind));
@@ -183,6 +184,10 @@ Layout layout(int kind, uint64_t items, uint64_t nseg) {
     l.off = 2 * data;
     l.scratch = l.off + r256((nseg + 1) * 8);
     l.total = l.scratch + r256(l.plan.scratch_bytes);
+    if (l.total > limit && l.plan.buckets) {
+        l.plan = origami::seg_plan(kind, items, nseg, true);
+        l.total = l.scratch + r256(l.plan.scratch_bytes);
+    }
     return l;
 }
 
@@ -261,7 +266,10 @@ struct origami_server {
     bool helpers_stop = false;
     std::vector<std::thread> helpers;
 
-    uint64_t need(int kind, uint64_t items, uint64_t nseg) const { return layout(kind, items, nseg).total; }
+    uint64_t need(int kind, uint64_t items, uint64_t nseg, uint64_t limit) const {
+        return layout(kind, items, nseg, limit).total;
+    }
+    uint64_t room() const { return budget > in_use ? budget - in_use : 0; }  // (mu held)
 
     // Large requests whose buffers the device can address, 16-byte aligned,
     // take the pipelined sort.
@@ -274,7 +282,7 @@ struct origami_server {
         return addressable(r.in) && addressable(r.out);
     }
     uint64_t need_of(const Request& r) const {
-        return pipe_ok(r) ? origami::host_pipe_bytes(r.kind, r.n) : need(r.kind, r.n, 1);
+        return pipe_ok(r) ? origami::host_pipe_bytes(r.kind, r.n) : need(r.kind, r.n, 1, budget);
     }
 
     static void CUDART_CB on_done(void* p) {
@@ -384,7 +392,7 @@ struct origami_server {
             }
             // the oldest request waits for memory rather than being overtaken,
             // so a large request is never starved by a stream of small ones
-            if (in_use + need(r->kind, items + r->n, b->reqs.size() + 1) > budget) {
+            if (in_use + need(r->kind, items + r->n, b->reqs.size() + 1, room()) > budget) {
                 if (b->reqs.empty() && !head) {
                     ++it;
                     continue;
@@ -402,7 +410,7 @@ struct origami_server {
         if (!b->pipe) {
             b->off.assign(b->reqs.size() + 1, 0);
             for (size_t i = 0; i < b->reqs.size(); ++i) b->off[i + 1] = b->off[i] + b->reqs[i]->n;
-            b->lay = layout(b->kind, items, b->reqs.size());
+            b->lay = layout(b->kind, items, b->reqs.size(), room());
             b->bytes = b->lay.total;
         }
         b->copied = true;

@@ -1,0 +1,162 @@
+"""Segmented sort by buckets (the default): lengths around the bucket, the tiles and
+the levels, segments that start at any item, heavy and clustered keys, samples that
+mislead, more buckets than the sort's grid, and the merge path as the other side.
+Integer work: the tolerance is zero."""
+import numpy as np
+import pytest
+
+import oracle as orc
+import origami_gpu as og
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+KINDS = [og.U32, og.U64, og.I64, og.KV64, og.KVU64]
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    import __graft_entry__ as g
+    g.build()
+    assert torch.cuda.is_available()
+
+
+def items(kind, k):
+    """Items with the 64-bit keys k (32-bit kinds: their upper halves)."""
+    a = orc.empty(kind, len(k))
+    if kind == og.U32:
+        a[:] = (k >> np.uint64(32)).astype(np.uint32)
+    elif a.dtype.names:
+        a["key"] = k.view(a.dtype["key"])
+        a["value"] = np.arange(len(k))
+    else:
+        a[:] = k.view(a.dtype)
+    return a
+
+
+def check(kind, a, lens):
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    d = torch.from_numpy(a.view(np.uint8).copy()).cuda()
+    og.sort_segmented(d, torch.from_numpy(off).cuda(), kind=kind)
+    got = d.cpu().numpy().view(a.dtype)
+    want = a.copy()
+    for s, e in zip(off[:-1], off[1:]):
+        x = a[s:e]
+        want[s:e] = x[np.argsort(x["key"], kind="stable")] if a.dtype.names else np.sort(x)
+    assert np.array_equal(got, want)
+
+
+def keys(dist, n, rng):
+    k = rng.integers(0, 2**64, n, dtype=np.uint64)
+    if dist == "equal":
+        k[:] = k[:1]
+    elif dist == "heavy":  # one key for half of the items, at one end of the order
+        k[rng.random(n) < 0.5] = ~np.uint64(0)
+    elif dist == "ids":  # a few thousand neighbouring keys
+        k = (k % np.uint64(3000)) << np.uint64(32)
+    elif dist == "zipf":
+        r = np.exp(rng.random(n) * np.log(2.0**20)).astype(np.uint64)
+        k = r * np.uint64(0x9E3779B97F4A7C15)
+    elif dist == "pairs":  # crowded bins of two heavy keys each
+        k = (k % np.uint64(40)) * np.uint64(1 << 58) + (k >> np.uint64(63) << np.uint64(33))
+    elif dist == "log":  # clusters in clusters
+        k >>= (k % np.uint64(32)).astype(np.uint64)
+    elif dist == "sorted":
+        k.sort()
+    return k
+
+
+# a bucket holds 6144 uint32 keys or 4096 wider items; tiles of the same size
+EDGES = [1, 0, 2, 33, 4095, 4096, 4097, 6143, 6144, 6145, 8191, 8193, 12289, 3 * 6144 + 1, 65537, 262147, 1]
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("dist", ["uniform", "equal", "heavy", "ids", "zipf", "pairs", "log", "sorted"])
+def test_lengths(kind, dist):
+    rng = np.random.default_rng(kind * 31 + len(dist))
+    check(kind, items(kind, np.concatenate([keys(dist, n, rng) for n in EDGES])), EDGES)
+
+
+@pytest.mark.parametrize("kind", [og.U32, og.I64, og.KV64])
+@pytest.mark.parametrize("dist", ["uniform", "zipf", "log"])
+def test_two_levels(kind, dist):
+    lens = [3, (1 << 21) + 77, 5000]
+    rng = np.random.default_rng(kind + 5)
+    check(kind, items(kind, np.concatenate([keys(dist, n, rng) for n in lens])), lens)
+
+
+def sampled(n, samples=2048):
+    j = np.arange(samples, dtype=np.uint64)
+    a = np.uint64(n) * j // np.uint64(samples)
+    gap = np.uint64(n) * (j + np.uint64(1)) // np.uint64(samples) - a
+    h = (j * np.uint64(2654435761) + np.uint64(12345)) & np.uint64(0xFFFFFFFF)
+    return (a + (h * gap >> np.uint64(32))).astype(np.int64)
+
+
+@pytest.mark.parametrize("kind", [og.U32, og.U64, og.KV64])
+def test_misleading_samples(kind):
+    # the first level's samples are spread over all keys, the other items lie in one
+    # of its slices and spread over their logarithms: the last level's slices are
+    # too long for a bucket and are sorted in global memory
+    n = 1200000 if kind == og.U32 else 800000
+    rng = np.random.default_rng(9)
+    k = np.exp(rng.random(n) * np.log(2.0**23)).astype(np.uint64) << np.uint64(32)
+    k |= rng.integers(0, 2**32, n, dtype=np.uint64)
+    p = sampled(n)
+    k[p] = rng.integers(0, 2**64, len(p), dtype=np.uint64)
+    check(kind, items(kind, k), [n])
+
+
+@pytest.mark.parametrize("kind", [og.U32, og.U64, og.KV64])
+def test_more_buckets_than_the_grid(kind):
+    # slices just over half a bucket, each followed by a slice of one item: twice as
+    # many buckets as half buckets in the segment
+    half = (6144 if kind == og.U32 else 4096) // 2 + 20
+    rng = np.random.default_rng(3)
+    k = []
+    for s in range(0, 256, 2):
+        k.append((np.uint64(s) << np.uint64(56)) + (np.uint64(1) << np.uint64(55)) +
+                 (rng.integers(0, 2**20, half, dtype=np.uint64) << np.uint64(32)))
+        k.append(np.array([((s + 1) << 56) + (1 << 55)], np.uint64))
+    k = np.concatenate(k)
+    check(kind, items(kind, rng.permutation(k)), [len(k)])
+
+
+@pytest.mark.parametrize("kind", [og.U32, og.KV64])
+def test_merges_when_tuned(kind, tmp_path):
+    rng = np.random.default_rng(2)
+    lens = rng.integers(1, 40000, 50)
+    a = items(kind, keys("zipf", int(lens.sum()), rng))
+    cls = int(lens.sum() // len(lens)).bit_length() - 1
+    f = tmp_path / "tuning"
+
+    def launched(on):
+        f.write_text(f"segbuckets {kind} {cls} {on}\n")
+        og.tuning_load(str(f))
+        og.profile_enable(True)
+        check(kind, a, lens)
+        names = set(og.profile_report())
+        og.profile_enable(False)
+        return {n for n in names if n.startswith("segbucket")}
+
+    try:
+        assert not launched(0)
+        og.tuning_save(str(f))
+        assert f"segbuckets {kind} {cls} 0" in f.read_text()
+    finally:
+        assert launched(1)
+
+
+@pytest.mark.parametrize("kind", [og.KV64])
+def test_pairs_report_expired_wait(kind):
+    # keys: test_gpu_timeout.py
+    lens = [1 << 16, 3 << 15]
+    a = items(kind, keys("uniform", sum(lens), np.random.default_rng(1)))
+    old = og.wait_limit()
+    og.set_wait_limit(0)
+    try:
+        with pytest.raises(og.OrigamiError) as e:
+            check(kind, a, lens)
+        assert e.value.code == og.ERR_TIMEOUT
+    finally:
+        og.set_wait_limit(old)
+    check(kind, a, lens)
