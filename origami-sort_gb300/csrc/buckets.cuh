@@ -1,9 +1,10 @@
 // Bucket sort: the default path (min_k = 0) of device sorts whose keys spread
-// evenly enough. Radix passes from the lowest digit up (radix.cuh) need one pass
-// per digit of the key; from the top down the array is cut into buckets that
-// fit shared memory after log2(n / bucket) bits, 16 for 2^28 keys, and one more
-// pass sorts every bucket whole. So a sort is two partition passes and a bucket
-// pass (one partition pass up to 256 buckets) whatever the width of the key.
+// evenly enough. A merge level moves every item once through HBM and doubles the
+// runs, a radix pass from the lowest digit up settles eight bits of the key; from the
+// top down the array is cut into buckets that fit shared memory after
+// log2(n / bucket) bits, 16 for 2^28 keys, and one more pass sorts every bucket
+// whole. So a sort is two partition passes and a bucket pass (one partition pass up
+// to 256 buckets) whatever the width of the key.
 //
 //   bk_sample_kernel  samples the keys of a segment, chooses the range that is
 //                     cut into 2^(b1+b2) equal slices, and sees whether a slice
@@ -13,7 +14,8 @@
 //                     can take; the next level's tiles
 //   bk_pass_kernel    one partition level for keys, one read and one write
 //   radix_pass_kernel the same for pairs, whose order has to be kept
-//   bk_sort_kernel    one bucket per CTA, sorted in shared memory
+//   bk_sort_kernel    one bucket per CTA, sorted in shared memory (64-bit keys:
+//                     sb_sort_kernel, seg_buckets.cuh)
 //
 // Measured (one GB300): 2^28 uint32 keys 3.79 ms by radix passes, 2.84 by buckets
 // (counting 2 x 0.20, partition 2 x 0.60, buckets 1.2); 2^27 uint64 keys 5.17 and
@@ -23,8 +25,10 @@
 // A slice is a monotone function of the key (keys outside the sampled range
 // fall into the end slices), so any data is sorted correctly as long as every
 // bucket fits. Where one does not (heavy duplicates, clustered keys), *route is
-// set on the device, the remaining kernels return at once, and the radix passes
-// that follow in the stream sort the array instead.
+// set on the device, the remaining kernels return at once, and what follows in the
+// stream sorts the array instead: radix passes for 32-bit keys (radix.cuh), the levels
+// of the segmented bucket sort for 64-bit keys (seg_buckets.cuh; from the slices of the
+// first level, where they are there already).
 //
 // Equal keys of keys-only items are identical, so their order does not matter:
 // bk_pass_kernel takes places with shared-memory atomics, one CTA per tile in
@@ -42,8 +46,8 @@
 
 namespace origami {
 
-// *route: 0 buckets; 1 radix passes from the input buffer; 2 radix passes from
-// the other buffer (the first partition pass has moved the items there).
+// *route: 0 buckets; 1 it gave up, the items are where they were; 2 it gave up, the
+// first partition pass has moved the items to the other buffer.
 enum BucketRoute : int { ROUTE_BUCKETS = 0, ROUTE_RADIX = 1, ROUTE_RADIX_MOVED = 2 };
 
 template <class T>
@@ -566,12 +570,32 @@ __device__ __forceinline__ void bk_byte_passes(T* sk, uint32_t* table, uint32_t*
     }
 }
 
-// The words a bucket sort shares beside its dynamic shared memory.
+// The words a bucket sort shares beside its dynamic shared memory. (Both are found by
+// name, also in functions that are not inlined: through pointer arguments the accesses
+// could be generic ones.)
 template <class T>
 struct BucketSortShared {
     uint32_t ws[BucketCfg<T>::S_NT / 32];
-    uint32_t rlo[2], rhi[2], widest;
+    uint32_t rlo[2], rhi[2], widest, listed;
 };
+template <class T>
+__device__ __forceinline__ BucketSortShared<T>& bk_shared() {
+    __shared__ BucketSortShared<T> s;
+    return s;
+}
+__device__ __forceinline__ unsigned char* bk_smem() {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    return smem_raw;
+}
+// threadIdx.x; read anew for 64-bit keys, so that what is computed from it is not kept
+// in registers over the sort (2^27 uint64 keys 0.85 ms instead of 1.00; 2^28 uint32
+// keys 1.22 instead of 1.20).
+template <class T>
+__device__ __forceinline__ int bk_tid() {
+    int t = threadIdx.x;
+    if (sizeof(typename Traits<T>::Key) == 8) asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return t;
+}
 // One warp sorts a crowded bin, items [s, s + c) of the bucket, if at most 32 of
 // them differ from the bin's commonest key (found in a sample of 32): the ranks of
 // those by comparison with each other, the others in between. Keys are sorted in
@@ -579,7 +603,7 @@ struct BucketSortShared {
 // bitmap of the places, one bit per item of the bucket, and its running counts.
 template <class T>
 __device__ __noinline__ bool bk_settle_bin(uint16_t* odd, T* sk, const uint16_t* si, uint32_t* map, int s, int c,
-                                           T* out, uint64_t xmask) {
+                                           T* out, uint64_t xout) {
     using K = typename Traits<T>::Key;
     constexpr bool ST = Traits<T>::kStable;
     constexpr int WORDS = BucketShape<T>::CAP / 32, PER = WORDS / 32;
@@ -644,9 +668,9 @@ __device__ __noinline__ bool bk_settle_bin(uint16_t* odd, T* sk, const uint16_t*
             const T y = sk[s + i];
             const int iy = si[s + i];
             if (Traits<T>::key(y) == h)
-                out[s + below + before[iy >> 5] + __popc(map[iy >> 5] & ((1u << (iy & 31)) - 1u))] = bk_flip(y, xmask);
+                out[s + below + before[iy >> 5] + __popc(map[iy >> 5] & ((1u << (iy & 31)) - 1u))] = bk_flip(y, xout);
         }
-        if (mine) out[at] = bk_flip(x, xmask);
+        if (mine) out[at] = bk_flip(x, xout);
         __syncwarp();
     } else {
         for (int i = below + lane; i < below + c - n; i += 32) sk[s + i] = h;
@@ -656,10 +680,11 @@ __device__ __noinline__ bool bk_settle_bin(uint16_t* odd, T* sk, const uint16_t*
 }
 // Clears the bins; no barrier needed before bk_sort_bucket.
 template <class T>
-__device__ __forceinline__ void bk_sort_init(unsigned char* smem_raw, BucketSortShared<T>& sh) {
+__device__ __forceinline__ void bk_sort_init() {
+    BucketSortShared<T>& sh = bk_shared<T>();
     using C = BucketCfg<T>;
-    uint32_t* tab = reinterpret_cast<uint32_t*>(smem_raw + BucketShape<T>::KEYS_BYTES);
-    const int tid = threadIdx.x;
+    uint32_t* tab = reinterpret_cast<uint32_t*>(bk_smem() + BucketShape<T>::KEYS_BYTES);
+    const int tid = bk_tid<T>();
     if (tid < 2) {
         sh.rlo[tid] = 0xFFFFFFFFu;
         sh.rhi[tid] = 0;
@@ -672,10 +697,12 @@ __device__ __forceinline__ void bk_sort_init(unsigned char* smem_raw, BucketSort
 // is (false is returned); its crowded bins settled by a warp each, and byte passes if
 // that fails.
 enum BkCrowded { BK_BYTES, BK_LEAVE, BK_SETTLE };
-// One bucket of cnt items (up to CAP), by the whole CTA. (src == out: in place.)
+// One bucket of cnt items (up to CAP), by the whole CTA. (src == out: in place.) xin
+// and xout: the sign flips of keys read and written.
 template <class T, BkCrowded CROWD>
-__device__ __forceinline__ bool bk_sort_bucket(unsigned char* smem_raw, BucketSortShared<T>& sh, const T* src, T* out,
-                                               int cnt, uint64_t xmask) {
+__device__ __forceinline__ bool bk_sort_bucket(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
+    unsigned char* smem_raw = bk_smem();
+    BucketSortShared<T>& sh = bk_shared<T>();
     using Sh = BucketShape<T>;
     using K = typename Traits<T>::Key;
     constexpr int NT = Sh::C::S_NT, IPT = Sh::C::S_IPT, BINS = Sh::C::BINS;
@@ -684,13 +711,12 @@ __device__ __forceinline__ bool bk_sort_bucket(unsigned char* smem_raw, BucketSo
     T* sk = reinterpret_cast<T*>(smem_raw) + Sh::SIDE;
     uint32_t* tab = reinterpret_cast<uint32_t*>(smem_raw + Sh::KEYS_BYTES);
     uint16_t* si = reinterpret_cast<uint16_t*>(tab + BINS);  // pairs: original places
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = bk_tid<T>(), lane = tid & 31, warp = tid >> 5;
     // crowded bins
     uint32_t* map = reinterpret_cast<uint32_t*>(smem_raw + Sh::KEYS_BYTES + Sh::BIN_BYTES) + warp * Sh::MAP_WORDS;
     uint16_t* odd = reinterpret_cast<uint16_t*>(smem_raw + Sh::KEYS_BYTES + Sh::BIN_BYTES + Sh::WARPS * Sh::MAP_WORDS * 4);
     uint16_t* bins = odd + Sh::WARPS * 32;
-    __shared__ uint32_t listed;
-    if (CROWD == BK_SETTLE && tid == 0) listed = 0;
+    if (CROWD == BK_SETTLE && tid == 0) sh.listed = 0;
     const int mine = cnt - tid;  // this thread's item i exists when i * NT < mine
     T v[IPT];
     const T* p = src + tid;
@@ -701,7 +727,7 @@ __device__ __forceinline__ bool bk_sort_bucket(unsigned char* smem_raw, BucketSo
     };
 #pragma unroll
     for (int i = 0; i < IPT; ++i)
-        if (i * NT < mine) v[i] = bk_flip(p[i * NT], xmask);
+        if (i * NT < mine) v[i] = bk_flip(p[i * NT], xin);
     uint32_t lo = 0xFFFFFFFFu, hi = 0;
 #pragma unroll
     for (int i = 0; i < IPT; ++i)
@@ -749,10 +775,10 @@ __device__ __forceinline__ bool bk_sort_bucket(unsigned char* smem_raw, BucketSo
         kr = hi - lo;
     }
     if (kr == 0) {  // one key: the bucket is sorted
-        if (src == out) return true;
+        if (src == out && xin == xout) return true;
 #pragma unroll
         for (int i = 0; i < IPT; ++i)
-            if (i * NT < mine) out[i * NT + tid] = bk_flip(v[i], xmask);
+            if (i * NT < mine) out[i * NT + tid] = bk_flip(v[i], xout);
         return true;
     }
     int c;
@@ -802,7 +828,7 @@ __device__ __forceinline__ bool bk_sort_bucket(unsigned char* smem_raw, BucketSo
         for (int i = 0; i < BPT; ++i) {
             const uint32_t x = h[i];
             crowded |= x > CROWDED;
-            if (CROWD == BK_SETTLE && x > CROWDED) bins[atomicAdd(&listed, 1u)] = (uint16_t)(tid * BPT + i);
+            if (CROWD == BK_SETTLE && x > CROWDED) bins[atomicAdd(&sh.listed, 1u)] = (uint16_t)(tid * BPT + i);
             wide = max(wide, x > CROWDED ? 0u : x);
             h[i] = sum;
             sum += x;
@@ -852,9 +878,9 @@ __device__ __forceinline__ bool bk_sort_bucket(unsigned char* smem_raw, BucketSo
     if (crowded) {
         bool mixed = false;
         if constexpr (CROWD == BK_SETTLE) {
-            for (int k = warp; k < (int)listed; k += Sh::WARPS) {
+            for (int k = warp; k < (int)sh.listed; k += Sh::WARPS) {
                 const int b = bins[k], s = b ? (int)tab[b - 1] : 0;
-                mixed |= !bk_settle_bin<T>(odd + warp * 32, sk, si, map, s, (int)tab[b] - s, out, xmask);
+                mixed |= !bk_settle_bin<T>(odd + warp * 32, sk, si, map, s, (int)tab[b] - s, out, xout);
             }
         } else if constexpr (!Sh::STABLE) {
             // keys only: a crowded bin of equal keys is in order
@@ -873,7 +899,7 @@ __device__ __forceinline__ bool bk_sort_bucket(unsigned char* smem_raw, BucketSo
                     if (i * NT < mine) sk[i * NT + tid] = v[i];
                 __syncthreads();
                 bk_byte_passes<T, NT, IPT>(sk, tab, sh.ws, cnt, klo, ((int)sizeof(K) * 8 - c + 7) / 8);
-                for (int i = tid; i < cnt; i += NT) out[i] = bk_flip(sk[i], xmask);
+                for (int i = tid; i < cnt; i += NT) out[i] = bk_flip(sk[i], xout);
                 return true;
             }
         }
@@ -889,7 +915,7 @@ __device__ __forceinline__ bool bk_sort_bucket(unsigned char* smem_raw, BucketSo
                 const int ix = (int)si[j];
                 for (int i = s; i < e; ++i) r += bk_before(sk[i], (int)si[i], x, ix) ? 1 : 0;
             }
-            out[r] = bk_flip(x, xmask);
+            out[r] = bk_flip(x, xout);
         }
     } else {
         const int w = (int)sh.widest;
@@ -902,7 +928,7 @@ __device__ __forceinline__ bool bk_sort_bucket(unsigned char* smem_raw, BucketSo
                 r += sk[j + k] < x ? 1 : 0;
                 r -= sk[j - k] > x ? 1 : 0;
             }
-            out[r] = bk_flip(x, xmask);
+            out[r] = bk_flip(x, xout);
         }
     }
     return true;
@@ -913,27 +939,27 @@ __device__ __forceinline__ bool bk_sort_bucket(unsigned char* smem_raw, BucketSo
 // registers: 2^27 pairs 1.4 and 1.8 ms. 32-bit keys, whose byte passes are few, are
 // better off with these in line: 2^28 keys 1.20 ms, with the call 1.38.)
 template <class T>
-__device__ __noinline__ void bk_sort_crowded(unsigned char* smem_raw, BucketSortShared<T>& sh, const T* src, T* out, int cnt,
-                                             uint64_t xmask) {
+__device__ __noinline__ void bk_sort_crowded(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
+    __builtin_assume(__isGlobal(src));
+    __builtin_assume(__isGlobal(out));
     __syncthreads();
-    bk_sort_init<T>(smem_raw, sh);
-    bk_sort_bucket<T, BK_SETTLE>(smem_raw, sh, src, out, cnt, xmask);
+    bk_sort_init<T>();
+    bk_sort_bucket<T, BK_SETTLE>(src, out, cnt, xin, xout);
 }
 
 template <class T>
 __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
-    bk_sort_kernel(const T* src, T* dst, const uint32_t* start, uint64_t xmask, uint32_t n, const int* route) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ BucketSortShared<T> sh;
-    bk_sort_init<T>(smem_raw, sh);
+    bk_sort_kernel(const T* src, T* dst, const uint32_t* start, uint64_t xin, uint64_t xout, uint32_t n,
+                   const int* route) {
+    bk_sort_init<T>();
     grid_dep_launch();
     grid_dep_wait();
     if (route_load(route) != ROUTE_BUCKETS) return;
     const uint32_t b0 = start[blockIdx.x], b1 = start[blockIdx.x + 1];
     if (b1 <= b0 || b1 > n || b1 - b0 > (uint32_t)BucketShape<T>::CAP) return;
     constexpr BkCrowded CROWD = sizeof(T) == 4 ? BK_BYTES : BK_LEAVE;
-    if (!bk_sort_bucket<T, CROWD>(smem_raw, sh, src + b0, dst + b0, (int)(b1 - b0), xmask))
-        bk_sort_crowded<T>(smem_raw, sh, src + b0, dst + b0, (int)(b1 - b0), xmask);
+    if (!bk_sort_bucket<T, CROWD>(src + b0, dst + b0, (int)(b1 - b0), xin, xout))
+        bk_sort_crowded<T>(src + b0, dst + b0, (int)(b1 - b0), xin, xout);
 }
 
 }  // namespace origami

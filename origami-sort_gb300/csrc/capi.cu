@@ -315,10 +315,10 @@ cudaError_t run_typed(int kind, void* d, void* tmp, uint64_t n, uint64_t sort_n,
     const uint64_t m = key_mask(kind);
     if (radix_takes(kind, n, sort_n, fan)) {
         switch (kind) {
-            case ORIGAMI_U32: return radix_sort_u32(d, tmp, n, sort_n, m, want, scratch, st);
+            case ORIGAMI_U32: return radix_sort_u32(d, tmp, n, sort_n, m, m, want, scratch, st);
             case ORIGAMI_U64:
-            case ORIGAMI_I64: return radix_sort_u64(d, tmp, n, sort_n, m, want, scratch, st);
-            default: return radix_sort_kv(d, tmp, n, sort_n, m, want, scratch, st);
+            case ORIGAMI_I64: return radix_sort_u64(d, tmp, n, sort_n, m, m, want, scratch, st);
+            default: return radix_sort_kv(d, tmp, n, sort_n, m, m, want, scratch, st);
         }
     }
     switch (kind) {

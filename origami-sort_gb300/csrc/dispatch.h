@@ -34,8 +34,8 @@ ORIGAMI_DECLARE_SORT(kv)
 #define ORIGAMI_DECLARE_RADIX(name)                                                                        \
     bool radix_fits_##name(uint64_t n, uint64_t sort_n);                                                   \
     uint64_t radix_scratch_bytes_##name(uint64_t n, uint64_t sort_n);                                      \
-    cudaError_t radix_sort_##name(void* d, void* tmp, uint64_t n, uint64_t sort_n, uint64_t key_mask, void* want, \
-                                  void* scratch, cudaStream_t st);
+    cudaError_t radix_sort_##name(void* d, void* tmp, uint64_t n, uint64_t sort_n, uint64_t key_mask,        \
+                                  uint64_t out_mask, void* want, void* scratch, cudaStream_t st);
 ORIGAMI_DECLARE_RADIX(u32)
 ORIGAMI_DECLARE_RADIX(u64)
 ORIGAMI_DECLARE_RADIX(kv)

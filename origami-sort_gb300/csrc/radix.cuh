@@ -1,5 +1,5 @@
-// Radix passes: what device sorts with min_k = 0 use where the bucket sort
-// (buckets.cuh) does not take the call or gives up; its partition of pairs is
+// Radix passes: what device sorts of 32-bit keys with min_k = 0 use where the bucket
+// sort (buckets.cuh) does not take the call or gives up; its partition of pairs is
 // the pass kernel here.
 //
 // A merge level moves every item once through HBM and doubles the runs; a
@@ -300,15 +300,25 @@ struct ByteDigit {
     }
 };
 
+// (32-bit keys are unsigned already)
+template <class T>
+__device__ __forceinline__ T radix_flip(const T& v, uint64_t x) {
+    if constexpr (sizeof(typename Traits<T>::Key) == 4)
+        return v;
+    else
+        return Traits<T>::flip(v, x);
+}
+
 // One pass: src -> dst by one digit. look: this pass's words, 256 per tile, zero
 // at launch; look_next (optional): the next pass's, cleared here. route
 // (optional): run only where it holds `run` (radix passes behind a bucket sort
-// run unless it is 0, the stable partition of a bucket sort while it is 0).
+// run unless it is 0, the stable partition of a bucket sort while it is 0). xflip:
+// applied to the keys as they are written.
 template <class T, class S, class G, class D>
 __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
     radix_pass_kernel(const T* __restrict__ src, T* __restrict__ dst, G geo, uint32_t tiles, D digit, S* look,
                       S* __restrict__ look_next, unsigned* __restrict__ claim, int* err, uint32_t spin,
-                      const int* route, bool buckets) {
+                      const int* route, bool buckets, uint64_t xflip) {
     using Sh = RadixShape<T>;
     using W = LookWord<S>;
     constexpr int NT = Sh::NT, IPT = Sh::IPT, NG = Sh::NG, TILE = Sh::TILE;
@@ -339,7 +349,7 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
             if (heavy && __syncthreads_or(h == (S)q.slen)) {
                 // one digit only: the segment keeps its order. (A tile of it
                 // takes no part in the look-back, like all the others.)
-                for (int i = tid; i < q.cnt; i += NT) dst[q.base + i] = src[q.base + i];
+                for (int i = tid; i < q.cnt; i += NT) dst[q.base + i] = radix_flip(src[q.base + i], xflip);
                 if (look_next)
                     for (int i = tid; i < RADIX_BINS; i += NT) look_next[(size_t)t * RADIX_BINS + i] = 0;
                 if (tid == 0) next_tile = atomicAdd(claim, 1u);
@@ -492,7 +502,7 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
             const T x = skeys[p];
             const S o = goff[digit(x)] + (S)p;
             // (o < slen always holds while the input does not change under the sort)
-            if (p < q.cnt && o < (S)q.slen) out[o] = x;
+            if (p < q.cnt && o < (S)q.slen) out[o] = radix_flip(x, xflip);
         }
         __syncthreads();
     }

@@ -1,5 +1,6 @@
-// Host launchers of the radix passes (radix.cuh) and the bucket sort
-// (buckets.cuh).
+// Host launchers of the bucket sort (buckets.cuh) and of what stands behind it: the
+// radix passes (radix.cuh) for 32-bit keys, the levels of the segmented bucket sort
+// (seg_buckets.cuh) for 64-bit keys.
 #pragma once
 #include <algorithm>
 #include <string>
@@ -8,6 +9,7 @@
 #include "pipeline.cuh"
 #include "profiler.h"
 #include "radix.cuh"
+#include "seg_bucket_host.cuh"
 
 namespace origami {
 
@@ -58,15 +60,32 @@ struct BucketPlan {
     bool on() const { return b1 > 0; }
 };
 
+// What stands behind the bucket sort, and sorts where it does not take the call. Radix
+// passes read the keys once more for every byte, the levels once more for every 256
+// slices, whatever the width; but the levels need more launches, and on clustered keys
+// a search. 2^20 / 2^22 / 2^28 uint32 Zipf keys: radix passes 0.084 / 0.20 / 6.5 ms,
+// levels 0.12 / 0.20 / 4.9; 2^20 / 2^22 / 2^27 uint64 Zipf keys 0.143 / 0.36 / 8.0 and
+// 0.147 / 0.24 / 3.65; 1.5M Zipf pairs 0.217 and 0.177, 2^26 5.1 and 3.4; normally
+// distributed keys, 2^27 uint64 7.6 and 4.0, 2^26 pairs 5.6 and 2.4.
+template <class T>
+constexpr bool levels_behind() {
+    return sizeof(typename Traits<T>::Key) == 8;
+}
+template <class T>
+SegBucketPlan<T> behind_plan(const RadixPlan<T>& p, const BucketPlan<T>& bk) {
+    return SegBucketPlan<T>(p.n, bk.b2 ? p.nseg << bk.b1 : p.nseg, p.len);
+}
+
 // Device scratch of one sort (each part 256-byte aligned):
-//   look 1/0   look-back words of the odd / even passes, 256 per tile
 //   bucket sort: slice starts and cursors of both levels, slice maps, tiles of
 //   the second level and their count
+//   look 1/0   look-back words of the odd / even radix passes, or of the second /
+//              first level of pairs, 256 per tile
 //   hist 1/2   counts of the bucket sort's levels
 //   hist       digit counts of the radix passes, [segment][digit][256]
-//   tail       256 bytes: the error word, the passes' tile counters (+64), the
-//              bucket sort's route (+128)
-// From `zero` on everything starts at 0 (one memset).
+//   words      the passes' tile counters, the bucket sort's route and tile count
+//   tail       256 bytes: the error word; the counters of the levels behind
+// From `zero` on everything starts at 0 (one memset). First of all the levels' scratch.
 template <class T>
 struct RadixScratch {
     using K = typename Traits<T>::Key;
@@ -81,7 +100,7 @@ struct RadixScratch {
     int *err = nullptr, *route = nullptr;
     unsigned* claim = nullptr;
     RadixScratch(void* base, const RadixPlan<T>& p, const BucketPlan<T>& bk) {
-        constexpr bool ST = BucketShape<T>::STABLE;
+        constexpr bool ST = BucketShape<T>::STABLE, LEVELS = levels_behind<T>();
         const uint64_t w = p.wide ? 8 : 4;
         char* b = static_cast<char*>(base);
         uint64_t o = 0;
@@ -91,6 +110,7 @@ struct RadixScratch {
             return r;
         };
         auto words = [&](uint64_t k) { return reinterpret_cast<uint32_t*>(take(k * 4)); };
+        if (LEVELS) o += SegBucketScratch<T>(nullptr, behind_plan(p, bk), nullptr, false).bytes;
         if (bk.on()) {
             start1 = words((p.nseg << bk.b1) + 1);
             if (!ST) cursor1 = words(p.nseg << bk.b1);
@@ -102,21 +122,22 @@ struct RadixScratch {
             }
         }
         // the second level's words: the first pass clears those of its own tiles
-        look[1] = take(std::max(p.tiles, ST ? bk.tiles2 : 0) * RADIX_BINS * w);
+        const bool look_pairs = ST && bk.on();
+        if (look_pairs ? bk.b2 > 0 : !LEVELS) look[1] = take(std::max(p.tiles, ST ? bk.tiles2 : 0) * RADIX_BINS * w);
         uint64_t z = o;
-        if (ST && bk.b2) z -= (bk.tiles2 - bk.tiles) * RADIX_BINS * w;
-        look[0] = take(p.tiles * RADIX_BINS * w);
-        if (!(ST && bk.on())) z = o;  // (cleared by radix_hist_kernel)
+        if (look_pairs && bk.b2) z -= (bk.tiles2 - bk.tiles) * RADIX_BINS * w;
+        if (look_pairs || !LEVELS) look[0] = take(p.tiles * RADIX_BINS * w);
+        if (!look_pairs) z = o;  // (cleared by radix_hist_kernel)
         if (bk.on()) {
             hist1 = words(p.nseg << bk.b1);
             if (bk.b2) hist2 = words(bk.nbuckets);
         }
-        hist = take(p.nseg * RadixShape<T>::DIGITS * RADIX_BINS * w);
+        if (!LEVELS) hist = take(p.nseg * RadixShape<T>::DIGITS * RADIX_BINS * w);
+        claim = words(16);
         err = reinterpret_cast<int*>(take(256));
         if (b) {
-            claim = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(err) + 64);
-            route = reinterpret_cast<int*>(reinterpret_cast<char*>(err) + 128);
-            count2 = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(err) + 132);
+            route = reinterpret_cast<int*>(claim + 12);
+            count2 = claim + 13;
             zero = b + z;
         }
         zero_bytes = o - z;
@@ -130,19 +151,10 @@ uint64_t radix_scratch_bytes(uint64_t n, uint64_t sort_n) {
     return RadixScratch<T>(nullptr, p, BucketPlan<T>(p)).bytes;
 }
 
-inline uint32_t resident_ctas(const void* kernel, int nt, size_t smem) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, nt, smem);
-    return (uint32_t)(sms * (per > 0 ? per : 1));
-}
-
 // The radix passes: d -> want (d or tmp). With `route` they stand behind a
 // bucket sort and run only where it gave up.
 template <class T, class S>
-void radix_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, uint64_t xmask, const RadixScratch<T>& sc,
+void radix_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, uint64_t xmask, uint64_t xout, const RadixScratch<T>& sc,
                   const int* route, cudaStream_t st) {
     using Sh = RadixShape<T>;
     using G = RadixUniform;
@@ -167,7 +179,7 @@ void radix_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, uint64_t xmask, 
             launch_dependent(radix_pass_kernel<T, S, G, D>, dim3(std::min(tiles, g_pass)), dim3(Sh::NT), Sh::SMEM, st,
                              (const T*)src, dst, geo, tiles, D(hist, xmask, b), static_cast<S*>(sc.look[b & 1]),
                              b + 1 < Sh::DIGITS ? static_cast<S*>(sc.look[(b + 1) & 1]) : (S*)nullptr, sc.claim + b,
-                             sc.err, wait_limit(), route, false);
+                             sc.err, wait_limit(), route, false, b + 1 < Sh::DIGITS ? 0ull : xmask ^ xout);
         });
         std::swap(src, dst);
     }
@@ -176,7 +188,7 @@ void radix_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, uint64_t xmask, 
 // The bucket sort: d -> want (d or tmp), *route set where it gives up.
 template <class T>
 void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPlan<T>& bk, uint64_t xmask,
-                   const RadixScratch<T>& sc, cudaStream_t st) {
+                   uint64_t xout, const RadixScratch<T>& sc, cudaStream_t st) {
     using Sh = BucketShape<T>;
     using RSh = RadixShape<T>;
     using K = typename Traits<T>::Key;
@@ -188,7 +200,8 @@ void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPla
     static const uint32_t g_hist = resident_ctas((const void*)bk_hist_kernel<T, G1>, 512, 0);
     static const uint32_t g_part = [] {
         cudaFuncSetAttribute(bk_sample_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SAMPLE_SMEM);
-        cudaFuncSetAttribute(bk_sort_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SORT_SMEM);
+        if constexpr (!levels_behind<T>())
+            cudaFuncSetAttribute(bk_sort_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SORT_SMEM);
         if constexpr (ST) {
             resident_ctas((const void*)radix_pass_kernel<T, uint32_t, G2, D>, RSh::NT, RSh::SMEM);
             return resident_ctas((const void*)radix_pass_kernel<T, uint32_t, G1, D>, RSh::NT, RSh::SMEM);
@@ -241,7 +254,7 @@ void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPla
                 launch_dependent(radix_pass_kernel<T, uint32_t, G, D>, dim3(std::min(tiles_l, g_part)), dim3(RSh::NT),
                                  RSh::SMEM, st, src, dst, geo_l, tiles_l, dig, static_cast<uint32_t*>(look),
                                  static_cast<uint32_t*>(look_next), claim, sc.err, wait_limit(), (const int*)sc.route,
-                                 true);
+                                 true, 0ull);
             } else {
                 launch_dependent(bk_pass_kernel<T, G>, dim3(tiles_l), dim3(Sh::C::NT), Sh::PASS_SMEM, st, src, dst, geo_l,
                                  tiles_l, (const SliceMap<K>*)sc.maps, map_shift, xmask, shift_l, bits_l, cursor, n32,
@@ -258,32 +271,45 @@ void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPla
               (void*)nullptr, sc.claim + 9);
         cur = d;
     }
-    launch(n_sort.c_str(), st, [&] {
+    // (the last kernel of the levels behind sorts these buckets too)
+    if constexpr (!levels_behind<T>()) launch(n_sort.c_str(), st, [&] {
         launch_dependent(bk_sort_kernel<T>, dim3((unsigned)bk.nbuckets), dim3(Sh::C::S_NT), Sh::SORT_SMEM, st, cur, want,
-                         (const uint32_t*)(bk.b2 ? sc.start2 : sc.start1), xmask, n32, (const int*)sc.route);
+                         (const uint32_t*)(bk.b2 ? sc.start2 : sc.start1), xmask, xout, n32, (const int*)sc.route);
     });
 }
 
 // Sorts d[0..n) in chunks of sort_n (0 = one full sort) into `want` (d or tmp):
-// by buckets where the geometry allows it, with the radix passes behind them
-// for what does not spread; else by radix passes. `scratch` holds
+// by buckets where the geometry allows it, with radix passes or levels behind them
+// for what does not spread; else by those. key_mask: the sign flip of keys
+// read; out_mask: of keys written. `scratch` holds
 // radix_scratch_bytes<T>(n, sort_n) bytes.
 template <class T>
-cudaError_t radix_sort(T* d, T* tmp, uint64_t n, uint64_t sort_n, uint64_t key_mask, T* want, void* scratch,
-                       cudaStream_t st) {
+cudaError_t radix_sort(T* d, T* tmp, uint64_t n, uint64_t sort_n, uint64_t key_mask, uint64_t out_mask, T* want,
+                       void* scratch, cudaStream_t st) {
     const RadixPlan<T> p(n, sort_n);
     const BucketPlan<T> bk(p);
     const RadixScratch<T> sc(scratch, p, bk);
     cudaMemsetAsync(sc.zero, 0, sc.zero_bytes, st);
     const int* route = nullptr;
     if (bk.on()) {
-        bucket_launch<T>(d, tmp, want, p, bk, key_mask, sc, st);
+        bucket_launch<T>(d, tmp, want, p, bk, key_mask, out_mask, sc, st);
         route = sc.route;
     }
-    if (p.wide)
-        radix_launch<T, uint64_t>(d, tmp, want, p, key_mask, sc, route, st);
-    else
-        radix_launch<T, uint32_t>(d, tmp, want, p, key_mask, sc, route, st);
+    if constexpr (levels_behind<T>()) {
+        const SegBucketPlan<T> q = behind_plan(p, bk);
+        const SegBucketScratch<T> seg(scratch, q, reinterpret_cast<SbCounts*>(sc.err), false);
+        const SbBuffers<T> buf{d, tmp, route, want == tmp};
+        const SbStarts plain{bk.on() ? (bk.b2 ? sc.start2 : sc.start1) : nullptr, (uint32_t)bk.nbuckets, !bk.b2};
+        const SbGiven given{route, sc.start1, p.n, p.len, (uint32_t)p.nseg, bk.b2 ? (uint32_t)(p.nseg << bk.b1) : 0u};
+        if (q.wide)
+            segbucket_levels<T, uint64_t>(buf, given, plain, q, key_mask, out_mask, seg, st);
+        else
+            segbucket_levels<T, uint32_t>(buf, given, plain, q, key_mask, out_mask, seg, st);
+    } else if (p.wide) {
+        radix_launch<T, uint64_t>(d, tmp, want, p, key_mask, out_mask, sc, route, st);
+    } else {
+        radix_launch<T, uint32_t>(d, tmp, want, p, key_mask, out_mask, sc, route, st);
+    }
     return cudaGetLastError();
 }
 

@@ -4,13 +4,17 @@
 
 namespace origami {
 
-bool radix_fits_u64(uint64_t n, uint64_t sort_n) { return RadixPlan<uint64_t>::fits(n, sort_n); }
+bool radix_fits_u64(uint64_t n, uint64_t sort_n) {
+    if (!RadixPlan<uint64_t>::fits(n, sort_n)) return false;
+    const RadixPlan<uint64_t> p(n, sort_n);
+    return behind_plan(p, BucketPlan<uint64_t>(p)).fits();
+}
 
 uint64_t radix_scratch_bytes_u64(uint64_t n, uint64_t sort_n) { return radix_scratch_bytes<uint64_t>(n, sort_n); }
 
-cudaError_t radix_sort_u64(void* d, void* tmp, uint64_t n, uint64_t sort_n, uint64_t key_mask, void* want,
+cudaError_t radix_sort_u64(void* d, void* tmp, uint64_t n, uint64_t sort_n, uint64_t key_mask, uint64_t out_mask, void* want,
                           void* scratch, cudaStream_t st) {
-    return radix_sort<uint64_t>(static_cast<uint64_t*>(d), static_cast<uint64_t*>(tmp), n, sort_n, key_mask, static_cast<uint64_t*>(want),
+    return radix_sort<uint64_t>(static_cast<uint64_t*>(d), static_cast<uint64_t*>(tmp), n, sort_n, key_mask, out_mask, static_cast<uint64_t*>(want),
                           scratch, st);
 }
 

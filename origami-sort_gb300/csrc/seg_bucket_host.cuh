@@ -5,25 +5,24 @@
 
 #include "pipeline.cuh"
 #include "profiler.h"
-#include "radix_host.cuh"
 #include "seg_buckets.cuh"
 
 namespace origami {
 
-// Geometry of the bucket sort of nseg segments of n items in all; their lengths
-// are on the device.
+// Geometry of the bucket sort of n items in segments whose lengths are on the device:
+// none longer than `longest`, at most nseg shorter than a bucket.
 template <class T>
 struct SegBucketPlan {
     using Sh = SegBucketShape<T>;
     uint64_t n, nseg, segs, tiles, recs;
     int levels;
     bool wide;  // 64-bit counts
-    SegBucketPlan(uint64_t n_, uint64_t nseg_) : n(n_), nseg(nseg_) {
-        // levels that 256 slices each need to cut one segment of n items into buckets
+    SegBucketPlan(uint64_t n_, uint64_t nseg_, uint64_t longest) : n(n_), nseg(nseg_) {
+        // levels that 256 slices each need to cut the longest segment into buckets
         // of 4/5 of the largest size, and one more for keys that are spread unevenly
         levels = 1;
-        for (uint64_t m = (uint64_t)Sh::CAP * 4 / 5 * RADIX_BINS; m < n && levels < SB_MAX_LEVELS; m *= RADIX_BINS) ++levels;
-        levels = n > (uint64_t)Sh::CAP ? std::min(levels + 1, SB_MAX_LEVELS) : 0;
+        for (uint64_t m = (uint64_t)Sh::CAP * 4 / 5 * RADIX_BINS; m < longest && levels < SB_MAX_LEVELS; m *= RADIX_BINS) ++levels;
+        levels = longest > (uint64_t)Sh::CAP ? std::min(levels + 1, SB_MAX_LEVELS) : 0;
         // a level's segments are longer than a bucket
         segs = n / (Sh::CAP + 1) + 1;
         tiles = n / Sh::TILE + segs;
@@ -43,7 +42,7 @@ struct SegBucketPlan {
 template <class T>
 struct SegBucketScratch {
     using K = typename Traits<T>::Key;
-    uint64_t bytes = 0, tail_at = 0;
+    uint64_t bytes = 0;
     SbSeg* list[2] = {nullptr, nullptr};
     SbMap<K>* maps = nullptr;
     K* splitters = nullptr;
@@ -54,7 +53,8 @@ struct SegBucketScratch {
     uint32_t* slow = nullptr;
     void* look = nullptr;  // pairs
     SbCounts* cn = nullptr;
-    SegBucketScratch(void* base, const SegBucketPlan<T>& p) {
+    // tail: where it is, if not here
+    SegBucketScratch(void* base, const SegBucketPlan<T>& p, SbCounts* tail = nullptr, bool tail_here = true) {
         const uint64_t w = p.wide ? 8 : 4;
         char* b = static_cast<char*>(base);
         uint64_t o = 0;
@@ -72,16 +72,25 @@ struct SegBucketScratch {
         recs = reinterpret_cast<SbRec*>(take(p.recs * sizeof(SbRec)));
         slow = reinterpret_cast<uint32_t*>(take(p.recs * 4));
         if (SegBucketShape<T>::STABLE) look = take(p.tiles * RADIX_BINS * w);
-        tail_at = o;
-        cn = reinterpret_cast<SbCounts*>(take(256));
+        cn = tail_here ? reinterpret_cast<SbCounts*>(take(256)) : tail;
         bytes = o;
     }
 };
 
+// Resident CTAs of a kernel on the whole GPU; sets its shared-memory limit.
+inline uint32_t resident_ctas(const void* kernel, int nt, size_t smem) {
+    int dev = 0, sms = 0, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, nt, smem);
+    return (uint32_t)(sms * (per > 0 ? per : 1));
+}
+
 // Grids of the kernels, found once per process.
 template <class T, class S>
 struct SegBucketGrids {
-    uint32_t sample, hist, pass, rest;
+    uint32_t sample, hist, pass, sort;
     static const SegBucketGrids& get() {
         using Sh = SegBucketShape<T>;
         static const SegBucketGrids g = [] {
@@ -94,93 +103,95 @@ struct SegBucketGrids {
                 r.pass = resident_ctas((const void*)sb_pass_kernel<T, S, true>, Sh::C::NT, Sh::PASS_SMEM);
                 resident_ctas((const void*)sb_pass_kernel<T, S, false>, Sh::C::NT, Sh::PASS_SMEM);
             }
-            resident_ctas((const void*)sb_sort_kernel<T>, Sh::Sort::C::S_NT, Sh::Sort::SORT_SMEM);
-            r.rest = resident_ctas((const void*)sb_rest_kernel<T>, Sh::Sort::C::S_NT, Sh::Sort::SORT_SMEM);
+            r.sort = resident_ctas((const void*)sb_sort_kernel<T>, Sh::Sort::C::S_NT, Sh::Sort::SORT_SMEM);
             return r;
         }();
         return g;
     }
 };
 
+// The levels and the bucket pass. given.nseg: behind a bucket sort that rarely gives up,
+// where no level's grid is larger than resident; else for the segments in the first list.
 template <class T, class S>
-cudaError_t segbucket_launch(T* d, T* tmp, const SegBucketPlan<T>& p, const uint64_t* off, uint64_t xmask,
-                             const SegBucketScratch<T>& sc, cudaStream_t st) {
+void segbucket_levels(const SbBuffers<T>& buf, const SbGiven& given, const SbStarts& plain, const SegBucketPlan<T>& p,
+                      uint64_t xin, uint64_t xout, const SegBucketScratch<T>& sc, cudaStream_t st) {
     using Sh = SegBucketShape<T>;
     using K = typename Traits<T>::Key;
     using C = typename Sh::C;
     const SegBucketGrids<T, S>& g = SegBucketGrids<T, S>::get();
-    static const std::string n_plan = std::string("segbucket_plan<") + TypeName<T>::v + ">";
     static const std::string n_sample = std::string("segbucket_sample<") + TypeName<T>::v + ">";
     static const std::string n_hist = std::string("segbucket_hist<") + TypeName<T>::v + ">";
     static const std::string n_pass = std::string("segbucket_pass<") + TypeName<T>::v + ">";
     static const std::string n_sort = std::string("segbucket_sort<") + TypeName<T>::v + ">";
-    static const std::string n_rest = std::string("segbucket_rest<") + TypeName<T>::v + ">";
     SbCounts* cn = sc.cn;
     S* hist = static_cast<S*>(sc.hist);
+    const bool behind = given.nseg != 0;
     const uint32_t segs = (uint32_t)p.segs, tiles = (uint32_t)p.tiles;
-    cudaMemsetAsync(cn, 0, 256, st);
-    launch(n_plan.c_str(), st, [&] {
-        sb_plan_kernel<T><<<(unsigned)((p.nseg + 255) / 256), 256, 0, st>>>(off, (uint32_t)p.nseg, p.n, sc.list[0], segs,
-                                                                           sc.recs, cn);
-    });
     for (int l = 0; l < p.levels; ++l) {
-        const T* src = (l & 1) ? tmp : d;
-        T* dst = (l & 1) ? d : tmp;
-        SbHandOn to;
+        SbHandOn to{};
         to.next = l + 1 < p.levels ? sc.list[(l + 1) & 1] : nullptr;
         to.next_count = &cn->segs[l + 1];
         to.recs = sc.recs;
         to.rec_count = &cn->recs;
-        to.flags = dst == tmp ? SbRec::TMP : 0;
-        to.stay = dst == d;
+        to.slow = sc.slow;
+        to.slow_count = &cn->slow;
+        const SbGiven none{};
+        const uint32_t samples = l == 0 && behind ? std::max(given.nseg, given.slices) : segs;
         launch(n_sample.c_str(), st, [&] {
-            launch_dependent(sb_sample_kernel<T, S>, dim3(std::min(segs, g.sample)), dim3(512), 0, st, src,
-                             (const SbSeg*)sc.list[l & 1], (const uint32_t*)&cn->segs[l], xmask, sc.maps, sc.splitters,
-                             hist, sc.done, sc.tiles, &cn->tiles[l], (const int*)&cn->err);
+            launch_dependent(sb_sample_kernel<T, S>, dim3(std::min(samples, g.sample)), dim3(512), 0, st, buf, l,
+                             l == 0 ? given : none, (const SbSeg*)sc.list[l & 1], &cn->segs[l], xin, sc.maps,
+                             sc.splitters, hist, sc.done, sc.tiles, &cn->tiles[l], sc.recs, &cn->recs,
+                             (const int*)&cn->err);
         });
         launch(n_hist.c_str(), st, [&] {
-            launch_dependent(sb_hist_kernel<T, S>, dim3(std::min(tiles, g.hist)), dim3(512), Sh::HIST_SMEM, st, src,
+            launch_dependent(sb_hist_kernel<T, S>, dim3(std::min(tiles, g.hist)), dim3(512), Sh::HIST_SMEM, st, buf, l,
                              (const SbTile*)sc.tiles, (const uint32_t*)&cn->tiles[l], (const SbMap<K>*)sc.maps,
-                             (const K*)sc.splitters, xmask, hist, sc.done, to, static_cast<S*>(sc.look), &cn->err,
+                             (const K*)sc.splitters, xin, hist, sc.done, to, static_cast<S*>(sc.look), &cn->err,
                              wait_limit());
         });
         launch(n_pass.c_str(), st, [&] {
             if constexpr (Sh::STABLE) {
                 launch_dependent(sb_stable_pass_kernel<T, S>, dim3(std::min(tiles, g.pass)), dim3(C::NT), Sh::PASS_SMEM, st,
-                                 src, dst, (const SbTile*)sc.tiles, (const uint32_t*)&cn->tiles[l],
-                                 (const SbMap<K>*)sc.maps, (const K*)sc.splitters, xmask, (const S*)hist,
+                                 buf, l, (const SbTile*)sc.tiles, (const uint32_t*)&cn->tiles[l],
+                                 (const SbMap<K>*)sc.maps, (const K*)sc.splitters, xin, (const S*)hist,
                                  static_cast<S*>(sc.look), &cn->claim[l], &cn->err, wait_limit());
             } else {
-                const bool loop = l > 0 && l + 1 == p.levels;
+                const bool loop = behind || (l > 0 && l + 1 == p.levels);
                 launch_dependent(loop ? sb_pass_kernel<T, S, true> : sb_pass_kernel<T, S, false>,
-                                 dim3(loop ? std::min(tiles, g.pass) : tiles), dim3(C::NT), Sh::PASS_SMEM, st, src, dst,
+                                 dim3(loop ? std::min(tiles, g.pass) : tiles), dim3(C::NT), Sh::PASS_SMEM, st, buf, l,
                                  (const SbTile*)sc.tiles, (const uint32_t*)&cn->tiles[l], (const SbMap<K>*)sc.maps,
-                                 (const K*)sc.splitters, xmask, hist, (const int*)&cn->err);
+                                 (const K*)sc.splitters, xin, hist, (const int*)&cn->err);
             }
         });
     }
-    // one CTA per bucket. Neighbouring buckets of a segment hold more than CAP items
-    // together, so few sorts have more than these; sb_rest_kernel takes the others
-    const uint32_t first = (uint32_t)std::min(p.recs, p.nseg + p.n * 9 / (4 * (uint64_t)Sh::CAP) + 1);
+    // one CTA per bucket: neighbouring buckets of a segment hold more than CAP items
+    // together, so few sorts have more than these, and few CTAs stand by for the rest
+    const uint32_t first = (uint32_t)std::min(p.recs, std::max<uint64_t>(plain.buckets, p.nseg + p.n * 9 / (4 * (uint64_t)Sh::CAP) + 1));
     launch(n_sort.c_str(), st, [&] {
-        launch_dependent(sb_sort_kernel<T>, dim3(first), dim3(Sh::Sort::C::S_NT), Sh::Sort::SORT_SMEM, st, d, tmp,
-                         (const SbRec*)sc.recs, sc.slow, cn, xmask);
+        launch_dependent(sb_sort_kernel<T>, dim3(std::max(first, plain.buckets) + std::min(first, g.sort / 4)),
+                         dim3(Sh::Sort::C::S_NT), Sh::Sort::SORT_SMEM, st, buf, plain, (const SbRec*)sc.recs,
+                         (const uint32_t*)sc.slow, (const SbCounts*)cn, first, xin, xout);
     });
-    launch(n_rest.c_str(), st, [&] {
-        launch_dependent(sb_rest_kernel<T>, dim3((unsigned)std::min<uint64_t>(p.recs, g.rest)), dim3(Sh::Sort::C::S_NT),
-                         Sh::Sort::SORT_SMEM, st, d, tmp, (const SbRec*)sc.recs, (const uint32_t*)sc.slow, (const SbCounts*)cn,
-                         first, xmask);
-    });
-    return cudaGetLastError();
 }
 
+// Segments [off[s], off[s+1]), sorted in place.
 template <class T>
 cudaError_t segbucket_run(T* d, T* tmp, const uint64_t* off, uint64_t nseg, uint64_t n, uint64_t xmask, void* scratch,
                           cudaStream_t st) {
-    const SegBucketPlan<T> p(n, nseg);
+    const SegBucketPlan<T> p(n, nseg, n);
     const SegBucketScratch<T> sc(scratch, p);
-    if (p.wide) return segbucket_launch<T, uint64_t>(d, tmp, p, off, xmask, sc, st);
-    return segbucket_launch<T, uint32_t>(d, tmp, p, off, xmask, sc, st);
+    static const std::string n_plan = std::string("segbucket_plan<") + TypeName<T>::v + ">";
+    cudaMemsetAsync(sc.cn, 0, 256, st);
+    launch(n_plan.c_str(), st, [&] {
+        sb_plan_kernel<T><<<(unsigned)((nseg + 255) / 256), 256, 0, st>>>(off, (uint32_t)nseg, n, sc.list[0],
+                                                                         (uint32_t)p.segs, sc.recs, sc.cn);
+    });
+    const SbBuffers<T> buf{d, tmp, nullptr, false};
+    if (p.wide)
+        segbucket_levels<T, uint64_t>(buf, SbGiven{}, SbStarts{}, p, xmask, xmask, sc, st);
+    else
+        segbucket_levels<T, uint32_t>(buf, SbGiven{}, SbStarts{}, p, xmask, xmask, sc, st);
+    return cudaGetLastError();
 }
 
 }  // namespace origami

@@ -4,10 +4,10 @@
 
 namespace origami {
 
-bool segbucket_fits_kv(uint64_t n, uint64_t nseg) { return SegBucketPlan<KV64>(n, nseg).fits(); }
+bool segbucket_fits_kv(uint64_t n, uint64_t nseg) { return SegBucketPlan<KV64>(n, nseg, n).fits(); }
 
 uint64_t segbucket_scratch_bytes_kv(uint64_t n, uint64_t nseg) {
-    return SegBucketScratch<KV64>(nullptr, SegBucketPlan<KV64>(n, nseg)).bytes;
+    return SegBucketScratch<KV64>(nullptr, SegBucketPlan<KV64>(n, nseg, n)).bytes;
 }
 
 cudaError_t segbucket_sort_kv(void* d, void* tmp, const uint64_t* off, uint64_t nseg, uint64_t n, uint64_t key_mask,

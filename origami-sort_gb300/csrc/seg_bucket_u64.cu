@@ -4,10 +4,10 @@
 
 namespace origami {
 
-bool segbucket_fits_u64(uint64_t n, uint64_t nseg) { return SegBucketPlan<uint64_t>(n, nseg).fits(); }
+bool segbucket_fits_u64(uint64_t n, uint64_t nseg) { return SegBucketPlan<uint64_t>(n, nseg, n).fits(); }
 
 uint64_t segbucket_scratch_bytes_u64(uint64_t n, uint64_t nseg) {
-    return SegBucketScratch<uint64_t>(nullptr, SegBucketPlan<uint64_t>(n, nseg)).bytes;
+    return SegBucketScratch<uint64_t>(nullptr, SegBucketPlan<uint64_t>(n, nseg, n)).bytes;
 }
 
 cudaError_t segbucket_sort_u64(void* d, void* tmp, const uint64_t* off, uint64_t nseg, uint64_t n, uint64_t key_mask,

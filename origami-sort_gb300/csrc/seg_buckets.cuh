@@ -16,7 +16,9 @@
 //   sb_stable_pass_kernel  the same for pairs, whose order has to be kept
 //   then
 //   sb_sort_kernel    sorts every bucket in shared memory
-//   sb_rest_kernel    the buckets it leaves
+//
+// The same levels stand behind the plain bucket sort of 64-bit keys (buckets.cuh), for
+// keys that it gives up on.
 //
 // How a segment is cut. Its keys' range, from the sample, in 256 slices of equal
 // width: a subtraction and a multiplication per key. Where one slice would take
@@ -88,6 +90,28 @@ struct SegBucketShape {
     // enclose it), pairs are read directly
     static constexpr size_t STAGE_BYTES = (TILE_BYTES + 16 + 127) & ~(size_t)127;
     static constexpr size_t HIST_SMEM = STABLE ? 0 : 2 * STAGE_BYTES;
+};
+
+// The two buffers of a sort. Level l moves the items from d to tmp where l is even and
+// back where it is odd; behind a bucket sort that gave up after its first partition the
+// other way round. The result is wanted in d or tmp.
+template <class T>
+struct SbBuffers {
+    T *d, *tmp;
+    const int* route;  // or null
+    bool want_tmp;
+    __device__ __forceinline__ bool moved() const { return route && route_load(route) == ROUTE_RADIX_MOVED; }
+    __device__ __forceinline__ bool from_tmp(int level) const { return ((level & 1) != 0) != moved(); }
+    __device__ __forceinline__ T* want() const { return want_tmp ? tmp : d; }
+};
+// The first level's segments behind a plain bucket sort (buckets.cuh): none where it
+// went on; else nseg segments of len of n items, or, after its first partition, the
+// `slices` of that.
+struct SbGiven {
+    const int* route;  // null: it was left out
+    const uint32_t* start1;
+    uint64_t n, len;
+    uint32_t nseg, slices;
 };
 
 // ------------------------------------------------------------------ lists ---
@@ -235,12 +259,14 @@ __global__ void sb_plan_kernel(const uint64_t* off, uint32_t nseg, uint64_t n, S
 }
 
 // ----------------------------------------------------------------- sample ---
-// One CTA per segment of the level. The linear range is the samples', widened by
-// 1/512 at each end.
+// One CTA per segment of the level (given.nseg: the first one behind a bucket sort;
+// segments that fit a bucket become one here). The linear range is the samples',
+// widened by 1/512 at each end.
 template <class T, class S>
 __global__ void __launch_bounds__(512)
-    sb_sample_kernel(const T* src, const SbSeg* list, const uint32_t* count, uint64_t xmask, SbMap<typename Traits<T>::Key>* maps, typename Traits<T>::Key* splitters, S* hist,
-                     uint32_t* done, SbTile* tiles, uint32_t* tile_count, const int* err) {
+    sb_sample_kernel(SbBuffers<T> buf, int level, SbGiven given, const SbSeg* list, uint32_t* count, uint64_t xmask,
+                     SbMap<typename Traits<T>::Key>* maps, typename Traits<T>::Key* splitters, S* hist, uint32_t* done,
+                     SbTile* tiles, uint32_t* tile_count, SbRec* recs, uint32_t* rec_count, const int* err) {
     using K = typename Traits<T>::Key;
     constexpr int NT = 512, PER = SB_SAMPLES / NT;
     constexpr uint32_t TILE = SegBucketShape<T>::TILE, MOST = SB_SAMPLES / 8;
@@ -248,14 +274,41 @@ __global__ void __launch_bounds__(512)
     __shared__ K smin[NT / 32], smax[NT / 32], scand;
     __shared__ uint32_t cnt[RADIX_BINS];
     __shared__ SbMap<K> smap;
-    __shared__ uint32_t stile;
+    __shared__ uint32_t stile, sid;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     grid_dep_launch();
     grid_dep_wait();
     // (segments that overlap would not fit the lists)
-    const uint32_t total = count_load((const uint32_t*)err) == ERR_BAD_OFFSETS ? 0u : count_load(count);
-    for (uint32_t sg = blockIdx.x; sg < total; sg += gridDim.x) {
-        const SbSeg q = list[sg];
+    uint32_t total;
+    bool slices = false;
+    if (given.nseg) {
+        const int route = given.route ? route_load(given.route) : (int)ROUTE_RADIX;
+        slices = route == ROUTE_RADIX_MOVED;
+        total = route == ROUTE_BUCKETS ? 0u : (slices ? given.slices : given.nseg);
+    } else {
+        total = count_load((const uint32_t*)err) == ERR_BAD_OFFSETS ? 0u : count_load(count);
+    }
+    if (blockIdx.x >= total) return;
+    const T* src = buf.from_tmp(level) ? buf.tmp : buf.d;
+    for (uint32_t at = blockIdx.x; at < total; at += gridDim.x) {
+        SbSeg q;
+        uint32_t sg = at;
+        if (given.nseg) {
+            q.base = slices ? given.start1[at] : at * given.len;
+            q.len = (slices ? given.start1[at + 1] : (given.n - q.base < given.len ? given.n : q.base + given.len)) - q.base;
+            const bool fits = q.len <= (uint64_t)SegBucketShape<T>::CAP;
+            if (tid == 0) {
+                if (!fits)
+                    sid = atomicAdd(count, 1u);
+                else if (q.len)
+                    recs[atomicAdd(rec_count, 1u)] = SbRec{q.base, q.len | (slices ? SbRec::TMP : 0)};
+            }
+            if (fits) continue;
+            __syncthreads();
+            sg = sid;
+        } else {
+            q = list[at];
+        }
         K v[PER], lo, hi;
 #pragma unroll
         for (int i = 0; i < PER; ++i) {
@@ -377,8 +430,9 @@ struct SbHandOn {
     SbSeg* next;
     uint32_t* next_count;
     SbRec* recs;
+    uint32_t *slow, *slow_count;
     uint32_t* rec_count;
-    uint64_t flags;
+    uint64_t flags;  // (set by the kernel, as stay)
     bool stay;
 };
 
@@ -445,7 +499,10 @@ __device__ __forceinline__ void sb_hand_on(const SbTile& q, S h, const Map& map,
     if (tid == RADIX_BINS - 1) at = atomicAdd(to.rec_count, o + nrec);
     if (tid < RADIX_BINS) goff[tid] = pure ? o : 0xFFFFFFFFu;
     __syncthreads();
-    if (nrec && !pure) to.recs[at + o] = SbRec{q.sbase + (uint64_t)gs[tid], len | flags | to.flags};
+    if (nrec && !pure) {
+        to.recs[at + o] = SbRec{q.sbase + (uint64_t)gs[tid], len | flags | to.flags};
+        if (flags & SbRec::SLOW) to.slow[atomicAdd(to.slow_count, 1u)] = at + o;
+    }
     // equal keys that have to move: pieces, by the whole CTA
     if (__syncthreads_or(pure && nrec)) {
         for (uint32_t k = 0; k < groups; ++k) {
@@ -471,7 +528,7 @@ __device__ __forceinline__ void sb_hand_on(const SbTile& q, S h, const Map& map,
 // cleared here.
 template <class T, class S>
 __global__ void __launch_bounds__(512)
-    sb_hist_kernel(const T* in, const SbTile* tiles, const uint32_t* tile_count,
+    sb_hist_kernel(SbBuffers<T> buf, int level, const SbTile* tiles, const uint32_t* tile_count,
                    const SbMap<typename Traits<T>::Key>* maps, const typename Traits<T>::Key* splitters, uint64_t xmask,
                    S* hist, uint32_t* done, SbHandOn to, S* look, int* err, uint32_t spin) {
     using Sh = SegBucketShape<T>;
@@ -495,6 +552,10 @@ __global__ void __launch_bounds__(512)
     const uint32_t t0 = (uint32_t)((uint64_t)total * blockIdx.x / gridDim.x);
     const uint32_t t1 = (uint32_t)((uint64_t)total * (blockIdx.x + 1) / gridDim.x);
     if (t0 >= t1) return;
+    const bool from_tmp = buf.from_tmp(level);
+    const T* in = from_tmp ? buf.tmp : buf.d;
+    to.flags = from_tmp ? 0 : SbRec::TMP;
+    to.stay = from_tmp != buf.want_tmp;
     for (int i = tid; i < RADIX_BINS * COPIES; i += NT) cnt[i] = 0;
     SbDigit<T> dig;
     dig.xmask = xmask;
@@ -609,7 +670,7 @@ __global__ void __launch_bounds__(512)
 // (a loop costs registers, and so resident warps).
 template <class T, class S, bool LOOP>
 __global__ void __launch_bounds__(SegBucketCfg<T>::NT, SegBucketCfg<T>::MINB)
-    sb_pass_kernel(const T* src, T* dst, const SbTile* tiles, const uint32_t* tile_count,
+    sb_pass_kernel(SbBuffers<T> buf, int level, const SbTile* tiles, const uint32_t* tile_count,
                    const SbMap<typename Traits<T>::Key>* maps, const typename Traits<T>::Key* splitters, uint64_t xmask,
                    S* cursor, const int* err) {
     using Sh = SegBucketShape<T>;
@@ -628,6 +689,9 @@ __global__ void __launch_bounds__(SegBucketCfg<T>::NT, SegBucketCfg<T>::MINB)
     SbTile q = tiles[t];  // (the list has room for the grid: one latency with the count)
     const uint32_t total = count_load(tile_count);
     if (t >= total || err_wait_set(err)) return;
+    const bool from_tmp = buf.from_tmp(level);
+    const T* src = from_tmp ? buf.tmp : buf.d;
+    T* dst = from_tmp ? buf.d : buf.tmp;
     SbDigit<T> dig;
     dig.xmask = xmask;
     dig.sp = sp;
@@ -765,7 +829,7 @@ __global__ void __launch_bounds__(SegBucketCfg<T>::NT, SegBucketCfg<T>::MINB)
 // the word and stop, later passes return at once.
 template <class T, class S>
 __global__ void __launch_bounds__(SegBucketCfg<T>::NT, SegBucketCfg<T>::MINB)
-    sb_stable_pass_kernel(const T* src, T* dst, const SbTile* tiles, const uint32_t* tile_count,
+    sb_stable_pass_kernel(SbBuffers<T> buf, int level, const SbTile* tiles, const uint32_t* tile_count,
                           const SbMap<typename Traits<T>::Key>* maps, const typename Traits<T>::Key* splitters,
                           uint64_t xmask, const S* start, S* look, unsigned* claim, int* err, uint32_t spin) {
     using Sh = SegBucketShape<T>;
@@ -786,6 +850,9 @@ __global__ void __launch_bounds__(SegBucketCfg<T>::NT, SegBucketCfg<T>::MINB)
     grid_dep_wait();
     const uint32_t total_tiles = count_load(tile_count);
     if (total_tiles == 0) return;
+    const bool from_tmp = buf.from_tmp(level);
+    const T* src = from_tmp ? buf.tmp : buf.d;
+    T* dst = from_tmp ? buf.d : buf.tmp;
     if (tid == 0) next_tile = atomicAdd(claim, 1u);
     if (__syncthreads_or(tid == 0 && err_wait_set(err))) return;
     SbDigit<T> dig;
@@ -987,19 +1054,24 @@ __device__ __forceinline__ void sb_byte_place(uint32_t* table, int mine, Digit d
 // its place in either buffer (a: where it is). Bytes that all keys share are skipped.
 // (Not inlined: its registers are not the other buckets'.)
 template <class T>
-__device__ __noinline__ void sb_sort_long(T* a, T* b, T* want, uint64_t len, uint32_t* table, uint64_t xmask) {
+__device__ __noinline__ void sb_sort_long(T* a, T* b, T* want, uint64_t len, uint64_t xin, uint64_t xout) {
+    unsigned char* smem_raw = bk_smem();
     using Sh = BucketShape<T>;
     using K = typename Traits<T>::Key;
     using Count = unsigned long long;
     constexpr int NT = Sh::C::S_NT, IPT = Sh::C::S_IPT;
-    __shared__ Count cnt[RADIX_BINS], place[RADIX_BINS], ws8[RADIX_BINS / 32];
-    __shared__ uint32_t ws[RADIX_BINS / 32];
+    // where a bucket's items stand otherwise (static shared memory would count for every bucket)
+    Count* cnt = reinterpret_cast<Count*>(smem_raw);
+    Count *place = cnt + RADIX_BINS, *ws8 = place + RADIX_BINS;
+    uint32_t* ws = reinterpret_cast<uint32_t*>(ws8 + RADIX_BINS / 32);
+    uint32_t* table = reinterpret_cast<uint32_t*>(smem_raw + Sh::KEYS_BYTES);
+    static_assert(Sh::KEYS_BYTES >= (2 * RADIX_BINS + RADIX_BINS / 32) * 8 + RADIX_BINS / 32 * 4, "they fit");
     const int tid = threadIdx.x, i0 = (tid >> 4) * (16 * IPT) + (tid & 15);
     T w[IPT];
 #pragma unroll 1
     for (int byte = 0; byte < (int)sizeof(K); ++byte) {
         auto digit_of = [&](const T& v) -> unsigned {
-            return (unsigned)(Traits<T>::key(bk_flip(v, xmask)) >> (8 * byte)) & 255u;
+            return (unsigned)(Traits<T>::key(bk_flip(v, xin)) >> (8 * byte)) & 255u;
         };
         auto digit = [&](int i) -> unsigned { return digit_of(w[i]); };
         if (tid < RADIX_BINS) cnt[tid] = 0;
@@ -1034,57 +1106,66 @@ __device__ __noinline__ void sb_sort_long(T* a, T* b, T* want, uint64_t len, uin
         a = b;
         b = x;
     }
-    if (a != want)
-        for (uint64_t i = tid; i < len; i += NT) want[i] = a[i];
+    if (a != want || xin != xout)
+        for (uint64_t i = tid; i < len; i += NT) want[i] = bk_flip(a[i], xin ^ xout);
 }
 
-// Buckets that sb_sort_kernel left: those beyond its grid (from `first` on), and
-// slices that did not fit.
-template <class T>
-__global__ void __launch_bounds__(BucketCfg<T>::S_NT, 2)
-    sb_rest_kernel(T* d, T* tmp, const SbRec* recs, const uint32_t* slow, const SbCounts* cn, uint32_t first,
-                   uint64_t xmask) {
-    using Sh = BucketShape<T>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ BucketSortShared<T> sh;
-    grid_dep_wait();
-    const uint32_t left = count_load(&cn->slow), all = count_load(&cn->recs);
-    const uint32_t total = left + (all > first ? all - first : 0u);
-    for (uint32_t h = blockIdx.x; h < total; h += gridDim.x) {
-        const SbRec r = recs[h < left ? slow[h] : first + (h - left)];
-        const uint64_t len = r.what & SbRec::LEN;
-        const bool moved = (r.what & SbRec::TMP) != 0;
-        T *a = (moved ? tmp : d) + r.base, *b = (moved ? d : tmp) + r.base, *want = d + r.base;
-        if (len <= (uint64_t)Sh::CAP) {
-            bk_sort_crowded<T>(smem_raw, sh, a, want, (int)len, xmask);
-        } else {
-            sb_sort_long<T>(a, b, want, len, reinterpret_cast<uint32_t*>(smem_raw + Sh::KEYS_BYTES), xmask);
-        }
-        __syncthreads();
-    }
-}
+// The buckets of a plain bucket sort that did not give up: [start[b], start[b + 1]) of d
+// or tmp.
+struct SbStarts {
+    const uint32_t* start;
+    uint32_t buckets;
+    bool in_tmp;
+};
 
-// Sorts every bucket of the list, one CTA each (bk_sort_bucket). A loop over
-// buckets would cost registers (1.24 ms became 1.67 at 2^28 uint32 keys); the few
-// buckets beyond the grid are left to sb_rest_kernel.
+// Sorts every bucket, one CTA each (bk_sort_bucket; a loop over buckets costs registers,
+// 2^28 uint32 keys 1.67 ms instead of 1.24): those of the list, or the plain bucket
+// sort's, so that no launch is for buckets of the other kind only (2 ns for every CTA
+// that finds nothing to do). The CTAs from `first` on take the rest of the list in turn:
+// the few buckets beyond the grid, and slices that did not fit.
 template <class T>
 __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
-    sb_sort_kernel(T* d, T* tmp, const SbRec* recs, uint32_t* slow, SbCounts* cn, uint64_t xmask) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ BucketSortShared<T> sh;
-    bk_sort_init<T>(smem_raw, sh);
+    sb_sort_kernel(SbBuffers<T> buf, SbStarts plain, const SbRec* recs, const uint32_t* slow, const SbCounts* cn,
+                   uint32_t first, uint64_t xin, uint64_t xout) {
+    bk_sort_init<T>();
     grid_dep_launch();
     grid_dep_wait();
-    const SbRec r = recs[blockIdx.x];  // (the list has room for the grid: one latency with the count)
-    if (blockIdx.x >= count_load(&cn->recs)) return;
-    if (r.what & SbRec::SLOW) {
-        if (threadIdx.x == 0) slow[atomicAdd(&cn->slow, 1u)] = blockIdx.x;
+    const uint32_t at = blockIdx.x;
+    const T* src;
+    uint64_t base;
+    int cnt;
+    // (32-bit keys: radix passes stand behind the plain bucket sort)
+    if (sizeof(typename Traits<T>::Key) == 8 && plain.start && route_load(buf.route) == ROUTE_BUCKETS) {
+        if (at >= plain.buckets) return;
+        const uint32_t b0 = plain.start[at], b1 = plain.start[at + 1];
+        if (b1 <= b0 || b1 - b0 > (uint32_t)BucketShape<T>::CAP) return;
+        src = plain.in_tmp ? buf.tmp : buf.d;
+        base = b0;
+        cnt = (int)(b1 - b0);
+    } else if (at < first) {
+        const SbRec r = recs[at];  // (the list has room for the grid: one latency with the count)
+        if (at >= count_load(&cn->recs) || (r.what & SbRec::SLOW)) return;
+        src = (r.what & SbRec::TMP) ? buf.tmp : buf.d;
+        base = r.base;
+        cnt = (int)(r.what & SbRec::LEN);
+    } else {
+        const uint32_t left = count_load(&cn->slow), all = count_load(&cn->recs);
+        const uint32_t total = left + (all > first ? all - first : 0u);
+        for (uint32_t h = at - first; h < total; h += gridDim.x - first) {
+            const SbRec r = recs[h < left ? slow[h] : first + (h - left)];
+            const uint64_t len = r.what & SbRec::LEN;
+            const bool moved = (r.what & SbRec::TMP) != 0;
+            T *a = (moved ? buf.tmp : buf.d) + r.base, *b = (moved ? buf.d : buf.tmp) + r.base;
+            if (len > (uint64_t)BucketShape<T>::CAP)
+                sb_sort_long<T>(a, b, buf.want() + r.base, len, xin, xout);
+            else
+                bk_sort_crowded<T>(a, buf.want() + r.base, (int)len, xin, xout);
+            __syncthreads();
+        }
         return;
     }
-    const T* src = ((r.what & SbRec::TMP) ? tmp : d) + r.base;
-    const int cnt = (int)(r.what & SbRec::LEN);
-    if (!bk_sort_bucket<T, BK_LEAVE>(smem_raw, sh, src, d + r.base, cnt, xmask))
-        bk_sort_crowded<T>(smem_raw, sh, src, d + r.base, cnt, xmask);
+    if (!bk_sort_bucket<T, BK_LEAVE>(src + base, buf.want() + base, cnt, xin, xout))
+        bk_sort_crowded<T>(src + base, buf.want() + base, cnt, xin, xout);
 }
 
 }  // namespace origami

@@ -1,5 +1,5 @@
-"""Bucket sort and the radix passes behind it (the default of device sorts from
-some size on): tile edges, ragged ends, one and two partition levels, digits
+"""Bucket sort and what stands behind it (the default of device sorts from some size
+on): tile edges, ragged ends, one and two partition levels, digits
 with one, two and sixteen values, clustered, duplicated and outlying keys, both
 result buffers, chunks, and the bounded waits. Integer work: the tolerance is
 zero."""
@@ -46,6 +46,10 @@ def keys(dist, n, seed):
     elif dist == "clusters":  # 100 neighbouring keys around each of many centres
         d = rng.integers(0, 2**64, max(1, n // 1000), dtype=np.uint64) & ~np.uint64(0x7F00000000)
         k = d[rng.integers(0, len(d), n)] + (rng.integers(0, 100, n).astype(np.uint64) << np.uint64(32))
+    elif dist == "zipf":  # a few heavy keys, spread over the range
+        k = np.exp(rng.random(n) * np.log(2.0**20)).astype(np.uint64) * np.uint64(0x9E3779B97F4A7C15)
+    elif dist == "log":  # clusters in clusters
+        k >>= (k % np.uint64(48)).astype(np.uint64)
     elif dist == "outliers":  # a narrow range and a few keys far outside it
         k = (k >> np.uint64(22)) + (np.uint64(5) << np.uint64(60))
         k[:: max(1, n // 5)] = rng.integers(0, 2**64, len(k[:: max(1, n // 5)]), dtype=np.uint64)
@@ -93,7 +97,7 @@ def test_radix_matches_stable_sort(kind, dist, n, in_tmp):
 
 # the largest one-level sort and the smallest two-level one of each kind are
 # 2^20 / 2^20 + 1 items (u32) and 2^19 / 2^19 + 1 (64-bit keys)
-@pytest.mark.parametrize("dist", ["uniform", "normal", "repeated", "clusters", "outliers"])
+@pytest.mark.parametrize("dist", ["uniform", "normal", "repeated", "clusters", "zipf", "log", "outliers"])
 @pytest.mark.parametrize("kind", [og.U32, og.U64, og.I64, og.KV64, og.KVU64])
 @pytest.mark.parametrize("n", [1 << 19, (1 << 19) + 1, 1 << 20, (1 << 20) + 1, (1 << 22) + 8191])
 def test_buckets_match_stable_sort(kind, dist, n):
@@ -103,10 +107,11 @@ def test_buckets_match_stable_sort(kind, dist, n):
 
 @pytest.mark.parametrize("kind", [og.U32, og.I64, og.KV64])
 @pytest.mark.parametrize("sort_n", [1 << 19, 1 << 20])
-def test_radix_chunks(kind, sort_n):
+@pytest.mark.parametrize("second", ["small", "zipf", "log"])
+def test_radix_chunks(kind, sort_n, second):
     n = (1 << 21) + 4099  # the last chunk is short
     a = items(kind, "uniform", n, seed=3)
-    a[sort_n:2 * sort_n] = items(kind, "small", sort_n, seed=4)  # one chunk with constant digits
+    a[sort_n:2 * sort_n] = items(kind, second, sort_n, seed=4)  # one chunk of other keys
     assert np.array_equal(device_sort(a, kind, sort_n=sort_n), expected(a, sort_n))
 
 
