@@ -310,17 +310,22 @@ int seg_shape_for(int kind, uint64_t n, uint64_t nseg) {
     return g_seg_tune[kind][seg_class(n, nseg)].load(std::memory_order_relaxed);
 }
 
+// The radix path, keys written with the sign flip xout.
+cudaError_t run_radix(int kind, void* d, void* tmp, uint64_t n, uint64_t sort_n, void* want, uint64_t xout,
+                      void* scratch, cudaStream_t st) {
+    const uint64_t m = key_mask(kind);
+    switch (kind) {
+        case ORIGAMI_U32: return radix_sort_u32(d, tmp, n, sort_n, m, xout, want, scratch, st);
+        case ORIGAMI_U64:
+        case ORIGAMI_I64: return radix_sort_u64(d, tmp, n, sort_n, m, xout, want, scratch, st);
+        default: return radix_sort_kv(d, tmp, n, sort_n, m, xout, want, scratch, st);
+    }
+}
+
 cudaError_t run_typed(int kind, void* d, void* tmp, uint64_t n, uint64_t sort_n, void* want,
                       int fan, void* scratch, cudaStream_t st) {
     const uint64_t m = key_mask(kind);
-    if (radix_takes(kind, n, sort_n, fan)) {
-        switch (kind) {
-            case ORIGAMI_U32: return radix_sort_u32(d, tmp, n, sort_n, m, m, want, scratch, st);
-            case ORIGAMI_U64:
-            case ORIGAMI_I64: return radix_sort_u64(d, tmp, n, sort_n, m, m, want, scratch, st);
-            default: return radix_sort_kv(d, tmp, n, sort_n, m, m, want, scratch, st);
-        }
-    }
+    if (radix_takes(kind, n, sort_n, fan)) return run_radix(kind, d, tmp, n, sort_n, want, m, scratch, st);
     switch (kind) {
         case ORIGAMI_U32: return sort_u32(d, tmp, n, sort_n, m, want, fan, scratch, st, nullptr);
         case ORIGAMI_U64:
@@ -600,15 +605,19 @@ struct HostPipePlan {
     bool slice_copies = false;
     uint64_t chunk_n = 0;
     int fan = 0, cfan = 0, mfan = 0;
-    // host input: the first chunk lands in this many pieces, each sorted as
-    // it lands, then merged into the chunk's run by one k-way pass
+    // chunks sort by the radix path with this pass shape code (0: by merges); a chunk
+    // shorter than RADIX_CHUNK merges
+    int radix = 0;
+    // host input of chunks that merge: the first chunk lands in this many pieces,
+    // each sorted as it lands, then merged into the chunk's run by one k-way pass
     int first_pieces = 1;
     uint64_t data = 0, ws = 0, wm = 0, total = 0;  // A and B (data each), lane scratch, merge scratch
 };
 
 uint64_t a256(uint64_t b) { return (b + 255) & ~255ull; }
 
-HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_k) {
+// merges: chunks do not sort by the radix path (its scratch could not be had).
+HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_k, bool merges = false) {
     HostPipePlan p;
     const uint64_t limit = (sort_n == 0 || sort_n >= n) ? n : sort_n;
     p.fan = shape_for(kind, n, min_k) & ~SHAPE_RADIX;
@@ -643,6 +652,17 @@ HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_
     p.first_pieces = shape_fan(p.cfan) >= 4 ? 4 : 1;
     p.ws = a256(std::max(typed_scratch_io(kind, p.chunk_n, 0, p.cfan, 0),
                          typed_scratch_io(kind, p.chunk_n, 0, p.cfan, p.chunk_n / p.first_pieces)));
+    const int code = shape_for(kind, p.chunk_n, min_k);
+    if (min_k == 0 && !merges && radix_takes(kind, p.chunk_n, 0, code)) {
+        // the chunk sorts keep up with the link (2^22 uint32 keys 0.10 ms, their
+        // transfer 0.08; Zipf keys 0.20). Per call from pinned memory, chunks by merges
+        // and by buckets: 2^26 uint32 3.50 and 3.03 ms, 2^28 13.2 and 11.4, 2^27 uint64
+        // 14.4 and 11.4, 2^25 pairs 6.65 and 5.80; Zipf keys: 2^26 uint32 3.43 and 3.46
+        // (six lanes; 3.48 with four), 2^25 uint64 3.75 and 3.40
+        p.radix = code;
+        p.first_pieces = 1;
+        p.ws = std::max(p.ws, a256(scratch_bytes(kind, p.chunk_n, 0, code)));
+    }
     // the merges across chunks are one k-way pass: bound by the host link it
     // writes (1 GiB in ~5.6 ms), which hides its cost per level
     const uint64_t need = (limit + p.chunk_n - 1) / p.chunk_n;
@@ -740,6 +760,13 @@ int host_pipe_run(int kind, void* host_in, void* host_out, const void* vin, void
                 cudaStreamWaitEvent(cst, event_on(sc), 0);
                 src = a + off * ib;
             }
+            if (p.radix && !device_in && cn >= RADIX_CHUNK) {
+                // keys stay in the internal order until the final pass
+                if (e == cudaSuccess)
+                    e = run_radix(kind, a + off * ib, b + off * ib, cn, 0, a + off * ib, 0, w[lane], cst);
+                if (e == cudaSuccess) e = watch.watch(w[lane] + scratch_bytes(kind, cn, 0, p.radix) - 256, cst);
+                continue;
+            }
             if (e == cudaSuccess)
                 e = typed_io(kind, src, a + off * ib, b + off * ib, a + off * ib, cn, 0, m, 0, 0, p.cfan, w[lane],
                              cst);
@@ -782,9 +809,15 @@ int host_pipe_run(int kind, void* host_in, void* host_out, const void* vin, void
 
 int sort_host_direct(int kind, void* host_in, void* host_out, const void* vin, void* vout, uint64_t n,
                      uint64_t sort_n, unsigned min_k, cudaStream_t st) {
-    const HostPipePlan p = host_pipe_plan(kind, n, sort_n, min_k);
+    HostPipePlan p = host_pipe_plan(kind, n, sort_n, min_k);
     void* block = nullptr;
-    CK(cudaMallocAsync(&block, p.total, st), "arena allocation");
+    cudaError_t e = cudaMallocAsync(&block, p.total, st);
+    if (e == cudaErrorMemoryAllocation && p.radix) {
+        cudaGetLastError();
+        p = host_pipe_plan(kind, n, sort_n, min_k, true);
+        e = cudaMallocAsync(&block, p.total, st);
+    }
+    CK(e, "arena allocation");
     const int rc = host_pipe_run(kind, host_in, host_out, vin, vout, n, sort_n, p, block, st);
     cudaFreeAsync(block, st);
     return rc;

@@ -134,6 +134,7 @@ void segbucket_levels(const SbBuffers<T>& buf, const SbGiven& given, const SbSta
         to.recs = sc.recs;
         to.rec_count = &cn->recs;
         to.slow = sc.slow;
+        to.stay = xin == xout;
         to.slow_count = &cn->slow;
         const SbGiven none{};
         const uint32_t samples = l == 0 && behind ? std::max(given.nseg, given.slices) : segs;

@@ -432,8 +432,8 @@ struct SbHandOn {
     SbRec* recs;
     uint32_t *slow, *slow_count;
     uint32_t* rec_count;
-    uint64_t flags;  // (set by the kernel, as stay)
-    bool stay;
+    uint64_t flags;  // (set by the kernel)
+    bool stay;       // equal keys need not be written again where they are wanted
 };
 
 // Turns a segment's counts (h: the count of slice tid, threads below 256) into
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(512)
     const bool from_tmp = buf.from_tmp(level);
     const T* in = from_tmp ? buf.tmp : buf.d;
     to.flags = from_tmp ? 0 : SbRec::TMP;
-    to.stay = from_tmp != buf.want_tmp;
+    to.stay = to.stay && from_tmp != buf.want_tmp;
     for (int i = tid; i < RADIX_BINS * COPIES; i += NT) cnt[i] = 0;
     SbDigit<T> dig;
     dig.xmask = xmask;

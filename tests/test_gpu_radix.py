@@ -115,6 +115,17 @@ def test_radix_chunks(kind, sort_n, second):
     assert np.array_equal(device_sort(a, kind, sort_n=sort_n), expected(a, sort_n))
 
 
+# five chunks, the last one short: their sorts leave signed keys in the internal order
+@pytest.mark.parametrize("dist", ["uniform", "equal", "zipf", "log", "repeated"])
+@pytest.mark.parametrize("kind", [og.U32, og.U64, og.I64, og.KV64, og.KVU64])
+def test_host_chunks(kind, dist):
+    n = (1 << 24) + (1 << 17) + 3
+    a = items(kind, dist, n, seed=kind)
+    b = a.copy()
+    og.sort(b, np.empty_like(b))
+    assert np.array_equal(b, expected(a))
+
+
 def test_radix_long_segment():
     # 2^30 items and more: the counts of one segment need the wide words
     n = (1 << 30) + 5
