@@ -11,7 +11,8 @@
 //                     is far too full
 //   bk_hist_kernel    counts a level's slices, one read
 //   bk_scan_kernel    slice starts; bucket sizes against what the last kernel
-//                     can take; the next level's tiles
+//                     can take; the next level's tiles (the first level of one
+//                     segment: the last CTA of bk_hist_kernel)
 //   bk_pass_kernel    one partition level for keys, one read and one write
 //   radix_pass_kernel the same for pairs, whose order has to be kept
 //   bk_sort_kernel    one bucket per CTA, sorted in shared memory (64-bit keys:
@@ -33,10 +34,11 @@
 // Equal keys of keys-only items are identical, so their order does not matter:
 // bk_pass_kernel takes places with shared-memory atomics, one CTA per tile in
 // any order, and claims each slice's output range with one global atomic. No
-// kernel here waits for another CTA. The kernels start early (programmatic
-// dependent launch), some while the buffers they will read are still being
-// written, so no pointer here is __restrict__ (no loads through the read-only
-// path) and everything shared is read after grid_dep_wait().
+// kernel here waits for another CTA. Each kernel starts while the last CTAs of the one
+// before it run (programmatic dependent launch; no kernel lets the next one in earlier,
+// its waiting CTAs would cost more than the launch: 2^20 uint32 keys 44 us with, 38
+// without), so no pointer here is __restrict__ (no loads through the read-only path)
+// and everything shared is read after grid_dep_wait().
 #pragma once
 #include <cstdint>
 
@@ -80,7 +82,9 @@ struct BucketShape {
     static constexpr int TILE = C::NT * C::IPT;
     static constexpr size_t PASS_SMEM = (size_t)TILE * sizeof(T);
     static constexpr int CAP = C::S_NT * C::S_IPT;  // largest bucket
-    static constexpr int CROWDED = 32;              // largest bin that neighbours settle
+    // largest bin that neighbours settle (32: 4000 Zipf uint32 keys 22 us, 16: 18; 2^27
+    // Zipf uint64 keys 3.76 and 3.28 ms)
+    static constexpr int CROWDED = 16;
     static constexpr int SIDE = STABLE ? 0 : CROWDED;  // guard keys on either side of the bucket
     static constexpr size_t KEYS_BYTES = (size_t)(CAP + 2 * SIDE) * sizeof(T);
     static constexpr size_t BIN_BYTES = (size_t)C::BINS * 4 + (STABLE ? (size_t)CAP * 2 : 0);  // bins, places (pairs)
@@ -97,8 +101,12 @@ struct BucketShape {
         KEYS_BYTES + (BIN_BYTES + CROWD_BYTES > BYTE_BYTES ? BIN_BYTES + CROWD_BYTES : BYTE_BYTES);
     static_assert(TILE == RadixShape<T>::TILE || !STABLE, "pairs partition by radix_pass_kernel");
 };
-constexpr int BK_SAMPLES = 8192;     // keys sampled per segment
+// keys sampled per segment; fewer up to one partition level (2^28 uint32 keys in chunks of
+// 2^19: samples 0.10 and 0.04 ms)
+constexpr int BK_SAMPLES = 8192, BK_FEW = 2048;
+constexpr uint64_t BK_FEW_UP_TO = 1 << 20;
 constexpr int BK_MAX_BITS = 16;      // slices of both levels
+constexpr uint64_t BK_SELF_CLEAR = 1 << 17;  // bytes
 
 // How a segment's keys map to slices: x = the key's distance from lo, scaled so
 // that hi's fills 32 bits; slice = x * mul >> 32. mul is a multiple of 2^b2, so
@@ -212,7 +220,7 @@ struct BkListed {
 template <class T>
 __global__ void __launch_bounds__(1024) bk_sample_kernel(const T* in, uint64_t n, uint64_t len, uint64_t xmask, int b1,
                                                          int b2, uint64_t cap, SliceMap<typename Traits<T>::Key>* maps,
-                                                         int* route) {
+                                                         int* route, uint4* zero, uint32_t nzero) {
     using K = typename Traits<T>::Key;
     constexpr int PER = BK_SAMPLES / 1024;
     extern __shared__ __align__(16) uint32_t half[];  // 2^(b1+b2) 16-bit counters
@@ -221,13 +229,19 @@ __global__ void __launch_bounds__(1024) bk_sample_kernel(const T* in, uint64_t n
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, bits = b1 + b2;
     const uint64_t base = (uint64_t)blockIdx.x * len;
     const uint64_t m = n - base < len ? n - base : len;
+    const int ns = m <= BK_FEW_UP_TO ? BK_FEW : BK_SAMPLES;
+    for (uint32_t i = tid; i < nzero; i += 1024) zero[i] = make_uint4(0, 0, 0, 0);
     K v[PER];
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
+        if (i * 1024 >= ns) {
+            v[i] = v[0];
+            continue;
+        }
         // evenly spaced, each moved inside its stretch by a hash
         const uint32_t j = (uint32_t)(i * 1024 + tid);
-        const uint64_t a = (m * j) / BK_SAMPLES;
-        const uint32_t gap = (uint32_t)((m * (j + 1)) / BK_SAMPLES - a);
+        const uint64_t a = (m * j) / (uint32_t)ns;
+        const uint32_t gap = (uint32_t)((m * (j + 1)) / (uint32_t)ns - a);
         const uint64_t p = a + __umulhi(j * 2654435761u, gap);
         v[i] = Traits<T>::key(bk_flip(in[base + (p < m ? p : m - 1)], xmask));
     }
@@ -268,14 +282,72 @@ __global__ void __launch_bounds__(1024) bk_sample_kernel(const T* in, uint64_t n
     bool full = false;
     const SliceMap<K> mp = map;
     // far too full: at least 16 samples, and twice the largest bucket by estimate
-    const uint32_t most = max(15u, (uint32_t)min((unsigned long long)(2 * cap * BK_SAMPLES / m), 60000ull));
+    const uint32_t most = max(15u, (uint32_t)min((unsigned long long)(2 * cap * (uint32_t)ns / m), 60000ull));
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
+        if (i * 1024 >= ns) break;
         const uint32_t s = __umulhi(mp.scaled(v[i]), mp.mul);
         const uint32_t h = (atomicAdd(&half[s >> 1], (s & 1) ? 0x10000u : 1u) >> ((s & 1) * 16) & 0xFFFFu) + 1;
         full |= h > most;
     }
     if (__syncthreads_or(full) && tid == 0) *route = ROUTE_RADIX;
+}
+
+// ------------------------------------------------------------------ scan ---
+// A segment's counts (h: the count of slice tid) become slice starts in start[] and
+// cursor[], and either the next level's tiles (tiles2 given) or the check that every
+// bucket fits. Every thread of the CTA calls it.
+struct BkScan {
+    uint32_t *start, *cursor;
+    BkTile* tiles2;
+    uint32_t* count2;
+    int* route;
+    int full_route;
+    uint64_t n;
+    uint32_t last_seg;
+};
+template <class T>
+__device__ __forceinline__ void bk_scan_segment(const BkScan& to, uint32_t seg, uint32_t base, int bits, uint32_t h) {
+    constexpr uint32_t TILE = BucketShape<T>::TILE;
+    __shared__ uint32_t ws[RADIX_BINS / 32], ws2[RADIX_BINS / 32], at2;
+    const int tid = threadIdx.x, nb = 1 << bits;
+    const size_t at = ((size_t)seg << bits) + tid;
+    const uint32_t s = base + radix_bin_scan<uint32_t>(h, ws);
+    if (tid < nb) {
+        to.start[at] = s;
+        if (to.cursor) to.cursor[at] = s;
+        if (seg == to.last_seg && tid == nb - 1) to.start[at + 1] = (uint32_t)to.n;
+    }
+    if (to.tiles2) {
+        // the segment's tiles stand together in the list, bucket by bucket
+        const uint32_t nt = (h + TILE - 1) / TILE;
+        uint32_t t0 = radix_bin_scan<uint32_t>(nt, ws2);
+        if (tid == RADIX_BINS - 1) at2 = atomicAdd(to.count2, t0 + nt);
+        __syncthreads();
+        t0 += at2;
+        for (uint32_t i = 0; i < nt; ++i) {
+            BkTile r;
+            r.sbase = s;
+            r.base = (uint64_t)s + (uint64_t)i * TILE;
+            r.slen = h;
+            r.seg = (seg << bits) + (uint32_t)tid;
+            r.ti = i;
+            r.cnt = h - i * TILE < TILE ? h - i * TILE : TILE;
+            to.tiles2[t0 + i] = r;
+        }
+    } else if (h > (uint32_t)BucketShape<T>::CAP) {
+        *to.route = to.full_route;
+    }
+}
+// One CTA per segment of the level (256 threads, one slice each).
+template <class T>
+__global__ void __launch_bounds__(RADIX_BINS)
+    bk_scan_kernel(const uint32_t* hist, int bits, const uint32_t* seg_start, uint64_t len, BkScan to) {
+    const uint32_t seg = blockIdx.x;
+    grid_dep_wait();
+    if (route_load(to.route) != ROUTE_BUCKETS) return;
+    const uint32_t h = threadIdx.x < (1u << bits) ? hist[((size_t)seg << bits) + threadIdx.x] : 0;
+    bk_scan_segment<T>(to, seg, seg_start ? seg_start[seg] : (uint32_t)(seg * len), bits, h);
 }
 
 // ------------------------------------------------------------------ hist ---
@@ -285,13 +357,12 @@ template <class T, class G>
 __global__ void __launch_bounds__(512) bk_hist_kernel(const T* in, G geo, uint32_t tiles,
                                                       const SliceMap<typename Traits<T>::Key>* maps,
                                                       uint32_t map_shift, uint64_t xmask, int shift, int bits,
-                                                      uint32_t* hist, const int* route) {
+                                                      uint32_t* hist, const int* route, BkScan to, uint32_t* done) {
     using Sh = BucketShape<T>;
     constexpr int COPIES = 16, TILE = Sh::TILE, V = Vec<T>::N, STEPS = TILE / V / 512;
     static_assert(STEPS * V * 512 == TILE, "whole vector steps");
     __shared__ uint32_t cnt[RADIX_BINS * COPIES];
     const int tid = threadIdx.x, col = tid & (COPIES - 1), nb = 1 << bits;
-    grid_dep_launch();
     grid_dep_wait();
     if (route_load(route) != ROUTE_BUCKETS) return;
     const uint32_t total = geo.total(tiles);
@@ -342,52 +413,16 @@ __global__ void __launch_bounds__(512) bk_hist_kernel(const T* in, G geo, uint32
         }
     }
     if (seg != 0xFFFFFFFFu) flush(seg);
-}
-
-// ------------------------------------------------------------------ scan ---
-// One CTA per segment of the level (256 threads, one slice each): slice starts
-// into start[] and cursor[], and either the next level's tiles (tiles2 given)
-// or the check that every bucket fits.
-template <class T>
-__global__ void __launch_bounds__(RADIX_BINS)
-    bk_scan_kernel(const uint32_t* hist, int bits, const uint32_t* seg_start, uint64_t len,
-                   uint32_t* start, uint32_t* cursor, uint64_t n, uint32_t last_seg,
-                   BkTile* tiles2, uint32_t* count2, int* route, int full_route) {
-    constexpr uint32_t TILE = BucketShape<T>::TILE;
-    __shared__ uint32_t ws[RADIX_BINS / 32], ws2[RADIX_BINS / 32], at2;
-    const int tid = threadIdx.x, nb = 1 << bits;
-    const uint32_t seg = blockIdx.x;
-    grid_dep_launch();
-    grid_dep_wait();
-    if (route_load(route) != ROUTE_BUCKETS) return;
-    const size_t at = ((size_t)seg << bits) + tid;
-    const uint32_t h = tid < nb ? hist[at] : 0;
-    const uint32_t base = seg_start ? seg_start[seg] : (uint32_t)(seg * len);
-    const uint32_t s = base + radix_bin_scan<uint32_t>(h, ws);
-    if (tid < nb) {
-        start[at] = s;
-        if (cursor) cursor[at] = s;
-        if (seg == last_seg && tid == nb - 1) start[at + 1] = (uint32_t)n;
-    }
-    if (tiles2) {
-        // the segment's tiles stand together in the list, bucket by bucket
-        const uint32_t nt = (h + TILE - 1) / TILE;
-        uint32_t t0 = radix_bin_scan<uint32_t>(nt, ws2);
-        if (tid == RADIX_BINS - 1) at2 = atomicAdd(count2, t0 + nt);
-        __syncthreads();
-        t0 += at2;
-        for (uint32_t i = 0; i < nt; ++i) {
-            BkTile r;
-            r.sbase = s;
-            r.base = (uint64_t)s + (uint64_t)i * TILE;
-            r.slen = h;
-            r.seg = (seg << bits) + (uint32_t)tid;
-            r.ti = i;
-            r.cnt = h - i * TILE < TILE ? h - i * TILE : TILE;
-            tiles2[t0 + i] = r;
-        }
-    } else if (h > (uint32_t)BucketShape<T>::CAP) {
-        *route = full_route;
+    if (!done) return;
+    // one segment: the CTA that adds its counts last turns them into starts
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(done, t1 - t0) + (t1 - t0) == total;
+    __syncthreads();
+    if (last) {
+        __threadfence();
+        bk_scan_segment<T>(to, 0, 0, bits, tid < nb ? look_load(hist + tid) : 0u);
     }
 }
 
@@ -412,7 +447,6 @@ __global__ void __launch_bounds__(BucketCfg<T>::NT, BucketCfg<T>::MINB)
     static_assert(NT == RADIX_BINS && IPT % 4 == 0, "one thread per slice; four digits to a register");
     const int tid = threadIdx.x, lane = tid & 31, nb = 1 << bits;
     tab[tid] = 0;
-    grid_dep_launch();
     grid_dep_wait();
     if (route_load(route) != ROUTE_BUCKETS) return;
     const uint32_t t = blockIdx.x;
@@ -952,7 +986,6 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
     bk_sort_kernel(const T* src, T* dst, const uint32_t* start, uint64_t xin, uint64_t xout, uint32_t n,
                    const int* route) {
     bk_sort_init<T>();
-    grid_dep_launch();
     grid_dep_wait();
     if (route_load(route) != ROUTE_BUCKETS) return;
     const uint32_t b0 = start[blockIdx.x], b1 = start[blockIdx.x + 1];
@@ -960,6 +993,17 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
     constexpr BkCrowded CROWD = sizeof(T) == 4 ? BK_BYTES : BK_LEAVE;
     if (!bk_sort_bucket<T, CROWD>(src + b0, dst + b0, (int)(b1 - b0), xin, xout))
         bk_sort_crowded<T>(src + b0, dst + b0, (int)(b1 - b0), xin, xout);
+}
+
+// A sort of one bucket: n items (up to CAP) by one CTA; clears the error word. (1000 uint32
+// keys 20 us by the tile sort of the merges, 10 here; 4000 uint64 keys 24 and 12, pairs 29
+// and 12.)
+template <class T>
+__global__ void __launch_bounds__(BucketCfg<T>::S_NT)
+    bk_one_kernel(const T* src, T* dst, int n, uint64_t xin, uint64_t xout, int* err) {
+    if (threadIdx.x == 0) *err = 0;
+    bk_sort_init<T>();
+    bk_sort_bucket<T, BK_SETTLE>(src, dst, n, xin, xout);
 }
 
 }  // namespace origami

@@ -878,13 +878,14 @@ int tune_load_file(const char* path) {
 struct TuneDefault {
     int kind, cls, fan, variant;
 };
-// First size class that sorts by radix passes. Below it the launches decide,
-// and a merge sort of a few levels has fewer: 131,072 uint32 keys take 43 us by
-// radix passes and 55 by the better merge shape, 65,536 keys 42 and 47, 32,768
-// keys are two merge levels (38); 131,072 uint64 keys 74 and 71, 262,144 keys 78
-// and 85; 131,072 pairs 74 and 83, 91,750 pairs
-// 83 by merges.
-constexpr int RADIX_FROM_U32 = 16, RADIX_FROM_U64 = 18, RADIX_FROM_KV = 17;
+// Size classes that sort by the radix path: the last one whose sorts can be one bucket
+// (where they are not, merges), and from where on several buckets pay. In between the
+// launches decide, and a merge sort of a few levels has fewer. Merges and buckets, us,
+// uniform / Zipf / all equal keys: 10,000 uint32 26 / 26 / 27 and 27 / 27 / 48; 20,000
+// 33 / 33 / 33 and 27 / 29 / 42; 50,000 46 / 46 / 44 and 29 / 38 / 44; 10,000 uint64
+// 38 / 37 / 36 and 27 / 33 / 40; 20,000 45 / 45 / 43 and 29 / 34 / 39; 20,000 pairs
+// 57 / 57 / 53 and 32 / 46 / 45.
+constexpr int RADIX_ONE = 12, RADIX_FROM_U32 = 15, RADIX_FROM_U64 = 14, RADIX_FROM_KV = 14;
 constexpr TuneDefault kTuneDefaults[] = {
     {ORIGAMI_U32, 18, 16, 0},  {ORIGAMI_U32, 19, 2, 3},   {ORIGAMI_U32, 20, 2, 3},   {ORIGAMI_U32, 21, 16, 0},
     {ORIGAMI_U32, 22, 2, 3},   {ORIGAMI_U32, 23, 2, 2},   {ORIGAMI_U32, 25, 16, 0},  {ORIGAMI_U64, 17, 16, 0},
@@ -902,7 +903,7 @@ int tune_builtin(int kind, int cls) {
     for (const TuneDefault& t : kTuneDefaults)
         if (t.kind == k && t.cls == cls) code = shape_code(t.fan, t.variant);
     const int from = k == ORIGAMI_U32 ? RADIX_FROM_U32 : (k == ORIGAMI_U64 ? RADIX_FROM_U64 : RADIX_FROM_KV);
-    return cls >= from ? code | SHAPE_RADIX : code;
+    return cls >= from || cls <= RADIX_ONE ? code | SHAPE_RADIX : code;
 }
 
 // Sets a class to a merge shape. The class's own built-in shape restores its

@@ -313,11 +313,12 @@ __device__ __forceinline__ T radix_flip(const T& v, uint64_t x) {
 // at launch; look_next (optional): the next pass's, cleared here. route
 // (optional): run only where it holds `run` (radix passes behind a bucket sort
 // run unless it is 0, the stable partition of a bucket sort while it is 0). xflip:
-// applied to the keys as they are written.
+// applied to the keys as they are written. (No early start of the next pass: its waiting
+// CTAs cost more than its launch, 2^20 uint32 Zipf keys 0.078 ms without and 0.111 with.)
 template <class T, class S, class G, class D>
 __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
-    radix_pass_kernel(const T* __restrict__ src, T* __restrict__ dst, G geo, uint32_t tiles, D digit, S* look,
-                      S* __restrict__ look_next, unsigned* __restrict__ claim, int* err, uint32_t spin,
+    radix_pass_kernel(const T* src, T* dst, G geo, uint32_t tiles, D digit, S* look,
+                      S* look_next, unsigned* claim, int* err, uint32_t spin,
                       const int* route, bool buckets, uint64_t xflip) {
     using Sh = RadixShape<T>;
     using W = LookWord<S>;

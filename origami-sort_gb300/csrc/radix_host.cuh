@@ -13,6 +13,8 @@
 
 namespace origami {
 
+constexpr uint64_t RADIX_LEAST = 1 << 14;
+
 // Segments of a radix sort: the whole array, or chunks of sort_n items.
 template <class T>
 struct RadixPlan {
@@ -29,10 +31,12 @@ struct RadixPlan {
             for (shift = 0; ((uint64_t)Sh::TILE << shift) < len;) ++shift;
         wide = len >= (1ull << 30);
     }
-    // Whole tiles per segment, and tile numbers that fit 31 bits.
+    // One bucket; else enough items for several launches (10,000 uint32 keys 27 us by
+    // buckets, 26 by merges), whole tiles per segment, and tile numbers that fit 31 bits.
     static bool fits(uint64_t n, uint64_t sort_n) {
         const uint64_t len = chunk_limit(n, sort_n);
-        return n >= 2 && (len == n || len % Sh::TILE == 0) && n / Sh::TILE < (1ull << 31) - 2;
+        if (n < 2 || (len == n && n <= (uint64_t)BucketShape<T>::CAP)) return n >= 2;
+        return n >= RADIX_LEAST && (len == n || len % Sh::TILE == 0) && n / Sh::TILE < (1ull << 31) - 2;
     }
 };
 
@@ -48,6 +52,8 @@ struct BucketPlan {
         if (p.n >= (1ull << 31)) return;
         int bits = 0;
         while ((p.len >> bits) > (1ull << Sh::C::LOG_TARGET)) ++bits;
+        // short sorts: one level can have up to 256 buckets, enough for every SM
+        while (bits < 8 && (p.nseg << bits) < RADIX_BINS && (p.len >> bits) > 256) ++bits;
         if (bits < 4 || bits > BK_MAX_BITS) return;
         if (p.nseg > 1 && (p.len % Sh::TILE != 0 || p.nseg > (1u << 20))) return;
         // two levels of about equal width: few slices would serialise the atomics
@@ -92,7 +98,7 @@ struct RadixScratch {
     uint64_t bytes = 0, zero_bytes = 0;
     char* zero = nullptr;
     void* look[2] = {nullptr, nullptr};
-    uint32_t *start1 = nullptr, *start2 = nullptr, *cursor1 = nullptr, *cursor2 = nullptr, *count2 = nullptr;
+    uint32_t *start1 = nullptr, *start2 = nullptr, *cursor1 = nullptr, *cursor2 = nullptr, *count2 = nullptr, *done = nullptr;
     SliceMap<K>* maps = nullptr;
     BkTile* tiles2 = nullptr;
     uint32_t *hist1 = nullptr, *hist2 = nullptr;
@@ -138,6 +144,7 @@ struct RadixScratch {
         if (b) {
             route = reinterpret_cast<int*>(claim + 12);
             count2 = claim + 13;
+            done = claim + 14;
             zero = b + z;
         }
         zero_bytes = o - z;
@@ -188,7 +195,7 @@ void radix_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, uint64_t xmask, 
 // The bucket sort: d -> want (d or tmp), *route set where it gives up.
 template <class T>
 void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPlan<T>& bk, uint64_t xmask,
-                   uint64_t xout, const RadixScratch<T>& sc, cudaStream_t st) {
+                   uint64_t xout, const RadixScratch<T>& sc, uint32_t nzero, cudaStream_t st) {
     using Sh = BucketShape<T>;
     using RSh = RadixShape<T>;
     using K = typename Traits<T>::Key;
@@ -225,21 +232,22 @@ void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPla
     const G1 geo{p.n, p.len, shift};
     launch(n_sample.c_str(), st, [&] {
         bk_sample_kernel<T><<<nseg, 1024, ((1u << bits) / 2 + 1) * 4, st>>>(d, p.n, p.len, xmask, bk.b1, bk.b2,
-                                                                            (uint64_t)Sh::CAP, sc.maps, sc.route);
+                                                                            (uint64_t)Sh::CAP, sc.maps, sc.route,
+                                                                            reinterpret_cast<uint4*>(sc.zero), nzero);
     });
     auto level = [&](auto geo_l, const T* src, T* dst, uint32_t tiles_l, int shift_l, int bits_l, uint32_t map_shift,
                      uint32_t segs, const uint32_t* seg_start, uint32_t* hist, uint32_t* start, uint32_t* cursor,
                      bool last, int full_route, void* look, void* look_next, unsigned* claim) {
         using G = decltype(geo_l);
+        const BkScan to{start, cursor, last ? (BkTile*)nullptr : sc.tiles2, sc.count2, sc.route, full_route, p.n, segs - 1};
         launch(n_hist.c_str(), st, [&] {
             launch_dependent(bk_hist_kernel<T, G>, dim3(std::min(tiles_l, g_hist)), dim3(512), 0, st, src, geo_l, tiles_l,
                              (const SliceMap<K>*)sc.maps, map_shift, xmask, shift_l, bits_l, hist,
-                             (const int*)sc.route);
+                             (const int*)sc.route, to, segs == 1 ? sc.done : (uint32_t*)nullptr);
         });
-        launch(n_scan.c_str(), st, [&] {
+        if (segs > 1) launch(n_scan.c_str(), st, [&] {
             launch_dependent(bk_scan_kernel<T>, dim3(segs), dim3(RADIX_BINS), 0, st, (const uint32_t*)hist, bits_l,
-                             seg_start, p.len, start, cursor, p.n, segs - 1, last ? (BkTile*)nullptr : sc.tiles2,
-                             sc.count2, sc.route, full_route);
+                             seg_start, p.len, to);
         });
         launch(n_pass.c_str(), st, [&] {
             if constexpr (ST) {
@@ -289,10 +297,26 @@ cudaError_t radix_sort(T* d, T* tmp, uint64_t n, uint64_t sort_n, uint64_t key_m
     const RadixPlan<T> p(n, sort_n);
     const BucketPlan<T> bk(p);
     const RadixScratch<T> sc(scratch, p, bk);
-    cudaMemsetAsync(sc.zero, 0, sc.zero_bytes, st);
+    if (p.nseg == 1 && n <= (uint64_t)BucketShape<T>::CAP) {
+        using Sh = BucketShape<T>;
+        static const std::string n_one = std::string("bucket_one<") + TypeName<T>::v + ">";
+        static const bool configured = [] {
+            cudaFuncSetAttribute(bk_one_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SORT_SMEM);
+            return true;
+        }();
+        (void)configured;
+        launch(n_one.c_str(), st, [&] {
+            bk_one_kernel<T><<<1, Sh::C::S_NT, Sh::SORT_SMEM, st>>>(d, want, (int)n, key_mask, out_mask, sc.err);
+        });
+        return cudaGetLastError();
+    }
+    // one segment's sample kernel clears what is not much by itself (2^20 uint32 keys: a
+    // memset takes 2 us)
+    const bool self = bk.on() && p.nseg == 1 && sc.zero_bytes <= BK_SELF_CLEAR;
+    if (!self) cudaMemsetAsync(sc.zero, 0, sc.zero_bytes, st);
     const int* route = nullptr;
     if (bk.on()) {
-        bucket_launch<T>(d, tmp, want, p, bk, key_mask, out_mask, sc, st);
+        bucket_launch<T>(d, tmp, want, p, bk, key_mask, out_mask, sc, self ? (uint32_t)(sc.zero_bytes / 16) : 0u, st);
         route = sc.route;
     }
     if constexpr (levels_behind<T>()) {

@@ -42,10 +42,8 @@
 // another CTA. Pairs are placed stably with a look-back over the tiles before
 // (sb_stable_pass_kernel). Every wait (look-back, bulk copies) is bounded.
 //
-// The kernels start early (programmatic dependent launch), some while the
-// buffers they will read are still being written, so no pointer here is
-// __restrict__ (no loads through the read-only path) and everything shared is
-// read after grid_dep_wait().
+// The kernels overlap as the plain bucket sort's do: no pointer here is __restrict__,
+// and everything shared is read after grid_dep_wait().
 #pragma once
 #include <cstdint>
 #include <type_traits>
@@ -235,7 +233,6 @@ template <class T>
 __global__ void sb_plan_kernel(const uint64_t* off, uint32_t nseg, uint64_t n, SbSeg* list, uint32_t most, SbRec* recs,
                                SbCounts* cn) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    grid_dep_launch();
     uint64_t a = 0, len = 0;
     if (s < nseg) {
         a = off[s];
@@ -276,7 +273,6 @@ __global__ void __launch_bounds__(512)
     __shared__ SbMap<K> smap;
     __shared__ uint32_t stile, sid;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    grid_dep_launch();
     grid_dep_wait();
     // (segments that overlap would not fit the lists)
     uint32_t total;
@@ -546,7 +542,6 @@ __global__ void __launch_bounds__(512)
         mbar_init(&bar[1], 1);
         mbar_init_fence();
     }
-    grid_dep_launch();
     grid_dep_wait();
     const uint32_t total = count_load(tile_count);
     const uint32_t t0 = (uint32_t)((uint64_t)total * blockIdx.x / gridDim.x);
@@ -683,7 +678,6 @@ __global__ void __launch_bounds__(SegBucketCfg<T>::NT, SegBucketCfg<T>::MINB)
     __shared__ K sp[SB_SPLITTERS + 1];
     static_assert(NT >= RADIX_BINS && IPT % 4 == 0, "one thread per slice; four digits to a register");
     const int tid = threadIdx.x, lane = tid & 31;
-    grid_dep_launch();
     grid_dep_wait();
     uint32_t t = blockIdx.x;
     SbTile q = tiles[t];  // (the list has room for the grid: one latency with the count)
@@ -1128,7 +1122,6 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
     sb_sort_kernel(SbBuffers<T> buf, SbStarts plain, const SbRec* recs, const uint32_t* slow, const SbCounts* cn,
                    uint32_t first, uint64_t xin, uint64_t xout) {
     bk_sort_init<T>();
-    grid_dep_launch();
     grid_dep_wait();
     const uint32_t at = blockIdx.x;
     const T* src;

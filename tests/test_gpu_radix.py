@@ -95,6 +95,17 @@ def test_radix_matches_stable_sort(kind, dist, n, in_tmp):
     assert np.array_equal(device_sort(a, kind, result_in_tmp=in_tmp), expected(a))
 
 
+# one bucket (up to 6144 uint32 keys, 4096 wider items), and the sizes around it and
+# around the smallest sort by several buckets
+@pytest.mark.parametrize("in_tmp", [False, True])
+@pytest.mark.parametrize("dist", ["uniform", "equal", "sixteen", "zipf", "clusters", "sorted"])
+@pytest.mark.parametrize("kind", [og.U32, og.U64, og.I64, og.KV64, og.KVU64])
+def test_one_bucket(kind, dist, in_tmp):
+    for n in (2, 3, 31, 255, 1000, 4095, 4096, 4097, 6143, 6144, 6145, 16383, 16384, 32767, 32768):
+        a = items(kind, dist, n, seed=n)
+        assert np.array_equal(device_sort(a, kind, result_in_tmp=in_tmp), expected(a)), n
+
+
 # the largest one-level sort and the smallest two-level one of each kind are
 # 2^20 / 2^20 + 1 items (u32) and 2^19 / 2^19 + 1 (64-bit keys)
 @pytest.mark.parametrize("dist", ["uniform", "normal", "repeated", "clusters", "zipf", "log", "outliers"])
