@@ -995,13 +995,13 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
         bk_sort_crowded<T>(src + b0, dst + b0, (int)(b1 - b0), xin, xout);
 }
 
-// A sort of one bucket: n items (up to CAP) by one CTA; clears the error word. (1000 uint32
+// A sort of one bucket: n items (up to CAP) by one CTA. (1000 uint32
 // keys 20 us by the tile sort of the merges, 10 here; 4000 uint64 keys 24 and 12, pairs 29
 // and 12.)
 template <class T>
 __global__ void __launch_bounds__(BucketCfg<T>::S_NT)
     bk_one_kernel(const T* src, T* dst, int n, uint64_t xin, uint64_t xout, int* err) {
-    if (threadIdx.x == 0) *err = 0;
+    if (err && threadIdx.x == 0) *err = 0;
     bk_sort_init<T>();
     bk_sort_bucket<T, BK_SETTLE>(src, dst, n, xin, xout);
 }

@@ -334,6 +334,25 @@ cudaError_t run_typed(int kind, void* d, void* tmp, uint64_t n, uint64_t sort_n,
     }
 }
 
+bool one_bucket(int kind, uint64_t n, uint64_t sort_n) {
+    switch (kind) {
+        case ORIGAMI_U32: return one_bucket_u32(n, sort_n);
+        case ORIGAMI_U64:
+        case ORIGAMI_I64: return one_bucket_u64(n, sort_n);
+        default: return one_bucket_kv(n, sort_n);
+    }
+}
+
+cudaError_t run_one_bucket(int kind, const void* d, void* want, uint64_t n, cudaStream_t st) {
+    const uint64_t m = key_mask(kind);
+    switch (kind) {
+        case ORIGAMI_U32: return bucket_one_u32(d, want, n, m, st);
+        case ORIGAMI_U64:
+        case ORIGAMI_I64: return bucket_one_u64(d, want, n, m, st);
+        default: return bucket_one_kv(d, want, n, m, st);
+    }
+}
+
 // Device-resident sort; the caller has validated the arguments. `watch`
 // (optional) collects the sort's device error word; with ORIGAMI_FLAG_SYNC and
 // no outer watch the call checks it itself and returns ORIGAMI_ERR_TIMEOUT
@@ -350,6 +369,13 @@ int sort_device_impl(int kind, void* d, void* tmp, uint64_t n, uint64_t sort_n, 
     if (n <= 1) {
         if (n == 1 && in_tmp)
             CK(cudaMemcpyAsync(tmp, d, item_bytes(kind), cudaMemcpyDeviceToDevice, st), "copy");
+        if (flags & ORIGAMI_FLAG_SYNC) CK(cudaStreamSynchronize(st), "stream sync");
+        return ORIGAMI_OK;
+    }
+    int fan = shape_for(kind, n, min_k);
+    if ((fan & SHAPE_RADIX) && one_bucket(kind, n, sort_n)) {
+        // one launch, without scratch or waits, whatever the buffers' alignment
+        CK(run_one_bucket(kind, d, in_tmp ? tmp : d, n, st), "sort launch");
         if (flags & ORIGAMI_FLAG_SYNC) CK(cudaStreamSynchronize(st), "stream sync");
         return ORIGAMI_OK;
     }
@@ -385,7 +411,6 @@ int sort_device_impl(int kind, void* d, void* tmp, uint64_t n, uint64_t sort_n, 
     }
     void* scratch = nullptr;
     if (!tmp) CK(cudaMallocAsync(&scratch, n * item_bytes(kind), st), "scratch allocation");
-    int fan = shape_for(kind, n, min_k);
     void* work = nullptr;
     cudaError_t e = cudaMallocAsync(&work, scratch_bytes(kind, n, sort_n, fan), st);
     if (e == cudaErrorMemoryAllocation && radix_takes(kind, n, sort_n, fan)) {

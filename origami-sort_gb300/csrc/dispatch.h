@@ -41,6 +41,16 @@ ORIGAMI_DECLARE_RADIX(u64)
 ORIGAMI_DECLARE_RADIX(kv)
 #undef ORIGAMI_DECLARE_RADIX
 
+// A sort of one bucket (bk_one_kernel): whether n items in chunks of sort_n are one, and
+// the sort, d -> want, any item alignment.
+#define ORIGAMI_DECLARE_ONE(name)                                                                   \
+    bool one_bucket_##name(uint64_t n, uint64_t sort_n);                                            \
+    cudaError_t bucket_one_##name(const void* d, void* want, uint64_t n, uint64_t key_mask, cudaStream_t st);
+ORIGAMI_DECLARE_ONE(u32)
+ORIGAMI_DECLARE_ONE(u64)
+ORIGAMI_DECLARE_ONE(kv)
+#undef ORIGAMI_DECLARE_ONE
+
 // Segmented sort by buckets (seg_buckets.cuh): whether it takes nseg segments of n
 // items in all, the scratch it needs (error word in its last 256 bytes), the sort
 // (result in d), and one-time kernel attributes (call outside stream capture).

@@ -286,6 +286,27 @@ void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPla
     });
 }
 
+// A sort of one bucket: d -> want by one launch, without scratch or waits. err (or null)
+// is cleared.
+template <class T>
+bool one_bucket(uint64_t n, uint64_t sort_n) {
+    return n >= 2 && n <= (uint64_t)BucketShape<T>::CAP && chunk_limit(n, sort_n) == n;
+}
+template <class T>
+cudaError_t bucket_one(const T* d, T* want, uint64_t n, uint64_t key_mask, uint64_t out_mask, int* err, cudaStream_t st) {
+    using Sh = BucketShape<T>;
+    static const std::string n_one = std::string("bucket_one<") + TypeName<T>::v + ">";
+    static const bool configured = [] {
+        cudaFuncSetAttribute(bk_one_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SORT_SMEM);
+        return true;
+    }();
+    (void)configured;
+    launch(n_one.c_str(), st, [&] {
+        bk_one_kernel<T><<<1, Sh::C::S_NT, Sh::SORT_SMEM, st>>>(d, want, (int)n, key_mask, out_mask, err);
+    });
+    return cudaGetLastError();
+}
+
 // Sorts d[0..n) in chunks of sort_n (0 = one full sort) into `want` (d or tmp):
 // by buckets where the geometry allows it, with radix passes or levels behind them
 // for what does not spread; else by those. key_mask: the sign flip of keys
@@ -297,19 +318,7 @@ cudaError_t radix_sort(T* d, T* tmp, uint64_t n, uint64_t sort_n, uint64_t key_m
     const RadixPlan<T> p(n, sort_n);
     const BucketPlan<T> bk(p);
     const RadixScratch<T> sc(scratch, p, bk);
-    if (p.nseg == 1 && n <= (uint64_t)BucketShape<T>::CAP) {
-        using Sh = BucketShape<T>;
-        static const std::string n_one = std::string("bucket_one<") + TypeName<T>::v + ">";
-        static const bool configured = [] {
-            cudaFuncSetAttribute(bk_one_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SORT_SMEM);
-            return true;
-        }();
-        (void)configured;
-        launch(n_one.c_str(), st, [&] {
-            bk_one_kernel<T><<<1, Sh::C::S_NT, Sh::SORT_SMEM, st>>>(d, want, (int)n, key_mask, out_mask, sc.err);
-        });
-        return cudaGetLastError();
-    }
+    if (one_bucket<T>(n, sort_n)) return bucket_one<T>(d, want, n, key_mask, out_mask, sc.err, st);
     // one segment's sample kernel clears what is not much by itself (2^20 uint32 keys: a
     // memset takes 2 us)
     const bool self = bk.on() && p.nseg == 1 && sc.zero_bytes <= BK_SELF_CLEAR;

@@ -18,4 +18,10 @@ cudaError_t radix_sort_kv(void* d, void* tmp, uint64_t n, uint64_t sort_n, uint6
                           scratch, st);
 }
 
+bool one_bucket_kv(uint64_t n, uint64_t sort_n) { return one_bucket<KV64>(n, sort_n); }
+
+cudaError_t bucket_one_kv(const void* d, void* want, uint64_t n, uint64_t key_mask, cudaStream_t st) {
+    return bucket_one<KV64>(static_cast<const KV64*>(d), static_cast<KV64*>(want), n, key_mask, key_mask, nullptr, st);
+}
+
 }  // namespace origami

@@ -14,4 +14,10 @@ cudaError_t radix_sort_u32(void* d, void* tmp, uint64_t n, uint64_t sort_n, uint
                           scratch, st);
 }
 
+bool one_bucket_u32(uint64_t n, uint64_t sort_n) { return one_bucket<uint32_t>(n, sort_n); }
+
+cudaError_t bucket_one_u32(const void* d, void* want, uint64_t n, uint64_t key_mask, cudaStream_t st) {
+    return bucket_one<uint32_t>(static_cast<const uint32_t*>(d), static_cast<uint32_t*>(want), n, key_mask, key_mask, nullptr, st);
+}
+
 }  // namespace origami

@@ -18,4 +18,10 @@ cudaError_t radix_sort_u64(void* d, void* tmp, uint64_t n, uint64_t sort_n, uint
                           scratch, st);
 }
 
+bool one_bucket_u64(uint64_t n, uint64_t sort_n) { return one_bucket<uint64_t>(n, sort_n); }
+
+cudaError_t bucket_one_u64(const void* d, void* want, uint64_t n, uint64_t key_mask, cudaStream_t st) {
+    return bucket_one<uint64_t>(static_cast<const uint64_t*>(d), static_cast<uint64_t*>(want), n, key_mask, key_mask, nullptr, st);
+}
+
 }  // namespace origami
