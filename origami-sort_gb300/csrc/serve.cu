@@ -287,13 +287,14 @@ struct origami_server {
 
     static void CUDART_CB on_done(void* p) {
         auto* b = static_cast<Batch*>(p);
+        auto* srv = b->srv;
         b->t_end = Clock::now();
-        {
-            std::lock_guard<std::mutex> lk(b->srv->mu);
-            b->finished.store(true);
-            ++b->srv->gen;
-        }
-        b->srv->cv_work.notify_one();
+        // notified under the lock: once it is free, the worker may free the batch, and its
+        // owner the server
+        std::lock_guard<std::mutex> lk(srv->mu);
+        b->finished.store(true);
+        ++srv->gen;
+        srv->cv_work.notify_one();
     }
 
     // Marks a batch finished from a helper thread.

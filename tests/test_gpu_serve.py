@@ -223,3 +223,19 @@ def test_large_requests_take_the_pipelined_sort():
     torch.cuda.synchronize()
     got = dev_in.cpu().numpy().view(np.uint64)
     assert np.array_equal(got, np.sort(dev_keep.cpu().numpy().view(np.uint64)))
+
+
+def test_many_batches_of_one_small_request():
+    # every batch finishes almost as soon as it starts: its completion must not touch it
+    # once the worker may have freed it
+    rng = np.random.default_rng(77)
+    a = make(og.U32, 1500, rng, pinned=True)
+    out = og.empty_host(og.U32, 1500, pinned=True)
+    want = np.sort(a)
+    for _ in range(10):
+        s = og.Server(hbm_budget_bytes=1 << 28, max_batch_items=1)
+        for _ in range(200):
+            out[:] = 0
+            s.wait(s.submit(a, out=out))
+            assert np.array_equal(out, want)
+        s.close()
