@@ -659,6 +659,7 @@ HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_
     p.chunked = n >= 4 * p.chunk_n && limit > p.chunk_n;
     p.data = a256(n * item_bytes(kind));
     if (!p.chunked) {
+        p.fan |= SHAPE_HOST_IN;
         p.ws = a256(typed_scratch_io(kind, n, sort_n, p.fan, 0));
         p.total = 2 * p.data + p.ws;
         return p;

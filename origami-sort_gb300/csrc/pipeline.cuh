@@ -12,6 +12,7 @@
 #include <utility>
 #include <vector>
 
+#include "buckets.cuh"
 #include "kway.cuh"
 #include "profiler.h"
 #include "sort_kernels.cuh"
@@ -190,6 +191,16 @@ static_assert(Config<uint32_t>::P2_TILE >= Config<uint32_t>::P_TILE && Config<ui
 // SHAPE_RADIX on top: the size class sorts by radix passes (radix.cuh) where
 // they take the call, and by the merge shape elsewhere.
 constexpr int SHAPE_RADIX = 1 << 16;
+// The first kernel reads its input from host memory, once.
+constexpr int SHAPE_HOST_IN = 1 << 17;
+// Shortest chunk that one CTA of the tile sort by buckets takes (2^22 items, block_sort
+// against it, us: uint32 keys in chunks of 1024 30 / 49, 2048 35 / 34, 4096 41 / 30;
+// uint64 keys in chunks of 256 59 / 100, 512 61 / 59, 4096 91 / 37; pairs 256 96 / 140,
+// 512 109 / 81, 4096 168 / 46).
+template <class T>
+constexpr uint64_t bucket_tile_least() {
+    return sizeof(typename Traits<T>::Key) == 8 ? 512 : 4096;
+}
 inline int shape_fan(int code) { return code & 0xFF; }
 inline int shape_variant(int code) { return (code >> 8) & 0xFF; }
 inline int shape_code(int fan, int variant) { return fan | (variant << 8); }
@@ -226,13 +237,24 @@ inline int next_pow2_int(uint64_t v) {
     return p;
 }
 
-// The merge passes after K1 for runs to reach `limit` (chunk size or n).
+// Runs that the first kernel leaves where the sort or chunk is not shorter: of 64-bit keys
+// those of bk_tile_kernel, unless the input is in host memory (crowded tiles are read
+// twice).
+template <class T>
+int first_run(int code) {
+    if constexpr (sizeof(typename Traits<T>::Key) == 8)
+        if (!(code & SHAPE_HOST_IN)) return BucketShape<T>::CAP;
+    return k1_tile<T>();
+}
+
+// The merge passes after the first kernel for runs to reach `limit` (chunk size or n).
 // fan == 2 gives the binary pipeline; fan in {4, 8, 16} the k-way one, whose
 // last pass uses the smallest fan-in that still reaches `limit`.
 template <class T>
-std::vector<PassPlan> plan_passes(uint64_t n, uint64_t limit, int fan, uint64_t start_run = 0) {
+std::vector<PassPlan> plan_passes(uint64_t n, uint64_t limit, int code, uint64_t start_run = 0) {
     std::vector<PassPlan> v;
-    uint64_t run = start_run ? start_run : k1_tile<T>();
+    const int fan = shape_fan(code);
+    uint64_t run = start_run ? start_run : first_run<T>(code);
     while (run < limit) {
         PassPlan p{run, 2, 0, 1};
         if (fan > 2) {
@@ -286,7 +308,7 @@ struct PipeScratch {
         };
         uint64_t bnd_b = 0, rng = 0;
         bool kway = false;
-        for (const PassPlan& p : plan_passes<T>(n, chunk_limit(n, sort_n), shape_fan(code), start_run)) {
+        for (const PassPlan& p : plan_passes<T>(n, chunk_limit(n, sort_n), code, start_run)) {
             if (p.fan <= 2) continue;
             kway = true;
             if (p.rpg > 1) bnd_b = std::max<uint64_t>(bnd_b, p.groups * (uint64_t)(p.rpg + 1) * KWAY_MAX * 8);
@@ -346,7 +368,7 @@ cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint
     if (n == 0) return cudaSuccess;
     const bool full = (sort_n == 0 || sort_n >= n);
     const uint64_t limit = chunk_limit(n, sort_n);
-    const std::vector<PassPlan> plan = plan_passes<T>(n, limit, fan, start_run);
+    const std::vector<PassPlan> plan = plan_passes<T>(n, limit, code, start_run);
     const int passes = (int)plan.size();
     if (start_run && passes == 0) return cudaErrorInvalidValue;
     const int k1_chunk = (int)(limit < (uint64_t)T1 ? (full ? T1 : limit) : T1);
@@ -362,8 +384,13 @@ cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint
     // samples for the first k-way pass: written by the tile sort, or gathered
     // from runs the caller gave (start_run)
     const bool kw_first = passes > 0 && plan[0].fan > 2;
-    K* k1_samp = (kw_first && !start_run) ? sc.samp[0] : nullptr;
-    K* k1_ssamp = (kw_first && !start_run) ? sc.ssamp[0] : nullptr;
+    // The tile sort by buckets: where it leaves the first run, sorts of one tile, and
+    // chunks of one tile that are not too short for a CTA each.
+    const bool by_buckets = !start_run && !(code & SHAPE_HOST_IN) &&
+                            (limit <= (uint64_t)BucketShape<T>::CAP ? limit >= bucket_tile_least<T>() || full
+                                                                    : first_run<T>(code) == BucketShape<T>::CAP);
+    K* k1_samp = (kw_first && !start_run && !by_buckets) ? sc.samp[0] : nullptr;
+    K* k1_ssamp = (kw_first && !start_run && !by_buckets) ? sc.ssamp[0] : nullptr;
 
     // kernel attributes, once per process (thread-safe static initialisation)
     static const bool configured = [] {
@@ -375,6 +402,8 @@ cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint
         } else
             cudaFuncSetAttribute(block_sort_kernel<T, C::K1_NT, C::K1_VTS, C::K1_VTM, C::STABLE>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k1_smem<T>());
+        cudaFuncSetAttribute(bk_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)BucketShape<T>::SORT_SMEM);
         PairMerge1<T>::configure();
         PairMerge2<T>::configure();
         PairMergeI<T>::configure();
@@ -409,7 +438,7 @@ cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint
                 k1_smem<T>());
             return (uint32_t)(sms * (per > 0 ? per : 1));
         }();
-        if (!start_run && tiles1 > wave) {
+        if (!start_run && !by_buckets && tiles1 > wave) {
             cudaPointerAttributes pa;
             if (cudaPointerGetAttributes(&pa, in) != cudaSuccess)
                 cudaGetLastError();  // not a CUDA pointer (pageable host memory): no prefetch
@@ -422,6 +451,12 @@ cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint
     if (!start_run) {
         T* k1_out = written_by(0);
         launch(n_k1.c_str(), st, [&] {
+            if (by_buckets) {
+                const uint32_t tile = (uint32_t)std::min<uint64_t>(limit, BucketShape<T>::CAP);
+                bk_tile_kernel<T><<<(unsigned)((n + tile - 1) / tile), BucketCfg<T>::S_NT, BucketShape<T>::SORT_SMEM, st>>>(
+                    in, k1_out, n, tile, xin, passes == 0 ? xout : 0, err);
+                return;
+            }
             if constexpr (C::WARP_K1) {
                 if (k1_samp)
                     warp_block_sort_kernel<T, C::K1_NW, C::K1_VT, C::K1_NWT, C::K1_MINB, true, C::K1_RUN0>
@@ -475,7 +510,7 @@ cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint
             const bool more = pi + 1 < passes && plan[pi + 1].fan > 2;
             K* s_out = more ? sc.samp[(pi + 1) & 1] : nullptr;
             K* ss_out = more ? sc.ssamp[(pi + 1) & 1] : nullptr;
-            if (pi == 0 && start_run) {
+            if (pi == 0 && (start_run || by_buckets)) {
                 const uint64_t ns = n / S;
                 const unsigned gb = (unsigned)std::min<uint64_t>((ns + 255) / 256 + 1, 152ull * 16);
                 launch(n_kg.c_str(), st, [&] { kb_gather_samples_kernel<T><<<gb, 256, 0, st>>>(cur, n, s_in, ss_in); });

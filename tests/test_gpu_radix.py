@@ -195,3 +195,15 @@ def test_tuning_selects_radix_or_merges(tmp_path):
         assert not launched()
     finally:
         og.tuning_set(og.U32, n, *prev)
+
+
+# the first kernel of the merge sorts: its tiles (4096 64-bit items), chunks of one tile,
+# sorts of one tile, and the k-way passes that sample its runs
+@pytest.mark.parametrize("dist", ["uniform", "equal", "zipf", "log", "sorted"])
+@pytest.mark.parametrize("kind", [og.U32, og.U64, og.I64, og.KV64, og.KVU64])
+@pytest.mark.parametrize("min_k", [2, 16])
+def test_merge_tiles(kind, dist, min_k):
+    for n, sort_n in ((1, 0), (17, 0), (4096, 0), (6145, 0), (8193, 0), (70_001, 0), (300_007, 0), (50_001, 256),
+                      (50_001, 512), (50_001, 2048), (50_001, 4096), (50_001, 8192)):
+        a = items(kind, dist, n, seed=n)
+        assert np.array_equal(device_sort(a, kind, min_k=min_k, sort_n=sort_n), expected(a, sort_n)), (n, sort_n)
