@@ -9,19 +9,22 @@
 //   bk_sample_kernel  samples the keys of a segment, chooses the range that is
 //                     cut into 2^(b1+b2) equal slices, and sees whether a slice
 //                     is far too full
-//   bk_hist_kernel    counts a level's slices, one read
-//   bk_scan_kernel    slice starts; bucket sizes against what the last kernel
-//                     can take; the next level's tiles (the first level of one
-//                     segment: the last CTA of bk_hist_kernel)
+//   bk_hist_all_kernel, bk_sum_kernel, bk_list_kernel
+//                     one segment of two levels: counts both levels' slices with one
+//                     read; bucket sizes against what the last kernel can take; slice
+//                     starts and the second level's tiles
+//   bk_hist_kernel    else: counts a level's slices, one read
+//   bk_scan_kernel    the same as sum and list, for one level (the first level of one
+//                     segment: by the last CTA of bk_hist_kernel)
 //   bk_pass_kernel    one partition level for keys, one read and one write
 //   radix_pass_kernel the same for pairs, whose order has to be kept
 //   bk_sort_kernel    one bucket per CTA, sorted in shared memory (64-bit keys:
 //                     sb_sort_kernel, seg_buckets.cuh)
 //
-// Measured (one GB300): 2^28 uint32 keys 3.79 ms by radix passes, 2.84 by buckets
-// (counting 2 x 0.20, partition 2 x 0.60, buckets 1.2); 2^27 uint64 keys 5.17 and
-// 2.21 (2 x 0.20, 2 x 0.47, 0.82); 2^27 pairs 8.47 and 4.27 (2 x 0.35, 2 x 1.08,
-// 1.38). A plain copy takes 0.32, 0.32 and 0.64 ms.
+// Measured (one GB300): 2^28 uint32 keys 7.38 ms by merges, 3.79 by eight-bit radix
+// passes, 2.63 by buckets (counting 0.22, partition 2 x 0.60, buckets 1.20); 2^27 uint64
+// keys 8.44, 5.17 and 2.02 (0.20, 2 x 0.47, 0.85); 2^27 pairs 14.0, 8.47 and 3.88 (0.33,
+// 2 x 1.07, 1.38). A plain copy takes 0.32, 0.32 and 0.64 ms.
 //
 // A slice is a monotone function of the key (keys outside the sampled range
 // fall into the end slices), so any data is sorted correctly as long as every
@@ -345,7 +348,7 @@ __global__ void __launch_bounds__(RADIX_BINS)
     bk_scan_kernel(const uint32_t* hist, int bits, const uint32_t* seg_start, uint64_t len, BkScan to) {
     const uint32_t seg = blockIdx.x;
     grid_dep_wait();
-    if (route_load(to.route) != ROUTE_BUCKETS) return;
+    if (__syncthreads_or(route_load(to.route) != ROUTE_BUCKETS)) return;  // (a CTA of this kernel may set it)
     const uint32_t h = threadIdx.x < (1u << bits) ? hist[((size_t)seg << bits) + threadIdx.x] : 0;
     bk_scan_segment<T>(to, seg, seg_start ? seg_start[seg] : (uint32_t)(seg * len), bits, h);
 }
@@ -423,6 +426,168 @@ __global__ void __launch_bounds__(512) bk_hist_kernel(const T* in, G geo, uint32
     if (last) {
         __threadfence();
         bk_scan_segment<T>(to, 0, 0, bits, tid < nb ? look_load(hist + tid) : 0u);
+    }
+}
+
+// ------------------------------------------------- both levels of a segment ---
+// Counts the slices of both levels with one read: up to 65536 counters of 16 bits in
+// shared memory, one CTA per SM, its counts to a row of its own. A counter that passes
+// CAP makes the sort give up, and so none can run over in a sort that goes on. Where the
+// 32 keys of a step share a slice (sorted input) one lane counts for all. 2^28 uint32
+// keys: two reads 0.43 ms, this one 0.22 (atomics; the read alone 0.16), 2^27 uint64
+// 0.44 and 0.20, 2^27 pairs 0.73 and 0.33.
+template <class T>
+__global__ void __launch_bounds__(1024)
+    bk_hist_all_kernel(const T* in, uint64_t n, const SliceMap<typename Traits<T>::Key>* maps, uint64_t xmask, int bits,
+                       uint32_t* rows, int* route) {
+    constexpr int NT = 1024, V = Vec<T>::N, TILE = BucketShape<T>::TILE, STEPS = TILE / V / NT;
+    constexpr uint32_t CAP = BucketShape<T>::CAP;
+    static_assert(STEPS * V * NT == TILE, "whole vector steps");
+    extern __shared__ __align__(16) uint32_t half[];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t words = 1u << (bits - 1);
+    for (uint32_t i = tid; i < words; i += NT) half[i] = 0;
+    grid_dep_wait();
+    if (__syncthreads_or(route_load(route) != ROUTE_BUCKETS)) return;  // (a CTA of this kernel may set it)
+    const SliceMap<typename Traits<T>::Key> map = maps[0];
+    __syncthreads();
+    bool over = false;
+    auto slice = [&](const T& v) -> uint32_t { return __umulhi(map.scaled(Traits<T>::key(bk_flip(v, xmask))), map.mul); };
+    auto add_to = [&](uint32_t s, uint32_t add) {
+        const uint32_t sh = (s & 1u) * 16u;
+        over |= ((atomicAdd(&half[s >> 1], add << sh) >> sh) & 0xFFFFu) >= CAP;
+    };
+    auto count = [&](const T& v, bool in) {
+        const uint32_t s = slice(v);
+        const uint32_t s0 = __shfl_sync(0xFFFFFFFFu, s, 0);
+        uint32_t add = in ? 1u : 0u;
+        if (__all_sync(0xFFFFFFFFu, in && s == s0)) add = lane == 0 ? 32u : 0u;
+        if (add) add_to(s, add);
+    };
+    const uint64_t tiles = (n + TILE - 1) / TILE;
+    const uint64_t t0 = tiles * blockIdx.x / gridDim.x, t1 = tiles * (blockIdx.x + 1) / gridDim.x;
+    uint4 x[STEPS];
+    auto fetch = [&](uint64_t t) {
+        if ((t + 1) * TILE <= n) {
+#pragma unroll
+            for (int j = 0; j < STEPS; ++j) x[j] = reinterpret_cast<const uint4*>(in + t * TILE)[j * NT + tid];
+        }
+    };
+    fetch(t0);
+    for (uint64_t t = t0; t < t1; ++t) {
+        if ((t + 1) * TILE <= n) {
+            uint4 y[STEPS];
+#pragma unroll
+            for (int j = 0; j < STEPS; ++j) y[j] = x[j];
+            if (t + 1 < t1) fetch(t + 1);
+            // (a warp whose first keys share a slice looks for such steps)
+            const uint32_t s = slice(*reinterpret_cast<const T*>(&y[0]));
+            const bool plain = !__all_sync(0xFFFFFFFFu, s == __shfl_sync(0xFFFFFFFFu, s, 0));
+#pragma unroll
+            for (int j = 0; j < STEPS; ++j) {
+                const T* e = reinterpret_cast<const T*>(&y[j]);
+                if (plain) {
+#pragma unroll
+                    for (int q = 0; q < V; ++q) add_to(slice(e[q]), 1u);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < V; ++q) count(e[q], true);
+                }
+            }
+        } else {
+            for (uint64_t i = t * TILE; i < n; i += NT) count(in[i + tid < n ? i + tid : n - 1], i + tid < n);
+        }
+    }
+    if (__syncthreads_or(over) && tid == 0) *route = ROUTE_RADIX;
+    for (uint32_t i = tid; i < words; i += NT) rows[(size_t)blockIdx.x * words + i] = half[i];
+}
+
+// Sums the rows: one CTA per first-level slice (256 threads, up to 128 words). hist2: the
+// second level's counts; hist1: the first level's.
+template <class T>
+__global__ void __launch_bounds__(256)
+    bk_sum_kernel(const uint32_t* rows, uint32_t nrows, int b1, int b2, uint32_t* hist1, uint32_t* hist2, int* route) {
+    __shared__ uint32_t lo2[128], hi2[128], total;
+    const int tid = threadIdx.x, w = tid & 127, part = tid >> 7, nw = 1 << (b2 - 1);
+    if (tid == 0) total = 0;
+    grid_dep_wait();
+    if (__syncthreads_or(route_load(route) != ROUTE_BUCKETS)) return;  // (a CTA of this kernel may set it)
+    const size_t words = (size_t)1 << (b1 + b2 - 1);
+    const uint32_t* p = rows + ((size_t)blockIdx.x << (b2 - 1)) + w;
+    uint32_t lo = 0, hi = 0;
+    if (w < nw) {
+#pragma unroll 8
+        for (uint32_t r = part; r < nrows; r += 2) {
+            const uint32_t x = p[r * words];
+            lo += x & 0xFFFFu;
+            hi += x >> 16;
+        }
+    }
+    if (part) {
+        lo2[w] = lo;
+        hi2[w] = hi;
+    }
+    __syncthreads();
+    uint32_t sum = 0;
+    bool over = false;
+    if (!part && w < nw) {
+        lo += lo2[w];
+        hi += hi2[w];
+        sum = lo + hi;
+        over = lo > (uint32_t)BucketShape<T>::CAP || hi > (uint32_t)BucketShape<T>::CAP;
+        reinterpret_cast<uint2*>(hist2 + ((size_t)blockIdx.x << b2))[w] = make_uint2(lo, hi);
+    }
+    sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+    if ((tid & 31) == 0 && sum) atomicAdd(&total, sum);
+    if (__syncthreads_or(over) && tid == 0) *route = ROUTE_RADIX;
+    if (tid == 0) hist1[blockIdx.x] = total;
+}
+
+// Starts, cursors and the second level's tiles: one CTA per first-level slice.
+template <class T>
+__global__ void __launch_bounds__(256)
+    bk_list_kernel(uint64_t n, int b1, int b2, const uint32_t* hist1, const uint32_t* hist2, uint32_t* start1,
+                   uint32_t* cursor1, uint32_t* start2, uint32_t* cursor2, BkTile* tiles2, uint32_t* count2,
+                   const int* route) {
+    constexpr uint32_t TILE = BucketShape<T>::TILE;
+    __shared__ uint32_t ws[RADIX_BINS / 32], ws2[RADIX_BINS / 32], ws3[RADIX_BINS / 32], mine[3];
+    const int tid = threadIdx.x, n1 = 1 << b1, n2 = 1 << b2;
+    const uint32_t seg = blockIdx.x;
+    grid_dep_wait();
+    if (route_load(route) != ROUTE_BUCKETS) return;
+    const uint32_t h1 = tid < n1 ? hist1[tid] : 0, nt = (h1 + TILE - 1) / TILE;
+    const uint32_t s1 = radix_bin_scan<uint32_t>(h1, ws), t1 = radix_bin_scan<uint32_t>(nt, ws2);
+    if (tid == (int)seg) {
+        mine[0] = s1;
+        mine[1] = h1;
+        mine[2] = t1;
+    }
+    if (seg == 0 && tid < n1) {
+        start1[tid] = s1;
+        if (cursor1) cursor1[tid] = s1;
+        if (tid == n1 - 1) {
+            start1[n1] = (uint32_t)n;
+            *count2 = t1 + nt;
+        }
+    }
+    const uint32_t h2 = tid < n2 ? hist2[((size_t)seg << b2) + tid] : 0;
+    const uint32_t r2 = radix_bin_scan<uint32_t>(h2, ws3);
+    __syncthreads();
+    const uint32_t base = mine[0], len = mine[1], at = mine[2];
+    if (tid < n2) {
+        start2[((size_t)seg << b2) + tid] = base + r2;
+        if (cursor2) cursor2[((size_t)seg << b2) + tid] = base + r2;
+        if (seg == (uint32_t)n1 - 1 && tid == n2 - 1) start2[(size_t)n1 << b2] = (uint32_t)n;
+    }
+    for (uint32_t i = tid; i * TILE < len; i += 256) {
+        BkTile r;
+        r.sbase = base;
+        r.base = (uint64_t)base + (uint64_t)i * TILE;
+        r.slen = len;
+        r.seg = seg;
+        r.ti = i;
+        r.cnt = len - i * TILE < TILE ? len - i * TILE : TILE;
+        tiles2[at + i] = r;
     }
 }
 

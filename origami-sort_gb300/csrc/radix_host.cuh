@@ -64,6 +64,11 @@ struct BucketPlan {
         nbuckets = p.nseg << bits;
     }
     bool on() const { return b1 > 0; }
+    // rows of counts where one read counts both levels (one segment): one for every SM,
+    // and four tiles each
+    uint32_t rows(const RadixPlan<T>& p) const {
+        return b2 && p.nseg == 1 ? (uint32_t)std::min<uint64_t>(152, (tiles + 3) / 4) : 0u;
+    }
 };
 
 // What stands behind the bucket sort, and sorts where it does not take the call. Radix
@@ -100,6 +105,7 @@ struct RadixScratch {
     void* look[2] = {nullptr, nullptr};
     uint32_t *start1 = nullptr, *start2 = nullptr, *cursor1 = nullptr, *cursor2 = nullptr, *count2 = nullptr, *done = nullptr;
     SliceMap<K>* maps = nullptr;
+    uint32_t* rows = nullptr;
     BkTile* tiles2 = nullptr;
     uint32_t *hist1 = nullptr, *hist2 = nullptr;
     void* hist = nullptr;
@@ -125,6 +131,7 @@ struct RadixScratch {
                 start2 = words(bk.nbuckets + 1);
                 if (!ST) cursor2 = words(bk.nbuckets);
                 tiles2 = reinterpret_cast<BkTile*>(take(bk.tiles2 * sizeof(BkTile)));
+                rows = words((uint64_t)bk.rows(p) << (bk.b1 + bk.b2 - 1));
             }
         }
         // the second level's words: the first pass clears those of its own tiles
@@ -235,17 +242,41 @@ void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPla
                                                                             (uint64_t)Sh::CAP, sc.maps, sc.route,
                                                                             reinterpret_cast<uint4*>(sc.zero), nzero);
     });
+    const uint32_t nrows = bk.rows(p);
+    if (nrows) {
+        static const std::string n_all = std::string("bucket_hist_all<") + TypeName<T>::v + ">";
+        static const std::string n_sum = std::string("bucket_sum<") + TypeName<T>::v + ">";
+        static const std::string n_list = std::string("bucket_list<") + TypeName<T>::v + ">";
+        static const bool configured = [] {
+            cudaFuncSetAttribute(bk_hist_all_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 << BK_MAX_BITS);
+            return true;
+        }();
+        (void)configured;
+        launch(n_all.c_str(), st, [&] {
+            launch_dependent(bk_hist_all_kernel<T>, dim3(nrows), dim3(1024), (size_t)2 << bits, st, (const T*)d, p.n,
+                             (const SliceMap<K>*)sc.maps, xmask, bits, sc.rows, sc.route);
+        });
+        launch(n_sum.c_str(), st, [&] {
+            launch_dependent(bk_sum_kernel<T>, dim3(1u << bk.b1), dim3(256), 0, st, (const uint32_t*)sc.rows, nrows, bk.b1,
+                             bk.b2, sc.hist1, sc.hist2, sc.route);
+        });
+        launch(n_list.c_str(), st, [&] {
+            launch_dependent(bk_list_kernel<T>, dim3(1u << bk.b1), dim3(256), 0, st, p.n, bk.b1, bk.b2,
+                             (const uint32_t*)sc.hist1, (const uint32_t*)sc.hist2, sc.start1, sc.cursor1, sc.start2,
+                             sc.cursor2, sc.tiles2, sc.count2, (const int*)sc.route);
+        });
+    }
     auto level = [&](auto geo_l, const T* src, T* dst, uint32_t tiles_l, int shift_l, int bits_l, uint32_t map_shift,
                      uint32_t segs, const uint32_t* seg_start, uint32_t* hist, uint32_t* start, uint32_t* cursor,
                      bool last, int full_route, void* look, void* look_next, unsigned* claim) {
         using G = decltype(geo_l);
         const BkScan to{start, cursor, last ? (BkTile*)nullptr : sc.tiles2, sc.count2, sc.route, full_route, p.n, segs - 1};
-        launch(n_hist.c_str(), st, [&] {
+        if (!nrows) launch(n_hist.c_str(), st, [&] {
             launch_dependent(bk_hist_kernel<T, G>, dim3(std::min(tiles_l, g_hist)), dim3(512), 0, st, src, geo_l, tiles_l,
                              (const SliceMap<K>*)sc.maps, map_shift, xmask, shift_l, bits_l, hist,
                              (const int*)sc.route, to, segs == 1 ? sc.done : (uint32_t*)nullptr);
         });
-        if (segs > 1) launch(n_scan.c_str(), st, [&] {
+        if (!nrows && segs > 1) launch(n_scan.c_str(), st, [&] {
             launch_dependent(bk_scan_kernel<T>, dim3(segs), dim3(RADIX_BINS), 0, st, (const uint32_t*)hist, bits_l,
                              seg_start, p.len, to);
         });
