@@ -15,7 +15,7 @@ template <class T>
 struct SegBucketPlan {
     using Sh = SegBucketShape<T>;
     uint64_t n, nseg, segs, tiles, recs;
-    int levels;
+    int levels, usual;  // usual: what segments of the mean length need
     bool wide;  // 64-bit counts
     SegBucketPlan(uint64_t n_, uint64_t nseg_, uint64_t longest) : n(n_), nseg(nseg_) {
         // levels that 256 slices each need to cut the longest segment into buckets
@@ -23,6 +23,9 @@ struct SegBucketPlan {
         levels = 1;
         for (uint64_t m = (uint64_t)Sh::CAP * 4 / 5 * RADIX_BINS; m < longest && levels < SB_MAX_LEVELS; m *= RADIX_BINS) ++levels;
         levels = longest > (uint64_t)Sh::CAP ? std::min(levels + 1, SB_MAX_LEVELS) : 0;
+        usual = 0;
+        for (uint64_t m = (uint64_t)Sh::CAP * 4 / 5; m < n / std::max<uint64_t>(nseg, 1); m *= RADIX_BINS) ++usual;
+        usual = std::max(usual, 1);
         // a level's segments are longer than a bucket
         segs = n / (Sh::CAP + 1) + 1;
         tiles = n / Sh::TILE + segs;
@@ -111,7 +114,10 @@ struct SegBucketGrids {
 };
 
 // The levels and the bucket pass. given.nseg: behind a bucket sort that rarely gives up,
-// where no level's grid is larger than resident; else for the segments in the first list.
+// where no level's grid is larger than resident; else for the segments in the first list,
+// one CTA per tile on the levels that segments of the mean length need, a resident grid
+// on those that few may (415M uint32 keys in 4096 segments: 0.33 ms of CTAs that found
+// nothing to do).
 template <class T, class S>
 void segbucket_levels(const SbBuffers<T>& buf, const SbGiven& given, const SbStarts& plain, const SegBucketPlan<T>& p,
                       uint64_t xin, uint64_t xout, const SegBucketScratch<T>& sc, cudaStream_t st) {
@@ -157,7 +163,7 @@ void segbucket_levels(const SbBuffers<T>& buf, const SbGiven& given, const SbSta
                                  (const SbMap<K>*)sc.maps, (const K*)sc.splitters, xin, (const S*)hist,
                                  static_cast<S*>(sc.look), &cn->claim[l], &cn->err, wait_limit());
             } else {
-                const bool loop = behind || (l > 0 && l + 1 == p.levels);
+                const bool loop = behind || l >= p.usual;
                 launch_dependent(loop ? sb_pass_kernel<T, S, true> : sb_pass_kernel<T, S, false>,
                                  dim3(loop ? std::min(tiles, g.pass) : tiles), dim3(C::NT), Sh::PASS_SMEM, st, buf, l,
                                  (const SbTile*)sc.tiles, (const uint32_t*)&cn->tiles[l], (const SbMap<K>*)sc.maps,
