@@ -507,9 +507,11 @@ bool is_pinned(const void* p) {
 }
 
 // Host buffers the device can address (view pointers vin / vout).
-//  * Small sorts, fan-in > 2, or chunk sizes of at most one chunk: one
-//    pipeline whose first kernel reads the host input and whose last pass
-//    writes the host output, with the passes in between in two arena buffers.
+//  * Sorts of one bucket: one launch that reads and writes the host buffers.
+//  * Other small sorts: copied in, sorted by buckets, copied out; where the
+//    buckets do not take them, one pipeline whose first kernel reads the host
+//    input and whose last pass writes the host output, with the passes in
+//    between in two arena buffers.
 //  * Large sorts: the input is cut into chunks of chunk_n (a power of two of
 //    at least 2^22 items; 4 to 16 chunks, more than 8 above 2^26 items). Each
 //    chunk lands in HBM (a copy-engine transfer for pinned memory, a copy
@@ -630,8 +632,8 @@ struct HostPipePlan {
     bool slice_copies = false;
     uint64_t chunk_n = 0;
     int fan = 0, cfan = 0, mfan = 0;
-    // chunks sort by the radix path with this pass shape code (0: by merges); a chunk
-    // shorter than RADIX_CHUNK merges
+    // chunks (or the whole of a sort that is not chunked) sort by the radix path with this
+    // pass shape code (0: by merges); a chunk shorter than RADIX_CHUNK merges
     int radix = 0;
     // host input of chunks that merge: the first chunk lands in this many pieces,
     // each sorted as it lands, then merged into the chunk's run by one k-way pass
@@ -640,6 +642,13 @@ struct HostPipePlan {
 };
 
 uint64_t a256(uint64_t b) { return (b + 255) & ~255ull; }
+
+// Sorts that are not chunked land in device memory, sort by the radix path and are copied
+// out from this size on; below it the merges, whose first kernel reads the host buffer and
+// whose last pass writes it. (Per call, merges and this, us:
+// 16,384 uint64 keys 55 and 44, 65,536 uint32 65 and 46, 2^20 uint32 151 and 95, uint64 233
+// and 162, pairs 350 and 262, Zipf pairs 336 and 311; 65,536 Zipf pairs 94 and 97.)
+constexpr uint64_t HOST_LAND = 1 << 14;
 
 // merges: chunks do not sort by the radix path (its scratch could not be had).
 HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_k, bool merges = false) {
@@ -658,6 +667,13 @@ HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_
     while (p.chunk_n * 16 < n) p.chunk_n <<= 1;
     p.chunked = n >= 4 * p.chunk_n && limit > p.chunk_n;
     p.data = a256(n * item_bytes(kind));
+    const int code = shape_for(kind, p.chunked ? p.chunk_n : n, min_k);
+    if (!p.chunked && min_k == 0 && !merges && n >= HOST_LAND && radix_takes(kind, n, sort_n, code)) {
+        p.radix = code;
+        p.ws = a256(scratch_bytes(kind, n, sort_n, code));
+        p.total = 2 * p.data + p.ws;
+        return p;
+    }
     if (!p.chunked) {
         p.fan |= SHAPE_HOST_IN;
         p.ws = a256(typed_scratch_io(kind, n, sort_n, p.fan, 0));
@@ -678,7 +694,6 @@ HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_
     p.first_pieces = shape_fan(p.cfan) >= 4 ? 4 : 1;
     p.ws = a256(std::max(typed_scratch_io(kind, p.chunk_n, 0, p.cfan, 0),
                          typed_scratch_io(kind, p.chunk_n, 0, p.cfan, p.chunk_n / p.first_pieces)));
-    const int code = shape_for(kind, p.chunk_n, min_k);
     if (min_k == 0 && !merges && radix_takes(kind, p.chunk_n, 0, code)) {
         // the chunk sorts keep up with the link (2^22 uint32 keys 0.10 ms, their
         // transfer 0.08; Zipf keys 0.20). Per call from pinned memory, chunks by merges
@@ -708,8 +723,9 @@ HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_
 // are in flight; the merge across chunks follows as one k-way pass that
 // writes the host output (or, with plan.slice_copies and pinned output, is
 // cut into output slices copied to the host while the next slices merge).
-// Small sorts run one pipeline whose first kernel reads the input and whose
-// last pass writes the output.
+// Other sorts land whole, sort by buckets and are copied out; where those do not
+// take them, one pipeline's first kernel reads the input and its last pass writes
+// the output.
 int host_pipe_run(int kind, void* host_in, void* host_out, const void* vin, void* vout, uint64_t n, uint64_t sort_n,
                   const HostPipePlan& p, void* block, cudaStream_t st) {
     const uint64_t ib = item_bytes(kind);
@@ -721,7 +737,22 @@ int host_pipe_run(int kind, void* host_in, void* host_out, const void* vin, void
     ErrWatch watch;  // every sort's error word, read after the final sync
     cudaError_t e = cudaSuccess;
     std::vector<cudaEvent_t> evs;
-    if (!p.chunked) {
+    auto land = [&](char* dst, uint64_t off_items, uint64_t items, cudaStream_t s) -> cudaError_t {
+        if (is_pinned(host_in))
+            return cudaMemcpyAsync(dst, static_cast<const char*>(host_in) + off_items * ib, items * ib,
+                                   cudaMemcpyHostToDevice, s);
+        return link_copy(static_cast<const char*>(vin) + off_items * ib, dst, items * ib, s);
+    };
+    if (!p.chunked && p.radix) {
+        // in, sort, out
+        char* w = b + p.data;
+        e = land(a, 0, n, st);
+        if (e == cudaSuccess) e = run_typed(kind, a, b, n, sort_n, a, p.radix, w, st);
+        if (e == cudaSuccess) e = watch.watch(w + scratch_bytes(kind, n, sort_n, p.radix) - 256, st);
+        if (e == cudaSuccess)
+            e = is_pinned(host_out) ? cudaMemcpyAsync(host_out, a, n * ib, cudaMemcpyDeviceToHost, st)
+                                    : link_copy(a, vout, n * ib, st);
+    } else if (!p.chunked) {
         void* w = b + p.data;
         e = typed_io(kind, vin, vout, a, b, n, sort_n, m, m, 0, p.fan, w, st);
         if (e == cudaSuccess)
@@ -742,12 +773,6 @@ int host_pipe_run(int kind, void* host_in, void* host_out, const void* vin, void
         cudaStream_t lanes[HOST_LANES - 1] = {st};
         for (int i = 1; i < HOST_LANES - 1; ++i) lanes[i] = aux_stream(i - 1);
         cudaStream_t sc = aux_stream(HOST_LANES - 1);
-        auto land = [&](char* dst, uint64_t off_items, uint64_t items) -> cudaError_t {
-            if (pinned_in)
-                return cudaMemcpyAsync(dst, static_cast<const char*>(host_in) + off_items * ib, items * ib,
-                                       cudaMemcpyHostToDevice, sc);
-            return link_copy(static_cast<const char*>(vin) + off_items * ib, dst, items * ib, sc);
-        };
         auto event_on = [&](cudaStream_t s) {
             cudaEvent_t ev;
             cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
@@ -770,7 +795,7 @@ int host_pipe_run(int kind, void* host_in, void* host_out, const void* vin, void
                 for (int q = 0; q < np && e == cudaSuccess; ++q) {
                     char* pa = a + q * pn * ib;
                     char* pb = b + q * pn * ib;
-                    e = land(pa, q * pn, pn);
+                    e = land(pa, q * pn, pn, sc);
                     cudaStreamWaitEvent(lanes[q], event_on(sc), 0);
                     if (e == cudaSuccess) e = typed_io(kind, pa, pb, pa, pb, pn, 0, m, 0, 0, p.cfan, w[q], lanes[q]);
                     if (e == cudaSuccess) e = watch.watch(w[q] + typed_scratch_io(kind, pn, 0, p.cfan, 0) - 256, lanes[q]);
@@ -782,7 +807,7 @@ int host_pipe_run(int kind, void* host_in, void* host_out, const void* vin, void
                 continue;
             }
             if (!device_in) {
-                e = land(a + off * ib, off, cn);
+                e = land(a + off * ib, off, cn, sc);
                 cudaStreamWaitEvent(cst, event_on(sc), 0);
                 src = a + off * ib;
             }
@@ -835,6 +860,13 @@ int host_pipe_run(int kind, void* host_in, void* host_out, const void* vin, void
 
 int sort_host_direct(int kind, void* host_in, void* host_out, const void* vin, void* vout, uint64_t n,
                      uint64_t sort_n, unsigned min_k, cudaStream_t st) {
+    if (min_k == 0 && one_bucket(kind, n, sort_n) && (shape_for(kind, n, 0) & SHAPE_RADIX)) {
+        // one launch that reads and writes the host buffers (1000 uint32 keys: 38 us
+        // a call by the merges' first kernel, 15 so)
+        CK(run_one_bucket(kind, vin, vout, n, st), "sort launch");
+        CK(cudaStreamSynchronize(st), "stream sync");
+        return ORIGAMI_OK;
+    }
     HostPipePlan p = host_pipe_plan(kind, n, sort_n, min_k);
     void* block = nullptr;
     cudaError_t e = cudaMallocAsync(&block, p.total, st);

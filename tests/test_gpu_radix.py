@@ -207,3 +207,19 @@ def test_merge_tiles(kind, dist, min_k):
                       (50_001, 512), (50_001, 2048), (50_001, 4096), (50_001, 8192)):
         a = items(kind, dist, n, seed=n)
         assert np.array_equal(device_sort(a, kind, min_k=min_k, sort_n=sort_n), expected(a, sort_n)), (n, sort_n)
+
+
+# host sorts of one bucket, and those that land in device memory: sizes around both
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("dist", ["uniform", "zipf", "equal", "log"])
+@pytest.mark.parametrize("kind", [og.U32, og.U64, og.I64, og.KV64, og.KVU64])
+def test_host_sizes(kind, dist, pinned):
+    for n in (2, 1000, 4096, 4097, 6144, 6145, 16383, 16384, 32768, 70_001, (1 << 20) + 5):
+        a = items(kind, dist, n, seed=n)
+        d, out = og.empty_host(kind, n, pinned=pinned), og.empty_host(kind, n, pinned=pinned)
+        d[:] = a
+        assert og.sort(d, out, result_in_tmp=True) is out
+        assert np.array_equal(out, expected(a)), n
+        assert np.array_equal(d, a)  # (the input is only read)
+        assert og.sort(d) is d
+        assert np.array_equal(d, expected(a)), n
