@@ -434,7 +434,7 @@ def main():
     bytes_per_launch = 2 * n * item
     achieved = bytes_per_launch / (per_launch_ms / 1e3) / 1e9
     passes = sum(c for name, (c, _) in report.items()
-                 if name.startswith(("block_sort", "pair_merge", "kway_merge"))) // args.steps
+                 if name.startswith(("block_sort", "pair_merge", "kway_merge", "bucket_pass", "bucket_sort"))) // args.steps
     ms_step = total_ms / args.steps
     # DRAM bytes per launch need an ncu capture, which this run does not make
     traffic = None

@@ -80,8 +80,8 @@ unsigned origami_item_bytes(int kind);
  *            Otherwise it must be a power of two.
  *   min_k    merge fan-in of each HBM pass (the reference's min_k, sorter.h:3875):
  *            2 = binary merge passes, 4/8/16 = k-way passes. 0 picks the tuned
- *            way to sort: from some size on radix passes (device buffers), else
- *            the tuned merge fan-in. The output is the same in every case.
+ *            way to sort: by buckets (nearly every size), else the tuned merge
+ *            fan-in. The output is the same in every case.
  *   result   receives d or tmp.
  * The call returns after the result is in place (host) or is enqueued on the
  * default stream (device pointers; add ORIGAMI_FLAG_SYNC to wait).
@@ -343,17 +343,18 @@ int origami_generate_device(int kind, void* d, uint64_t n, int dist, uint64_t se
  * sizes about as large as L2, other binary shapes for others; binary passes
  * with shape 0 elsewhere). min_k = 2 keeps the table's merge shape with
  * binary passes; larger min_k forces that fan-in. Beside its merge shape an
- * entry says whether the class sorts by radix passes (the built-in choice for
- * larger classes); device sorts with min_k = 0 then do, where the chunk size
+ * entry says whether the class sorts by buckets, with radix passes behind them
+ * for keys that are too uneven (called "radix" below; the built-in choice of all
+ * but a few small classes); sorts with min_k = 0 then do, where the chunk size
  * allows it, and fall back to the merge shape when their scratch cannot be
  * allocated.
- *   origami_autotune   times every shape and the radix passes on n generated
+ *   origami_autotune   times every shape and the buckets on n generated
  *                      device items and stores the fastest for n's size class;
  *                      `report` (may be NULL) receives one "fan= variant= ms="
  *                      line per shape and one "radix ms=" line.
  *   get / set          read or write one entry's merge shape. Setting the
  *                      class's built-in shape restores its built-in choice,
- *                      radix passes included; any other selects merge passes.
+ *                      buckets included; any other selects merge passes.
  *   save / load        the entries other than binary passes with shape 0 as
  *                      "kind class fan variant"
  *                      lines, radix choices that differ from the built-in ones

@@ -79,7 +79,7 @@ uint32_t wait_limit() { return g_wait_limit.load(std::memory_order_relaxed); }
 // 2^16 / 2^18 / 2^20 / 2^21 keys take 2.15 / 2.07 / 2.01 / 2.77 ms by buckets, 2.92 /
 // 3.66 / 4.41 / 4.78 by merge passes; shorter chunks have too few buckets.
 constexpr uint64_t RADIX_CHUNK = 1 << 16;
-// Whether the radix path (bucket sort, radix passes behind it) sorts n items in
+// Whether the radix path (bucket sort, radix passes or levels behind it) sorts n items in
 // chunks of sort_n under this shape code: the size class asks for it, the
 // geometry fits, and the chunks are long enough. Its cost hardly depends on the
 // chunk size, a merge sort's is one level less for every halving.
@@ -286,7 +286,7 @@ int size_class(uint64_t n) {
 void tune_init();
 
 // Pass shape code for a sort of n items: min_k = 0 takes the table's choice
-// (radix passes included), min_k <= 2 binary passes with the table's tile shape,
+// (the radix path included), min_k <= 2 binary passes with the table's tile shape,
 // larger min_k k-way.
 int shape_for(int kind, uint64_t n, unsigned min_k) {
     std::call_once(g_tune_once, tune_init);
@@ -886,7 +886,7 @@ void tune_store(int kind, int cls, int code);
 
 // Tuning file: one entry per line. "kind class fan variant": the plain sort's
 // merge shape for a size class; "radix kind class on": whether the class sorts
-// by radix passes, after its shape line; "seg kind class shape": the segmented
+// by the radix path, after its shape line; "seg kind class shape": the segmented
 // sort's merge shape for a class of mean segment length; "segbuckets kind class
 // on": whether it sorts by buckets, after its shape line. Other lines are skipped.
 int tune_load_file(const char* path) {
@@ -953,8 +953,8 @@ constexpr TuneDefault kTuneDefaults[] = {
     {ORIGAMI_KV64, 25, 2, 1},  {ORIGAMI_KV64, 26, 2, 1},   {ORIGAMI_KV64, 27, 2, 1},   {ORIGAMI_KV64, 28, 2, 1},
 };
 
-// Built-in choice of a size class: the merge shape above, and radix passes from
-// the class on where they were faster (RADIX_FROM below).
+// Built-in choice of a size class: the merge shape above, and the radix path (buckets)
+// where it was faster (RADIX_ONE, RADIX_FROM above).
 int tune_builtin(int kind, int cls) {
     const int k = kind == ORIGAMI_I64 ? ORIGAMI_U64 : (kind == ORIGAMI_KVU64 ? ORIGAMI_KV64 : kind);
     int code = shape_code(2, 0);
@@ -965,7 +965,7 @@ int tune_builtin(int kind, int cls) {
 }
 
 // Sets a class to a merge shape. The class's own built-in shape restores its
-// built-in choice (radix passes included); any other shape selects merge passes.
+// built-in choice (the radix path included); any other shape selects merge passes.
 void tune_store(int kind, int cls, int code) {
     const int b = tune_builtin(kind, cls);
     g_tune[kind][cls].store(code == (b & ~SHAPE_RADIX) ? b : code, std::memory_order_relaxed);
