@@ -651,7 +651,10 @@ uint64_t a256(uint64_t b) { return (b + 255) & ~255ull; }
 constexpr uint64_t HOST_LAND = 1 << 14;
 
 // merges: chunks do not sort by the radix path (its scratch could not be had).
-HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_k, bool merges = false) {
+// beside: other batches run beside the sort (the serving loop); chunks that merge take
+// binary passes, whose launches interleave with theirs.
+HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_k, bool merges = false,
+                            bool beside = false) {
     HostPipePlan p;
     const uint64_t limit = (sort_n == 0 || sort_n >= n) ? n : sort_n;
     p.fan = shape_for(kind, n, min_k) & ~SHAPE_RADIX;
@@ -686,7 +689,7 @@ HostPipePlan host_pipe_plan(int kind, uint64_t n, uint64_t sort_n, unsigned min_
     // from the different streams interleave, 14.46 with the persistent binary
     // kernel and 14.27 with 8-way passes); min_k = 2 keeps binary passes of the
     // interleaving shape, larger min_k that fan-in
-    p.cfan = min_k > 2 ? shape_code(fan_of(min_k), 0) : (min_k == 2 ? shape_code(2, 2) : shape_code(16, 0));
+    p.cfan = min_k > 2 ? shape_code(fan_of(min_k), 0) : (min_k == 2 || beside ? shape_code(2, 2) : shape_code(16, 0));
     // the GPU would wait for a whole first chunk before any sorting starts:
     // copied in four pieces it starts after a quarter (1 GiB u32 call from
     // pinned memory 13.33-13.40 -> 13.25-13.28 ms); needs chunk passes of
@@ -1025,13 +1028,20 @@ int sort_host_impl(int kind, void* d, void* tmp, uint64_t n, uint64_t sort_n, un
 }  // namespace
 
 namespace origami {
-// The serving loop's large requests: the pipelined host sort with binary
-// passes of the interleaving shape for the chunks (min_k = 2), because the
-// loop's other batches run beside it; persistent 16-way chunk sorts hold
-// every SM while they run (400 requests/s: p50 0.35 -> 3.6 ms, p99 14 -> 108 ms).
-uint64_t host_pipe_bytes(int kind, uint64_t n) { return host_pipe_plan(kind, n, 0, 2).total; }
+// The serving loop's large requests: the pipelined host sort with chunks sorted by
+// buckets, or by binary passes of the interleaving shape where `limit` bytes do not hold
+// the buckets' scratch, because the loop's other batches run beside it; persistent
+// 16-way chunk sorts hold every SM while they run (400 requests/s: p50 0.35 -> 3.6 ms,
+// p99 14 -> 108 ms). Chunks by binary passes and by buckets, 128 requests of 2^10 to
+// 2^26 items at once: 8.1 and 9.2 Gkeys/s, p99 43 and 38 ms (medians of runs taken in
+// turn); at 400 requests/s no difference (p50 0.26 and 0.27 ms).
+static HostPipePlan beside_plan(int kind, uint64_t n, uint64_t limit) {
+    const HostPipePlan p = host_pipe_plan(kind, n, 0, 0, false, true);
+    return p.total <= limit ? p : host_pipe_plan(kind, n, 0, 0, true, true);
+}
+uint64_t host_pipe_bytes(int kind, uint64_t n, uint64_t limit) { return beside_plan(kind, n, limit).total; }
 
-int host_pipe_sort(int kind, const void* in, void* out, uint64_t n, void* block, cudaStream_t st) {
+int host_pipe_sort(int kind, const void* in, void* out, uint64_t n, void* block, uint64_t bytes, cudaStream_t st) {
     auto view = [](const void* p) -> void* {
         if (is_device_pointer(p)) return const_cast<void*>(p);
         return device_view(const_cast<void*>(p));
@@ -1040,7 +1050,7 @@ int host_pipe_sort(int kind, const void* in, void* out, uint64_t n, void* block,
     void* vout = view(out);
     if (!vin || !vout || ((((uintptr_t)vin) | ((uintptr_t)vout)) & 15))
         return fail(ORIGAMI_ERR_INVALID, "buffers the device cannot address directly");
-    HostPipePlan p = host_pipe_plan(kind, n, 0, 2);
+    HostPipePlan p = beside_plan(kind, n, bytes);
     p.slice_copies = true;  // the loop's other batches run beside this one
     return host_pipe_run(kind, const_cast<void*>(in), out, vin, vout, n, 0, p, block, st);
 }

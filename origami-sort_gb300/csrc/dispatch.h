@@ -106,11 +106,12 @@ inline bool err_word_timeout(int w) { return w == 1 || w == 3; }
 // address (host memory the GPU reads through its mapping or page tables, or
 // device memory): chunks copied in while earlier chunks sort, then one k-way
 // pass whose output slices leave while later slices merge. host_pipe_bytes is
-// the device memory it needs (one block, caller-owned); host_pipe_sort runs it
+// the device memory it needs (one block, caller-owned; more than `limit` only where no
+// plan needs less); host_pipe_sort runs it in a block of that many bytes
 // on `st` and the calling thread's helper streams and returns once the result
 // is in `out` (ORIGAMI_ERR_INVALID when a buffer is not device-addressable).
-uint64_t host_pipe_bytes(int kind, uint64_t n);
-int host_pipe_sort(int kind, const void* in, void* out, uint64_t n, void* block, cudaStream_t st);
+uint64_t host_pipe_bytes(int kind, uint64_t n, uint64_t limit);
+int host_pipe_sort(int kind, const void* in, void* out, uint64_t n, void* block, uint64_t bytes, cudaStream_t st);
 
 // capi.cu: sets the thread's last-error message; makes the stream-ordered pool
 // the caching device arena (returns an ORIGAMI_* status).

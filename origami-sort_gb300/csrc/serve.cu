@@ -61,6 +61,7 @@ struct Request {
     int mem_out = MEM_PAGEABLE;
     int state = PENDING;
     int status = ORIGAMI_OK;
+    bool lean = false;  // the device had no memory for it: by merges, which need less scratch
     Clock::time_point t_submit, t_done;
 };
 
@@ -269,7 +270,8 @@ struct origami_server {
     uint64_t need(int kind, uint64_t items, uint64_t nseg, uint64_t limit) const {
         return layout(kind, items, nseg, limit).total;
     }
-    uint64_t room() const { return budget > in_use ? budget - in_use : 0; }  // (mu held)
+    // (mu held) What a batch of this first request may take.
+    uint64_t room(const Request& r) const { return r.lean || in_use >= budget ? 0 : budget - in_use; }
 
     // Large requests whose buffers the device can address, 16-byte aligned,
     // take the pipelined sort.
@@ -282,7 +284,7 @@ struct origami_server {
         return addressable(r.in) && addressable(r.out);
     }
     uint64_t need_of(const Request& r) const {
-        return pipe_ok(r) ? origami::host_pipe_bytes(r.kind, r.n) : need(r.kind, r.n, 1, budget);
+        return pipe_ok(r) ? origami::host_pipe_bytes(r.kind, r.n, budget) : need(r.kind, r.n, 1, budget);
     }
 
     static void CUDART_CB on_done(void* p) {
@@ -360,7 +362,7 @@ struct origami_server {
                     ++it;
                     continue;
                 }
-                const uint64_t nb = origami::host_pipe_bytes(r->kind, r->n);
+                const uint64_t nb = origami::host_pipe_bytes(r->kind, r->n, room(*r));
                 if (in_use + nb > budget) {
                     if (head) return nullptr;  // the oldest waits for memory; nothing overtakes it
                     ++it;
@@ -393,7 +395,7 @@ struct origami_server {
             }
             // the oldest request waits for memory rather than being overtaken,
             // so a large request is never starved by a stream of small ones
-            if (in_use + need(r->kind, items + r->n, b->reqs.size() + 1, room()) > budget) {
+            if (in_use + need(r->kind, items + r->n, b->reqs.size() + 1, room(b->reqs.empty() ? *r : *b->reqs.front())) > budget) {
                 if (b->reqs.empty() && !head) {
                     ++it;
                     continue;
@@ -411,7 +413,7 @@ struct origami_server {
         if (!b->pipe) {
             b->off.assign(b->reqs.size() + 1, 0);
             for (size_t i = 0; i < b->reqs.size(); ++i) b->off[i + 1] = b->off[i] + b->reqs[i]->n;
-            b->lay = layout(b->kind, items, b->reqs.size(), room());
+            b->lay = layout(b->kind, items, b->reqs.size(), room(*b->reqs.front()));
             b->bytes = b->lay.total;
         }
         b->copied = true;
@@ -441,7 +443,7 @@ struct origami_server {
             std::lock_guard<std::mutex> lk(mu);
             post([this, pb] {
                 const Request& r = *pb->reqs[0];
-                pb->status = origami::host_pipe_sort(pb->kind, r.in, r.out, r.n, pb->block, cur_stream);
+                pb->status = origami::host_pipe_sort(pb->kind, r.in, r.out, r.n, pb->block, pb->bytes, cur_stream);
                 pb->t_end = Clock::now();
                 helper_done(*pb);
             });
@@ -605,7 +607,9 @@ struct origami_server {
                     in_use -= b.bytes;
                     --batches;
                     if (b.pipe) --pipe_batches;
-                    if (inflight.empty()) {
+                    bool lean = true;
+                    for (auto& r : b.reqs) lean &= r->lean, r->lean |= inflight.empty();
+                    if (inflight.empty() && lean) {
                         // nothing will return memory: the request cannot be served
                         for (auto& r : b.reqs) {
                             r->state = FAILED;
@@ -622,7 +626,7 @@ struct origami_server {
                     }
                 }
                 max_concurrent = std::max<uint64_t>(max_concurrent, inflight.size());
-                if (back.empty()) continue;
+                if (back.empty() || inflight.empty()) continue;  // (what no memory was had for: leaner now, or failed)
             }
             if (!fin.empty()) continue;
             if (stop && inflight.empty()) break;  // destroy() cancelled everything pending

@@ -239,3 +239,31 @@ def test_many_batches_of_one_small_request():
             s.wait(s.submit(a, out=out))
             assert np.array_equal(out, want)
         s.close()
+
+
+@pytest.mark.parametrize("kind", [og.U32, og.KVU64])
+def test_large_request_at_the_least_budget(kind):
+    # a pipelined request whose budget does not hold the bucket sort's scratch
+    # sorts by merges, down to the least budget that takes it; all of them exact
+    n = (1 << 24) + 77
+    a = make(kind, n, np.random.default_rng(7), pinned=True)
+    want = expected(a)
+
+    def taken(budget):
+        out = og.empty_host(kind, n, pinned=True)
+        with og.Server(hbm_budget_bytes=budget) as s:
+            try:
+                r = s.submit(a, out=out)
+            except og.OrigamiError as e:
+                assert e.code == og.ERR_OOM
+                return False
+            s.wait(r)
+            assert s.stats()["peak_bytes_reserved"] <= budget
+        assert np.array_equal(out, want)
+        return True
+
+    lo, hi = 2 * a.nbytes, 4 * a.nbytes
+    assert not taken(lo) and taken(hi)
+    while hi - lo > 1 << 20:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if taken(mid) else (mid, hi)
