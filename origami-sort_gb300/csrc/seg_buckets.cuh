@@ -1146,6 +1146,7 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
         const uint32_t total = left + (all > first ? all - first : 0u);
         for (uint32_t h = at - first; h < total; h += gridDim.x - first) {
             const SbRec r = recs[h < left ? slow[h] : first + (h - left)];
+            if (h >= left && (r.what & SbRec::SLOW)) continue;  // (once, by its place in `slow`)
             const uint64_t len = r.what & SbRec::LEN;
             const bool moved = (r.what & SbRec::TMP) != 0;
             T *a = (moved ? buf.tmp : buf.d) + r.base, *b = (moved ? buf.d : buf.tmp) + r.base;

@@ -121,6 +121,33 @@ def test_more_buckets_than_the_grid(kind):
     check(kind, items(kind, rng.permutation(k)), [len(k)])
 
 
+@pytest.mark.parametrize("kind", [og.U32, og.U64, og.KV64])
+def test_long_slices_beyond_the_grid(kind):
+    # more buckets than the grid, and among those beyond it slices that are too long:
+    # two segments of alternating slices (as above), then one whose first level's
+    # samples mislead, so that the last level cuts 100 buckets' worth of items into 127
+    # uneven slices. (By the slices' definition some 600 buckets, 444 of them in the
+    # grid, about 20 too long, 10 of them beyond the grid.)
+    cap = 6144 if kind == og.U32 else 4096
+    rng = np.random.default_rng(11)
+
+    def alternating():
+        k = [np.array([(255 << 56) + (1 << 55)], np.uint64)]
+        for s in range(0, 186, 2):
+            k.append((np.uint64(s) << np.uint64(56)) + (np.uint64(1) << np.uint64(55)) +
+                     (rng.integers(0, 2**20, cap // 2 + 20, dtype=np.uint64) << np.uint64(32)))
+            k.append(np.array([((s + 1) << 56) + (1 << 55)], np.uint64))
+        return rng.permutation(np.concatenate(k))
+
+    n = 102 * cap
+    k = (np.uint64(77) << np.uint64(56)) + (np.uint64(1) << np.uint64(54))
+    k = k + (rng.random(n) ** 4 * 2.0**55).astype(np.uint64)
+    p = sampled(n)
+    k[p] = rng.integers(0, 2**64, len(p), dtype=np.uint64)
+    segs = [alternating(), alternating(), k]
+    check(kind, items(kind, np.concatenate(segs)), [len(s) for s in segs])
+
+
 @pytest.mark.parametrize("kind", [og.U32, og.KV64])
 def test_merges_when_tuned(kind, tmp_path):
     rng = np.random.default_rng(2)
