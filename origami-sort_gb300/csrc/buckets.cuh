@@ -48,6 +48,7 @@
 #include "bulk.cuh"
 #include "common.cuh"
 #include "radix.cuh"
+#include "warp_sort.cuh"
 
 namespace origami {
 
@@ -88,6 +89,7 @@ struct BucketShape {
     // largest bin that neighbours settle (32: 4000 Zipf uint32 keys 22 us, 16: 18; 2^27
     // Zipf uint64 keys 3.76 and 3.28 ms)
     static constexpr int CROWDED = 16;
+    static constexpr int SETTLED = 33;  // items of a bin that a warp settles whatever their keys
     static constexpr int SIDE = STABLE ? 0 : CROWDED;  // guard keys on either side of the bucket
     static constexpr size_t KEYS_BYTES = (size_t)(CAP + 2 * SIDE) * sizeof(T);
     static constexpr size_t BIN_BYTES = (size_t)C::BINS * 4 + (STABLE ? (size_t)CAP * 2 : 0);  // bins, places (pairs)
@@ -96,12 +98,15 @@ struct BucketShape {
     static constexpr int WARPS = C::S_NT / 32, MOST_CROWDED = CAP / (CROWDED + 1);
     static constexpr int MAP_WORDS = STABLE ? CAP / 32 + CAP / 64 : 0;
     static constexpr size_t CROWD_BYTES = (size_t)WARPS * MAP_WORDS * 4 + ((size_t)MOST_CROWDED + WARPS * 32) * 2;
-    // or the byte passes' words. (For pairs two CTAs of 96 KB and little more just fit a
-    // shared memory of 196 KB; 1.2 KB more, and an L1 of 28 KB slowed the scattered
-    // stores: 2^27 pairs 1.55 ms, not 1.38.)
+    // or what bins by splitters need (BkSplit), or the words of byte passes. (For pairs two
+    // CTAs of 96 KB and little more just fit a shared memory of 196 KB; 1.2 KB more, and an
+    // L1 of 28 KB slowed the scattered stores: 2^27 pairs 1.55 ms, not 1.38.)
     static constexpr size_t BYTE_BYTES = (size_t)(C::S_NT / 16) * RADIX_BINS * 4;
-    static constexpr size_t SORT_SMEM =
-        KEYS_BYTES + (BIN_BYTES + CROWD_BYTES > BYTE_BYTES ? BIN_BYTES + CROWD_BYTES : BYTE_BYTES);
+    static constexpr int SPLITTERS = 256;
+    static constexpr size_t SPLIT_BYTES = SPLITTERS * sizeof(typename Traits<T>::Key) + (2 * SPLITTERS + 32) * 4 +
+                                          (size_t)CAP * (STABLE ? 4 : 2) + (STABLE ? CAP / 32 + CAP / 32 * 48 : 64);
+    static constexpr size_t MORE_BYTES = BIN_BYTES + CROWD_BYTES > BYTE_BYTES ? BIN_BYTES + CROWD_BYTES : BYTE_BYTES;
+    static constexpr size_t SORT_SMEM = KEYS_BYTES + (SPLIT_BYTES > MORE_BYTES ? SPLIT_BYTES : MORE_BYTES);
     static_assert(TILE == RadixShape<T>::TILE || !STABLE, "pairs partition by radix_pass_kernel");
 };
 // keys sampled per segment; fewer up to one partition level (2^28 uint32 keys in chunks of
@@ -707,10 +712,9 @@ __global__ void __launch_bounds__(BucketCfg<T>::NT, BucketCfg<T>::MINB)
 // bin of the bucket: conflict-free loads, no bin bounds, one trip count for the
 // CTA. (Pairs compare original positions on equal keys and so are stable.)
 // Crowded bins (heavy keys, a few distinct keys, or clustered ones): where every
-// crowded bin holds one key only, keys are in order as placed. Otherwise one warp
-// each sorts them, where few of a bin's items differ from its commonest key; a
-// bucket with any other crowded bin is sorted by stable byte passes over the keys'
-// distance from the smallest, in shared memory.
+// crowded bin holds one key only, keys are in order as placed. Other buckets take bins by
+// splitters (bk_sort_crowded; uint32 keys of plain sorts byte passes over the keys'
+// distance from the smallest).
 template <class T>
 __device__ __forceinline__ bool bk_before(const T& a, int ia, const T& b, int ib) {
     return less(a, b) || (!less(b, a) && ia < ib);
@@ -892,9 +896,8 @@ __device__ __forceinline__ void bk_sort_init() {
 #pragma unroll
     for (int i = 0; i < C::BINS / C::S_NT; ++i) tab[i * C::S_NT + tid] = 0;
 }
-// What becomes of a bucket with crowded bins of several keys: byte passes; left as it
-// is (false is returned); its crowded bins settled by a warp each, and byte passes if
-// that fails.
+// What becomes of a bucket with crowded bins of several keys: byte passes; left as it is
+// (false is returned); its crowded bins settled by a warp each, and left if that fails.
 enum BkCrowded { BK_BYTES, BK_LEAVE, BK_SETTLE };
 // One bucket of cnt items (up to CAP), by the whole CTA. (src == out: in place.) xin
 // and xout: the sign flips of keys read and written.
@@ -1090,7 +1093,16 @@ __device__ __forceinline__ bool bk_sort_bucket(const T* src, T* out, int cnt, ui
             }
         }
         if (__syncthreads_or(mixed)) {
-            if constexpr (CROWD == BK_LEAVE) {
+            if constexpr (CROWD != BK_BYTES) {
+                if constexpr (CROWD == BK_SETTLE && Sh::STABLE) {
+                    // settled bins were written: in place, the items are put back
+                    if (src == out) {
+#pragma unroll
+                        for (int i = 0; i < IPT; ++i)
+                            if (i * NT < mine) out[i * NT + tid] = bk_flip(v[i], xin);
+                    }
+                    __syncthreads();
+                }
                 return false;
             } else {
 #pragma unroll
@@ -1133,17 +1145,265 @@ __device__ __forceinline__ bool bk_sort_bucket(const T* src, T* out, int cnt, ui
     return true;
 }
 
-// A bucket that bk_sort_bucket left. (A call of its own, from the start: in line, or
-// with the items kept in registers over it, this code costs the other buckets
-// registers: 2^27 pairs 1.4 and 1.8 ms. 32-bit keys, whose byte passes are few, are
-// better off with these in line: 2^28 keys 1.20 ms, with the call 1.38.)
+// Bins by splitters, for buckets whose crowded bins a warp each does not settle: 256 of the
+// bucket's own keys are the splitters, and the keys equal to each have a bin of their own.
+// Then the bins hold few items of different keys however the keys are spread, and each
+// item's rank in its bin is counted; equal keys are in order as placed (pairs after their
+// original places are ranked, many equal ones by a bitmap of the places, a warp a bin).
+// Bounded by the search, eight steps of a random shared load a key, twice, and the ranks:
+// 21 instructions an item in all, 55 % of issue slots. A bin that is wide all the same
+// (samples that mislead) sends the bucket to byte passes.
+// Those took every such bucket before, up to eight passes: groups of 200 log-uniform keys,
+// 2^25 in all, uint32 11.9 ms and now 3.4, uint64 20.8 and 3.6, pairs 38.5 and 5.8; groups
+// of 1000 3.0 / 1.1, 5.0 / 1.5, 9.1 / 1.9; 2^24 uint64 keys in clusters 1.78 and 0.88. (Tried:
+// 512 splitters, groups of 200 twice as long, larger ones the same; merges through registers
+// in shared memory, groups of 5000 3.0 ms instead of 2.5.)
+template <class T>
+struct BkSplit {
+    using K = typename Traits<T>::Key;
+    static constexpr int SPLITTERS = BucketShape<T>::SPLITTERS, BINS = 2 * SPLITTERS + 1;
+    static constexpr int FEW = 256;  // up to here: no bins
+    static constexpr int MANY = 64;  // equal pairs from here on: by bitmap
+    static constexpr uint32_t WIDE = 256;
+    static constexpr int CAP = BucketShape<T>::CAP, PLACES = BucketShape<T>::STABLE ? CAP : 1;
+    static constexpr int MAPS = BucketShape<T>::STABLE ? 8 : 1, WORDS = BucketShape<T>::STABLE ? CAP / 32 : 1;
+    K sp[SPLITTERS];
+    uint32_t tab[BINS + 31];
+    uint16_t bin[CAP];             // by original place
+    uint16_t at[PLACES];           // pairs: original places
+    uint16_t list[BucketShape<T>::STABLE ? CAP / MANY : 1];  // bins of many equal pairs
+    uint32_t map[MAPS][WORDS];     // one bit per item of the bucket
+    uint16_t before[MAPS][WORDS];  // its running counts
+};
+// (This and what follows are calls of their own, from the start: in line, or with the items
+// kept in registers over them, they cost the other buckets registers, 2^27 pairs 1.4 and 1.8
+// ms; which of them are calls was chosen by the registers that the others keep. 32-bit keys
+// of plain sorts, whose byte passes are few, are better off with these in line: 2^28 keys
+// 1.20 ms, with a call 1.38.)
+template <class T>
+__device__ __noinline__ void bk_sort_bytes(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
+    using Sh = BucketShape<T>;
+    __builtin_assume(__isGlobal(src));
+    __builtin_assume(__isGlobal(out));
+    T* sk = reinterpret_cast<T*>(bk_smem());
+    uint32_t* table = reinterpret_cast<uint32_t*>(bk_smem() + Sh::KEYS_BYTES);
+    constexpr int NT = Sh::C::S_NT;
+    for (int i = threadIdx.x; i < cnt; i += NT) sk[i] = bk_flip(src[i], xin);
+    __syncthreads();
+    bk_byte_passes<T, NT, Sh::C::S_IPT>(sk, table, bk_shared<T>().ws, cnt, 0, (int)sizeof(typename Traits<T>::Key));
+    for (int i = threadIdx.x; i < cnt; i += NT) out[i] = bk_flip(sk[i], xout);
+}
+template <class T>
+__device__ __noinline__ void bk_sort_split(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
+    using Sh = BucketShape<T>;
+    using W = BkSplit<T>;
+    using K = typename Traits<T>::Key;
+    constexpr int NT = Sh::C::S_NT, NS = W::SPLITTERS;
+    static_assert(Sh::KEYS_BYTES + sizeof(W) <= Sh::SORT_SMEM, "it fits");
+    __builtin_assume(__isGlobal(src));
+    __builtin_assume(__isGlobal(out));
+    T* sk = reinterpret_cast<T*>(bk_smem());
+    W& w = *reinterpret_cast<W*>(bk_smem() + Sh::KEYS_BYTES);
+    BucketSortShared<T>& sh = bk_shared<T>();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __syncthreads();
+    if (cnt <= W::FEW) {
+        // every item's rank by comparison with all
+        T x;
+        if (tid < cnt) sk[tid] = x = bk_flip(src[tid], xin);
+        __syncthreads();
+        if (tid < cnt) {
+            int r = 0;
+#pragma unroll 4
+            for (int i = 0; i < tid; ++i) r += less(x, sk[i]) ? 0 : 1;
+#pragma unroll 4
+            for (int i = tid + 1; i < cnt; ++i) r += less(sk[i], x) ? 1 : 0;
+            out[r] = bk_flip(x, xout);
+        }
+        return;
+    }
+    for (int i = tid; i < W::BINS; i += NT) w.tab[i] = 0;
+    if (tid < NS) {
+        // evenly spaced, each moved inside its stretch by a hash
+        const int a = cnt * tid / NS, gap = cnt * (tid + 1) / NS - a;
+        const int p = a + (int)__umulhi((uint32_t)tid * 2654435761u + 12345u, (uint32_t)gap);
+        w.sp[tid] = Traits<T>::key(bk_flip(src[min(p, cnt - 1)], xin));
+    }
+    if (tid == 0) sh.widest = sh.listed = 0;
+    __syncthreads();
+    if (warp == 0) {
+        K s[NS / 32];
+#pragma unroll
+        for (int k = 0; k < NS / 32; ++k) s[k] = w.sp[k * 32 + lane];
+        warp_sort<K, NS / 32>(s, NS);
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < NS / 32; ++k) w.sp[lane * (NS / 32) + k] = s[k];
+    }
+    __syncthreads();
+    // 2i: between splitters i-1 and i; 2i+1: equal to splitter i
+    auto bin = [&](K k) -> uint32_t {
+        uint32_t p = 0;
+#pragma unroll
+        for (int s = NS / 2; s; s >>= 1)
+            if (w.sp[p + s - 1] < k) p += s;
+        const K x = w.sp[p];
+        return 2 * p + (x < k ? 2u : (x == k ? 1u : 0u));
+    };
+#pragma unroll 4
+    for (int i = tid; i < cnt; i += NT) {
+        const uint32_t b = bin(Traits<T>::key(bk_flip(src[i], xin)));
+        w.bin[i] = (uint16_t)b;
+        atomicAdd(&w.tab[b], 1u);
+    }
+    __syncthreads();
+    // starts: thread t has the bins below and of splitter t, the last one also that above all
+    static_assert(NS == RADIX_BINS, "one thread a splitter");
+    uint32_t mixed = 0, pure = 0;
+    if (tid < NS) {
+        mixed = w.tab[2 * tid];
+        pure = w.tab[2 * tid + 1];
+    }
+    const uint32_t first = radix_bin_scan<uint32_t>(mixed + pure, sh.ws);
+    if (tid < NS) {
+        w.tab[2 * tid] = first;
+        w.tab[2 * tid + 1] = first + mixed;
+        if (Sh::STABLE && pure > (uint32_t)W::MANY) w.list[atomicAdd(&sh.listed, 1u)] = (uint16_t)(2 * tid + 1);
+        uint32_t wide = mixed;
+        if (tid == NS - 1) {
+            wide = max(wide, w.tab[2 * NS]);
+            w.tab[2 * NS] = first + mixed + pure;
+        }
+        wide = __reduce_max_sync(0xFFFFFFFFu, wide);
+        if (lane == 0) atomicMax(&sh.widest, wide);
+    }
+    __syncthreads();
+    if (sh.widest > W::WIDE) {
+        bk_sort_bytes<T>(src, out, cnt, xin, xout);
+        return;
+    }
+#pragma unroll 4
+    for (int i = tid; i < cnt; i += NT) {
+        const uint32_t r = atomicAdd(&w.tab[w.bin[i]], 1u);
+        sk[r] = bk_flip(src[i], xin);
+        if constexpr (Sh::STABLE) w.at[r] = (uint16_t)i;
+    }
+    __syncthreads();
+    // a bin's word is its end now, and so the start of the next
+    if constexpr (Sh::STABLE) {
+        constexpr int PER = W::WORDS / 32;
+        if (warp < W::MAPS)
+            for (int k = warp; k < (int)sh.listed; k += W::MAPS) {
+                uint32_t* map = w.map[warp];
+                const int b = w.list[k], s = (int)w.tab[b - 1], e = (int)w.tab[b];
+#pragma unroll
+                for (int i = 0; i < PER; ++i) map[lane * PER + i] = 0;
+                __syncwarp();
+                for (int i = s + lane; i < e; i += 32) atomicOr(&map[w.at[i] >> 5], 1u << (w.at[i] & 31));
+                __syncwarp();
+                int sum = 0;
+#pragma unroll
+                for (int i = 0; i < PER; ++i) sum += __popc(map[lane * PER + i]);
+                int inc = sum;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                    if (lane >= o) inc += u;
+                }
+                int run = inc - sum;
+#pragma unroll
+                for (int i = 0; i < PER; ++i) {
+                    w.before[warp][lane * PER + i] = (uint16_t)run;
+                    run += __popc(map[lane * PER + i]);
+                }
+                __syncwarp();
+                for (int i = s + lane; i < e; i += 32) {
+                    const int o = w.at[i];
+                    out[s + w.before[warp][o >> 5] + __popc(map[o >> 5] & ((1u << (o & 31)) - 1u))] = bk_flip(sk[i], xout);
+                }
+                __syncwarp();
+            }
+    }
+    for (int j = tid; j < cnt; j += NT) {
+        const T x = sk[j];
+        const uint32_t b = bin(Traits<T>::key(x));
+        const int e = (int)w.tab[b], s = b ? (int)w.tab[b - 1] : 0;
+        int r = s;
+        if constexpr (Sh::STABLE) {
+            if ((b & 1u) && e - s > W::MANY) continue;
+            const int ix = (int)w.at[j];
+            for (int i = s; i < e; ++i) r += bk_before(sk[i], (int)w.at[i], x, ix) ? 1 : 0;
+        } else if (b & 1u) {
+            r = j;
+        } else {
+            for (int i = s; i < j; ++i) r += sk[i] <= x ? 1 : 0;
+            for (int i = j + 1; i < e; ++i) r += sk[i] < x ? 1 : 0;
+        }
+        out[r] = bk_flip(x, xout);
+    }
+}
+
+// Crowded bins, each settled by a warp, and whether that was all.
+template <class T>
+__device__ __noinline__ bool bk_settle_bucket(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
+    __builtin_assume(__isGlobal(src));
+    __builtin_assume(__isGlobal(out));
+    bk_sort_init<T>();
+    const bool done = bk_sort_bucket<T, BK_SETTLE>(src, out, cnt, xin, xout);
+    __syncthreads();
+    return done;
+}
+template <class T>
+__device__ __noinline__ void bk_sort_settled(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
+    __syncthreads();
+    if (!bk_settle_bucket<T>(src, out, cnt, xin, xout)) bk_sort_split<T>(src, out, cnt, xin, xout);
+}
+// A bucket that bk_sort_bucket<T, BK_LEAVE> left just now. Where a quarter of 64 items
+// stand in bins of more items than a warp settles, and are alone with their keys among 32,
+// no bin of theirs would be settled (groups of 200 log-uniform uint64 keys 3.6 ms, 5.2 if
+// that is tried first; Zipf pairs in groups of 1000, which are settled, 1.45, by splitters
+// 1.87).
 template <class T>
 __device__ __noinline__ void bk_sort_crowded(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
     __builtin_assume(__isGlobal(src));
     __builtin_assume(__isGlobal(out));
+    using Sh = BucketShape<T>;
+    using K = typename Traits<T>::Key;
+    constexpr int BINS = Sh::C::BINS, TRIED = 64;
+    BucketSortShared<T>& sh = bk_shared<T>();
+    const uint32_t* tab = reinterpret_cast<const uint32_t*>(bk_smem() + Sh::KEYS_BYTES);
+    const int tid = threadIdx.x;
     __syncthreads();
-    bk_sort_init<T>();
-    bk_sort_bucket<T, BK_SETTLE>(src, out, cnt, xin, xout);
+    bool odd = false;
+    if (tid < TRIED) {
+        // bins as in bk_sort_bucket, from the range found there
+        K klo = sh.rlo[0], kr = sh.rhi[0] - sh.rlo[0];
+        int c;
+        uint32_t xr, b;
+        if constexpr (sizeof(K) == 8) {
+            klo = kr ? klo << 32 : (klo << 32 | sh.rlo[1]);
+            kr = kr ? kr << 32 | 0xFFFFFFFFu : (K)(sh.rhi[1] - sh.rlo[1]);
+            c = __clzll((long long)kr);
+            xr = (uint32_t)((kr << c) >> 32);
+        } else {
+            c = __clz((int)kr);
+            xr = kr << c;
+        }
+        const uint32_t mul = (uint32_t)(((float)BINS * 4294967296.0f) / ((float)xr + 512.0f)) - 1u;
+        const int p = cnt > TRIED ? cnt * tid / TRIED : min(tid, cnt - 1);
+        const K k = Traits<T>::key(bk_flip(src[p], xin));
+        const unsigned same = __match_any_sync(0xFFFFFFFFu, k);
+        if constexpr (sizeof(K) == 8)
+            b = __umulhi((uint32_t)(((k - klo) << c) >> 32), mul);
+        else
+            b = __umulhi((k - klo) << c, mul);
+        // (of keys the bins' words are their ends already, of pairs their starts)
+        const int s = Sh::STABLE ? (int)tab[b] : (b ? (int)tab[b - 1] : 0);
+        const int e = Sh::STABLE ? (b + 1 < BINS ? (int)tab[b + 1] : cnt) : (int)tab[b];
+        odd = tid < cnt && (same & (same - 1u)) == 0 && e - s > Sh::SETTLED;
+    }
+    if (__syncthreads_count(odd) >= TRIED / 4 || !bk_settle_bucket<T>(src, out, cnt, xin, xout))
+        bk_sort_split<T>(src, out, cnt, xin, xout);
 }
 
 template <class T>
@@ -1168,7 +1428,12 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT)
     bk_one_kernel(const T* src, T* dst, int n, uint64_t xin, uint64_t xout, int* err) {
     if (err && threadIdx.x == 0) *err = 0;
     bk_sort_init<T>();
-    bk_sort_bucket<T, BK_SETTLE>(src, dst, n, xin, xout);
+    if (bk_sort_bucket<T, BK_SETTLE>(src, dst, n, xin, xout)) return;
+    __syncthreads();
+    if (sizeof(T) == 4)  // (four byte passes: one CTA is done in 28 us, by splitters in 46)
+        bk_sort_bytes<T>(src, dst, n, xin, xout);
+    else
+        bk_sort_split<T>(src, dst, n, xin, xout);
 }
 
 // The first kernel of a merge sort: sorts every `tile` items (up to CAP). 2^24 uint64 keys in

@@ -1153,13 +1153,14 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
             if (len > (uint64_t)BucketShape<T>::CAP)
                 sb_sort_long<T>(a, b, buf.want() + r.base, len, xin, xout);
             else
-                bk_sort_crowded<T>(a, buf.want() + r.base, (int)len, xin, xout);
+                bk_sort_settled<T>(a, buf.want() + r.base, (int)len, xin, xout);
             __syncthreads();
         }
         return;
     }
-    if (!bk_sort_bucket<T, BK_LEAVE>(src + base, buf.want() + base, cnt, xin, xout))
-        bk_sort_crowded<T>(src + base, buf.want() + base, cnt, xin, xout);
+    src += base;
+    T* const out = buf.want() + base;
+    if (!bk_sort_bucket<T, BK_LEAVE>(src, out, cnt, xin, xout)) bk_sort_crowded<T>(src, out, cnt, xin, xout);
 }
 
 }  // namespace origami
