@@ -89,6 +89,7 @@ struct BucketShape {
     // largest bin that neighbours settle (32: 4000 Zipf uint32 keys 22 us, 16: 18; 2^27
     // Zipf uint64 keys 3.76 and 3.28 ms)
     static constexpr int CROWDED = 16;
+    static constexpr int FEW = 256;  // buckets up to here: ranked by comparison with all instead
     static constexpr int SETTLED = 33;  // items of a bin that a warp settles whatever their keys
     static constexpr int SIDE = STABLE ? 0 : CROWDED;  // guard keys on either side of the bucket
     static constexpr size_t KEYS_BYTES = (size_t)(CAP + 2 * SIDE) * sizeof(T);
@@ -881,6 +882,33 @@ __device__ __noinline__ bool bk_settle_bin(uint16_t* odd, T* sk, const uint16_t*
     }
     return true;
 }
+// Keys only: settles every crowded bin of the bucket that stands in its bins, and whether
+// that could be done; by the whole CTA. (A call of its own, as bk_sort_crowded below. Zipf
+// keys in groups of 5000, 2^25 in all: uint32 0.52 ms when such a bucket was loaded and put
+// in its bins once more first, 0.38 now; uint64 1.22 and 0.95.)
+template <class T>
+__device__ __noinline__ bool bk_settle_keys() {
+    using Sh = BucketShape<T>;
+    constexpr int NT = Sh::C::S_NT, BINS = Sh::C::BINS;
+    unsigned char* smem_raw = bk_smem();
+    BucketSortShared<T>& sh = bk_shared<T>();
+    T* sk = reinterpret_cast<T*>(smem_raw) + Sh::SIDE;
+    const uint32_t* tab = reinterpret_cast<const uint32_t*>(smem_raw + Sh::KEYS_BYTES);
+    uint16_t* odd = reinterpret_cast<uint16_t*>(smem_raw + Sh::KEYS_BYTES + Sh::BIN_BYTES);
+    uint16_t* bins = odd + Sh::WARPS * 32;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    if (tid == 0) sh.listed = 0;
+    __syncthreads();
+    for (int b = tid; b < BINS; b += NT)
+        if (tab[b] - (b ? tab[b - 1] : 0u) > (uint32_t)Sh::CROWDED) bins[atomicAdd(&sh.listed, 1u)] = (uint16_t)b;
+    __syncthreads();
+    bool mixed = false;
+    for (int k = warp; k < (int)sh.listed; k += Sh::WARPS) {
+        const int b = bins[k], s = b ? (int)tab[b - 1] : 0;
+        mixed |= !bk_settle_bin<T>(odd + warp * 32, sk, nullptr, nullptr, s, (int)tab[b] - s, nullptr, 0);
+    }
+    return !__syncthreads_or(mixed);
+}
 // Clears the bins; no barrier needed before bk_sort_bucket.
 template <class T>
 __device__ __forceinline__ void bk_sort_init() {
@@ -897,7 +925,8 @@ __device__ __forceinline__ void bk_sort_init() {
     for (int i = 0; i < C::BINS / C::S_NT; ++i) tab[i * C::S_NT + tid] = 0;
 }
 // What becomes of a bucket with crowded bins of several keys: byte passes; left as it is
-// (false is returned); its crowded bins settled by a warp each, and left if that fails.
+// (false is returned; keys only: if a warp a bin can't settle them); pairs: settled by a
+// warp each, and left if that fails.
 enum BkCrowded { BK_BYTES, BK_LEAVE, BK_SETTLE };
 // One bucket of cnt items (up to CAP), by the whole CTA. (src == out: in place.) xin
 // and xout: the sign flips of keys read and written.
@@ -1061,7 +1090,7 @@ __device__ __forceinline__ bool bk_sort_bucket(const T* src, T* out, int cnt, ui
     }
     __syncthreads();
     if (CROWD == BK_LEAVE && Sh::STABLE && crowded) return false;
-    static_assert(CROWD != BK_BYTES || !Sh::STABLE, "pairs are not in order as placed");
+    static_assert(CROWD == BK_LEAVE || (CROWD == BK_SETTLE) == Sh::STABLE, "pairs are not in order as placed");
 #pragma unroll
     for (int i = 0; i < IPT; ++i)
         if (i * NT < mine) {
@@ -1092,9 +1121,11 @@ __device__ __forceinline__ bool bk_sort_bucket(const T* src, T* out, int cnt, ui
                 mixed |= e - s > CROWDED && sk[j] != sk[s];
             }
         }
-        if (__syncthreads_or(mixed)) {
+        mixed = __syncthreads_or(mixed);
+        if constexpr (CROWD == BK_LEAVE && !Sh::STABLE) mixed = mixed && (cnt <= Sh::FEW || !bk_settle_keys<T>());
+        if (mixed) {
             if constexpr (CROWD != BK_BYTES) {
-                if constexpr (CROWD == BK_SETTLE && Sh::STABLE) {
+                if constexpr (CROWD == BK_SETTLE) {
                     // settled bins were written: in place, the items are put back
                     if (src == out) {
 #pragma unroll
@@ -1154,15 +1185,14 @@ __device__ __forceinline__ bool bk_sort_bucket(const T* src, T* out, int cnt, ui
 // 21 instructions an item in all, 55 % of issue slots. A bin that is wide all the same
 // (samples that mislead) sends the bucket to byte passes.
 // Those took every such bucket before, up to eight passes: groups of 200 log-uniform keys,
-// 2^25 in all, uint32 11.9 ms and now 3.4, uint64 20.8 and 3.6, pairs 38.5 and 5.8; groups
-// of 1000 3.0 / 1.1, 5.0 / 1.5, 9.1 / 1.9; 2^24 uint64 keys in clusters 1.78 and 0.88. (Tried:
+// 2^25 in all, uint32 11.9 ms and now 3.2, uint64 20.8 and 3.5, pairs 38.5 and 5.8; groups
+// of 1000 3.0 / 1.2, 5.0 / 1.6, 9.1 / 1.9; 2^24 uint64 keys in clusters 1.78 and 0.88. (Tried:
 // 512 splitters, groups of 200 twice as long, larger ones the same; merges through registers
 // in shared memory, groups of 5000 3.0 ms instead of 2.5.)
 template <class T>
 struct BkSplit {
     using K = typename Traits<T>::Key;
     static constexpr int SPLITTERS = BucketShape<T>::SPLITTERS, BINS = 2 * SPLITTERS + 1;
-    static constexpr int FEW = 256;  // up to here: no bins
     static constexpr int MANY = 64;  // equal pairs from here on: by bitmap
     static constexpr uint32_t WIDE = 256;
     static constexpr int CAP = BucketShape<T>::CAP, PLACES = BucketShape<T>::STABLE ? CAP : 1;
@@ -1175,7 +1205,7 @@ struct BkSplit {
     uint32_t map[MAPS][WORDS];     // one bit per item of the bucket
     uint16_t before[MAPS][WORDS];  // its running counts
 };
-// (This and what follows are calls of their own, from the start: in line, or with the items
+// (These are calls of their own, from the start: in line, or with the items
 // kept in registers over them, they cost the other buckets registers, 2^27 pairs 1.4 and 1.8
 // ms; which of them are calls was chosen by the registers that the others keep. 32-bit keys
 // of plain sorts, whose byte passes are few, are better off with these in line: 2^28 keys
@@ -1207,7 +1237,7 @@ __device__ __noinline__ void bk_sort_split(const T* src, T* out, int cnt, uint64
     BucketSortShared<T>& sh = bk_shared<T>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     __syncthreads();
-    if (cnt <= W::FEW) {
+    if (cnt <= Sh::FEW) {
         // every item's rank by comparison with all
         T x;
         if (tid < cnt) sk[tid] = x = bk_flip(src[tid], xin);
@@ -1349,20 +1379,21 @@ __device__ __noinline__ bool bk_settle_bucket(const T* src, T* out, int cnt, uin
     __builtin_assume(__isGlobal(src));
     __builtin_assume(__isGlobal(out));
     bk_sort_init<T>();
-    const bool done = bk_sort_bucket<T, BK_SETTLE>(src, out, cnt, xin, xout);
+    const bool done = bk_sort_bucket<T, BucketShape<T>::STABLE ? BK_SETTLE : BK_LEAVE>(src, out, cnt, xin, xout);
     __syncthreads();
     return done;
 }
+// One bucket of a CTA that takes several.
 template <class T>
 __device__ __noinline__ void bk_sort_settled(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
     __syncthreads();
     if (!bk_settle_bucket<T>(src, out, cnt, xin, xout)) bk_sort_split<T>(src, out, cnt, xin, xout);
 }
-// A bucket that bk_sort_bucket<T, BK_LEAVE> left just now. Where a quarter of 64 items
-// stand in bins of more items than a warp settles, and are alone with their keys among 32,
-// no bin of theirs would be settled (groups of 200 log-uniform uint64 keys 3.6 ms, 5.2 if
-// that is tried first; Zipf pairs in groups of 1000, which are settled, 1.45, by splitters
-// 1.87).
+// A bucket that bk_sort_bucket<T, BK_LEAVE> left just now. Keys: by splitters. Pairs: where
+// a quarter of 64 items stand in bins of more items than a warp settles, and are alone with
+// their keys among 32, no bin of theirs would be settled. (2^25 pairs, groups of 200, keys
+// spread over their logarithms: 5.8 ms, 8.3 if settling is tried first; Zipf keys in groups
+// of 1000, which are settled, 1.47, by splitters 1.87.)
 template <class T>
 __device__ __noinline__ void bk_sort_crowded(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
     __builtin_assume(__isGlobal(src));
@@ -1370,6 +1401,7 @@ __device__ __noinline__ void bk_sort_crowded(const T* src, T* out, int cnt, uint
     using Sh = BucketShape<T>;
     using K = typename Traits<T>::Key;
     constexpr int BINS = Sh::C::BINS, TRIED = 64;
+    static_assert(Sh::STABLE, "pairs");
     BucketSortShared<T>& sh = bk_shared<T>();
     const uint32_t* tab = reinterpret_cast<const uint32_t*>(bk_smem() + Sh::KEYS_BYTES);
     const int tid = threadIdx.x;
@@ -1378,31 +1410,27 @@ __device__ __noinline__ void bk_sort_crowded(const T* src, T* out, int cnt, uint
     if (tid < TRIED) {
         // bins as in bk_sort_bucket, from the range found there
         K klo = sh.rlo[0], kr = sh.rhi[0] - sh.rlo[0];
-        int c;
-        uint32_t xr, b;
-        if constexpr (sizeof(K) == 8) {
-            klo = kr ? klo << 32 : (klo << 32 | sh.rlo[1]);
-            kr = kr ? kr << 32 | 0xFFFFFFFFu : (K)(sh.rhi[1] - sh.rlo[1]);
-            c = __clzll((long long)kr);
-            xr = (uint32_t)((kr << c) >> 32);
-        } else {
-            c = __clz((int)kr);
-            xr = kr << c;
-        }
+        klo = kr ? klo << 32 : (klo << 32 | sh.rlo[1]);
+        kr = kr ? kr << 32 | 0xFFFFFFFFu : (K)(sh.rhi[1] - sh.rlo[1]);
+        const int c = __clzll((long long)kr);
+        const uint32_t xr = (uint32_t)((kr << c) >> 32);
         const uint32_t mul = (uint32_t)(((float)BINS * 4294967296.0f) / ((float)xr + 512.0f)) - 1u;
         const int p = cnt > TRIED ? cnt * tid / TRIED : min(tid, cnt - 1);
         const K k = Traits<T>::key(bk_flip(src[p], xin));
         const unsigned same = __match_any_sync(0xFFFFFFFFu, k);
-        if constexpr (sizeof(K) == 8)
-            b = __umulhi((uint32_t)(((k - klo) << c) >> 32), mul);
-        else
-            b = __umulhi((k - klo) << c, mul);
-        // (of keys the bins' words are their ends already, of pairs their starts)
-        const int s = Sh::STABLE ? (int)tab[b] : (b ? (int)tab[b - 1] : 0);
-        const int e = Sh::STABLE ? (b + 1 < BINS ? (int)tab[b + 1] : cnt) : (int)tab[b];
+        // (the bins' words are their starts)
+        const uint32_t b = __umulhi((uint32_t)(((k - klo) << c) >> 32), mul);
+        const int s = (int)tab[b], e = b + 1 < BINS ? (int)tab[b + 1] : cnt;
         odd = tid < cnt && (same & (same - 1u)) == 0 && e - s > Sh::SETTLED;
     }
     if (__syncthreads_count(odd) >= TRIED / 4 || !bk_settle_bucket<T>(src, out, cnt, xin, xout))
+        bk_sort_split<T>(src, out, cnt, xin, xout);
+}
+template <class T>
+__device__ __forceinline__ void bk_sort_left(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
+    if constexpr (BucketShape<T>::STABLE)
+        bk_sort_crowded<T>(src, out, cnt, xin, xout);
+    else
         bk_sort_split<T>(src, out, cnt, xin, xout);
 }
 
@@ -1417,7 +1445,7 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
     if (b1 <= b0 || b1 > n || b1 - b0 > (uint32_t)BucketShape<T>::CAP) return;
     constexpr BkCrowded CROWD = sizeof(T) == 4 ? BK_BYTES : BK_LEAVE;
     if (!bk_sort_bucket<T, CROWD>(src + b0, dst + b0, (int)(b1 - b0), xin, xout))
-        bk_sort_crowded<T>(src + b0, dst + b0, (int)(b1 - b0), xin, xout);
+        bk_sort_left<T>(src + b0, dst + b0, (int)(b1 - b0), xin, xout);
 }
 
 // A sort of one bucket: n items (up to CAP) by one CTA. (1000 uint32
@@ -1428,7 +1456,7 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT)
     bk_one_kernel(const T* src, T* dst, int n, uint64_t xin, uint64_t xout, int* err) {
     if (err && threadIdx.x == 0) *err = 0;
     bk_sort_init<T>();
-    if (bk_sort_bucket<T, BK_SETTLE>(src, dst, n, xin, xout)) return;
+    if (bk_sort_bucket<T, BucketShape<T>::STABLE ? BK_SETTLE : BK_LEAVE>(src, dst, n, xin, xout)) return;
     __syncthreads();
     if (sizeof(T) == 4)  // (four byte passes: one CTA is done in 28 us, by splitters in 46)
         bk_sort_bytes<T>(src, dst, n, xin, xout);
@@ -1447,7 +1475,7 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
     if (blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
     bk_sort_init<T>();
     if (!bk_sort_bucket<T, BK_LEAVE>(in + base, out + base, cnt, xin, xout))
-        bk_sort_crowded<T>(in + base, out + base, cnt, xin, xout);
+        bk_sort_left<T>(in + base, out + base, cnt, xin, xout);
 }
 
 }  // namespace origami

@@ -1160,7 +1160,7 @@ __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
     }
     src += base;
     T* const out = buf.want() + base;
-    if (!bk_sort_bucket<T, BK_LEAVE>(src, out, cnt, xin, xout)) bk_sort_crowded<T>(src, out, cnt, xin, xout);
+    if (!bk_sort_bucket<T, BK_LEAVE>(src, out, cnt, xin, xout)) bk_sort_left<T>(src, out, cnt, xin, xout);
 }
 
 }  // namespace origami
