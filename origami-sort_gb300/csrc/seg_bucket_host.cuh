@@ -18,11 +18,14 @@ struct SegBucketPlan {
     int levels, usual;  // usual: what segments of the mean length need
     bool wide;  // 64-bit counts
     SegBucketPlan(uint64_t n_, uint64_t nseg_, uint64_t longest) : n(n_), nseg(nseg_) {
-        // levels that 256 slices each need to cut the longest segment into buckets
-        // of 4/5 of the largest size, and one more for keys that are spread unevenly
-        levels = 1;
-        for (uint64_t m = (uint64_t)Sh::CAP * 4 / 5 * RADIX_BINS; m < longest && levels < SB_MAX_LEVELS; m *= RADIX_BINS) ++levels;
-        levels = longest > (uint64_t)Sh::CAP ? std::min(levels + 1, SB_MAX_LEVELS) : 0;
+        // levels that splitters need to cut the longest segment into buckets of half the
+        // largest size; from two levels on for four times fewer items, so that a key of some 9 % of
+        // them does not send the first level to splitters (6,000,000 Zipf uint64 keys in two
+        // levels, by splitters, 375 us, in three 233)
+        levels = longest > (uint64_t)Sh::CAP ? 1 : 0;
+        for (uint64_t m = (uint64_t)Sh::CAP / 2 << SB_SURE_BITS; levels && m < longest && levels < SB_MAX_LEVELS;
+             m <<= levels == 2 ? SB_SURE_BITS - 2 : SB_SURE_BITS)
+            ++levels;
         usual = 0;
         for (uint64_t m = (uint64_t)Sh::CAP * 4 / 5; m < n / std::max<uint64_t>(nseg, 1); m *= RADIX_BINS) ++usual;
         usual = std::max(usual, 1);
@@ -146,7 +149,7 @@ void segbucket_levels(const SbBuffers<T>& buf, const SbGiven& given, const SbSta
         const uint32_t samples = l == 0 && behind ? std::max(given.nseg, given.slices) : segs;
         launch(n_sample.c_str(), st, [&] {
             launch_dependent(sb_sample_kernel<T, S>, dim3(std::min(samples, g.sample)), dim3(512), 0, st, buf, l,
-                             l == 0 ? given : none, (const SbSeg*)sc.list[l & 1], &cn->segs[l], xin, sc.maps,
+                             p.levels - 1 - l, l == 0 ? given : none, (const SbSeg*)sc.list[l & 1], &cn->segs[l], xin, sc.maps,
                              sc.splitters, hist, sc.done, sc.tiles, &cn->tiles[l], sc.recs, &cn->recs,
                              (const int*)&cn->err);
         });

@@ -22,19 +22,22 @@
 //
 // How a segment is cut. Its keys' range, from the sample, in 256 slices of equal
 // width: a subtraction and a multiplication per key. Where one slice would take
-// more than 1/8 of the samples because of one key, that key gets a slice of its
+// too many of the samples because of one key, that key gets a slice of its
 // own, which needs no sorting. Where slices are uneven beyond that (clusters,
 // several heavy keys), 127 sampled keys are the splitters instead, each with a
 // slice of its own for the keys equal to it: seven steps of search per key, but
 // slices of bounded size for any keys. All three are monotone functions of the
 // key, so the sample decides only how even the slices are, never the result.
+// Too many: 1/8 of the samples, and what the levels that follow would not cut into
+// buckets by splitters. (With 1/8 alone clusters in clusters of 11 % of the keys
+// left slices longer than a bucket: 838,000 uint64 keys 1.08 ms instead of 0.13, 2^27
+// 19.3 instead of 3.45, by merges 8.4.)
 //
 // Segment lengths are on the device, so every list is made there: the host
-// launches a fixed sequence (as many levels as one segment of all items would
-// need, and one more for keys that are spread unevenly; a level without segments
-// returns at once) and never waits. Slices of the last level that still do not
-// fit, possible only when samples mislead several levels in a row, are sorted by
-// one CTA each in global memory.
+// launches a fixed sequence (as many levels as one segment of all items may
+// need by splitters; a level without segments returns at once) and never waits.
+// Slices of the last level that still do not fit, possible only when samples
+// mislead, are sorted by one CTA each in global memory.
 //
 // Equal keys of keys-only items are identical, so their order does not matter:
 // sb_pass_kernel takes places with shared-memory atomics, tiles in any order, and
@@ -55,6 +58,9 @@ namespace origami {
 constexpr int SB_SPLITTERS = 127;  // two slices each, and one above them
 constexpr int SB_SAMPLES = 2048;   // keys sampled per segment
 constexpr int SB_MAX_LEVELS = 4;
+// A level by splitters cuts any segment by this: a slice is 16 of the samples, 1/128 of the
+// segment, give or take a quarter.
+constexpr int SB_SURE_BITS = 6;
 
 // The tiles of a level's segments: 6144 uint32 keys, 4096 uint64 keys or pairs.
 // (uint32: 8192 keys at three CTAs per SM pass 2^28 in 0.66 ms, 6144 at four in
@@ -258,15 +264,19 @@ __global__ void sb_plan_kernel(const uint64_t* off, uint32_t nseg, uint64_t n, S
 // ----------------------------------------------------------------- sample ---
 // One CTA per segment of the level (given.nseg: the first one behind a bucket sort;
 // segments that fit a bucket become one here). The linear range is the samples',
-// widened by 1/512 at each end.
+// widened by 1/512 at each end. more: the levels that follow this one.
 template <class T, class S>
 __global__ void __launch_bounds__(512)
-    sb_sample_kernel(SbBuffers<T> buf, int level, SbGiven given, const SbSeg* list, uint32_t* count, uint64_t xmask,
+    sb_sample_kernel(SbBuffers<T> buf, int level, int more, SbGiven given, const SbSeg* list, uint32_t* count, uint64_t xmask,
                      SbMap<typename Traits<T>::Key>* maps, typename Traits<T>::Key* splitters, S* hist, uint32_t* done,
                      SbTile* tiles, uint32_t* tile_count, SbRec* recs, uint32_t* rec_count, const int* err) {
     using K = typename Traits<T>::Key;
     constexpr int NT = 512, PER = SB_SAMPLES / NT;
-    constexpr uint32_t TILE = SegBucketShape<T>::TILE, MOST = SB_SAMPLES / 8;
+    constexpr uint32_t TILE = SegBucketShape<T>::TILE;
+    // longest slice, by the samples, that the levels that follow are sure to cut (half a
+    // bucket where there are none: a share of 32 samples is one of 18 to 46)
+    constexpr int CAP = SegBucketShape<T>::CAP;
+    const uint64_t sure = more ? (uint64_t)(CAP * 3 / 4) << (SB_SURE_BITS * more) : (uint64_t)(CAP / 2);
     __shared__ K smp[SB_SAMPLES];
     __shared__ K smin[NT / 32], smax[NT / 32], scand;
     __shared__ uint32_t cnt[RADIX_BINS];
@@ -361,9 +371,10 @@ __global__ void __launch_bounds__(512)
         map.heavy = 0;
         map.heavy_slice = 0;
         bool full = false;
+        const uint32_t most = (uint32_t)min((uint64_t)(SB_SAMPLES / 8), SB_SAMPLES * sure / q.len);
 #pragma unroll
         for (int i = 0; i < PER; ++i)
-            if (atomicAdd(&cnt[map.linear(v[i])], 1u) >= MOST) {
+            if (atomicAdd(&cnt[map.linear(v[i])], 1u) >= most) {
                 full = true;
                 scand = v[i];  // a key of a crowded slice (any of them)
             }
@@ -376,7 +387,7 @@ __global__ void __launch_bounds__(512)
             full = false;
 #pragma unroll
             for (int i = 0; i < PER; ++i)
-                if (v[i] != map.heavy) full |= atomicAdd(&cnt[map.linear(v[i])], 1u) >= MOST;
+                if (v[i] != map.heavy) full |= atomicAdd(&cnt[map.linear(v[i])], 1u) >= most;
             map.mode = __syncthreads_or(full) ? SB_SEARCH : SB_HEAVY;
             map.heavy_slice = map.linear(map.heavy) + 1;
         }
