@@ -132,7 +132,8 @@ __device__ __forceinline__ typename Traits<T>::Key ckey(const T& v, uint64_t xin
 template <class T, class Lists>
 __global__ void __launch_bounds__(256) kway_split_kernel(const Lists lists, int rpg, uint64_t xin,
                                                          int64_t* __restrict__ bnd,
-                                                         int* __restrict__ err) {
+                                                         int* __restrict__ err, const int* route = nullptr) {
+    if (route && *route == 0) return;  // (as kb_cut_kernel)
     using K = typename Traits<T>::Key;
     __shared__ int64_t lo[KWAY_MAX], hi[KWAY_MAX];
     __shared__ unsigned long long nlo[KWAY_MAX], nhi[KWAY_MAX];

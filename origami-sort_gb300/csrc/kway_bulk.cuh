@@ -185,13 +185,15 @@ struct KbCuts {
 // tiles[0 .. *ntiles) (*ntiles is 0 at launch). bnd0 (rpg > 1):
 // kway_split_kernel's super-sample counts per range boundary,
 // [g * (rpg+1) + b][KWAY_MAX]. The first CTA resets the merge kernel's claim
-// counter.
+// counter. route (optional): the pass stands behind a bucket sort, nothing to do where it
+// holds 0 (and so no tiles for the merge kernel).
 template <class T>
 __global__ void __launch_bounds__(KB_CUT_NT) kb_cut_kernel(const typename Traits<T>::Key* __restrict__ samp,
                                                           uint64_t n, uint64_t run, int fan, int rpg,
                                                           const int64_t* __restrict__ bnd0, KbCuts cuts,
                                                           uint32_t* __restrict__ tiles, unsigned* __restrict__ ntiles,
-                                                          unsigned* __restrict__ claim, int* __restrict__ err) {
+                                                          unsigned* __restrict__ claim, int* __restrict__ err,
+                                                          const int* route = nullptr) {
     using Sh = KbShape<T>;
     using K = typename Sh::K;
     using E = typename Sh::E;
@@ -213,6 +215,7 @@ __global__ void __launch_bounds__(KB_CUT_NT) kb_cut_kernel(const typename Traits
     const uint64_t g = bid / (uint64_t)rpg;
     const int b = (int)(bid % (uint64_t)rpg);
     const KbGroup grp(g, n, run, fan);
+    if (route && *route == 0) return;
     if (bid == 0 && tid == 0) *claim = 0;
     // a wait of an earlier kernel expired: the runs are not sorted, no tiles
     if (__syncthreads_or(tid == 0 && err_wait_set(err))) return;

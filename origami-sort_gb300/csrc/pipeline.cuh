@@ -110,6 +110,16 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
+// Resident CTAs of a kernel on the whole GPU; sets its shared-memory limit.
+inline uint32_t resident_ctas(const void* kernel, int nt, size_t smem) {
+    int dev = 0, sms = 0, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, nt, smem);
+    return (uint32_t)(sms * (per > 0 ? per : 1));
+}
+
 // One binary-pass merge shape: pair_merge_kernel (one tile per CTA, cp.async
 // staging) or, with BULK, pair_merge_bulk_kernel (persistent, double-buffered
 // bulk copies, as many CTAs as fit on the GPU at once).
@@ -355,10 +365,17 @@ uint64_t pipeline_scratch_bytes(uint64_t n, uint64_t sort_n, int code, uint64_t 
 // only the merge passes from there to the chunk size run (at least one).
 // `scratch` holds pipeline_scratch_bytes<T>(n, sort_n, fan, start_run) bytes of
 // device memory.
+// behind (optional): the passes, all k-way, stand behind a bucket sort (buckets.cuh) of
+// chunks of 32-bit keys, and run only where it gave up.
+template <class T>
+struct PipeBehind {
+    const int* route;
+    int* err;  // its error word
+};
 template <class T>
 cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint64_t sort_n, uint64_t xin,
                              uint64_t xout, uint64_t start_run, int code, void* scratch, cudaStream_t st,
-                             LaunchStats* stats) {
+                             LaunchStats* stats, const PipeBehind<T>* behind = nullptr) {
     using C = Config<T>;
     using KC = KwayCfg<T>;
     constexpr int T1 = k1_tile<T>();
@@ -378,7 +395,8 @@ cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint
     const T* cur = start_run ? in : written_by(0);
     const PipeScratch<T> sc(scratch, n, sort_n, code, start_run);
     int64_t* splits = sc.splits;
-    int* err = sc.err;
+    int* err = behind ? behind->err : sc.err;
+    const int* route = behind ? behind->route : nullptr;
     unsigned* claim = sc.claim;
     using K = typename Traits<T>::Key;
     // samples for the first k-way pass: written by the tile sort, or gathered
@@ -448,7 +466,18 @@ cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint
     }
     // the error word starts at 0: the tile sort clears it, else a memset
     if (start_run) cudaMemsetAsync(err, 0, sizeof(int), st);
-    if (!start_run) {
+    if (behind) {
+        if constexpr (sizeof(T) == 4) {
+            constexpr auto kernel =
+                warp_block_sort_kernel<T, C::K1_NW, C::K1_VT, C::K1_NWT, C::K1_MINB, true, C::K1_RUN0, true>;
+            static const uint32_t wave = resident_ctas((const void*)kernel, C::K1_NWT * 32, k1_smem<T>());
+            const unsigned grid = (unsigned)std::min<uint64_t>(tiles1, wave);
+            launch(n_k1.c_str(), st, [&] {
+                kernel<<<grid, C::K1_NWT * 32, k1_smem<T>(), st>>>(in, written_by(0), n, k1_chunk, xin, 0, grid, nullptr,
+                                                                  sc.samp[0], sc.ssamp[0], route, sc.tcount);
+            });
+        }
+    } else if (!start_run) {
         T* k1_out = written_by(0);
         launch(n_k1.c_str(), st, [&] {
             if (by_buckets) {
@@ -519,7 +548,7 @@ cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint
             if (p.rpg > 1) {
                 launch(n_ks.c_str(), st, [&] {
                     kway_split_kernel<K, RunLists<K>><<<(unsigned)(p.groups * (p.rpg + 1)), 256, 0, st>>>(
-                        RunLists<K>{ss_in, n / (S * SS), p.run / (S * SS), p.fan}, p.rpg, 0, sc.bnd0, err);
+                        RunLists<K>{ss_in, n / (S * SS), p.run / (S * SS), p.fan}, p.rpg, 0, sc.bnd0, err, route);
                 });
                 if (stats) stats->kernels++;
             }
@@ -527,10 +556,10 @@ cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint
             // pass pi lists its tiles in tcount[pi & 1]; the first k-way pass's
             // counter starts at 0 here, each merge kernel zeroes the next one
             unsigned* tc = sc.tcount + (pi & 1);
-            if (pi == 0) cudaMemsetAsync(tc, 0, sizeof(unsigned), st);
+            if (pi == 0 && !behind) cudaMemsetAsync(tc, 0, sizeof(unsigned), st);
             launch(n_kc.c_str(), st, [&] {
                 kb_cut_kernel<T><<<(unsigned)ranges, KB_CUT_NT, KbShape<T>::CUT_SMEM, st>>>(
-                    s_in, n, p.run, p.fan, p.rpg, sc.bnd0, sc.cuts, sc.tiles, tc, claim, err);
+                    s_in, n, p.run, p.fan, p.rpg, sc.bnd0, sc.cuts, sc.tiles, tc, claim, err, route);
             });
             const uint64_t nslots = ranges * (uint64_t)KbShape<T>::TPR;
             const uint64_t grid = std::min<uint64_t>(nslots, kb_resident<T>());

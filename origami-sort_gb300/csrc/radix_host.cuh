@@ -14,6 +14,7 @@
 namespace origami {
 
 constexpr uint64_t RADIX_LEAST = 1 << 14;
+constexpr uint64_t BK_MOST = 1ull << 31;  // items of a bucket sort: fewer
 
 // Segments of a radix sort: the whole array, or chunks of sort_n items.
 template <class T>
@@ -33,8 +34,11 @@ struct RadixPlan {
     }
     // One bucket; else enough items for several launches (10,000 uint32 keys 27 us by
     // buckets, 26 by merges), whole tiles per segment, and tile numbers that fit 31 bits.
+    // Not chunks of 2^31 uint32 keys in all and more, which the bucket sort does not take:
+    // radix passes, 6.6 ms for 2^28 Zipf keys, have merges of 3.3 to 5.1 ms against them.
     static bool fits(uint64_t n, uint64_t sort_n) {
         const uint64_t len = chunk_limit(n, sort_n);
+        if (sizeof(typename Traits<T>::Key) == 4 && len < n && n >= BK_MOST) return false;
         if (n < 2 || (len == n && n <= (uint64_t)BucketShape<T>::CAP)) return n >= 2;
         return n >= RADIX_LEAST && (len == n || len % Sh::TILE == 0) && n / Sh::TILE < (1ull << 31) - 2;
     }
@@ -49,7 +53,7 @@ struct BucketPlan {
     int b1 = 0, b2 = 0;
     uint64_t tiles = 0, tiles2 = 0, nbuckets = 0;
     BucketPlan(const RadixPlan<T>& p) {
-        if (p.n >= (1ull << 31)) return;
+        if (p.n >= BK_MOST) return;
         int bits = 0;
         while ((p.len >> bits) > (1ull << Sh::C::LOG_TARGET)) ++bits;
         // short sorts: one level can have up to 256 buckets, enough for every SM
@@ -71,16 +75,33 @@ struct BucketPlan {
     }
 };
 
-// What stands behind the bucket sort, and sorts where it does not take the call. Radix
-// passes read the keys once more for every byte, the levels once more for every 256
-// slices, whatever the width; but the levels need more launches, and on clustered keys
-// a search. 2^20 / 2^22 / 2^28 uint32 Zipf keys: radix passes 0.084 / 0.20 / 6.5 ms,
-// levels 0.12 / 0.20 / 4.9; 2^20 / 2^22 / 2^27 uint64 Zipf keys 0.143 / 0.36 / 8.0 and
-// 0.147 / 0.24 / 3.65; 1.5M Zipf pairs 0.217 and 0.177, 2^26 5.1 and 3.4; normally
-// distributed keys, 2^27 uint64 7.6 and 4.0, 2^26 pairs 5.6 and 2.4.
+// What stands behind the bucket sort, and sorts where it does not take the call.
+//   64-bit keys: the levels. Radix passes would read the keys once more for every byte, the
+// levels do for every 256 slices, whatever the width: 2^27 uint64 Zipf keys 8.0 ms by radix
+// passes and 3.4 by levels, 2^26 pairs 5.1 and 3.3, normally distributed keys 7.6 and 4.0,
+// 5.6 and 2.4.
+//   uint32 keys, one segment: radix passes, four of them and fewer launches (2^20 Zipf keys
+// 0.074 ms, by levels some 0.11; 2^28 6.5 and 4.9, which one more path would not be for).
+//   uint32 keys in chunks: by merges chunks took the less the shorter they are, so radix
+// passes lost up to 2.4 times there. 2^28 keys, ms, merges alone / radix passes, levels,
+// merges behind the bucket sort:
+//     chunks of      2^16                    2^17                    2^19
+//     Zipf keys      2.9 / 6.9, 6.4, 4.2     3.3 / 6.7, 7.0, 4.2     4.0 / 6.7, 5.4, 5.1
+//     log-uniform    2.9 / 6.6, 5.4, 3.9     3.3 / 6.6, 4.9, 4.2     4.0 / 6.6, 4.9, 5.0
+//     one chunk Zipf 2.9 / 4.3, 3.9, 4.1     3.3 / 4.2, 3.7, 4.4     4.0 / 4.0, 3.5, 5.2
+// Merges up to 2^17 keys a chunk (one 16-way pass after the tile sort: three launches), the
+// levels up to 2^20 (from there on one crowded chunk costs them a partition: chunks of 2^21
+// 4.1 by radix passes, 5.8) in sorts of 2^25 keys and more: their launches, two more than
+// radix passes', cost 2^22 uniform keys 7 of 69 us.
+enum class Behind { RADIX, LEVELS, MERGES };
+constexpr uint64_t MERGES_CHUNK = 1 << 17, MERGES_FROM = 1 << 22, LEVELS_CHUNK = 1 << 20, LEVELS_FROM = 1 << 25;
+constexpr int MERGES_CODE = 16;  // shape: 16-way
 template <class T>
-constexpr bool levels_behind() {
-    return sizeof(typename Traits<T>::Key) == 8;
+Behind behind(const RadixPlan<T>& p, const BucketPlan<T>& bk) {
+    if (sizeof(typename Traits<T>::Key) == 8) return Behind::LEVELS;
+    if (!bk.on() || p.nseg <= 1) return Behind::RADIX;
+    if (p.len <= MERGES_CHUNK) return p.n >= MERGES_FROM ? Behind::MERGES : Behind::RADIX;
+    return p.len <= LEVELS_CHUNK && p.n >= LEVELS_FROM ? Behind::LEVELS : Behind::RADIX;
 }
 template <class T>
 SegBucketPlan<T> behind_plan(const RadixPlan<T>& p, const BucketPlan<T>& bk) {
@@ -96,7 +117,8 @@ SegBucketPlan<T> behind_plan(const RadixPlan<T>& p, const BucketPlan<T>& bk) {
 //   hist       digit counts of the radix passes, [segment][digit][256]
 //   words      the passes' tile counters, the bucket sort's route and tile count
 //   tail       256 bytes: the error word; the counters of the levels behind
-// From `zero` on everything starts at 0 (one memset). First of all the levels' scratch.
+// From `zero` on everything starts at 0 (one memset). First of all the scratch of the
+// levels or merges behind.
 template <class T>
 struct RadixScratch {
     using K = typename Traits<T>::Key;
@@ -112,7 +134,9 @@ struct RadixScratch {
     int *err = nullptr, *route = nullptr;
     unsigned* claim = nullptr;
     RadixScratch(void* base, const RadixPlan<T>& p, const BucketPlan<T>& bk) {
-        constexpr bool ST = BucketShape<T>::STABLE, LEVELS = levels_behind<T>();
+        constexpr bool ST = BucketShape<T>::STABLE;
+        const Behind rest = behind(p, bk);
+        const bool passes = rest == Behind::RADIX;
         const uint64_t w = p.wide ? 8 : 4;
         char* b = static_cast<char*>(base);
         uint64_t o = 0;
@@ -122,7 +146,8 @@ struct RadixScratch {
             return r;
         };
         auto words = [&](uint64_t k) { return reinterpret_cast<uint32_t*>(take(k * 4)); };
-        if (LEVELS) o += SegBucketScratch<T>(nullptr, behind_plan(p, bk), nullptr, false).bytes;
+        if (rest == Behind::LEVELS) o += SegBucketScratch<T>(nullptr, behind_plan(p, bk), nullptr, false).bytes;
+        if (rest == Behind::MERGES) o += PipeScratch<T>(nullptr, p.n, p.len, MERGES_CODE, 0).bytes;
         if (bk.on()) {
             start1 = words((p.nseg << bk.b1) + 1);
             if (!ST) cursor1 = words(p.nseg << bk.b1);
@@ -136,16 +161,16 @@ struct RadixScratch {
         }
         // the second level's words: the first pass clears those of its own tiles
         const bool look_pairs = ST && bk.on();
-        if (look_pairs ? bk.b2 > 0 : !LEVELS) look[1] = take(std::max(p.tiles, ST ? bk.tiles2 : 0) * RADIX_BINS * w);
+        if (look_pairs ? bk.b2 > 0 : passes) look[1] = take(std::max(p.tiles, ST ? bk.tiles2 : 0) * RADIX_BINS * w);
         uint64_t z = o;
         if (look_pairs && bk.b2) z -= (bk.tiles2 - bk.tiles) * RADIX_BINS * w;
-        if (look_pairs || !LEVELS) look[0] = take(p.tiles * RADIX_BINS * w);
+        if (look_pairs || passes) look[0] = take(p.tiles * RADIX_BINS * w);
         if (!look_pairs) z = o;  // (cleared by radix_hist_kernel)
         if (bk.on()) {
             hist1 = words(p.nseg << bk.b1);
             if (bk.b2) hist2 = words(bk.nbuckets);
         }
-        if (!LEVELS) hist = take(p.nseg * RadixShape<T>::DIGITS * RADIX_BINS * w);
+        if (passes) hist = take(p.nseg * RadixShape<T>::DIGITS * RADIX_BINS * w);
         claim = words(16);
         err = reinterpret_cast<int*>(take(256));
         if (b) {
@@ -214,7 +239,7 @@ void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPla
     static const uint32_t g_hist = resident_ctas((const void*)bk_hist_kernel<T, G1>, 512, 0);
     static const uint32_t g_part = [] {
         cudaFuncSetAttribute(bk_sample_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SAMPLE_SMEM);
-        if constexpr (!levels_behind<T>())
+        if constexpr (sizeof(K) == 4)
             cudaFuncSetAttribute(bk_sort_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SORT_SMEM);
         if constexpr (ST) {
             resident_ctas((const void*)radix_pass_kernel<T, uint32_t, G2, D>, RSh::NT, RSh::SMEM);
@@ -310,8 +335,8 @@ void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPla
               (void*)nullptr, sc.claim + 9);
         cur = d;
     }
-    // (the last kernel of the levels behind sorts these buckets too)
-    if constexpr (!levels_behind<T>()) launch(n_sort.c_str(), st, [&] {
+    // (64-bit keys: the last kernel of the levels behind sorts these buckets too)
+    if constexpr (sizeof(K) == 4) launch(n_sort.c_str(), st, [&] {
         launch_dependent(bk_sort_kernel<T>, dim3((unsigned)bk.nbuckets), dim3(Sh::C::S_NT), Sh::SORT_SMEM, st, cur, want,
                          (const uint32_t*)(bk.b2 ? sc.start2 : sc.start1), xmask, xout, n32, (const int*)sc.route);
     });
@@ -359,20 +384,31 @@ cudaError_t radix_sort(T* d, T* tmp, uint64_t n, uint64_t sort_n, uint64_t key_m
         bucket_launch<T>(d, tmp, want, p, bk, key_mask, out_mask, sc, self ? (uint32_t)(sc.zero_bytes / 16) : 0u, st);
         route = sc.route;
     }
-    if constexpr (levels_behind<T>()) {
+    const Behind rest = behind(p, bk);
+    if (rest == Behind::LEVELS) {
         const SegBucketPlan<T> q = behind_plan(p, bk);
         const SegBucketScratch<T> seg(scratch, q, reinterpret_cast<SbCounts*>(sc.err), false);
         const SbBuffers<T> buf{d, tmp, route, want == tmp};
-        const SbStarts plain{bk.on() ? (bk.b2 ? sc.start2 : sc.start1) : nullptr, (uint32_t)bk.nbuckets, !bk.b2};
+        SbStarts plain{};
+        if (bk.on() && sizeof(typename Traits<T>::Key) == 8)
+            plain = SbStarts{bk.b2 ? sc.start2 : sc.start1, (uint32_t)bk.nbuckets, !bk.b2};
         const SbGiven given{route, sc.start1, p.n, p.len, (uint32_t)p.nseg, bk.b2 ? (uint32_t)(p.nseg << bk.b1) : 0u};
         if (q.wide)
             segbucket_levels<T, uint64_t>(buf, given, plain, q, key_mask, out_mask, seg, st);
         else
             segbucket_levels<T, uint32_t>(buf, given, plain, q, key_mask, out_mask, seg, st);
-    } else if (p.wide) {
-        radix_launch<T, uint64_t>(d, tmp, want, p, key_mask, out_mask, sc, route, st);
-    } else {
-        radix_launch<T, uint32_t>(d, tmp, want, p, key_mask, out_mask, sc, route, st);
+        return cudaGetLastError();
+    }
+    if constexpr (sizeof(typename Traits<T>::Key) == 4) {
+        if (rest == Behind::MERGES) {
+            const PipeBehind<T> after{route, sc.err};
+            return sort_pipeline_io<T>(d, want, want == d ? tmp : d, want, n, sort_n, key_mask, out_mask, 0, MERGES_CODE,
+                                       scratch, st, nullptr, &after);
+        }
+        if (p.wide)
+            radix_launch<T, uint64_t>(d, tmp, want, p, key_mask, out_mask, sc, route, st);
+        else
+            radix_launch<T, uint32_t>(d, tmp, want, p, key_mask, out_mask, sc, route, st);
     }
     return cudaGetLastError();
 }

@@ -83,20 +83,10 @@ struct SegBucketScratch {
     }
 };
 
-// Resident CTAs of a kernel on the whole GPU; sets its shared-memory limit.
-inline uint32_t resident_ctas(const void* kernel, int nt, size_t smem) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, nt, smem);
-    return (uint32_t)(sms * (per > 0 ? per : 1));
-}
-
 // Grids of the kernels, found once per process.
 template <class T, class S>
 struct SegBucketGrids {
-    uint32_t sample, hist, pass, sort;
+    uint32_t sample, hist, pass, sort, rest;  // (rest: 32-bit keys)
     static const SegBucketGrids& get() {
         using Sh = SegBucketShape<T>;
         static const SegBucketGrids g = [] {
@@ -109,7 +99,9 @@ struct SegBucketGrids {
                 r.pass = resident_ctas((const void*)sb_pass_kernel<T, S, true>, Sh::C::NT, Sh::PASS_SMEM);
                 resident_ctas((const void*)sb_pass_kernel<T, S, false>, Sh::C::NT, Sh::PASS_SMEM);
             }
-            r.sort = resident_ctas((const void*)sb_sort_kernel<T>, Sh::Sort::C::S_NT, Sh::Sort::SORT_SMEM);
+            r.sort = resident_ctas((const void*)sb_sort_kernel<T, false>, Sh::Sort::C::S_NT, Sh::Sort::SORT_SMEM);
+            if constexpr (sizeof(typename Traits<T>::Key) == 4)
+                r.rest = resident_ctas((const void*)sb_sort_kernel<T, true>, Sh::Sort::C::S_NT, Sh::Sort::SORT_SMEM);
             return r;
         }();
         return g;
@@ -174,14 +166,18 @@ void segbucket_levels(const SbBuffers<T>& buf, const SbGiven& given, const SbSta
             }
         });
     }
+    auto sort = [&](auto kernel, uint32_t grid, uint32_t first) {
+        launch(n_sort.c_str(), st, [&] {
+            launch_dependent(kernel, dim3(grid), dim3(Sh::Sort::C::S_NT), Sh::Sort::SORT_SMEM, st, buf, plain,
+                             (const SbRec*)sc.recs, (const uint32_t*)sc.slow, (const SbCounts*)cn, first, xin, xout);
+        });
+    };
+    if constexpr (sizeof(K) == 4)
+        if (behind) return sort(sb_sort_kernel<T, true>, g.rest, 0u);
     // one CTA per bucket: neighbouring buckets of a segment hold more than CAP items
     // together, so few sorts have more than these, and few CTAs stand by for the rest
     const uint32_t first = (uint32_t)std::min(p.recs, std::max<uint64_t>(plain.buckets, p.nseg + p.n * 9 / (4 * (uint64_t)Sh::CAP) + 1));
-    launch(n_sort.c_str(), st, [&] {
-        launch_dependent(sb_sort_kernel<T>, dim3(std::max(first, plain.buckets) + std::min(first, g.sort / 4)),
-                         dim3(Sh::Sort::C::S_NT), Sh::Sort::SORT_SMEM, st, buf, plain, (const SbRec*)sc.recs,
-                         (const uint32_t*)sc.slow, (const SbCounts*)cn, first, xin, xout);
-    });
+    sort(sb_sort_kernel<T, false>, std::max(first, plain.buckets) + std::min(first, g.sort / 4), first);
 }
 
 // Segments [off[s], off[s+1]), sorted in place.

@@ -1128,17 +1128,44 @@ struct SbStarts {
 // sort's, so that no launch is for buckets of the other kind only (2 ns for every CTA
 // that finds nothing to do). The CTAs from `first` on take the rest of the list in turn:
 // the few buckets beyond the grid, and slices that did not fit.
-template <class T>
+// LOOP (32-bit keys behind a plain bucket sort, whose last kernel is one of its own):
+// resident CTAs take all of the list in turn, so that few find nothing to do in the usual
+// case (one CTA a bucket would cost 2^28 keys 0.2 ms there). The loop's variable stands in
+// shared memory.
+template <class T, bool LOOP>
 __global__ void __launch_bounds__(BucketCfg<T>::S_NT, BucketCfg<T>::S_MINB)
     sb_sort_kernel(SbBuffers<T> buf, SbStarts plain, const SbRec* recs, const uint32_t* slow, const SbCounts* cn,
                    uint32_t first, uint64_t xin, uint64_t xout) {
+    if constexpr (LOOP) {
+        __shared__ volatile uint32_t next;
+        if (threadIdx.x == 0) next = blockIdx.x;
+        grid_dep_wait();
+#pragma unroll 1
+        while (true) {
+            __syncthreads();
+            const uint32_t at = next;
+            if (at >= count_load(&cn->recs)) return;
+            const SbRec r = recs[at];
+            const bool moved = (r.what & SbRec::TMP) != 0;
+            T *a = (moved ? buf.tmp : buf.d) + r.base, *out = buf.want() + r.base;
+            if (r.what & SbRec::SLOW) {
+                sb_sort_long<T>(a, (moved ? buf.d : buf.tmp) + r.base, out, r.what & SbRec::LEN, xin, xout);
+            } else {
+                const int cnt = (int)(r.what & SbRec::LEN);
+                bk_sort_init<T>();
+                if (!bk_sort_bucket<T, BK_LEAVE>(a, out, cnt, xin, xout)) bk_sort_left<T>(a, out, cnt, xin, xout);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) next = next + gridDim.x;
+        }
+    }
     bk_sort_init<T>();
     grid_dep_wait();
     const uint32_t at = blockIdx.x;
     const T* src;
     uint64_t base;
     int cnt;
-    // (32-bit keys: radix passes stand behind the plain bucket sort)
+    // (32-bit keys: the plain bucket sort has a last kernel of its own)
     if (sizeof(typename Traits<T>::Key) == 8 && plain.start && route_load(buf.route) == ROUTE_BUCKETS) {
         if (at >= plain.buckets) return;
         const uint32_t b0 = plain.start[at], b1 = plain.start[at + 1];

@@ -119,14 +119,19 @@ struct WarpSortShape {
 // the first thread. SAMPLES: also writes the samples of the sorted tiles to
 // samp / ssamp for a k-way pass that follows (kway_bulk.cuh); a separate
 // instantiation, so that the plain tile sort keeps its registers.
-template <class T, int NW, int VT, int NWT = NW, int MINB = 1, bool SAMPLES = false, int RUN0 = 32 * VT>
+// BEHIND: the tile sort stands behind a bucket sort of one partition level (buckets.cuh):
+// nothing to do where that went on (*route 0); resident CTAs, so that few of them find
+// nothing. tcount: the two tile counters of the passes that follow, 0 whatever the route.
+template <class T, int NW, int VT, int NWT = NW, int MINB = 1, bool SAMPLES = false, int RUN0 = 32 * VT, bool BEHIND = false>
 __global__ void __launch_bounds__(NWT * 32, MINB) warp_block_sort_kernel(const T* __restrict__ in,
                                                                         T* __restrict__ out, uint64_t n,
                                                                         int chunk, uint64_t xin,
                                                                         uint64_t xout, uint32_t ahead = 0,
                                                                         int* err = nullptr,
                                                                         typename Traits<T>::Key* samp = nullptr,
-                                                                        typename Traits<T>::Key* ssamp = nullptr) {
+                                                                        typename Traits<T>::Key* ssamp = nullptr,
+                                                                        const int* route = nullptr,
+                                                                        unsigned* tcount = nullptr) {
     using Sh = WarpSortShape<T, NW, VT, NWT>;
     static_assert(NWT >= NW, "the sorting warps take part in the merge rounds");
     constexpr int TILE = Sh::TILE, WT = Sh::WTILE;
@@ -140,88 +145,95 @@ __global__ void __launch_bounds__(NWT * 32, MINB) warp_block_sort_kernel(const T
     __shared__ int split[TILE / (VT - 1) + TILE / (2 * R0) + 4];
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
-    const uint64_t base = (uint64_t)blockIdx.x * TILE;
     static_assert(VT % Vec<T>::N == 0, "lanes load whole vectors");
-    const int valid = (int)((n - base) < (uint64_t)TILE ? (n - base) : (uint64_t)TILE);
     const int w0 = warp * WT;
-    if (err && blockIdx.x == 0 && tid == 0) *err = 0;
-    if (ahead && tid == 0) {
-        const uint64_t pb = base + (uint64_t)ahead * TILE;
-        if (pb + TILE <= n) bulk_prefetch_l2(in + pb, (uint32_t)(TILE * sizeof(T)));
+    uint64_t base = (uint64_t)blockIdx.x * TILE;
+    if constexpr (BEHIND) {
+        if (blockIdx.x == 0 && tid < 2) tcount[tid] = 0;
+        if (*route == 0) return;
     }
+    do {
+        const int valid = (int)((n - base) < (uint64_t)TILE ? (n - base) : (uint64_t)TILE);
+        if (err && blockIdx.x == 0 && tid == 0) *err = 0;
+        if (ahead && tid == 0) {
+            const uint64_t pb = base + (uint64_t)ahead * TILE;
+            if (pb + TILE <= n) bulk_prefetch_l2(in + pb, (uint32_t)(TILE * sizeof(T)));
+        }
 
-    // each lane loads VT keys with 16-byte vector loads; a partial tail is
-    // filled with the largest key. When a chunk spans the warp's whole run the
-    // lanes' keys may come from anywhere in it, so the loads are striped
-    // (each instruction reads 512 contiguous bytes); smaller chunks need each
-    // lane to hold its own VT consecutive keys (blocked).
-    constexpr int V = Vec<T>::N;
-    T v[VT];
-    const bool sorter = warp < NW;
-    if (sorter) {
-        const bool striped = chunk >= WT;
-#pragma unroll
-        for (int j = 0; j < VT / V; ++j) {
-            const int i0 = striped ? w0 + j * 32 * V + lane * V : w0 + lane * VT + j * V;
-            const T* src = in + base + i0;
-            if (i0 + V <= valid) {
-                const uint4 q = *reinterpret_cast<const uint4*>(src);
-                const T* e = reinterpret_cast<const T*>(&q);
-#pragma unroll
-                for (int k = 0; k < V; ++k) v[j * V + k] = Traits<T>::flip(e[k], xin);
-            } else {
-#pragma unroll
-                for (int k = 0; k < V; ++k)
-                    v[j * V + k] = (i0 + k < valid) ? Traits<T>::flip(src[k], xin) : Traits<T>::max_item();
-            }
-        }
-        warp_sort<T, VT>(v, chunk < R0 ? chunk : R0);
-    }
-    if (R0 < TILE && R0 < chunk) {
+        // each lane loads VT keys with 16-byte vector loads; a partial tail is
+        // filled with the largest key. When a chunk spans the warp's whole run the
+        // lanes' keys may come from anywhere in it, so the loads are striped
+        // (each instruction reads 512 contiguous bytes); smaller chunks need each
+        // lane to hold its own VT consecutive keys (blocked).
+        constexpr int V = Vec<T>::N;
+        T v[VT];
+        const bool sorter = warp < NW;
         if (sorter) {
+            const bool striped = chunk >= WT;
 #pragma unroll
-            for (int k = 0; k < VT; ++k) sa[pad<T>(w0 + lane * VT + k)] = v[k];
-        }
-        __syncthreads();
-        merge_round_uniform<T, Sh::NTM, VT, false, PadIdx<T>>(sa, sb, R0, TILE, split);
-        T* src = sb;
-        T* dst = sa;
-        for (int w = 2 * R0; w < TILE && w < chunk; w <<= 1) {
-            merge_round_uniform<T, Sh::NTM, VT, false, LinIdx>(src, dst, w, TILE, split);
-            T* t = src;
-            src = dst;
-            dst = t;
-        }
-        // coalesced 16-byte stores of the sorted tile
-        const int nvec = valid / V;
-        for (int i = tid; i < nvec; i += Sh::NTM) {
-            const uint4 q = *reinterpret_cast<const uint4*>(src + (size_t)i * V);
-            T e[V];
-            const T* qe = reinterpret_cast<const T*>(&q);
+            for (int j = 0; j < VT / V; ++j) {
+                const int i0 = striped ? w0 + j * 32 * V + lane * V : w0 + lane * VT + j * V;
+                const T* src = in + base + i0;
+                if (i0 + V <= valid) {
+                    const uint4 q = *reinterpret_cast<const uint4*>(src);
+                    const T* e = reinterpret_cast<const T*>(&q);
 #pragma unroll
-            for (int k = 0; k < V; ++k) e[k] = Traits<T>::flip(qe[k], xout);
-            *reinterpret_cast<uint4*>(out + base + (size_t)i * V) = *reinterpret_cast<const uint4*>(e);
-        }
-        for (int i = nvec * V + tid; i < valid; i += Sh::NTM) out[base + i] = Traits<T>::flip(src[i], xout);
-        if constexpr (SAMPLES) kb_emit_samples<T>(src, base, valid, samp, ssamp, Sh::NTM);
-    } else if (sorter) {
-        // runs end at the warp (or chunk) size: each lane stores its own keys
-        const int i0 = w0 + lane * VT;
-        T* dp = out + base + i0;
+                    for (int k = 0; k < V; ++k) v[j * V + k] = Traits<T>::flip(e[k], xin);
+                } else {
 #pragma unroll
-        for (int j = 0; j < VT / V; ++j) {
-            if (i0 + (j + 1) * V <= valid) {
+                    for (int k = 0; k < V; ++k)
+                        v[j * V + k] = (i0 + k < valid) ? Traits<T>::flip(src[k], xin) : Traits<T>::max_item();
+                }
+            }
+            warp_sort<T, VT>(v, chunk < R0 ? chunk : R0);
+        }
+        if (R0 < TILE && R0 < chunk) {
+            if (sorter) {
+#pragma unroll
+                for (int k = 0; k < VT; ++k) sa[pad<T>(w0 + lane * VT + k)] = v[k];
+            }
+            __syncthreads();
+            merge_round_uniform<T, Sh::NTM, VT, false, PadIdx<T>>(sa, sb, R0, TILE, split);
+            T* src = sb;
+            T* dst = sa;
+            for (int w = 2 * R0; w < TILE && w < chunk; w <<= 1) {
+                merge_round_uniform<T, Sh::NTM, VT, false, LinIdx>(src, dst, w, TILE, split);
+                T* t = src;
+                src = dst;
+                dst = t;
+            }
+            // coalesced 16-byte stores of the sorted tile
+            const int nvec = valid / V;
+            for (int i = tid; i < nvec; i += Sh::NTM) {
+                const uint4 q = *reinterpret_cast<const uint4*>(src + (size_t)i * V);
                 T e[V];
+                const T* qe = reinterpret_cast<const T*>(&q);
 #pragma unroll
-                for (int k = 0; k < V; ++k) e[k] = Traits<T>::flip(v[j * V + k], xout);
-                *reinterpret_cast<uint4*>(dp + j * V) = *reinterpret_cast<const uint4*>(e);
-            } else {
+                for (int k = 0; k < V; ++k) e[k] = Traits<T>::flip(qe[k], xout);
+                *reinterpret_cast<uint4*>(out + base + (size_t)i * V) = *reinterpret_cast<const uint4*>(e);
+            }
+            for (int i = nvec * V + tid; i < valid; i += Sh::NTM) out[base + i] = Traits<T>::flip(src[i], xout);
+            if constexpr (SAMPLES) kb_emit_samples<T>(src, base, valid, samp, ssamp, Sh::NTM);
+        } else if (sorter) {
+            // runs end at the warp (or chunk) size: each lane stores its own keys
+            const int i0 = w0 + lane * VT;
+            T* dp = out + base + i0;
 #pragma unroll
-                for (int k = 0; k < V; ++k)
-                    if (i0 + j * V + k < valid) dp[j * V + k] = Traits<T>::flip(v[j * V + k], xout);
+            for (int j = 0; j < VT / V; ++j) {
+                if (i0 + (j + 1) * V <= valid) {
+                    T e[V];
+#pragma unroll
+                    for (int k = 0; k < V; ++k) e[k] = Traits<T>::flip(v[j * V + k], xout);
+                    *reinterpret_cast<uint4*>(dp + j * V) = *reinterpret_cast<const uint4*>(e);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < V; ++k)
+                        if (i0 + j * V + k < valid) dp[j * V + k] = Traits<T>::flip(v[j * V + k], xout);
+                }
             }
         }
-    }
+        if (BEHIND) __syncthreads();
+    } while (BEHIND && (base += (uint64_t)gridDim.x * TILE) < n);
 }
 
 // Geometry of one binary pass: runs of `run` items (the last one may be short)

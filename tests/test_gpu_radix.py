@@ -126,6 +126,66 @@ def test_radix_chunks(kind, sort_n, second):
     assert np.array_equal(device_sort(a, kind, sort_n=sort_n), expected(a, sort_n))
 
 
+def device_keys(dist, n, sort_n):
+    """n uint32 keys (int32 storage): all of one distribution, or one chunk of it."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    k = torch.randint(-(2**31), 2**31, (n,), dtype=torch.int32, device="cuda", generator=g)
+    u = torch.rand(n, device="cuda", dtype=torch.float64, generator=g)
+    if dist == "zipf":
+        return (torch.exp(u * np.log(2.0**20)).long() * 0x9E3779B1).to(torch.int32)
+    if dist == "log":
+        return torch.exp2(u * 30.99).to(torch.int32)
+    if dist == "sixteen":
+        return (k & 15) * 0x1E3779B1
+    if dist == "one chunk":
+        k[sort_n:2 * sort_n] = (torch.exp(u[:sort_n] * np.log(2.0**20)).long() * 0x9E3779B1).to(torch.int32)
+    return k
+
+
+def merged(src, sort_n):
+    d, t = src.clone(), torch.empty_like(src)
+    return og.sort(d, t, kind=og.U32, sort_n=sort_n, min_k=2)
+
+
+# chunks of uint32 keys that the buckets give up: merges stand behind them up to chunks of
+# 2^17 keys (sorts of 2^22 and more), levels up to 2^20 (2^25), radix passes elsewhere; the
+# sizes on either side, a short last chunk
+@pytest.mark.parametrize("n, sort_n", [(1 << 22, 1 << 16), ((1 << 22) - 1, 1 << 16), ((1 << 22) + 8191, 1 << 17),
+                                       ((1 << 22) + 1, 1 << 18), ((1 << 25) + 77, 1 << 17), (1 << 25, 1 << 18),
+                                       ((1 << 25) + 4099, 1 << 20), ((1 << 25) - 1, 1 << 20), ((1 << 25) + 1, 1 << 21)])
+@pytest.mark.parametrize("dist", ["uniform", "zipf", "log", "sixteen", "one chunk"])
+@pytest.mark.parametrize("in_tmp", [False, True])
+def test_skewed_chunks(n, sort_n, dist, in_tmp):
+    src = device_keys(dist, n, sort_n)
+    d, t = src.clone(), torch.empty_like(src)
+    got = og.sort(d, t, kind=og.U32, sort_n=sort_n, result_in_tmp=in_tmp)
+    assert got.data_ptr() == (t if in_tmp else d).data_ptr()
+    assert torch.equal(got, merged(src, sort_n))
+
+
+@pytest.mark.parametrize("sort_n, dist, most", [(1 << 16, "zipf", 1.75), (1 << 17, "zipf", 1.6), (1 << 19, "sixteen", 1.2),
+                                                (1 << 20, "zipf", 1.35)])
+def test_skewed_chunks_keep_pace(sort_n, dist, most):
+    # against merges, 1.41, 1.25, 0.75 and 1.18 times their time (radix passes 2.31, 1.93,
+    # 1.57 and 1.41)
+    src = device_keys(dist, 1 << 26, sort_n)
+    d, t = torch.empty_like(src), torch.empty_like(src)
+
+    def ms(min_k):
+        best = 1e9
+        for _ in range(6):
+            d.copy_(src)
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            og.sort(d, t, kind=og.U32, sort_n=sort_n, min_k=min_k)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    assert ms(0) < most * ms(2)
+
+
 # five chunks, the last one short: their sorts leave signed keys in the internal order
 @pytest.mark.parametrize("dist", ["uniform", "equal", "zipf", "log", "repeated"])
 @pytest.mark.parametrize("kind", [og.U32, og.U64, og.I64, og.KV64, og.KVU64])
