@@ -1396,9 +1396,11 @@ int origami_tuning_save(const char* path) {
     for (int k = 0; k < 5; ++k)
         for (int c = 0; c < TUNE_CLASSES; ++c) {
             const int code = g_tune[k][c].load(std::memory_order_relaxed), shape = code & ~SHAPE_RADIX;
-            if (shape != shape_code(2, 0)) std::fprintf(f, "%d %d %d %d\n", k, c, shape_fan(code), shape_variant(code));
-            // the radix choice, where loading the shape alone would give another
             const int b = tune_builtin(k, c);
+            // the shape, where it is not the built-in one, and where it is not the common one
+            if (shape != shape_code(2, 0) || shape != (b & ~SHAPE_RADIX))
+                std::fprintf(f, "%d %d %d %d\n", k, c, shape_fan(code), shape_variant(code));
+            // the radix choice, where loading the shape alone would give another
             if (code != (shape == (b & ~SHAPE_RADIX) ? b : shape))
                 std::fprintf(f, "radix %d %d %d\n", k, c, (code & SHAPE_RADIX) ? 1 : 0);
         }

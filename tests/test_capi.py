@@ -133,6 +133,28 @@ def test_tuning_table_roundtrip(lib, tmp_path):
     og.tuning_set(og.KV64, 1 << 27, *built_in_kv)
 
 
+@pytest.mark.parametrize("kind, cls, shape", [(0, 18, (2, 0)), (0, 20, (2, 0)), (3, 27, (2, 0)), (1, 20, (16, 0)), (1, 21, (2, 2))])
+def test_tuning_file_restores_a_fresh_process(lib, tmp_path, kind, cls, shape):
+    # classes with other built-in shapes set to the common one, and the other way round: a
+    # process that loads the file has the same table, and would save the same file
+    import subprocess
+    import sys
+    path = tmp_path / "tune.txt"
+    run = ("import sys; sys.path.insert(0, sys.argv[1]); import origami_gpu as og; k, c = int(sys.argv[2]), int(sys.argv[3])\n"
+           "{}\nprint(*og.tuning_get(k, 1 << c)); og.tuning_save(sys.argv[4])")
+
+    def process(do, out):
+        pkg = os.path.dirname(os.path.dirname(os.path.abspath(og.__file__)))
+        r = subprocess.run([sys.executable, "-c", run.format(do), pkg, str(kind), str(cls), str(out)],
+                           capture_output=True, text=True, check=True)
+        return tuple(int(x) for x in r.stdout.split())
+
+    assert process(f"og.tuning_set(k, 1 << c, *{shape})", path) == shape
+    again = tmp_path / "again.txt"
+    assert process(f"og.tuning_load({str(path)!r})", again) == shape
+    assert again.read_text() == path.read_text()
+
+
 def test_noalloc_rejects_bad_arguments_on_the_host(lib):
     # pure host checks, made before the library looks for a device: no buffer
     # below is ever read or written (they are small host arrays)
