@@ -110,14 +110,23 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
+// SMs of the current device.
+inline uint32_t sm_count() {
+    static const uint32_t n = [] {
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        return (uint32_t)(sms > 0 ? sms : 1);
+    }();
+    return n;
+}
+
 // Resident CTAs of a kernel on the whole GPU; sets its shared-memory limit.
 inline uint32_t resident_ctas(const void* kernel, int nt, size_t smem) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int per = 0;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, nt, smem);
-    return (uint32_t)(sms * (per > 0 ? per : 1));
+    return sm_count() * (uint32_t)(per > 0 ? per : 1);
 }
 
 // One binary-pass merge shape: pair_merge_kernel (one tile per CTA, cp.async

@@ -34,10 +34,8 @@
 //
 // What bounds it (2^28 uint32 keys, one GB300): the shared-memory pipe. A step
 // of 32 keys costs about 25 cycles of it (five random accesses of 3.5 bank
-// conflicts each), 0.86 ms a pass against 0.32 ms of HBM traffic; 2^27 uint64
-// keys 0.60, 2^26 pairs 0.51 ms, where the look-back is 0.1 of it. Whole sorts:
-// 1 GiB uint32 7.38 -> 3.79 ms, 1 GiB uint64 8.44 -> 5.17, 2^27 pairs 14.0 ->
-// 8.47 ms.
+// conflicts each), 0.86 ms a pass against 0.32 ms of HBM traffic. Whole sorts:
+// 1 GiB uint32 7.38 ms by merges, 3.79 by radix passes alone.
 //
 // Every wait is bounded (`spin` polls): on expiry the CTA records
 // ERR_WAIT_EXPIRED and stops, waiting CTAs see the word and stop, later passes
@@ -61,14 +59,12 @@ struct RadixCfg<uint32_t> {
     static constexpr int HIST_COPIES = 8;
 };
 template <>
-struct RadixCfg<uint64_t> {
+struct RadixCfg<uint64_t> {  // (whole tiles a chunk only)
     static constexpr int NT = 256, IPT = 16, MINB = 3;  // 4096 keys, 32 KiB
-    static constexpr int HIST_COPIES = 8;
 };
 template <>
-struct RadixCfg<KV64> {
+struct RadixCfg<KV64> {  // (the partition of the bucket sort)
     static constexpr int NT = 256, IPT = 16, MINB = 2;  // 4096 pairs, 64 KiB
-    static constexpr int HIST_COPIES = 8;
 };
 
 template <class T>
@@ -79,19 +75,11 @@ struct RadixShape {
     static constexpr int DIGITS = (int)sizeof(typename Traits<T>::Key);  // 8-bit digits of a key
     static constexpr size_t KEYS_BYTES = (size_t)TILE * sizeof(T);
     static constexpr size_t SMEM = KEYS_BYTES + (size_t)NG * RADIX_BINS * 4;
-    static constexpr size_t HIST_SMEM = (size_t)DIGITS * RADIX_BINS * C::HIST_COPIES * 4;
     static_assert(NT >= RADIX_BINS, "one thread per bin");
 };
 
-// Digit `byte` of an item's key, in the order of the sort: `dx` flips the sign
-// bit of signed keys (nonzero for the top digit only).
-__device__ __forceinline__ unsigned radix_digit(uint32_t k, int byte, unsigned dx) {
-    return __byte_perm(k, 0, 0x4440 | byte) ^ dx;
-}
-__device__ __forceinline__ unsigned radix_digit(uint64_t k, int byte, unsigned dx) {
-    const uint32_t w = byte >= 4 ? (uint32_t)(k >> 32) : (uint32_t)k;
-    return __byte_perm(w, 0, 0x4440 | (byte & 3)) ^ dx;
-}
+// Digit `byte` of a key.
+__device__ __forceinline__ unsigned radix_digit(uint32_t k, int byte) { return __byte_perm(k, 0, 0x4440 | byte); }
 
 // Lanes of the warp whose digit equals this lane's: eight ballots, each turned
 // round where this lane's bit is 0. (Written as PTX: from C++ the same ballots
@@ -177,9 +165,13 @@ struct RadixUniform {
 // there yet (the passes are an even number and end where they start).
 // route (optional): the radix passes stand behind a bucket sort (buckets.cuh);
 // 0: it has done the work, return; 2: the items are in `moved` instead of `in`.
+template <class T>
+constexpr size_t radix_hist_smem() {
+    return (size_t)RadixShape<T>::DIGITS * RADIX_BINS * RadixCfg<T>::HIST_COPIES * 4;
+}
 template <class T, class S, class G>
 __global__ void __launch_bounds__(512) radix_hist_kernel(const T* in0, const T* moved, T* want, G geo, uint32_t tiles,
-                                                         uint64_t xmask, S* hist, S* look0, const int* route) {
+                                                         S* hist, S* look0, const int* route) {
     using Sh = RadixShape<T>;
     constexpr int D = Sh::DIGITS, C = Sh::C::HIST_COPIES, TILE = Sh::TILE;
     extern __shared__ __align__(16) uint32_t cnt_sm[];
@@ -213,9 +205,9 @@ __global__ void __launch_bounds__(512) radix_hist_kernel(const T* in0, const T* 
         __syncthreads();
     };
     auto count = [&](const T& v) {
-        const auto k = Traits<T>::key(Traits<T>::flip(v, xmask));
+        const auto k = Traits<T>::key(v);
 #pragma unroll
-        for (int b = 0; b < D; ++b) atomicAdd(&cnt_sm[(b * RADIX_BINS + radix_digit(k, b, 0)) * C + col], 1u);
+        for (int b = 0; b < D; ++b) atomicAdd(&cnt_sm[(b * RADIX_BINS + radix_digit(k, b)) * C + col], 1u);
     };
     uint32_t seg = 0xFFFFFFFFu;
     for (uint32_t t = t0; t < t1; ++t) {
@@ -257,7 +249,8 @@ __global__ void __launch_bounds__(512) radix_hist_kernel(const T* in0, const T* 
 }
 
 // Exclusive scan over the 256 bins (one value per thread of the first 8 warps;
-// `ws` is 8 values of scratch). Every thread of the CTA calls it; two barriers.
+// `ws` is 8 values of scratch). Every thread of the CTA calls it. One barrier inside,
+// and `ws` is read behind it: it is free again only after another one.
 template <class S>
 __device__ __forceinline__ S radix_bin_scan(S v, S* ws) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -282,13 +275,9 @@ template <class T, class S>
 struct ByteDigit {
     static constexpr bool kHeavy = true;  // any share of the items may have one digit
     const S* hist;
-    uint64_t xmask;
     int byte;
-    unsigned dx;
-    ByteDigit(const S* h, uint64_t x, int b) : hist(h), xmask(x), byte(b), dx((unsigned)(x >> (8 * b)) & 255u) {}
-    __device__ __forceinline__ unsigned operator()(const T& v) const {
-        return radix_digit(Traits<T>::key(v), byte, dx);
-    }
+    ByteDigit(const S* h, int b) : hist(h), byte(b) {}
+    __device__ __forceinline__ unsigned operator()(const T& v) const { return radix_digit(Traits<T>::key(v), byte); }
     __device__ __forceinline__ void enter(uint32_t) {}  // a tile of this segment follows
     __device__ __forceinline__ S count(uint32_t seg, int bin) const {
         return hist[((size_t)seg * RadixShape<T>::DIGITS + byte) * RADIX_BINS + bin];
@@ -300,26 +289,16 @@ struct ByteDigit {
     }
 };
 
-// (32-bit keys are unsigned already)
-template <class T>
-__device__ __forceinline__ T radix_flip(const T& v, uint64_t x) {
-    if constexpr (sizeof(typename Traits<T>::Key) == 4)
-        return v;
-    else
-        return Traits<T>::flip(v, x);
-}
-
 // One pass: src -> dst by one digit. look: this pass's words, 256 per tile, zero
 // at launch; look_next (optional): the next pass's, cleared here. route
 // (optional): run only where it holds `run` (radix passes behind a bucket sort
-// run unless it is 0, the stable partition of a bucket sort while it is 0). xflip:
-// applied to the keys as they are written. (No early start of the next pass: its waiting
+// run unless it is 0, the stable partition of a bucket sort while it is 0). (No early start of the next pass: its waiting
 // CTAs cost more than its launch, 2^20 uint32 Zipf keys 0.078 ms without and 0.111 with.)
 template <class T, class S, class G, class D>
 __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
     radix_pass_kernel(const T* src, T* dst, G geo, uint32_t tiles, D digit, S* look,
                       S* look_next, unsigned* claim, int* err, uint32_t spin,
-                      const int* route, bool buckets, uint64_t xflip) {
+                      const int* route, bool buckets) {
     using Sh = RadixShape<T>;
     using W = LookWord<S>;
     constexpr int NT = Sh::NT, IPT = Sh::IPT, NG = Sh::NG, TILE = Sh::TILE;
@@ -350,7 +329,7 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
             if (heavy && __syncthreads_or(h == (S)q.slen)) {
                 // one digit only: the segment keeps its order. (A tile of it
                 // takes no part in the look-back, like all the others.)
-                for (int i = tid; i < q.cnt; i += NT) dst[q.base + i] = radix_flip(src[q.base + i], xflip);
+                for (int i = tid; i < q.cnt; i += NT) dst[q.base + i] = src[q.base + i];
                 if (look_next)
                     for (int i = tid; i < RADIX_BINS; i += NT) look_next[(size_t)t * RADIX_BINS + i] = 0;
                 if (tid == 0) next_tile = atomicAdd(claim, 1u);
@@ -503,7 +482,7 @@ __global__ void __launch_bounds__(RadixCfg<T>::NT, RadixCfg<T>::MINB)
             const T x = skeys[p];
             const S o = goff[digit(x)] + (S)p;
             // (o < slen always holds while the input does not change under the sort)
-            if (p < q.cnt && o < (S)q.slen) out[o] = radix_flip(x, xflip);
+            if (p < q.cnt && o < (S)q.slen) out[o] = x;
         }
         __syncthreads();
     }

@@ -45,8 +45,9 @@ struct RadixPlan {
 };
 
 // Bucket sort of a full sort or of chunks: bits per level, 0 when it does not
-// take the call (buckets would be larger than half of what fits, or the items
-// too few for 16 buckets).
+// take the call: more than 65,536 buckets of the mean size (2^LOG_TARGET: two thirds of
+// what fits for uint32 keys, half for wider items), so sorts and chunks of 2^28 + 65,536
+// uint32 keys, 2^27 + 65,536 wider items and more; or fewer than 16 buckets.
 template <class T>
 struct BucketPlan {
     using Sh = BucketShape<T>;
@@ -71,7 +72,7 @@ struct BucketPlan {
     // rows of counts where one read counts both levels (one segment): one for every SM,
     // and four tiles each
     uint32_t rows(const RadixPlan<T>& p) const {
-        return b2 && p.nseg == 1 ? (uint32_t)std::min<uint64_t>(152, (tiles + 3) / 4) : 0u;
+        return b2 && p.nseg == 1 ? (uint32_t)std::min<uint64_t>(sm_count(), (tiles + 3) / 4) : 0u;
     }
 };
 
@@ -193,13 +194,13 @@ uint64_t radix_scratch_bytes(uint64_t n, uint64_t sort_n) {
 // The radix passes: d -> want (d or tmp). With `route` they stand behind a
 // bucket sort and run only where it gave up.
 template <class T, class S>
-void radix_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, uint64_t xmask, uint64_t xout, const RadixScratch<T>& sc,
-                  const int* route, cudaStream_t st) {
+void radix_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const RadixScratch<T>& sc, const int* route,
+                  cudaStream_t st) {
     using Sh = RadixShape<T>;
     using G = RadixUniform;
     using D = ByteDigit<T, S>;
     // kernel attributes and grids, once per process
-    static const uint32_t g_hist = resident_ctas((const void*)radix_hist_kernel<T, S, G>, 512, Sh::HIST_SMEM);
+    static const uint32_t g_hist = resident_ctas((const void*)radix_hist_kernel<T, S, G>, 512, radix_hist_smem<T>());
     static const uint32_t g_pass = resident_ctas((const void*)radix_pass_kernel<T, S, G, D>, Sh::NT, Sh::SMEM);
     static const std::string n_hist = std::string("radix_hist<") + TypeName<T>::v + ">";
     static const std::string n_pass = std::string("radix_pass<") + TypeName<T>::v + ">";
@@ -207,8 +208,8 @@ void radix_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, uint64_t xmask, 
     const G geo{p.n, p.len, p.shift};
     S* hist = static_cast<S*>(sc.hist);
     launch(n_hist.c_str(), st, [&] {
-        launch_dependent(radix_hist_kernel<T, S, G>, dim3(std::min(tiles, g_hist)), dim3(512), Sh::HIST_SMEM, st,
-                         (const T*)d, (const T*)tmp, want, geo, tiles, xmask, hist, static_cast<S*>(sc.look[0]), route);
+        launch_dependent(radix_hist_kernel<T, S, G>, dim3(std::min(tiles, g_hist)), dim3(512), radix_hist_smem<T>(), st,
+                         (const T*)d, (const T*)tmp, want, geo, tiles, hist, static_cast<S*>(sc.look[0]), route);
     });
     T* src = want;
     T* dst = want == d ? tmp : d;
@@ -216,9 +217,9 @@ void radix_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, uint64_t xmask, 
     for (int b = 0; b < Sh::DIGITS; ++b) {
         launch(n_pass.c_str(), st, [&] {
             launch_dependent(radix_pass_kernel<T, S, G, D>, dim3(std::min(tiles, g_pass)), dim3(Sh::NT), Sh::SMEM, st,
-                             (const T*)src, dst, geo, tiles, D(hist, xmask, b), static_cast<S*>(sc.look[b & 1]),
+                             (const T*)src, dst, geo, tiles, D(hist, b), static_cast<S*>(sc.look[b & 1]),
                              b + 1 < Sh::DIGITS ? static_cast<S*>(sc.look[(b + 1) & 1]) : (S*)nullptr, sc.claim + b,
-                             sc.err, wait_limit(), route, false, b + 1 < Sh::DIGITS ? 0ull : xmask ^ xout);
+                             sc.err, wait_limit(), route, false);
         });
         std::swap(src, dst);
     }
@@ -318,7 +319,7 @@ void bucket_launch(T* d, T* tmp, T* want, const RadixPlan<T>& p, const BucketPla
                 launch_dependent(radix_pass_kernel<T, uint32_t, G, D>, dim3(std::min(tiles_l, g_part)), dim3(RSh::NT),
                                  RSh::SMEM, st, src, dst, geo_l, tiles_l, dig, static_cast<uint32_t*>(look),
                                  static_cast<uint32_t*>(look_next), claim, sc.err, wait_limit(), (const int*)sc.route,
-                                 true, 0ull);
+                                 true);
             } else {
                 launch_dependent(bk_pass_kernel<T, G>, dim3(tiles_l), dim3(Sh::C::NT), Sh::PASS_SMEM, st, src, dst, geo_l,
                                  tiles_l, (const SliceMap<K>*)sc.maps, map_shift, xmask, shift_l, bits_l, cursor, n32,
@@ -406,9 +407,9 @@ cudaError_t radix_sort(T* d, T* tmp, uint64_t n, uint64_t sort_n, uint64_t key_m
                                        scratch, st, nullptr, &after);
         }
         if (p.wide)
-            radix_launch<T, uint64_t>(d, tmp, want, p, key_mask, out_mask, sc, route, st);
+            radix_launch<T, uint64_t>(d, tmp, want, p, sc, route, st);
         else
-            radix_launch<T, uint32_t>(d, tmp, want, p, key_mask, out_mask, sc, route, st);
+            radix_launch<T, uint32_t>(d, tmp, want, p, sc, route, st);
     }
     return cudaGetLastError();
 }

@@ -129,7 +129,6 @@ struct __align__(16) SbTile {  // one tile of a level
 struct __align__(16) SbRec {  // one bucket
     uint64_t base, what;      // first item; length and flags
     static constexpr uint64_t TMP = 1ull << 62;   // the items are in tmp (else in d)
-    static constexpr uint64_t COPY = 1ull << 61;  // equal keys: move only
     static constexpr uint64_t SLOW = 1ull << 60;  // does not fit: sorted in global memory
     static constexpr uint64_t LEN = (1ull << 60) - 1;
 };
@@ -518,7 +517,7 @@ __device__ __forceinline__ void sb_hand_on(const SbTile& q, S h, const Map& map,
             for (uint64_t i = tid; i * CAP < pl; i += NT) {
                 const uint64_t rest = pl - i * CAP;
                 to.recs[at + goff[k] + i] =
-                    SbRec{q.sbase + p0 + i * CAP, (rest < (uint64_t)CAP ? rest : (uint64_t)CAP) | SbRec::COPY | to.flags};
+                    SbRec{q.sbase + p0 + i * CAP, (rest < (uint64_t)CAP ? rest : (uint64_t)CAP) | to.flags};
             }
         }
     }
@@ -1005,7 +1004,7 @@ __global__ void __launch_bounds__(SegBucketCfg<T>::NT, SegBucketCfg<T>::MINB)
 }
 
 // ------------------------------------------------------------ bucket sort ---
-// One step of a stable byte pass, as bk_stable_pass_kernel ranks: every 16 lanes
+// One step of a stable byte pass, as radix_pass_kernel ranks: every 16 lanes
 // own a stretch of items and 256 words of `table`; the words hold the items' next
 // places when it returns from sb_byte_count (which gives thread b < 256 the count
 // of digit b), and sb_byte_place calls put(place, i) for every item i.
