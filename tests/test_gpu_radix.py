@@ -212,6 +212,73 @@ def test_radix_long_segment():
         assert bool((x[1:] >= x[:-1]).all())
 
 
+def mix(i):
+    """A bijection of 64-bit words."""
+    i = i * -0x61C8864680B583EB
+    i = i ^ (i >> 32 & 0xFFFFFFFF)
+    return i * -0x3B314601E57A13AD
+
+
+def unmix(k):
+    inv = lambda m: pow(m, -1, 2**64) - 2**64  # noqa: E731  (as a negative number)
+    k = k * torch.tensor(inv(-0x3B314601E57A13AD & 2**64 - 1), device=k.device)
+    k = k ^ (k >> 32 & 0xFFFFFFFF)
+    return k * torch.tensor(inv(-0x61C8864680B583EB & 2**64 - 1), device=k.device)
+
+
+# the longest sorts that buckets take and the shortest that they don't (levels alone), and
+# those whose counts need 64 bits: pairs from 2^30 items, keys from 2^32
+@pytest.mark.parametrize("kind, n", [("u64", (1 << 27) + 65535), ("u64", (1 << 27) + 65536), ("kvu64", (1 << 27) + 65535),
+                                     ("kvu64", (1 << 27) + 65537), ("kvu64", (1 << 30) + 3), ("u64", (1 << 32) + 5)])
+def test_long_sorts(kind, n):
+    pairs = kind == "kvu64"
+    piece = 1 << 27
+    d = torch.empty((n, 2) if pairs else n, dtype=torch.int64, device="cuda")
+    for i in range(0, n, piece):
+        x = torch.arange(i, min(n, i + piece), device="cuda")
+        if pairs:  # every key twice
+            d[i:i + piece, 0] = mix(x >> 1)
+            d[i:i + piece, 1] = x
+        else:
+            d[i:i + piece] = mix(x)
+    t = torch.empty_like(d)
+    out = og.sort(d.view(-1), t.view(-1), kind=kind).view(d.shape)
+    del t
+    for i in range(0, n, piece):
+        x = out[i:i + piece + 1]
+        k = (x[:, 0] if pairs else x) ^ -(2**63)
+        v = x[:, 1] if pairs else unmix(x)
+        # strictly ascending (key, value), of values that belong to them: a permutation
+        assert bool((v >= 0).all()) and bool((v < n).all())
+        if pairs:
+            assert torch.equal(mix(v >> 1), x[:, 0])
+            assert bool(((k[1:] > k[:-1]) | ((k[1:] == k[:-1]) & (v[1:] > v[:-1]))).all())
+        else:
+            assert bool((k[1:] > k[:-1]).all())
+
+
+@pytest.mark.parametrize("n", [(1 << 28) + 65535, (1 << 28) + 65536])
+def test_long_uint32_sorts(n):
+    g = torch.Generator(device="cuda").manual_seed(4)
+    src = torch.randint(-(2**31), 2**31, (n,), dtype=torch.int32, device="cuda", generator=g)
+    out = og.sort(src.clone(), torch.empty_like(src), kind="u32")
+    assert torch.equal(out ^ -(2**31), torch.sort(src ^ -(2**31)).values)
+
+
+# (2^31 keys in chunks and more: merges, as the bucket sort does not take them)
+def test_chunks_beyond_the_bucket_sort():
+    n, sort_n = (1 << 31) + 9, 1 << 20
+    g = torch.Generator(device="cuda").manual_seed(6)
+    src = torch.randint(-(2**31), 2**31, (n,), dtype=torch.int32, device="cuda", generator=g)
+    d, t = src.clone(), torch.empty_like(src)
+    out = og.sort(d, t, kind="u32", sort_n=sort_n) ^ -(2**31)
+    for i in range(0, n, 1 << 28):
+        want = src[i:i + (1 << 28)] ^ -(2**31)
+        whole = len(want) // sort_n * sort_n
+        assert torch.equal(out[i:i + whole], torch.sort(want[:whole].view(-1, sort_n)).values.view(-1))
+        assert torch.equal(out[i + whole:i + len(want)], torch.sort(want[whole:]).values)
+
+
 @pytest.mark.parametrize("kind", [og.U32, og.KV64])
 def test_radix_reports_expired_wait_then_recovers(kind):
     n = 1 << 20

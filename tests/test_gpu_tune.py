@@ -102,3 +102,28 @@ def test_concurrent_streams(kind, variant):
             assert np.array_equal(r.cpu().numpy().view(a.dtype), expected(a))
     finally:
         og.tuning_set(kind, n, *prev)
+
+
+# a class's built-in merge shape: set, it restores the built-in choice, buckets; by a file the
+# class sorts by merges of that shape
+@pytest.mark.parametrize("kind, n", [(og.U32, 300_007), (og.U32, (1 << 22) + 9), (og.U32, (1 << 23) + 1), (og.U64, 300_007),
+                                     (og.I64, (1 << 21) + 5), (og.KV64, (1 << 22) + 9), (og.KVU64, (1 << 25) + 3)])
+def test_built_in_merge_shape(kind, n, tmp_path):
+    a = make(kind, n, seed=n + kind)
+    fan, variant = og.tuning_get(kind, n)
+    f = tmp_path / "tuning"
+    f.write_text(f"radix {kind} {n.bit_length() - 1} 0\n")
+    try:
+        og.tuning_load(str(f))
+        assert og.tuning_get(kind, n) == (fan, variant)
+        d = torch.from_numpy(a.view(np.uint8).copy()).cuda()
+        og.profile_enable(True)
+        r = og.sort(d, torch.empty_like(d), kind=kind)
+        torch.cuda.synchronize()
+        names = {k.split("<")[0] for k in og.profile_report()}
+        og.profile_enable(False)
+        assert ("kway_merge" if fan > 2 else "pair_merge") in names and "bucket_sample" not in names
+        assert np.array_equal(r.cpu().numpy().view(a.dtype), expected(a))
+    finally:
+        og.profile_enable(False)
+        og.tuning_set(kind, n, fan, variant)
