@@ -1390,10 +1390,10 @@ __device__ __noinline__ void bk_sort_settled(const T* src, T* out, int cnt, uint
     if (!bk_settle_bucket<T>(src, out, cnt, xin, xout)) bk_sort_split<T>(src, out, cnt, xin, xout);
 }
 // A bucket that bk_sort_bucket<T, BK_LEAVE> left just now. Keys: by splitters. Pairs: where
-// a quarter of 64 items stand in bins of more items than a warp settles, and are alone with
-// their keys among 32, no bin of theirs would be settled. (2^25 pairs, groups of 200, keys
-// spread over their logarithms: 5.8 ms, 8.3 if settling is tried first; Zipf keys in groups
-// of 1000, which are settled, 1.47, by splitters 1.87.)
+// a quarter of 64 items share a bin of more items than a warp settles with one of 32 that
+// has another key, those bins would not be settled. (2^25 pairs, groups of 200, keys spread
+// over their logarithms: 5.8 ms, 8.3 if settling is tried first; Zipf keys in groups of 1000,
+// which are settled, 1.47, by splitters 1.87.)
 template <class T>
 __device__ __noinline__ void bk_sort_crowded(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
     __builtin_assume(__isGlobal(src));
@@ -1417,11 +1417,11 @@ __device__ __noinline__ void bk_sort_crowded(const T* src, T* out, int cnt, uint
         const uint32_t mul = (uint32_t)(((float)BINS * 4294967296.0f) / ((float)xr + 512.0f)) - 1u;
         const int p = cnt > TRIED ? cnt * tid / TRIED : min(tid, cnt - 1);
         const K k = Traits<T>::key(bk_flip(src[p], xin));
-        const unsigned same = __match_any_sync(0xFFFFFFFFu, k);
         // (the bins' words are their starts)
         const uint32_t b = __umulhi((uint32_t)(((k - klo) << c) >> 32), mul);
         const int s = (int)tab[b], e = b + 1 < BINS ? (int)tab[b + 1] : cnt;
-        odd = tid < cnt && (same & (same - 1u)) == 0 && e - s > Sh::SETTLED;
+        const unsigned others = __match_any_sync(0xFFFFFFFFu, b) & ~__match_any_sync(0xFFFFFFFFu, k);
+        odd = tid < cnt && others && e - s > Sh::SETTLED;
     }
     if (__syncthreads_count(odd) >= TRIED / 4 || !bk_settle_bucket<T>(src, out, cnt, xin, xout))
         bk_sort_split<T>(src, out, cnt, xin, xout);

@@ -26,6 +26,14 @@ struct SegBucketPlan {
         for (uint64_t m = (uint64_t)Sh::CAP / 2 << SB_SURE_BITS; levels && m < longest && levels < SB_MAX_LEVELS;
              m <<= levels == 2 ? SB_SURE_BITS - 2 : SB_SURE_BITS)
             ++levels;
+        // many segments: their work, not the launches, decides, and slices of equal width are
+        // the cheaper ones, so a level more than those need (2^26 normally distributed uint64
+        // keys in segments of 2^17: one level by splitters 1.43 ms, two levels 0.95)
+        if (levels && longest < n) {
+            int wide = 2;
+            for (uint64_t m = (uint64_t)Sh::CAP * 4 / 5 * RADIX_BINS; m < longest && wide < SB_MAX_LEVELS; m *= RADIX_BINS) ++wide;
+            levels = std::max(levels, wide);
+        }
         usual = 0;
         for (uint64_t m = (uint64_t)Sh::CAP * 4 / 5; m < n / std::max<uint64_t>(nseg, 1); m *= RADIX_BINS) ++usual;
         usual = std::max(usual, 1);
