@@ -29,6 +29,11 @@ ORIGAMI_DECLARE_SORT(u64)
 ORIGAMI_DECLARE_SORT(kv)
 #undef ORIGAMI_DECLARE_SORT
 
+// The k-way passes as what stands behind the bucket sort of chunks: sort_io for where
+// `route` says so, errors in `err`.
+cudaError_t sort_behind_u32(const void* in, void* out, void* wa, void* wb, uint64_t n, uint64_t sort_n, uint64_t xin,
+                            uint64_t xout, int fan, void* scratch, const int* route, int* err, cudaStream_t st);
+
 // Radix passes (radix.cuh): whether they take a sort of n items in chunks of
 // sort_n, the scratch they need (error word in its last 256 bytes) and the sort.
 #define ORIGAMI_DECLARE_RADIX(name)                                                                        \

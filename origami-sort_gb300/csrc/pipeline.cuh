@@ -376,7 +376,6 @@ uint64_t pipeline_scratch_bytes(uint64_t n, uint64_t sort_n, int code, uint64_t 
 // device memory.
 // behind (optional): the passes, all k-way, stand behind a bucket sort (buckets.cuh) of
 // chunks of 32-bit keys, and run only where it gave up.
-template <class T>
 struct PipeBehind {
     const int* route;
     int* err;  // its error word
@@ -384,7 +383,7 @@ struct PipeBehind {
 template <class T>
 cudaError_t sort_pipeline_io(const T* in, T* out, T* wa, T* wb, uint64_t n, uint64_t sort_n, uint64_t xin,
                              uint64_t xout, uint64_t start_run, int code, void* scratch, cudaStream_t st,
-                             LaunchStats* stats, const PipeBehind<T>* behind = nullptr) {
+                             LaunchStats* stats, const PipeBehind* behind = nullptr) {
     using C = Config<T>;
     using KC = KwayCfg<T>;
     constexpr int T1 = k1_tile<T>();

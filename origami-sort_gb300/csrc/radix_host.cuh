@@ -6,6 +6,7 @@
 #include <string>
 
 #include "buckets.cuh"
+#include "dispatch.h"
 #include "pipeline.cuh"
 #include "profiler.h"
 #include "radix.cuh"
@@ -394,17 +395,13 @@ cudaError_t radix_sort(T* d, T* tmp, uint64_t n, uint64_t sort_n, uint64_t key_m
         if (bk.on() && sizeof(typename Traits<T>::Key) == 8)
             plain = SbStarts{bk.b2 ? sc.start2 : sc.start1, (uint32_t)bk.nbuckets, !bk.b2};
         const SbGiven given{route, sc.start1, p.n, p.len, (uint32_t)p.nseg, bk.b2 ? (uint32_t)(p.nseg << bk.b1) : 0u};
-        if (q.wide)
-            segbucket_levels<T, uint64_t>(buf, given, plain, q, key_mask, out_mask, seg, st);
-        else
-            segbucket_levels<T, uint32_t>(buf, given, plain, q, key_mask, out_mask, seg, st);
+        segbucket_behind(buf, given, plain, q, key_mask, out_mask, seg, st);
         return cudaGetLastError();
     }
     if constexpr (sizeof(typename Traits<T>::Key) == 4) {
         if (rest == Behind::MERGES) {
-            const PipeBehind<T> after{route, sc.err};
-            return sort_pipeline_io<T>(d, want, want == d ? tmp : d, want, n, sort_n, key_mask, out_mask, 0, MERGES_CODE,
-                                       scratch, st, nullptr, &after);
+            return sort_behind_u32(d, want, want == d ? tmp : d, want, n, sort_n, key_mask, out_mask, MERGES_CODE,
+                                   scratch, route, sc.err, st);
         }
         if (p.wide)
             radix_launch<T, uint64_t>(d, tmp, want, p, sc, route, st);

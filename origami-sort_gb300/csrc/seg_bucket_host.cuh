@@ -188,6 +188,27 @@ void segbucket_levels(const SbBuffers<T>& buf, const SbGiven& given, const SbSta
     sort(sb_sort_kernel<T, false>, std::max(first, plain.buckets) + std::min(first, g.sort / 4), first);
 }
 
+// The levels as what stands behind a bucket sort (radix_host.cuh). Defined with the
+// segmented sort, in seg_bucket_*.cu: a kernel is launched from one translation unit only,
+// since each has a copy of it, and what is set once per process (shared-memory limits,
+// grids) is set for one copy.
+#define ORIGAMI_DECLARE_BEHIND(T)                                                                                        \
+    void segbucket_behind(const SbBuffers<T>& buf, const SbGiven& given, const SbStarts& plain, const SegBucketPlan<T>& p, \
+                          uint64_t xin, uint64_t xout, const SegBucketScratch<T>& sc, cudaStream_t st);
+ORIGAMI_DECLARE_BEHIND(uint32_t)
+ORIGAMI_DECLARE_BEHIND(uint64_t)
+ORIGAMI_DECLARE_BEHIND(KV64)
+#undef ORIGAMI_DECLARE_BEHIND
+
+template <class T>
+void segbucket_run(const SbBuffers<T>& buf, const SbGiven& given, const SbStarts& plain, const SegBucketPlan<T>& p,
+                   uint64_t xin, uint64_t xout, const SegBucketScratch<T>& sc, cudaStream_t st) {
+    if (p.wide)
+        segbucket_levels<T, uint64_t>(buf, given, plain, p, xin, xout, sc, st);
+    else
+        segbucket_levels<T, uint32_t>(buf, given, plain, p, xin, xout, sc, st);
+}
+
 // Segments [off[s], off[s+1]), sorted in place.
 template <class T>
 cudaError_t segbucket_run(T* d, T* tmp, const uint64_t* off, uint64_t nseg, uint64_t n, uint64_t xmask, void* scratch,
@@ -200,11 +221,7 @@ cudaError_t segbucket_run(T* d, T* tmp, const uint64_t* off, uint64_t nseg, uint
         sb_plan_kernel<T><<<(unsigned)((nseg + 255) / 256), 256, 0, st>>>(off, (uint32_t)nseg, n, sc.list[0],
                                                                          (uint32_t)p.segs, sc.recs, sc.cn);
     });
-    const SbBuffers<T> buf{d, tmp, nullptr, false};
-    if (p.wide)
-        segbucket_levels<T, uint64_t>(buf, SbGiven{}, SbStarts{}, p, xmask, xmask, sc, st);
-    else
-        segbucket_levels<T, uint32_t>(buf, SbGiven{}, SbStarts{}, p, xmask, xmask, sc, st);
+    segbucket_run<T>(SbBuffers<T>{d, tmp, nullptr, false}, SbGiven{}, SbStarts{}, p, xmask, xmask, sc, st);
     return cudaGetLastError();
 }
 

@@ -15,6 +15,11 @@ cudaError_t segbucket_sort_kv(void* d, void* tmp, const uint64_t* off, uint64_t 
     return segbucket_run<KV64>(static_cast<KV64*>(d), static_cast<KV64*>(tmp), off, nseg, n, key_mask, scratch, st);
 }
 
+void segbucket_behind(const SbBuffers<KV64>& buf, const SbGiven& given, const SbStarts& plain, const SegBucketPlan<KV64>& p,
+                      uint64_t xin, uint64_t xout, const SegBucketScratch<KV64>& sc, cudaStream_t st) {
+    segbucket_run<KV64>(buf, given, plain, p, xin, xout, sc, st);
+}
+
 void segbucket_prepare_kv() {
     SegBucketGrids<KV64, uint32_t>::get();
     SegBucketGrids<KV64, uint64_t>::get();

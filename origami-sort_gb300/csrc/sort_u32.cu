@@ -17,6 +17,13 @@ cudaError_t sort_io_u32(const void* in, void* out, void* wa, void* wb, uint64_t 
                                 static_cast<uint32_t*>(wb), n, sort_n, xin, xout, start_run, fan, scratch, st, nullptr);
 }
 
+cudaError_t sort_behind_u32(const void* in, void* out, void* wa, void* wb, uint64_t n, uint64_t sort_n, uint64_t xin,
+                            uint64_t xout, int fan, void* scratch, const int* route, int* err, cudaStream_t st) {
+    const PipeBehind behind{route, err};
+    return sort_pipeline_io<uint32_t>(static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), static_cast<uint32_t*>(wa),
+                                static_cast<uint32_t*>(wb), n, sort_n, xin, xout, 0, fan, scratch, st, nullptr, &behind);
+}
+
 uint64_t scratch_bytes_io_u32(uint64_t n, uint64_t sort_n, int fan, uint64_t start_run) {
     return pipeline_scratch_bytes<uint32_t>(n, sort_n, fan, start_run);
 }

@@ -273,3 +273,52 @@ def test_pairs_report_expired_wait(kind):
     finally:
         og.set_wait_limit(old)
     check(kind, a, lens)
+
+
+ORDER = """
+import sys
+import numpy as np, torch, oracle as orc, origami_gpu as og
+kind = int(sys.argv[1])
+def buf(n):
+    a = orc.empty(kind, n)
+    k = np.random.default_rng(9).integers(0, 1 << 31, n).astype(np.uint32)
+    if a.dtype.names:
+        a["key"], a["value"] = k, np.arange(n)
+    else:
+        a[:] = k
+    return a
+def segmented():
+    a = buf(30000)
+    d, off = torch.from_numpy(a.view(np.uint8).copy()).cuda(), torch.tensor([0, 7, 30000], device="cuda")
+    og.SegmentedPlan(d, off, torch.empty_like(d), kind).launch(torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    return d, a, [(0, 7), (7, 30000)]
+def plain(n, sort_n, min_k=0):
+    a = buf(n)
+    d = torch.from_numpy(a.view(np.uint8).copy()).cuda()
+    o = og.sort(d, torch.empty_like(d), kind=kind, sort_n=sort_n, min_k=min_k)
+    torch.cuda.synchronize()
+    s = sort_n or n
+    return o, a, [(i, min(i + s, n)) for i in range(0, n, s)]
+calls = {"segmented": segmented, "levels": lambda: plain(1 << 25, 1 << 18 if kind == og.U32 else 0),
+         "merges": lambda: plain(1 << 22, 0, 16), "chunks": lambda: plain(1 << 22, 1 << 17)}
+for c in sys.argv[2:]:
+    d, a, segs = calls[c]()
+    got = d.cpu().numpy().view(a.dtype)
+    for s, e in segs:
+        x = a[s:e]
+        want = x[np.argsort(x["key"], kind="stable")] if a.dtype.names else np.sort(x)
+        assert np.array_equal(got[s:e], want), c
+"""
+
+
+@pytest.mark.parametrize("order", [("segmented", "levels"), ("levels", "segmented"), ("merges", "chunks"), ("chunks", "merges")])
+@pytest.mark.parametrize("kind", [og.U32, og.U64, og.KV64])
+def test_first_calls_in_either_order(kind, order):
+    # what a process sets up once for the kernels of its first call is there for the second
+    import os
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-c", ORDER, str(kind), *order], capture_output=True, text=True,
+                       env={**os.environ, "PYTHONPATH": os.pathsep.join(p for p in sys.path if p)})
+    assert r.returncode == 0, r.stderr[-800:]
