@@ -343,9 +343,9 @@ int origami_generate_device(int kind, void* d, uint64_t n, int dist, uint64_t se
  * sizes about as large as L2, other binary shapes for others; binary passes
  * with shape 0 elsewhere). min_k = 2 keeps the table's merge shape with
  * binary passes; larger min_k forces that fan-in. Beside its merge shape an
- * entry says whether the class sorts by buckets, with radix passes behind them
- * for keys that are too uneven (called "radix" below; the built-in choice of all
- * but a few small classes); sorts with min_k = 0 then do, where the chunk size
+ * entry says whether the class sorts by buckets, with radix passes, further levels
+ * or merges behind them for keys that are too uneven (called "radix" below; the
+ * built-in choice of all but a few small classes); sorts with min_k = 0 then do, where the chunk size
  * allows it, and fall back to the merge shape when their scratch cannot be
  * allocated.
  *   origami_autotune   times every shape and the buckets on n generated
@@ -354,11 +354,14 @@ int origami_generate_device(int kind, void* d, uint64_t n, int dist, uint64_t se
  *                      line per shape and one "radix ms=" line.
  *   get / set          read or write one entry's merge shape. Setting the
  *                      class's built-in shape restores its built-in choice,
- *                      buckets included; any other selects merge passes.
- *   save / load        the entries other than binary passes with shape 0 as
- *                      "kind class fan variant"
- *                      lines, radix choices that differ from the built-in ones
- *                      as "radix kind class on" lines, and the segmented
+ *                      buckets included; any other selects merge passes. (Merges
+ *                      of the built-in shape: min_k = 2, or a "radix" line.)
+ *   save / load        the entries whose shape is not their class's built-in
+ *                      one, and those other than binary passes with shape 0, as
+ *                      "kind class fan variant" lines (loading one sets it, as
+ *                      above), the choices of buckets or merges that those lines
+ *                      alone would not give as "radix kind class on" lines (a file
+ *                      may hold them for any class), and the segmented
  *                      table's (below) as "seg kind class shape" and
  *                      "segbuckets kind class on" lines. The file named by
  *                      ORIGAMI_TUNING, if set, is loaded at first use.

@@ -23,16 +23,17 @@
 //
 // Measured (one GB300): 2^28 uint32 keys 7.38 ms by merges, 3.79 by eight-bit radix
 // passes, 2.63 by buckets (counting 0.22, partition 2 x 0.60, buckets 1.20); 2^27 uint64
-// keys 8.44, 5.17 and 2.02 (0.20, 2 x 0.47, 0.85); 2^27 pairs 14.0, 8.47 and 3.88 (0.33,
+// keys 8.44 by merges and 2.02 (0.20, 2 x 0.47, 0.85); 2^27 pairs 14.0 and 3.88 (0.33,
 // 2 x 1.07, 1.38). A plain copy takes 0.32, 0.32 and 0.64 ms.
 //
 // A slice is a monotone function of the key (keys outside the sampled range
 // fall into the end slices), so any data is sorted correctly as long as every
 // bucket fits. Where one does not (heavy duplicates, clustered keys), *route is
 // set on the device, the remaining kernels return at once, and what follows in the
-// stream sorts the array instead: radix passes for 32-bit keys (radix.cuh), the levels
-// of the segmented bucket sort for 64-bit keys (seg_buckets.cuh; from the slices of the
-// first level, where they are there already).
+// stream sorts the array instead (radix_host.cuh, Behind): the levels of the segmented
+// bucket sort for 64-bit keys (seg_buckets.cuh; from the slices of the first level, where
+// they are there already), radix passes for 32-bit keys (radix.cuh), for chunks of them
+// merges or levels.
 //
 // Equal keys of keys-only items are identical, so their order does not matter:
 // bk_pass_kernel takes places with shared-memory atomics, one CTA per tile in
@@ -178,7 +179,7 @@ struct SliceDigit {
 // The same for radix_pass_kernel, with the slice starts of the scan.
 template <class T>
 struct SliceDigitStable : SliceDigit<T> {
-    static constexpr bool kHeavy = false;  // the sample sends crowded slices to the radix passes
+    static constexpr bool kHeavy = false;  // no digit of most of the items: the sample gives up on such slices
     const SliceMap<typename Traits<T>::Key>* maps;
     uint32_t map_shift;
     const uint32_t* start;

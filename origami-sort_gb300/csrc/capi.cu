@@ -77,9 +77,11 @@ uint32_t wait_limit() { return g_wait_limit.load(std::memory_order_relaxed); }
 
 // Smallest chunk that sorts by the radix path: 2^28 uint32 keys in chunks of
 // 2^16 / 2^18 / 2^20 / 2^21 keys take 2.15 / 2.07 / 2.01 / 2.77 ms by buckets, 2.92 /
-// 3.66 / 4.41 / 4.78 by merge passes; shorter chunks have too few buckets.
+// 3.66 / 4.41 / 4.78 by merge passes; shorter chunks have too few buckets. (Zipf keys, on
+// which the buckets give up, in chunks of 2^16 / 2^17 / 2^20 / 2^21: 4.2 / 4.2 / 5.1 / 6.7
+// by what stands behind them, 2.9 / 3.3 / 4.4 / 4.8 by merges.)
 constexpr uint64_t RADIX_CHUNK = 1 << 16;
-// Whether the radix path (bucket sort, radix passes or levels behind it) sorts n items in
+// Whether the radix path (bucket sort, and what stands behind it) sorts n items in
 // chunks of sort_n under this shape code: the size class asks for it, the
 // geometry fits, and the chunks are long enough. Its cost hardly depends on the
 // chunk size, a merge sort's is one level less for every halving.
