@@ -782,6 +782,7 @@ template <class T>
 struct BucketSortShared {
     uint32_t ws[BucketCfg<T>::S_NT / 32];
     uint32_t rlo[2], rhi[2], widest, listed;
+    int odd;  // pairs that leave: how many of BK_TRIED items share a deep bin with another key
 };
 template <class T>
 __device__ __forceinline__ BucketSortShared<T>& bk_shared() {
@@ -925,6 +926,7 @@ __device__ __forceinline__ void bk_sort_init() {
 #pragma unroll
     for (int i = 0; i < C::BINS / C::S_NT; ++i) tab[i * C::S_NT + tid] = 0;
 }
+constexpr int BK_TRIED = 64;  // items of a crowded bucket of pairs that are looked at
 // What becomes of a bucket with crowded bins of several keys: byte passes; left as it is
 // (false is returned; keys only: if a warp a bin can't settle them); pairs: settled by a
 // warp each, and left if that fails.
@@ -1090,7 +1092,21 @@ __device__ __forceinline__ bool bk_sort_bucket(const T* src, T* out, int cnt, ui
         }
     }
     __syncthreads();
-    if (CROWD == BK_LEAVE && Sh::STABLE && crowded) return false;
+    if constexpr (CROWD == BK_LEAVE && Sh::STABLE)
+        if (crowded) {
+            bool other = false;
+            if (tid < BK_TRIED) {  // (the first ones)
+                const bool here = tid < cnt;
+                const K k = here ? Traits<T>::key(v[0]) : 0;
+                const uint32_t b = here ? bp[0] & 0xFFFFu : 0u;
+                const int s = (int)tab[b], e = b + 1 < BINS ? (int)tab[b + 1] : cnt;
+                const unsigned with = __match_any_sync(0xFFFFFFFFu, b) & ~__match_any_sync(0xFFFFFFFFu, k);
+                other = here && with && e - s > Sh::SETTLED;
+            }
+            const int odd = __syncthreads_count(other);
+            if (tid == 0) sh.odd = odd;
+            return false;
+        }
     static_assert(CROWD == BK_LEAVE || (CROWD == BK_SETTLE) == Sh::STABLE, "pairs are not in order as placed");
 #pragma unroll
     for (int i = 0; i < IPT; ++i)
@@ -1186,7 +1202,7 @@ __device__ __forceinline__ bool bk_sort_bucket(const T* src, T* out, int cnt, ui
 // 21 instructions an item in all, 55 % of issue slots. A bin that is wide all the same
 // (samples that mislead) sends the bucket to byte passes.
 // Those took every such bucket before, up to eight passes: groups of 200 log-uniform keys,
-// 2^25 in all, uint32 11.9 ms and now 3.2, uint64 20.8 and 3.5, pairs 38.5 and 5.8; groups
+// 2^25 in all, uint32 11.9 ms and now 3.2, uint64 20.8 and 3.5, pairs 38.5 and 5.7; groups
 // of 1000 3.0 / 1.2, 5.0 / 1.6, 9.1 / 1.9; 2^24 uint64 keys in clusters 1.78 and 0.88. (Tried:
 // 512 splitters, groups of 200 twice as long, larger ones the same; merges through registers
 // in shared memory, groups of 5000 3.0 ms instead of 2.5.)
@@ -1393,38 +1409,16 @@ __device__ __noinline__ void bk_sort_settled(const T* src, T* out, int cnt, uint
 // A bucket that bk_sort_bucket<T, BK_LEAVE> left just now. Keys: by splitters. Pairs: where
 // a quarter of 64 items share a bin of more items than a warp settles with one of 32 that
 // has another key, those bins would not be settled. (2^25 pairs, groups of 200, keys spread
-// over their logarithms: 5.8 ms, 8.3 if settling is tried first; Zipf keys in groups of 1000,
-// which are settled, 1.47, by splitters 1.87.)
+// over their logarithms: 5.7 ms, 8.3 if settling is tried first; Zipf keys in groups of 1000,
+// which are settled, 1.31, by splitters 1.87. The test on items still in registers; read
+// again for it here, Zipf groups took 1.47, chunks of 4096 0.086 instead of 0.078.)
 template <class T>
 __device__ __noinline__ void bk_sort_crowded(const T* src, T* out, int cnt, uint64_t xin, uint64_t xout) {
     __builtin_assume(__isGlobal(src));
     __builtin_assume(__isGlobal(out));
-    using Sh = BucketShape<T>;
-    using K = typename Traits<T>::Key;
-    constexpr int BINS = Sh::C::BINS, TRIED = 64;
-    static_assert(Sh::STABLE, "pairs");
-    BucketSortShared<T>& sh = bk_shared<T>();
-    const uint32_t* tab = reinterpret_cast<const uint32_t*>(bk_smem() + Sh::KEYS_BYTES);
-    const int tid = threadIdx.x;
+    static_assert(BucketShape<T>::STABLE, "pairs");
     __syncthreads();
-    bool odd = false;
-    if (tid < TRIED) {
-        // bins as in bk_sort_bucket, from the range found there
-        K klo = sh.rlo[0], kr = sh.rhi[0] - sh.rlo[0];
-        klo = kr ? klo << 32 : (klo << 32 | sh.rlo[1]);
-        kr = kr ? kr << 32 | 0xFFFFFFFFu : (K)(sh.rhi[1] - sh.rlo[1]);
-        const int c = __clzll((long long)kr);
-        const uint32_t xr = (uint32_t)((kr << c) >> 32);
-        const uint32_t mul = (uint32_t)(((float)BINS * 4294967296.0f) / ((float)xr + 512.0f)) - 1u;
-        const int p = cnt > TRIED ? cnt * tid / TRIED : min(tid, cnt - 1);
-        const K k = Traits<T>::key(bk_flip(src[p], xin));
-        // (the bins' words are their starts)
-        const uint32_t b = __umulhi((uint32_t)(((k - klo) << c) >> 32), mul);
-        const int s = (int)tab[b], e = b + 1 < BINS ? (int)tab[b + 1] : cnt;
-        const unsigned others = __match_any_sync(0xFFFFFFFFu, b) & ~__match_any_sync(0xFFFFFFFFu, k);
-        odd = tid < cnt && others && e - s > Sh::SETTLED;
-    }
-    if (__syncthreads_count(odd) >= TRIED / 4 || !bk_settle_bucket<T>(src, out, cnt, xin, xout))
+    if (bk_shared<T>().odd >= BK_TRIED / 4 || !bk_settle_bucket<T>(src, out, cnt, xin, xout))
         bk_sort_split<T>(src, out, cnt, xin, xout);
 }
 template <class T>
